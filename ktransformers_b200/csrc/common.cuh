@@ -41,6 +41,17 @@ void count_launch(int n = 1);
     } while (0)
 
 int num_sms(int device);
+// stream-ordered scratch from a bounded pool (runtime.cu); ScratchBlock gives it back behind the work already queued on the stream
+cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out);
+struct ScratchBlock {
+    void* ptr = nullptr;
+    cudaStream_t stream;
+    explicit ScratchBlock(cudaStream_t s) : stream(s) {}
+    ScratchBlock(const ScratchBlock&) = delete;
+    ScratchBlock& operator=(const ScratchBlock&) = delete;
+    cudaError_t take(int device, size_t bytes) { return scratch_alloc(device, bytes, stream, &ptr); }
+    ~ScratchBlock() { if (ptr) cudaFreeAsync(ptr, stream); }
+};
 
 #ifdef __CUDACC__
 // launch with the programmatic-stream-serialization attribute (KTB200_PDL=0 disables it library-wide)

@@ -10,6 +10,7 @@
 //     grid = (ceil(N / 128) row tiles, K splits), two CTAs per SM; 192 threads: warp 0 TMA producer (4-stage ring), warp 1 issuer,
 //     warps 2-5 quantise x for the CTA's K range while the first weight boxes are in flight, then run the epilogue.
 // K splits add their fp32 partial sums with atomics into a zeroed workspace; the last CTA of a row tile converts and re-zeroes.
+// Batches of more than kFT tokens take fp8_gemm_kernel below: tokens on the MMA's rows, so that the weights are read once per 128 of them.
 #include <cuda.h>
 #include <cuda_fp8.h>
 
@@ -71,7 +72,8 @@ __device__ __forceinline__ void fp8_load4(const void* x, long off, int hidden_ty
     }
 }
 // batches of more than 2 tokens: quantise x ONCE (one warp per block) instead of once per row tile
-__global__ void __launch_bounds__(256) fp8_act_quant_kernel(const void* x, int hidden_type, int T, int K, uint8_t* xq, float* xs) {
+// (scales [token][block], or with spitch > 0 [block][spitch] for the GEMM)
+__global__ void __launch_bounds__(256) fp8_act_quant_kernel(const void* x, int hidden_type, int T, int K, uint8_t* xq, float* xs, int spitch) {
     const int lane = threadIdx.x & 31, blk = blockIdx.x * 8 + (threadIdx.x >> 5), nkb = K / 128;
     griddep_launch_dependents();
     if (blk >= T * nkb) return;
@@ -81,7 +83,7 @@ __global__ void __launch_bounds__(256) fp8_act_quant_kernel(const void* x, int h
     uint32_t packed;
     const float s = fp8_quant_block(v, packed);
     reinterpret_cast<uint32_t*>(xq + (long)t * K + (long)kb * 128)[lane] = packed;
-    if (lane == 0) xs[t * nkb + kb] = s;
+    if (lane == 0) xs[spitch ? (long)kb * spitch + t : (long)t * nkb + kb] = s;
 }
 
 __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constant__ CUtensorMap wmap, const Fp8Params p) {
@@ -236,6 +238,177 @@ __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constan
     }
 }
 
+// Prompt portions (more than kFT tokens): y = xq . W^T as a persistent GEMM.  The pass kernel above streams all of W again for every 16
+// tokens (2000 tokens, 7168 -> 18432: 125 passes, 7.9 ms); here a tile is 128 tokens x BN weight rows, both operands come by TMA in the
+// 128-byte-swizzle layout, and what bounds it is the tensor pipe (K = 128 of a 128 x 256 tile: 512 cycles of MMA) beside the promotion of
+// the partial dot to fp32 after every 128 of K that the two block scales ask for (128 fused multiply-adds per thread and 128 of K).
+//     warp 0 TMA ring (4 to 8 stages, 192 KB), warp 1 issuer, warps 2-9 epilogue: a thread owns one token and half of the tile's columns;
+//     lanes are tokens, so the token scale is a register and acc += dot * (a_s * b_s) is ONE fma per value and 128 of K.
+//     Two TMEM buffers of BN columns: the MMAs of one K block run while the block before it is promoted.
+// BN: 256 leaves the tensor pipe shared-memory headroom (96 of 128 B per cycle); 128 and 64 keep the chip full when there are few tiles.
+// Tiles run token tile fastest inside groups of kFGroupM, so that the CTAs of a wave share the weight rows and the tokens through L2.
+constexpr int kFGemmThreads = 320, kFGroupM = 16, kFGemmRing = 192 * 1024, kFGemmTokens = 4096;
+struct Fp8GemmMisc {
+    unsigned long long full[8], free[8], d_full[2], d_free[2];
+    uint32_t tmem_base;
+};
+constexpr int kFGemmSmem = kFGemmRing + (int)sizeof(Fp8GemmMisc) + 1024;
+
+struct Fp8GemmParams {
+    const float* xs;          // [nkb][tpad] token scales, token fastest
+    const float* scale_inv;   // [ceil(N/128)][nkb]
+    void* y;                  // [T][N]
+    const int* bsz;
+    int hidden_type, T, N, nkb, tpad, mt, nt, t0, vec;
+};
+
+// TWO: fp32 results, where the order of a long fp32 chain shows (K = 12032: 2.0e-7 off in one chain, 1.2e-7 with K splits): the chain is cut
+// every 8 blocks into a second accumulator.
+template <int BN, bool TWO>
+__global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Fp8GemmParams p) {
+    constexpr int kStageB = 128 * 128 + BN * 128, kStages = kFGemmRing / kStageB, kCols = 2 * BN;
+    static_assert(kStages <= 8, "barriers");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    Fp8GemmMisc& misc = *reinterpret_cast<Fp8GemmMisc*>(smem_raw + (base - raw) + kFGemmRing);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        for (int s = 0; s < kStages; s++) { bar_init(smem_u32(&misc.full[s]), 1); bar_init(smem_u32(&misc.free[s]), 1); }
+        for (int b = 0; b < 2; b++) { bar_init(smem_u32(&misc.d_full[b]), 1); bar_init(smem_u32(&misc.d_free[b]), 8); }
+        bar_fence_init();
+        tma_prefetch_desc(&xmap);
+        tma_prefetch_desc(&wmap);
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&misc.tmem_base), kCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = misc.tmem_base;
+    const int tiles = p.mt * p.nt;
+    auto place = [&](int tile, int& m0, int& n0) {      // groups of kFGroupM token tiles; inside a group the token tile is fastest
+        const int per = kFGroupM * p.nt, g = tile / per, r = tile - g * per, gm = min(kFGroupM, p.mt - g * kFGroupM);
+        n0 = (r / gm) * BN;
+        m0 = (g * kFGroupM + r % gm) * 128;
+    };
+    griddep_wait();      // the quantised tokens and their scales come from the kernel before this one
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0, ph = 1;
+            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+                int m0, n0;
+                place(tile, m0, n0);
+                for (int kb = 0; kb < p.nkb; kb++) {
+                    bar_wait(smem_u32(&misc.free[s]), ph);
+                    const uint32_t bar = smem_u32(&misc.full[s]), dst = base + s * kStageB;
+                    bar_expect_tx(bar, kStageB);
+                    tma_load_2d(dst, &xmap, bar, kb * 128, m0);
+                    tma_load_2d(dst + 128 * 128, &wmap, bar, kb * 128, n0);
+                    if (++s == kStages) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = instr_desc(1, 0, 0, 0, 0, 128, BN);   // f32 += e4m3 . e4m3, K-major both
+        int s = 0, ph = 0;
+        unsigned it = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+            for (int kb = 0; kb < p.nkb; kb++, it++) {
+                const int buf = it & 1;
+                bar_wait(smem_u32(&misc.full[s]), ph);
+                bar_wait(smem_u32(&misc.d_free[buf]), ((it >> 1) & 1) ^ 1);
+                tc_fence_after();
+                const uint32_t a = base + s * kStageB, b = a + 128 * 128;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    mma_f8(tmem + buf * BN, smem_desc(a + j * 32, 16, 1024, kLayoutSw128), smem_desc(b + j * 32, 16, 1024, kLayoutSw128), idesc, j != 0);
+                mma_commit(smem_u32(&misc.free[s]));
+                mma_commit(smem_u32(&misc.d_full[buf]));
+                if (++s == kStages) { s = 0; ph ^= 1; }
+            }
+    } else {
+        constexpr int kHalf = BN / 2;
+        const int sp = warp & 3, ch = (warp - 2) >> 2;
+        const uint32_t tcol = tmem + ((uint32_t)(32 * sp) << 16) + ch * kHalf;
+        const int live = p.bsz ? max(0, min(p.T, *p.bsz - p.t0)) : p.T;
+        unsigned it = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            int m0, n0;
+            place(tile, m0, n0);
+            const int t = m0 + 32 * sp + lane, nb = n0 + ch * kHalf;
+            const float* xs = p.xs + t;                                                     // t < tpad
+            const float* sinv = p.scale_inv + (long)min(nb / 128, (p.N - 1) / 128) * p.nkb;
+            float acc[kHalf], sum[TWO ? kHalf : 1];
+#pragma unroll
+            for (int i = 0; i < kHalf; i++) {
+                acc[i] = 0.f;
+                if (TWO) sum[i] = 0.f;
+            }
+            float a_s = __ldg(xs), b_s = __ldg(sinv);
+            for (int kb = 0; kb < p.nkb; kb++, it++) {
+                const int buf = it & 1;
+                const float f = a_s * b_s;
+                if (kb + 1 < p.nkb) { a_s = __ldg(xs + (long)(kb + 1) * p.tpad); b_s = __ldg(sinv + kb + 1); }
+                bar_wait(smem_u32(&misc.d_full[buf]), (it >> 1) & 1);
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < kHalf; c += 16) {
+                    uint32_t d[16];
+                    tmem_ld16(tcol + buf * BN + c, d);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; i++) acc[c + i] = __fmaf_rn(__uint_as_float(d[i]), f, acc[c + i]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(smem_u32(&misc.d_free[buf]));
+                if (TWO && ((kb & 7) == 7 || kb + 1 == p.nkb)) {
+#pragma unroll
+                    for (int i = 0; i < kHalf; i++) { sum[i] += acc[i]; acc[i] = 0.f; }
+                }
+            }
+            if (TWO) {
+#pragma unroll
+                for (int i = 0; i < kHalf; i++) acc[i] = sum[i];
+            }
+            if (t < live) {
+                const long o = (long)t * p.N + nb;
+#pragma unroll
+                for (int c = 0; c < kHalf; c += 8) {
+                    if (p.vec && nb + c + 8 <= p.N) {
+                        if (p.hidden_type == KTB200_TYPE_F32) {
+                            float4* y = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.y) + o + c);
+                            y[0] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+                            y[1] = make_float4(acc[c + 4], acc[c + 5], acc[c + 6], acc[c + 7]);
+                        } else {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                const float lo = acc[c + 2 * i], hi = acc[c + 2 * i + 1];
+                                w[i] = p.hidden_type == KTB200_TYPE_BF16 ? (uint32_t)f32_to_bf16_ggml(lo) | ((uint32_t)f32_to_bf16_ggml(hi) << 16)
+                                                                         : (uint32_t)__half_as_ushort(__float2half_rn(lo)) | ((uint32_t)__half_as_ushort(__float2half_rn(hi)) << 16);
+                            }
+                            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.y) + o + c) = make_uint4(w[0], w[1], w[2], w[3]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            if (nb + c + i < p.N) store_hidden(p.y, o + c + i, p.hidden_type, acc[c + i]);
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kCols);
+    }
+}
+
 typedef CUresult (*EncodeTiledFn8)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                    CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFn8 encode_tiled8() {
@@ -259,6 +432,59 @@ struct ktb200_fp8_linear {
     uint8_t* xq;   // [kFT][K] e4m3
     float* xs;     // [kFT][nkb]
 };
+
+namespace ktb {
+// one box of `rows` x 128 bytes of a row-major byte matrix [n][K]
+static int fp8_map(CUtensorMap* map, const void* ptr, int K, int n, int rows) {
+    const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)n};
+    const cuuint64_t gstr[1] = {(cuuint64_t)K};
+    const cuuint32_t box[2] = {128, (cuuint32_t)rows}, estr[2] = {1, 1};
+    const CUresult cr = encode_tiled8()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) { set_error("fp8_linear: cuTensorMapEncodeTiled failed (%d)", (int)cr); return KTB200_ECUDA; }
+    return KTB200_OK;
+}
+template <int BN, bool TWO>
+static cudaError_t launch_fp8_gemm(const CUtensorMap& xmap, const CUtensorMap& wmap, const Fp8GemmParams& p, int grid, cudaStream_t s) {
+    const cudaError_t e = cudaFuncSetAttribute(fp8_gemm_kernel<BN, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFGemmSmem);
+    return e != cudaSuccess ? e : launch_pdl(fp8_gemm_kernel<BN, TWO>, dim3(grid), dim3(kFGemmThreads), (size_t)kFGemmSmem, s, xmap, wmap, p);
+}
+static int fp8_forward_gemm(ktb200_fp8_linear* l, int qlen, const void* x, void* y, const int* bsz, cudaStream_t s) {
+    const size_t hb = type_size(l->hidden_type);
+    for (int t0 = 0; t0 < qlen; t0 += kFGemmTokens) {
+        Fp8GemmParams p{};
+        p.T = qlen - t0 < kFGemmTokens ? qlen - t0 : kFGemmTokens;
+        p.N = l->N; p.nkb = l->nkb; p.t0 = t0; p.bsz = bsz; p.hidden_type = l->hidden_type; p.scale_inv = l->scale_inv;
+        p.mt = (p.T + 127) / 128; p.tpad = p.mt * 128;
+        p.y = reinterpret_cast<uint8_t*>(y) + (size_t)t0 * l->N * hb;
+        p.vec = (size_t)l->N * hb % 16 == 0 && (uintptr_t)y % 16 == 0;
+        ScratchBlock mem(s);
+        const size_t xs_bytes = (size_t)l->nkb * p.tpad * sizeof(float);
+        KTB_CUDA_CHECK(mem.take(l->device, (size_t)p.T * l->K + xs_bytes));
+        float* xs = reinterpret_cast<float*>(mem.ptr);
+        uint8_t* xq = reinterpret_cast<uint8_t*>(mem.ptr) + xs_bytes;
+        p.xs = xs;
+        const void* xc = reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * l->K * hb;
+        fp8_act_quant_kernel<<<(unsigned)(((long)p.T * l->nkb + 7) / 8), 256, 0, s>>>(xc, l->hidden_type, p.T, l->K, xq, xs, p.tpad);
+        // the widest tile that still gives every SM one
+        const int sms = num_sms(l->device);
+        const bool two = l->hidden_type == KTB200_TYPE_F32;      // (twice the accumulators: no room for 256 columns)
+        int bn = two ? 128 : 256;
+        while (bn > 64 && (long)p.mt * ((l->N + bn - 1) / bn) < sms) bn >>= 1;
+        p.nt = (l->N + bn - 1) / bn;
+        CUtensorMap xmap, wmap;
+        int rc = fp8_map(&xmap, xq, l->K, p.T, 128);
+        if (rc == KTB200_OK) rc = fp8_map(&wmap, l->w, l->K, l->N, bn);
+        if (rc) return rc;
+        const int grid = p.mt * p.nt < sms ? p.mt * p.nt : sms;
+        const auto go = two ? (bn == 128 ? launch_fp8_gemm<128, true> : launch_fp8_gemm<64, true>)
+                            : (bn == 256 ? launch_fp8_gemm<256, false> : bn == 128 ? launch_fp8_gemm<128, false> : launch_fp8_gemm<64, false>);
+        KTB_CUDA_CHECK(go(xmap, wmap, p, grid, s));
+        count_launch(2);
+    }
+    return KTB200_OK;
+}
+}  // namespace ktb
 
 extern "C" {
 
@@ -316,8 +542,9 @@ int ktb200_fp8_linear_forward(ktb200_fp8_linear* l, int qlen, const void* x, voi
     if (!l || !x || !y) { set_error("fp8_linear: null pointer"); return KTB200_EINVAL; }
     if (qlen <= 0) return KTB200_OK;
     DeviceGuard g(l->device);
+    if (qlen > kFT) return fp8_forward_gemm(l, qlen, x, y, bsz, (cudaStream_t)stream);
     const size_t hb = type_size(l->hidden_type);
-    for (int t0 = 0; t0 < qlen; t0 += kFT) {   // decode-sized passes; a prefill batch re-streams the weights every 16 tokens
+    for (int t0 = 0; t0 < qlen; t0 += kFT) {
         Fp8Params p{};
         p.x = reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * l->K * hb;
         p.y = reinterpret_cast<uint8_t*>(y) + (size_t)t0 * l->N * hb;
@@ -326,7 +553,7 @@ int ktb200_fp8_linear_forward(ktb200_fp8_linear* l, int qlen, const void* x, voi
         p.kb_per_split = l->kb_per_split; p.ksplit = l->ksplit;
         if (p.T > 2) {   // quantise once, then the GEMM as a programmatic dependent launch: its weight boxes stream while the quantiser drains
             p.xq = l->xq; p.xs = l->xs;
-            fp8_act_quant_kernel<<<(p.T * l->nkb + 7) / 8, 256, 0, (cudaStream_t)stream>>>(p.x, l->hidden_type, p.T, l->K, l->xq, l->xs);
+            fp8_act_quant_kernel<<<(p.T * l->nkb + 7) / 8, 256, 0, (cudaStream_t)stream>>>(p.x, l->hidden_type, p.T, l->K, l->xq, l->xs, 0);
             KTB_CUDA_CHECK(launch_pdl(fp8_linear_kernel, dim3(l->row_tiles, l->ksplit), dim3(192), (size_t)kFSmem, (cudaStream_t)stream, l->map, p));
             count_launch(2);
         } else {

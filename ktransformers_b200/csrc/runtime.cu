@@ -3,6 +3,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <atomic>
+#include <mutex>
 
 #include "gemv_bulk.cuh"
 
@@ -33,6 +34,32 @@ int num_sms(int device) {
         cached[device] = n;
     }
     return cached[device];
+}
+
+// Scratch of one call, taken and given back in stream order from a pool of this library's own (one per device): safe for any number of
+// threads and streams, and under stream capture (the graph then owns the memory).  The pool keeps at most kScratchKeep bytes between
+// calls, so that a prompt's layers do not pay for mapping memory each; what exceeds it goes back to the driver at the next synchronisation.
+constexpr unsigned long long kScratchKeep = 1ull << 30;
+cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out) {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!pools[device]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            const cudaError_t e = cudaMemPoolCreate(&pools[device], &props);
+            if (e != cudaSuccess) { pools[device] = nullptr; return e; }
+            unsigned long long keep = kScratchKeep;
+            cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        pool = pools[device];
+    }
+    return cudaMallocFromPoolAsync(out, bytes, pool, stream);
 }
 
 }  // namespace ktb
