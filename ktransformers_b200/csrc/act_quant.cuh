@@ -20,8 +20,8 @@ namespace ktb {
 //     fused multiply-add (what gcc emits for the reference on every FMA-capable x86-64 build).
 //   * an all-zero block gives d = 0, q = 0 (bsums forced to 0; the reference leaves them stale but
 //     they are only ever multiplied by d == 0).
-__device__ __forceinline__ void warp_quantize_q8k_block(const float (&x)[8], int lane, uint32_t* q8_out,
-                                                        float* d_out, int16_t* bsums_out, int16_t* bs32_out = nullptr) {
+// The core: the lane's 8 quants as two words of 4 int8, the block scale d (every lane) and the lane's sum of quants.
+__device__ __forceinline__ void warp_q8k_words(const float (&x)[8], uint32_t& w0, uint32_t& w1, float& d, int& s) {
     // local first-max scan
     float amax = 0.f, mx = 0.f;
 #pragma unroll
@@ -38,9 +38,7 @@ __device__ __forceinline__ void warp_quantize_q8k_block(const float (&x)[8], int
         mx = __shfl_sync(0xffffffffu, mx, src);
         amax = __uint_as_float(gmax);
     }
-    uint32_t w0 = 0, w1 = 0;
-    int s = 0;
-    float d = 0.f;
+    w0 = 0; w1 = 0; s = 0; d = 0.f;
     if (amax != 0.f) {
         const float iscale = __fdiv_rn(-127.f, mx);
         int q[8];
@@ -57,6 +55,13 @@ __device__ __forceinline__ void warp_quantize_q8k_block(const float (&x)[8], int
              ((uint32_t)(q[7] & 0xff) << 24);
         d = __frcp_rn(iscale);   // correctly rounded reciprocal == 1.f / iscale
     }
+}
+__device__ __forceinline__ void warp_quantize_q8k_block(const float (&x)[8], int lane, uint32_t* q8_out,
+                                                        float* d_out, int16_t* bsums_out, int16_t* bs32_out = nullptr) {
+    uint32_t w0, w1;
+    float d;
+    int s;
+    warp_q8k_words(x, w0, w1, d, s);
     q8_out[2 * lane] = w0;
     q8_out[2 * lane + 1] = w1;
     int s2 = s + __shfl_xor_sync(0xffffffffu, s, 1);

@@ -8,6 +8,7 @@
 #include "gemv_bulk.cuh"
 #include "dense_bulk.cuh"
 #include "handles.cuh"
+#include "kq_gemm.cuh"
 
 namespace ktb {
 
@@ -572,12 +573,12 @@ extern "C++" {
 namespace ktb {
 bool grouped_ok(const ktb200_moe* m, int k);
 int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, const float* weights, const void* input, void* output, const int* bsz, cudaStream_t s);
-void grouped_set_trace(long long* t);
 }
 }
 // qlen from which the per-expert tensor-core GEMMs (grouped.cu) replace the per-pair GEMV kernels: the reference makes the
 // same split between MOE::forward_one and MOE::forward_many (moe.cpp:367-377, threshold group_min_len)
-void ktb200_debug_grouped(long long* trace_dev) { ktb::grouped_set_trace(trace_dev); }
+// (kept for callers that look it up: the kernel whose stamps it asked for is gone)
+void ktb200_debug_grouped(long long*) {}
 static int grouped_min_qlen() {
     static const int v = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : 48; }();
     return v;
@@ -721,6 +722,10 @@ struct ktb200_linear {
     bool loaded, soa;
 };
 
+// rows from which a linear runs as a tensor-core GEMM (kq_gemm.cu): the row kernels keep up to 8 rows of activations on the SM and read the weights
+// once for them; beyond, once more for every row
+constexpr int kLinearGemmMin = 9;
+
 int ktb200_linear_create(int in_size, int out_size, const void* proj, int proj_type, int hidden_type, int group_max_len,
                          int device, ktb200_linear** out) {
     if (!out || !proj) { set_error("null argument"); return KTB200_EINVAL; }
@@ -756,12 +761,17 @@ int ktb200_linear_forward(ktb200_linear* l, int qlen, const void* input, void* o
     if (qlen <= 0) return KTB200_OK;
     if (!input || !output) { set_error("forward: null pointer"); return KTB200_EINVAL; }
     DeviceGuard g(l->device);
+    const FmtId fmt = pick_fmt(l->proj_type, l->soa);
+    if (qlen >= kLinearGemmMin) {
+        const int rc = kq_linear(fmt, l->proj, l->out_size, l->in_size, input, l->hidden_type, qlen, output, bias, bsz, l->device, (cudaStream_t)stream);
+        if (rc != 1) return rc;
+    }
     RowsParams rp{};
     rp.shared_token = -1;
     rp.w0 = l->proj; rp.w1 = nullptr; rp.type0 = rp.type1 = l->proj_type; rp.n_experts = 1; rp.rows = l->out_size;
     rp.ncols = l->in_size; rp.slots = 1; rp.ids = nullptr; rp.id_offset = 0; rp.x = input; rp.hidden_type = l->hidden_type;
     rp.use_silu = 0; rp.out_f32 = nullptr; rp.out_hidden = output; rp.bias = bias; rp.bsz = bsz;
-    return launch_rows<false>(pick_fmt(l->proj_type, l->soa), rp, qlen, l->device, (cudaStream_t)stream);
+    return launch_rows<false>(fmt, rp, qlen, l->device, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------------------------------ mlp

@@ -1,4 +1,4 @@
-"""Tensor-core products of prompt-sized batches (csrc/fp8_linear.cu) through the C-ABI, at the edges of their tiles, against plain torch in 64 bits
+"""Tensor-core products of prompt-sized batches (csrc/fp8_linear.cu, csrc/kq_gemm.cu) through the C-ABI, at the edges of their tiles, against plain torch in 64 bits
 on the same quantised operands.  The operands' products are exact, so a result is off by its fp32 sums (n ~ 100 terms of one rounding each: well
 below 4e-6 of the largest value) and its last rounding (half a unit: 2^-9 of a bf16, 2^-12 of an fp16)."""
 import ctypes as C
@@ -7,10 +7,13 @@ import pytest
 import torch
 
 from ktransformers_b200 import native
+from ktransformers_b200.util.synth import synth_blocks
+from oracle.bindings import Oracle
 
 pytestmark = pytest.mark.gpu
 
 F32, F16, BF16 = 0, 1, 30
+Q4_K, Q5_K, Q6_K = 12, 13, 14
 TORCH = {F32: torch.float32, F16: torch.float16, BF16: torch.bfloat16}
 HALF_UNIT = {F32: 2.0 ** -24, F16: 2.0 ** -11, BF16: 2.0 ** -8}      # twice the half unit: a sum at the edge may fall to the other side
 
@@ -56,3 +59,71 @@ def test_fp8_prompt_batches(T, K, N, hid):
     _check(y, want, hid)
     _rows_untouched(call, y, T - 5, y)
     lib.ktb200_fp8_linear_destroy(h)
+
+
+def _q8(x):
+    """Q8_K rounding of activations, in 64 bits: 256 int8 and the fp32 scale of their block"""
+    f = x.float().reshape(-1, 256)
+    most = f.gather(1, f.abs().argmax(-1, keepdim=True))
+    inv = torch.full_like(most, -127.0) / most
+    q = (inv.double() * f.double()).round().clamp(max=127.0)
+    return (q * (torch.ones_like(inv) / inv).double()).reshape(x.shape)
+
+
+# 9 rows: the first batch of this path; 64 / 65: one tile of tokens and a ragged second; R ragged against the 128 rows of a matrix and the 256 of a
+# tile; one block of K, two blocks (no parts), many (K in parts); every weight type and, for Q6_K, its 8-row groups; 4100: two passes
+@pytest.mark.parametrize("type,T,K,R,hid", [(Q4_K, 9, 256, 64, BF16), (Q4_K, 64, 7168, 300, F32), (Q4_K, 65, 512, 40002, BF16), (Q4_K, 200, 1536, 2051, F16), (Q5_K, 16, 2560, 129, F32),
+                                            (Q5_K, 130, 256, 38000, BF16), (Q6_K, 17, 768, 1000, F32), (Q6_K, 257, 3072, 520, BF16), (Q6_K, 33, 256, 38400, F16), (Q4_K, 4100, 256, 272, BF16)])
+def test_k_quant_prompt_batches(type, T, K, R, hid):
+    blocks = synth_blocks(type, R * K, "cuda", T + K + R)
+    dense = torch.from_numpy(Oracle().to_float(blocks.cpu().numpy(), type, R * K)).cuda().view(R, K)
+    g = torch.Generator(device="cuda").manual_seed(T + R)
+    x = torch.randn((T, K), generator=g, device="cuda").to(TORCH[hid])
+    bias = torch.randn(R, generator=g, device="cuda")
+    lib, h = native.lib(), C.c_void_p()
+    native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), type, hid, T, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, _stream()))
+
+    def call(y, bsz=None):
+        native.check(lib.ktb200_linear_forward(h, T, x.data_ptr(), y.data_ptr(), bias.data_ptr(), bsz.data_ptr() if bsz is not None else None, _stream()))
+
+    y = torch.zeros((T, R), dtype=TORCH[hid], device="cuda")
+    call(y)
+    _check(y, _q8(x) @ dense.double().T + bias.double(), hid)
+    _rows_untouched(call, y, T - 3, y)
+    lib.ktb200_linear_destroy(h)
+
+
+# experts with no token, one token, 64, 65 and all tokens; an expert named twice by a token and ids beyond the experts; gate and up of one
+# 128-row tile and of several; down in both layouts
+@pytest.mark.parametrize("gu,down,H,I,T", [(Q4_K, Q6_K, 256, 256, 48), (Q4_K, Q4_K, 512, 256, 131), (Q4_K, Q6_K, 1024, 768, 200), (Q4_K, Q6_K, 2048, 512, 1100), (Q5_K, Q5_K, 768, 512, 100),
+                                           (Q6_K, Q6_K, 512, 256, 70)])
+def test_experts_of_a_prompt_at_tile_edges(gu, down, H, I, T):
+    import gpu_util as G
+    E, k = 6, 3
+    gate, up, dn = synth_blocks(gu, E * I * H, "cuda", 1), synth_blocks(gu, E * I * H, "cuda", 2), synth_blocks(down, E * H * I, "cuda", 3)
+    orc = Oracle()
+    dense = [torch.from_numpy(orc.to_float(t.cpu().numpy(), q, t_n)).cuda().view(E, r, c) for t, q, t_n, r, c in
+             ((gate, gu, E * I * H, I, H), (up, gu, E * I * H, I, H), (dn, down, E * H * I, H, I))]
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, H), generator=gen, device="cuda") / 10
+    w = torch.rand((T, k), generator=gen, device="cuda")
+    ids = torch.full((T, k), 0, dtype=torch.int64, device="cuda")      # expert 0: every token
+    ids[:, 1] = 1 + (torch.arange(T, device="cuda") >= min(65, T - 1)).long() * 4      # expert 1: 65 tokens, expert 5: the others
+    ids[:, 2] = -1
+    ids[:min(64, T), 2] = 3                                             # expert 3: 64 tokens
+    ids[T - 1, 2] = 4                                                   # expert 4: one token; expert 2: none
+    ids[0, 1] = 0                                                       # twice the same expert
+    ids[1, 2] = E + 7
+    m = G.Moe(E, k, H, I, gate, up, dn, gu, gu, down, F32, max_tokens=T)
+    got = torch.from_numpy(m.forward(ids.cpu().numpy(), w.cpu().numpy(), x.cpu().numpy())).cuda()
+    x8, want = _q8(x), torch.zeros((T, H), dtype=torch.float64, device="cuda")
+    for e in range(E):
+        tok, slot = torch.where(ids == e)
+        if len(tok):
+            a = torch.nn.functional.silu(x8[tok] @ dense[0][e].double().T) * (x8[tok] @ dense[1][e].double().T)
+            want.index_add_(0, tok, (_q8(a) @ dense[2][e].double().T) * w[tok, slot].double().unsqueeze(-1))
+    # an activation at the edge of two int8 steps may fall to either side: a unit of 1/127 of its block's largest, in a few values of a row
+    assert (got.double() - want).norm() <= 1e-3 * want.norm()
+    assert (got.double() - want).abs().max() <= 2e-2 * want.abs().max()
+    m.close()
