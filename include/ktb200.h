@@ -337,6 +337,13 @@ int ktb200_mla_prep(const void* q_dev, int num_heads, int qk_nope_head_dim, cons
                     float eps, const float* cos_dev, const float* sin_dev, void* kv_cache_dev, int page_size, const int* page_idx_dev,
                     const int* page_offset_dev, void* q_pe_out_dev, int n_tokens, void* stream);
 
+/* ktb200_mla_prep for one new token per sequence, from the positions themselves (int64, `position_stride` elements apart): cos / sin of
+ * position * inv_freq[32], the cache row of `cache_position` (one for all sequences) in the static cache whose sequence b owns pages
+ * [b * max_pages, (b + 1) * max_pages), and kv_len_out[b] = position + 1. */
+int ktb200_mla_step_prep(const void* q_dev, int num_heads, int qk_nope_head_dim, const void* kv_a_out_dev, const void* kv_a_norm_weight_dev, float eps,
+                         const float* inv_freq_dev, const long long* positions_dev, long position_stride, const long long* cache_position_dev, void* kv_cache_dev,
+                         int page_size, int max_pages, void* q_pe_out_dev, int* kv_len_out_dev, int batch, void* stream);
+
 /* The two absorb products of MLA decode (attention.py:428-431, 470-472): batches of one-row GEMVs over the per-head bf16
  * halves of kv_b_proj — q_abs[t][h][:] = q_nope[t][h][:] . W_UK[h] ([heads][nope][512]; q addressed by element strides so the
  * q_nope slice of the q_b output needs no copy) and out[t][h][:] = attn_latent[t][h][:] . W_UV[h]^T ([heads][v][512]). */

@@ -107,9 +107,69 @@ __global__ void __launch_bounds__(256) mla_prep_kernel(const __nv_bfloat16* q, i
     if (threadIdx.x < R) dst[LAT + threadIdx.x] = __float2bfloat16_rn(rope(row + LAT, threadIdx.x));
 }
 
+// The same for one new token per sequence straight from the positions (KDeepseekV2Attention's decode step): the rotation's cosines and sines, the
+// cache row and the sequence length are worked out here, which takes the ~30 small launches around them off the host (the whole layer
+// was bound by issuing them: 675 us for one token where its kernels take about 75).  Products stay in fp32 and are rounded once.
+// grid (1 + ceil(heads / 16), sequences), 256 threads: CTA 0 of a sequence does the latent row, the others 16 heads' q_pe each.
+__global__ void __launch_bounds__(256) mla_step_prep_kernel(const __nv_bfloat16* q, int num_heads, int q_head_dim, int nope_dim, const __nv_bfloat16* kva, const __nv_bfloat16* kv_norm_w,
+                                                            float eps, const float* inv_freq, const long long* pos, long pos_stride, const long long* cache_pos,
+                                                            __nv_bfloat16* kv_cache, int page_size, int max_pages, __nv_bfloat16* q_pe_out, int* kv_len_out) {
+    constexpr int R = 64, LAT = 512, kHeads = 16;
+    __shared__ float red[8], cs[R / 2], sn[R / 2];
+    griddep_launch_dependents();
+    griddep_wait();
+    const long b = blockIdx.y;
+    const long long at = pos[b * pos_stride];
+    if (threadIdx.x < R / 2) {
+        const float a = (float)at * inv_freq[threadIdx.x];
+        sincosf(a, &sn[threadIdx.x], &cs[threadIdx.x]);
+    }
+    __syncthreads();
+    // pairs (2i, 2i + 1) turn together and come out at i and i + 32
+    auto turn = [&](const __nv_bfloat16* x, __nv_bfloat16* y, int i) {
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(x + 2 * i));
+        y[i] = __float2bfloat16_rn(v.x * cs[i] - v.y * sn[i]);
+        y[i + R / 2] = __float2bfloat16_rn(v.y * cs[i] + v.x * sn[i]);
+    };
+    if (blockIdx.x > 0) {
+        const int h0 = (blockIdx.x - 1) * kHeads;
+        for (int u = threadIdx.x; u < kHeads * (R / 2); u += 256) {
+            const int h = h0 + u / (R / 2);
+            if (h < num_heads) turn(q + (b * num_heads + h) * q_head_dim + nope_dim, q_pe_out + (b * num_heads + h) * R, u % (R / 2));
+        }
+        return;
+    }
+    if (threadIdx.x == 0) kv_len_out[b] = (int)at + 1;
+    const __nv_bfloat16* row = kva + b * (LAT + R);
+    const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + 2 * threadIdx.x));
+    const float inv = rsqrtf(block_sum(v.x * v.x + v.y * v.y, red) / (float)LAT + eps);
+    const long long cp = *cache_pos;
+    if (cp < 0 || cp >= (long long)max_pages * page_size) return;      // beyond the cache: nothing to write to
+    __nv_bfloat16* dst = kv_cache + ((b * max_pages + cp / page_size) * page_size + cp % page_size) * (LAT + R);
+    *reinterpret_cast<__nv_bfloat162*>(dst + 2 * threadIdx.x) = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(kv_norm_w + 2 * threadIdx.x), __floats2bfloat162_rn(v.x * inv, v.y * inv));
+    if (threadIdx.x < R / 2) turn(row + LAT, dst + LAT, threadIdx.x);
+}
+
 }  // namespace ktb
 
 using namespace ktb;
+
+extern "C" int ktb200_mla_step_prep(const void* q, int num_heads, int qk_nope_head_dim, const void* kv_a_out, const void* kv_a_norm_weight, float eps, const float* inv_freq,
+                                    const long long* positions, long position_stride, const long long* cache_position, void* kv_cache, int page_size, int max_pages,
+                                    void* q_pe_out, int* kv_len_out, int batch, void* stream) {
+    if (!q || !kv_a_out || !kv_a_norm_weight || !inv_freq || !positions || !cache_position || !kv_cache || !q_pe_out || !kv_len_out || num_heads <= 0 || qk_nope_head_dim <= 0 ||
+        qk_nope_head_dim % 2 || page_size <= 0 || max_pages <= 0) {
+        set_error("mla_step_prep: null pointer / bad shape");
+        return KTB200_EINVAL;
+    }
+    if (((uintptr_t)q | (uintptr_t)kv_a_out | (uintptr_t)kv_a_norm_weight | (uintptr_t)kv_cache | (uintptr_t)q_pe_out) & 3) { set_error("mla_step_prep: 4-byte aligned rows"); return KTB200_EINVAL; }
+    if (batch <= 0) return KTB200_OK;
+    KTB_CUDA_CHECK(launch_pdl(mla_step_prep_kernel, dim3(1 + (num_heads + 15) / 16, batch), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)q, num_heads, qk_nope_head_dim + 64,
+                              qk_nope_head_dim, (const __nv_bfloat16*)kv_a_out, (const __nv_bfloat16*)kv_a_norm_weight, eps, inv_freq, positions, position_stride, cache_position,
+                              (__nv_bfloat16*)kv_cache, page_size, max_pages, (__nv_bfloat16*)q_pe_out, kv_len_out));
+    count_launch();
+    return KTB200_OK;
+}
 
 extern "C" int ktb200_add_rmsnorm(void* residual, const void* delta, const void* weight, float eps, void* out, int n_tokens, int hidden, void* stream) {
     if (!residual || !weight || !out || n_tokens < 0 || hidden <= 0 || hidden % 2 || hidden > 2 * kNormPairs * kNormThreads) { set_error("add_rmsnorm: bad argument (bf16, even hidden <= 8192)"); return KTB200_EINVAL; }

@@ -15,7 +15,8 @@ from typing import Optional, Tuple
 import torch
 
 from .. import native
-from ..models.modeling_deepseek_v3 import DeepseekV3Attention, apply_rotary_pos_emb
+from ..models.custom_cache import StaticCache
+from ..models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3RMSNorm, DeepseekV3RotaryEmbedding, apply_rotary_pos_emb
 from .base_operator import BaseInjectedModule
 from .flashinfer_wrapper import MLAWrapperSingleton
 
@@ -37,6 +38,59 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
             object.__setattr__(self, "out_absorb", kv_b[:, self.qk_nope_head_dim:, :].contiguous())
         return self.q_absorb, self.out_absorb
 
+    def _step(self, hidden_states, position_ids, cache, cache_position):
+        """One new token per sequence with everything between the projections in this library's launches (`ktb200_mla_step_prep` is the latent norm,
+        both rotations, the cache write and the lengths): bf16, plain norms and rotation, the static cache.  None for any other form, which the
+        module-by-module path below takes.  (The reference's decode branch: archive/ktransformers/operators/attention.py:395-478.)"""
+        rot, kv_norm, x = self.rotary_emb, self.kv_a_layernorm, hidden_states
+        bf16 = torch.bfloat16
+        if not (x.dtype == bf16 and x.is_cuda and type(rot) is DeepseekV3RotaryEmbedding and type(kv_norm) is DeepseekV3RMSNorm and type(cache) is StaticCache
+                and kv_norm.weight.dtype == bf16 and kv_norm.weight.device == x.device and self.kv_lora_rank == 512 and self.qk_rope_head_dim == 64):
+            return None
+        for t in (position_ids, cache_position):
+            if t is None or t.dtype != torch.int64 or t.device != x.device:
+                return None
+        bsz, heads, nope = x.shape[0], self.num_heads, self.qk_nope_head_dim
+        if tuple(position_ids.shape) != (bsz, 1) or cache_position.numel() != 1 or cache.max_batch_size < bsz or rot.inv_freq.dtype != torch.float32 or nope % 2:
+            return None
+        lib, stream = native.lib(), torch.cuda.current_stream(x.device).cuda_stream
+        if self.q_lora_rank is None:
+            q = self.q_proj(x)
+        else:
+            qa, norm = self.q_a_proj(x), self.q_a_layernorm
+            if type(norm) is DeepseekV3RMSNorm and norm.weight.dtype == bf16 == qa.dtype and qa.is_contiguous() and self.q_lora_rank % 2 == 0 and self.q_lora_rank <= 8192:
+                qn = torch.empty_like(qa)
+                native.check(lib.ktb200_add_rmsnorm(qa.data_ptr(), None, norm.weight.data_ptr(), float(norm.variance_epsilon), qn.data_ptr(), bsz, self.q_lora_rank, stream))
+            else:
+                qn = norm(qa)
+            q = self.q_b_proj(qn)
+        kva = self.kv_a_proj_with_mqa(x)
+        q_absorb, out_absorb = self.get_absorbed()
+        if not (q.dtype == bf16 == kva.dtype == q_absorb.dtype and q.is_contiguous() and kva.is_contiguous()):
+            return None
+        inv_freq = rot.inv_freq.to(x.device)
+        kv = cache.key_cache[self.layer_idx]
+        w = self.mla_wrapper
+        if w is None:
+            w = self.mla_wrapper = MLAWrapperSingleton.get_instance(str(x.device), bsz, cache.max_pages * bsz, use_cuda_graph=True)
+        if w.need_plan:
+            indptr = torch.arange(0, bsz + 1, dtype=torch.int32, device=x.device) * cache.max_pages
+            w.plan(None, indptr, cache.page_table_list[self.layer_idx].reshape(-1), (position_ids[:, 0] + 1).to(torch.int32), None, heads, 512, 64, cache.page_size, self.softmax_scale, bf16, kv.dtype)
+            w.max_pages_per_seq = cache.max_pages
+        q_pe = torch.empty((bsz, heads, 64), dtype=bf16, device=x.device)
+        q_abs = torch.empty((bsz, heads, 512), dtype=bf16, device=x.device)
+        native.check(lib.ktb200_mla_step_prep(q.data_ptr(), heads, nope, kva.data_ptr(), kv_norm.weight.data_ptr(), float(kv_norm.variance_epsilon), inv_freq.data_ptr(),
+                                              position_ids.data_ptr(), position_ids.stride(0), cache_position.data_ptr(), kv.data_ptr(), cache.page_size, cache.max_pages, q_pe.data_ptr(),
+                                              w.kv_len_arr_buf.data_ptr(), bsz, stream))
+        native.check(lib.ktb200_mla_absorb_q(q.data_ptr(), nope + 64, heads * (nope + 64), q_absorb.data_ptr(), heads, nope, 512, q_abs.data_ptr(), bsz, stream))
+        if not torch.cuda.is_current_stream_capturing():
+            cache.past_tokens[self.layer_idx] += 1
+        pages = kv.view(-1, cache.page_size, 576)
+        lat = w.run(q_abs, q_pe, pages[..., :512], pages[..., 512:])
+        o = torch.empty((bsz, 1, heads * self.v_head_dim), dtype=bf16, device=x.device)
+        native.check(lib.ktb200_mla_absorb_o(lat.data_ptr(), out_absorb.data_ptr(), heads, self.v_head_dim, 512, o.data_ptr(), bsz, stream))
+        return self.o_proj(o)
+
     def forward(self, hidden_states: torch.Tensor, attention_mask: Optional[torch.Tensor] = None,
                 position_ids: Optional[torch.Tensor] = None, past_key_value=None, output_attentions: bool = False,
                 use_cache: bool = False, cache_position: Optional[torch.Tensor] = None, **kwargs):
@@ -44,6 +98,10 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         if q_len != 1 and not self.absorb_for_prefill:
             raise NotImplementedError("KDeepseekV2Attention: the B200 path covers absorbed decode (q_len == 1)")
         assert past_key_value is not None, "decode needs the paged latent cache (models/custom_cache.StaticCache)"
+        if q_len == 1:
+            out = self._step(hidden_states, position_ids, past_key_value, cache_position)
+            if out is not None:
+                return out, None, past_key_value
         q = self.q_proj(hidden_states) if self.q_lora_rank is None else self.q_b_proj(self.q_a_layernorm(self.q_a_proj(hidden_states)))
         q = q.view(bsz, q_len, self.num_heads, self.q_head_dim)
         q_nope, q_pe = torch.split(q, [self.qk_nope_head_dim, self.qk_rope_head_dim], dim=-1)

@@ -1,0 +1,46 @@
+"""The decode step of KDeepseekV2Attention with its launches fused (`ktb200_mla_step_prep`) against the module-by-module path of the same operator on
+the same inputs: the same cache row up to a unit of bf16 in the last place (its products are rounded once instead of three times), the same lengths,
+the same output within the reach of those roundings (4 x 2^-8 of the largest value)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bsz,heads,q_rank,pos", [(1, 128, 256, 0), (3, 16, None, 63), (2, 17, 130, 64), (1, 32, 64, 4095)])
+def test_step_equals_the_module_path(bsz, heads, q_rank, pos):
+    from ktransformers_b200 import native
+    from ktransformers_b200.models.custom_cache import StaticCache
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3Config, DeepseekV3RotaryEmbedding
+    from ktransformers_b200.operators.attention import KDeepseekV2Attention
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapper
+
+    class OtherRotary(DeepseekV3RotaryEmbedding):      # any other module than the plain one takes the module path
+        pass
+
+    torch.manual_seed(pos + heads)
+    cfg = DeepseekV3Config(hidden_size=512, num_attention_heads=heads, q_lora_rank=q_rank, num_hidden_layers=1)
+    plain = DeepseekV3Attention(cfg, layer_idx=0).to(device="cuda", dtype=torch.bfloat16)
+    plain.rotary_emb = DeepseekV3RotaryEmbedding(64).to("cuda")
+    outs, rows, lens = [], [], []
+    x = torch.randn(bsz, 1, 512, device="cuda").to(torch.bfloat16)
+    past = torch.randn(bsz, max(pos, 1), 576, device="cuda").to(torch.bfloat16)
+    for rot in (DeepseekV3RotaryEmbedding(64).to("cuda"), OtherRotary(64).to("cuda")):
+        plain.rotary_emb = rot
+        op = KDeepseekV2Attention("blk.0.self_attn", None, cfg, plain, "cuda", "cuda")
+        cache = StaticCache(cfg, max_batch_size=bsz, max_cache_len=pos + 2, device="cuda")
+        seq = cache.key_cache[0].view(bsz, -1, 576)
+        if pos:
+            seq[:, :pos].copy_(past)
+        op.mla_wrapper = MLAWrapper(bsz, cache.max_pages * bsz)
+        where = torch.full((bsz, 1), pos, dtype=torch.int64, device="cuda")
+        n0 = native.launch_count()
+        with torch.no_grad():
+            y, _, _ = op(x, position_ids=where, past_key_value=cache, cache_position=torch.tensor([pos], device="cuda"))
+        launches = native.launch_count() - n0
+        assert launches == (5 + (q_rank is not None) if type(rot) is DeepseekV3RotaryEmbedding else 5), launches      # prep | cache write, absorb, attention, merge, absorb (+ norm)
+        outs.append(y.float()); rows.append(seq[:, pos].float().clone()); lens.append(op.mla_wrapper.kv_len_arr_buf[:bsz].clone())
+        assert cache.get_seq_length(0) == 1
+    assert torch.equal(lens[0], lens[1]) and (lens[0] == pos + 1).all()
+    assert ((rows[0] - rows[1]).abs() <= 2.0 ** -6 * rows[1].abs() + 2.0 ** -7).all()
+    assert (outs[0] - outs[1]).abs().max() <= 2.0 ** -6 * outs[1].abs().max()
