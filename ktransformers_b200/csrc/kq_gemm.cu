@@ -17,8 +17,13 @@
 //     weights.  The pairs come out as (0, 2), (1, 3) of four; the activations are stored in that order (kq_pos4).
 //   * a scale per 256-block needs the accumulator drained per 256-block: two matrices of 128 rows per CTA (gate and up of the same experts, or
 //     256 rows of one) take turns, one drained while the other multiplies, and share the activation tiles.
-// CTA: 20 warps.  0-3 / 4-7 producers of matrix 0 / 1: cp.async ring of raw blocks private to the warp (32 rows) -> registers -> TMEM;
-//      8 TMA of activations, 9 / 10 MMA issuers of matrix 0 / 1; 12-15 / 16-19 epilogue of matrix 0 / 1.
+// CTA: 28 warps in 7 groups of 4.  Groups 0-3 producers: (matrix 0, first operand stage), (matrix 1, first), (0, second), (1, second), a warp = 32 rows:
+//      raw blocks from a TMA ring -> registers -> TMEM; warp 16 TMA of activations, 17 / 18 MMA issuers of matrix 0 / 1, 19 TMA of weights;
+//      groups 5 / 6 epilogue of matrix 0 / 1.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
+//      warps took a third of the issue slots, and the four roles' code is kept in rolled loops: unrolled it overran the instruction cache (10,000
+//      cycles for a block of two matrices; now 3,400; HBM brings one every 1,550).  What is left is the chain product -> drain -> product of
+//      a matrix beside producers that issue ~8,000 instructions per block; measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 6556 us with one
+//      int32 accumulator per 32 values and operands through shared memory, 2500 us; Q4_K linear 777 x 1536 -> 24576 172 us (345 TFLOP/s).
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
 #include <cuda_fp16.h>
 
@@ -33,27 +38,24 @@ using namespace umma;
 template <int FMT>
 struct KqCfg {
     static constexpr bool kQ6 = FMT == KQ_Q6K_T4 || FMT == KQ_Q6K_SOA8;
-    static constexpr int kRow = FMT == KQ_Q4K ? 144 : FMT == KQ_Q5K ? 176 : 208;      // bytes of a row's block in a ring slot: 16-byte words, an odd number of them (conflict-free)
-    static constexpr int kTail = kQ6 ? 4 : 0;                                         // + the word that holds a Q6_K block's d
-    static constexpr int kRing = FMT == KQ_Q4K ? 3 : 2;
-    static constexpr int kWarpSlot = 32 * (kRow + kTail);
+    static constexpr int kRow = FMT == KQ_Q4K ? 144 : FMT == KQ_Q5K ? 176 : 208;      // bytes of a row's block in a ring slot (Q6_K: without d)
     static constexpr int kStages = kQ6 ? 4 : 2;                                       // operand stages per block
     static constexpr float kScale = FMT == KQ_Q4K ? 1.f : FMT == KQ_Q5K ? 2.f : 4.f;  // what the fp16 integers were divided by
-    // registers: producers, issuers, epilogue.  They draw on the launch's 5 x 96 per warp group
-    static constexpr int kRegsP = 88, kRegsI = 64, kRegsE = 120;
-    static_assert(2 * kRegsP + kRegsI + 2 * kRegsE == 5 * 96, "register split");
+    // registers: producers, issuers, epilogue.  They draw on the launch's 7 x 72 per warp group
+    static constexpr int kRegsP = 48, kRegsI = 72, kRegsE = 120;
+    static_assert(4 * kRegsP + kRegsI + 2 * kRegsE == 7 * 72, "register split");
     // shared memory
-    static constexpr int kB = kKqN * 512, kOffSums = 2 * kB, kSums = kQ6 ? 0 : kKqN * 32;
-    static constexpr int kOffMins = kOffSums + 2 * kSums, kMins = kQ6 ? 0 : 128 * 32;                            // [matrix][2]
-    static constexpr int kOffRing = kOffMins + 4 * kMins, kOffMisc = kOffRing + kRing * 8 * kWarpSlot;
+    static constexpr int kRing = 3, kMat = 128 * kRow, kSlot = 2 * kMat;
+    static constexpr int kB = kKqN * 512, kOffRing = 2 * kB, kOffMins = kOffRing + kRing * kSlot, kMins = kQ6 ? 0 : 128 * 32;        // minima: [matrix][2]
+    static constexpr int kOffSums = kOffMins + 4 * kMins, kSums = kQ6 ? 0 : kKqN * 32, kOffMisc = kOffSums + 2 * kSums;
 };
 struct KqMisc {
-    unsigned long long b_full[2], b_free[2], dx_full[4], dx_free[4], a_full[2][2], a_free[2][2], acc_full[2], acc_free[2], hdr_free[2][2];
+    unsigned long long b_full[2], b_free[2], dx_full[4], dx_free[4], raw_full[3], raw_free[3], a_full[2][2], a_free[2][2], acc_full[2], acc_free[2], hdr_free[2][2];
     uint32_t tmem_base, pad[3];
     float dx[4][kKqN];
-    uint32_t hdr[2][2][128];      // half2 (d, dmin) of a row's block
+    uint32_t hdr[2][2][128];      // Q4_K, Q5_K: half2 (d, dmin) of a row's block
 };
-constexpr int kKqThreads = 640;
+constexpr int kKqThreads = 896;
 template <int FMT>
 constexpr int kq_smem() { return KqCfg<FMT>::kOffMisc + (int)sizeof(KqMisc) + 1024; }
 static_assert(kq_smem<KQ_Q4K>() <= 232448 && kq_smem<KQ_Q5K>() <= 232448 && kq_smem<KQ_Q6K_T4>() <= 232448, "shared memory budget");
@@ -78,15 +80,19 @@ __device__ __forceinline__ int kq_pos4(int e0, bool q6) {      // first of the p
     return 64 * (e0 >> 6) + 8 * j + 4 * ((e0 >> 5) & 1);
 }
 
-__device__ __forceinline__ void kq_cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void kq_cp4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void kq_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void kq_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 template <int N>
 __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
 __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3, int c4) {
+    asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(c1),
+                 "r"(c2), "r"(c3), "r"(c4)
+                 : "memory");
+}
+__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 __device__ __forceinline__ void kq_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
@@ -127,25 +133,6 @@ __device__ __forceinline__ void mma_f16_ta8(uint32_t tmem_d, uint32_t tmem_a, ui
         "r"(tmem_a), "l"(desc_b), "l"(next), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// bar_wait (umma.cuh) with a long suspension per poll: 18 warps that poll at the default rate take a third of the issue slots
-__device__ __forceinline__ bool kq_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < (1u << 19); it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    atomicAdd(&g_bar_wait_gave_up, 1u);
-    return false;
-}
-
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 constexpr uint32_t kMagic = 0x64006400u;      // fp16 1024, 1024: a small integer or-ed into the mantissa adds itself
@@ -209,11 +196,11 @@ __device__ __forceinline__ KqTile kq_tile(const KqParams& p, int tile) {
     return t;
 }
 
-// 32 columns (64 weights of a row) of an operand stage from 8 words of quants; sl / sh: scales of the low / high nibbles' values
-__device__ __forceinline__ void kq_unpack4(const uint32_t (&w)[8], __half2 sl, __half2 sh, uint32_t (&o)[32]) {
+// 16 columns (32 weights of a row) of an operand stage from 4 words of quants; sl / sh: scales of the low / high nibbles' values
+__device__ __forceinline__ void kq_unpack4(const uint32_t* w, __half2 sl, __half2 sh, uint32_t (&o)[16]) {
     const __half2 cl = __hmul2(sl, __float2half2_rn(-1024.f)), s16 = __hmul2(sh, __float2half2_rn(1.f / 16.f)), ch = __hmul2(sh, __float2half2_rn(-64.f));
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
+    for (int j = 0; j < 4; j++) {
         const uint32_t a = w[j], b = a >> 8;
         o[4 * j] = as_u32(__hfma2(magic_and<0x000f000fu>(a), sl, cl));
         o[4 * j + 1] = as_u32(__hfma2(magic_and<0x000f000fu>(b), sl, cl));
@@ -222,10 +209,10 @@ __device__ __forceinline__ void kq_unpack4(const uint32_t (&w)[8], __half2 sl, _
     }
 }
 // Q5_K, halved: the fifth bits are bits 0 (low nibbles) and 1 (high nibbles) of the bytes of t
-__device__ __forceinline__ void kq_unpack5(const uint32_t (&w)[8], const uint32_t (&q)[8], int shift, __half2 sl, __half2 sh, uint32_t (&o)[32]) {
+__device__ __forceinline__ void kq_unpack5(const uint32_t* w, const uint32_t* q, int shift, __half2 sl, __half2 sh, uint32_t (&o)[16]) {
     const __half2 s2 = __hmul2(sl, __float2half2_rn(0.5f)), cl = __hmul2(sl, __float2half2_rn(-512.f)), s32 = __hmul2(sh, __float2half2_rn(1.f / 32.f)), ch = __hmul2(sh, __float2half2_rn(-32.f));
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
+    for (int j = 0; j < 4; j++) {
         const uint32_t a = w[j], b = a >> 8, t = q[j] >> shift;
         o[4 * j] = as_u32(__hfma2(as_h2((a & 0x000f000fu) | ((t << 4) & 0x00100010u) | kMagic), s2, cl));
         o[4 * j + 1] = as_u32(__hfma2(as_h2((b & 0x000f000fu) | ((t >> 4) & 0x00100010u) | kMagic), s2, cl));
@@ -233,13 +220,22 @@ __device__ __forceinline__ void kq_unpack5(const uint32_t (&w)[8], const uint32_
         o[4 * j + 3] = as_u32(__hfma2(as_h2((b & 0x00f000f0u) | ((t >> 1) & 0x01000100u) | kMagic), s32, ch));
     }
 }
-__device__ __forceinline__ void kq_words8(const uint8_t* src, uint32_t (&w)[8]) {
-    const uint4 a = reinterpret_cast<const uint4*>(src)[0], b = reinterpret_cast<const uint4*>(src)[1];
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+__device__ __forceinline__ void kq_words8(const uint8_t* a, const uint8_t* b, uint32_t (&w)[8]) {
+    const uint4 x = *reinterpret_cast<const uint4*>(a), y = *reinterpret_cast<const uint4*>(b);
+    w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w; w[4] = y.x; w[5] = y.y; w[6] = y.z; w[7] = y.w;
 }
+// where 16-byte word c (0-7 ql, 8-11 qh, 12 scales) of row r's Q6_K block sits in a matrix's part of a ring slot
+template <int FMT>
+__device__ __forceinline__ int kq_q6_word(int r, int c) {
+    if (FMT == KQ_Q6K_T4) return (r >> 2) * 832 + c * 64 + (r & 3) * 16;                       // [4-row item][word][row], as it lies in memory
+    if (c < 8) return r * 128 + ((c ^ (r & 7)) << 4);                                          // 128-byte swizzle
+    if (c < 12) return 128 * 128 + r * 64 + (((c - 8) ^ ((r >> 1) & 3)) << 4);                 // 64-byte swizzle
+    return 128 * 192 + r * 16;
+}
+struct KqMaps { CUtensorMap q, sums, w[2][3]; };      // activations, their sums; weights of matrix 0 / 1 (Q6_K in 8-row groups: ql, qh, scales)
 
 template <int FMT>
-__global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap smap, const KqParams p) {
+__global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_constant__ KqMaps maps, const KqParams p) {
     using C = KqCfg<FMT>;
     constexpr bool Q6 = C::kQ6;
     constexpr int kAccCols = Q6 ? kKqN : 2 * kKqN, kColA = 2 * kAccCols;      // per matrix: accumulator (and minima); then the operand stages
@@ -256,130 +252,77 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
             for (int j = 0; j < 2; j++) { bar_init(smem_u32(&misc.a_full[i][j]), 4); bar_init(smem_u32(&misc.a_free[i][j]), 1); bar_init(smem_u32(&misc.hdr_free[i][j]), 4); }
         }
         for (int i = 0; i < 4; i++) { bar_init(smem_u32(&misc.dx_full[i]), 1); bar_init(smem_u32(&misc.dx_free[i]), 8); }
+        for (int i = 0; i < C::kRing; i++) { bar_init(smem_u32(&misc.raw_full[i]), 1); bar_init(smem_u32(&misc.raw_free[i]), 16); }
         bar_fence_init();
-        tma_prefetch_desc(&qmap);
-        if (!Q6) tma_prefetch_desc(&smap);
     }
-    if (warp == 9) tmem_alloc(smem_u32(&misc.tmem_base), 512);
+    if (warp == 17) tmem_alloc(smem_u32(&misc.tmem_base), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = misc.tmem_base;
     const int total = p.n_tiles ? *p.n_tiles * p.tiles_mul : p.total;
 
-    if (warp < 8) {
+    if (warp < 16) {
         // ========================================================================== producers
         regs_down<C::kRegsP>();
-        const int mat = warp >> 2, r = tid & 127;                  // weight row of the tile's matrix = TMEM lane
-        const uint32_t ring = base + C::kOffRing + warp * C::kWarpSlot;
-        const uint8_t* ring_p = smem + C::kOffRing + warp * C::kWarpSlot;
-        constexpr int kSlot = 8 * C::kWarpSlot;
-        // fetch cursor, kRing blocks ahead of the conversion and across tile boundaries
-        int ftile = blockIdx.x, fs = 0, fn = 0, fslot = 0, fblk = 0;
-        const uint8_t* fbase = nullptr;
-        int frow = 0;                                              // warp's first row (matrix coordinates)
-        auto enter = [&]() {
-            if (ftile >= total) return;
-            const KqTile t = kq_tile(p, ftile);
-            fbase = p.w[p.pair ? mat : 0] + (long)t.e * p.expert_bytes;
-            frow = t.row0 + (p.pair ? 0 : 128 * mat) + 32 * (warp & 3);
-            fs = 0; fn = t.nsb; fblk = t.sb0;
-        };
-        auto fetch = [&]() {
-            if (ftile < total) {
-                const uint32_t dst = ring + fslot * kSlot;
-                const int last = p.R - 1;                          // rows beyond the matrix read its last row and are never stored
-                if (!Q6) {
-                    constexpr int kCh = C::kRow / 16, kDr = 32 / kCh, kDp = 32 - kDr * kCh;
-                    int rr = lane / kCh, part = lane - rr * kCh;
-#pragma unroll 3
-                    for (int i = 0; i < kCh; i++) {                // 16-byte words of the warp's 32 blocks, a row's words on consecutive lanes
-                        kq_cp16(dst + (i * 32 + lane) * 16, fbase + ((uint32_t)(min(frow + rr, last) * p.nblk + fblk) * (unsigned long long)C::kRow + part * 16));
-                        rr += kDr; part += kDp;
-                        if (part >= kCh) { part -= kCh; rr++; }
-                    }
-                } else if (FMT == KQ_Q6K_T4) {                     // 4-row items of 16-byte planes (repack_q6k4t): a lane fetches its row's 13 words
-                    const int row = min(frow + lane, last), f = (row & 3) * p.nblk + fblk, plane = 4 * p.nblk * 16;
-                    const uint8_t* item = fbase + (long)(row >> 2) * 4 * p.nblk * SZ_Q6_K;
-                    const uint8_t* src = item + f * 16;
-#pragma unroll 4
-                    for (int c = 0; c < 13; c++, src += plane) kq_cp16(dst + lane * C::kRow + c * 16, src);
-                    kq_cp4(dst + 32 * C::kRow + lane * 4, item + 13L * plane + (f >> 1) * 4);
-                } else {                                           // 8-row groups of ql | qh | scales | d (repack_q6k)
-                    auto group = [&](int row) { return fbase + (long)(row >> 3) * 8 * p.nblk * SZ_Q6_K; };
-                    auto at = [&](int row) { return (row & 7) * p.nblk + fblk; };
-#pragma unroll 2
-                    for (int i = 0; i < 8; i++) {
-                        const int rr = 4 * i + (lane >> 3), c = lane & 7, row = min(frow + rr, last);
-                        kq_cp16(dst + rr * C::kRow + c * 16, group(row) + at(row) * 128 + c * 16);
-                    }
-#pragma unroll 2
-                    for (int i = 0; i < 4; i++) {
-                        const int rr = 8 * i + (lane >> 2), c = lane & 3, row = min(frow + rr, last);
-                        kq_cp16(dst + rr * C::kRow + 128 + c * 16, group(row) + 1024 * p.nblk + at(row) * 64 + c * 16);
-                    }
-                    const int row = min(frow + lane, last);
-                    kq_cp16(dst + lane * C::kRow + 192, group(row) + 1536 * p.nblk + at(row) * 16);
-                    kq_cp4(dst + 32 * C::kRow + lane * 4, group(row) + 1664 * p.nblk + (at(row) >> 1) * 4);
-                }
-                fslot = fslot == C::kRing - 1 ? 0 : fslot + 1;
-                fblk++;
-                if (++fs == fn) { ftile += gridDim.x; enter(); }
-            }
-            kq_cp_commit();
-        };
-        enter();
-        for (int i = 0; i < C::kRing; i++) fetch();
-        int slot = 0;
-        unsigned it = 0, stage = 0;      // blocks and operand stages so far
+        const int mat = (warp >> 2) & 1, half = warp >> 3, r = tid & 127, grp = warp >> 2;      // row of the tile's matrix = TMEM lane; operand stages half, half + 2
+        const bool leader = (warp & 3) == 0;
+        const uint32_t dst = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kColA + (mat * 2 + half) * 64;
+        int slot = 0, sphase = 0;
+        unsigned it = 0, uses = 0;       // blocks, and uses of this group's operand stage, so far
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-            const KqTile t = kq_tile(p, tile);
-            const int row = min(t.row0 + (p.pair ? 0 : 128 * mat) + r, p.R - 1);
-            for (int s = 0; s < t.nsb; s++, it++) {
-                kq_cp_wait<C::kRing - 1>();
-                __syncwarp();
-                const uint8_t* src = ring_p + slot * kSlot + lane * C::kRow;
-                kq_wait(smem_u32(&misc.hdr_free[mat][it & 1]), ((it >> 1) & 1) ^ 1);
-                KqScales k{};
-                uint32_t qh[8];
-                if (!Q6) {
-                    const uint4 head = *reinterpret_cast<const uint4*>(src);
-                    k = kq_scales(head.y, head.z, head.w);
-                    misc.hdr[mat][it & 1][r] = head.x;
-                    // minima, each twice, against the sixteen 16-value activation sums: K-major core matrices of 8 rows x 16 bytes
-                    uint8_t* m = smem + C::kOffMins + (mat * 2 + (it & 1)) * C::kMins + (r >> 3) * 256 + (r & 7) * 16;
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                        *reinterpret_cast<uint4*>(m + h * 128) = make_uint4(as_u32(h2_of(byte_of(k.mn[h], 0))), as_u32(h2_of(byte_of(k.mn[h], 1))), as_u32(h2_of(byte_of(k.mn[h], 2))),
-                                                                            as_u32(h2_of(byte_of(k.mn[h], 3))));
-                    fence_async_smem();
-                    if (FMT == KQ_Q5K) kq_words8(src + 16, qh);
-                } else {
-                    const uint32_t tail = *reinterpret_cast<const uint32_t*>(ring_p + slot * kSlot + 32 * C::kRow + lane * 4);
-                    const int f = FMT == KQ_Q6K_T4 ? (row & 3) * p.nblk + t.sb0 + s : (row & 7) * p.nblk + t.sb0 + s;
-                    misc.hdr[mat][it & 1][r] = (f & 1) ? tail >> 16 : tail & 0xffffu;
-                }
-                // (rolled: four roles of fully unrolled code overran the instruction cache, 10,000 cycles a block where this takes less than 2,000)
+            const int nsb = kq_tile(p, tile).nsb;
+            for (int s = 0; s < nsb; s++, it++) {
+                const uint8_t* src = smem + C::kOffRing + slot * C::kSlot + mat * C::kMat;
+                if (leader) bar_wait(smem_u32(&misc.raw_full[slot]), sphase);
 #pragma unroll 1
-                for (int h = 0; h < C::kStages; h++, stage++) {
-                    kq_wait(smem_u32(&misc.a_free[mat][stage & 1]), ((stage >> 1) & 1) ^ 1);
+                for (int h = half; h < C::kStages; h += 2, uses++) {
+                    if (leader) {
+                        bar_wait(smem_u32(&misc.a_free[mat][half]), (uses & 1) ^ 1);
+                        if (!Q6 && !half) bar_wait(smem_u32(&misc.hdr_free[mat][it & 1]), ((it >> 1) & 1) ^ 1);
+                    }
+                    group_sync(1 + grp);
                     tc_fence_after();
-                    const uint32_t dst = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kColA + (mat * 2 + (stage & 1)) * 64;
-                    uint32_t w[8], o[32];
-                    if (!Q6) {      // chunk c = 2h + part: low nibbles are sub-block 2c, high nibbles sub-block 2c + 1
+                    uint32_t w[8], o[16];
+                    if (!Q6) {
+                        src += r * C::kRow;
+                        const uint4 head = *reinterpret_cast<const uint4*>(src);
+                        const KqScales k = kq_scales(head.y, head.z, head.w);
+                        uint32_t sc = h ? k.sc[1] : k.sc[0];
 #pragma unroll 1
-                        for (int part = 0; part < 2; part++) {
-                            const uint32_t sc = (h ? k.sc[1] : k.sc[0]) >> (16 * part);
-                            kq_words8(src + C::kRow - 128 + 32 * (2 * h + part), w);
-                            if (FMT == KQ_Q4K) kq_unpack4(w, h2_of(sc & 0xff), h2_of((sc >> 8) & 0xff), o);
-                            else kq_unpack5(w, qh, 2 * (2 * h + part), h2_of(sc & 0xff), h2_of((sc >> 8) & 0xff), o);
-                            tmem_st32(dst + 32 * part, o);
+                        for (int part = 0; part < 2; part++, sc >>= 16) {      // chunk c = 2h + part: low nibbles are sub-block 2c, high nibbles sub-block 2c + 1
+                            const uint8_t* q = src + C::kRow - 128 + 32 * (2 * h + part);
+                            kq_words8(q, q + 16, w);
+                            if (FMT == KQ_Q4K) {
+#pragma unroll
+                                for (int i = 0; i < 2; i++) {
+                                    kq_unpack4(w + 4 * i, h2_of(sc & 0xff), h2_of((sc >> 8) & 0xff), o);
+                                    tmem_st16(dst + 32 * part + 16 * i, o);
+                                }
+                            } else {
+                                uint32_t qh[8];
+                                kq_words8(src + 16, src + 32, qh);
+#pragma unroll
+                                for (int i = 0; i < 2; i++) {
+                                    kq_unpack5(w + 4 * i, qh + 4 * i, 2 * (2 * h + part), h2_of(sc & 0xff), h2_of((sc >> 8) & 0xff), o);
+                                    tmem_st16(dst + 32 * part + 16 * i, o);
+                                }
+                            }
+                        }
+                        if (!half) {      // this group also hands on (d, dmin) and the minima, each twice, against the sixteen 16-value activation sums
+                            misc.hdr[mat][it & 1][r] = head.x;
+                            uint8_t* m = smem + C::kOffMins + (mat * 2 + (it & 1)) * C::kMins + (r >> 3) * 256 + (r & 7) * 16;      // K-major core matrices of 8 rows x 16 bytes
+#pragma unroll
+                            for (int i = 0; i < 2; i++)
+                                *reinterpret_cast<uint4*>(m + i * 128) = make_uint4(as_u32(h2_of(byte_of(k.mn[i], 0))), as_u32(h2_of(byte_of(k.mn[i], 1))), as_u32(h2_of(byte_of(k.mn[i], 2))),
+                                                                                    as_u32(h2_of(byte_of(k.mn[i], 3))));
+                            fence_async_smem();
                         }
                     } else {
                         // quarter (hh, pp) of the block: elements 128 hh + 32 pp + l (ql low nibbles, qh bits 2 pp) and + 64 (high nibbles, bits 4 + 2 pp), l < 32;
                         // first 32 columns sc * low four bits / 4, last 32 columns sc * (16 * high two bits - 32) / 4; a scale per 16 elements
                         const int hh = h >> 1, pp = h & 1;
-                        const uint2 sc = *reinterpret_cast<const uint2*>(src + 192 + 8 * hh);
+                        const uint2 sc = *reinterpret_cast<const uint2*>(src + kq_q6_word<FMT>(r, 12) + 8 * hh);
                         const __half2 quarter = __float2half2_rn(0.25f);
                         __half2 sl[2], sh[2];
 #pragma unroll
@@ -387,94 +330,119 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
                             sl[i] = __hmul2(__half2half2(__int2half_rn((int)(int8_t)((sc.x >> (16 * pp + 8 * i)) & 0xff))), quarter);
                             sh[i] = __hmul2(__half2half2(__int2half_rn((int)(int8_t)((sc.y >> (16 * pp + 8 * i)) & 0xff))), quarter);
                         }
-                        kq_words8(src + 32 * h, w);
+                        kq_words8(src + kq_q6_word<FMT>(r, 2 * h), src + kq_q6_word<FMT>(r, 2 * h + 1), w);
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
-                            const __half2 cl = __hmul2(sl[i], __float2half2_rn(-1024.f)), s16 = __hmul2(sh[i], __float2half2_rn(1.f / 16.f)), ch = __hmul2(sh[i], __float2half2_rn(-64.f));
-#pragma unroll
-                            for (int j = 4 * i; j < 4 * i + 4; j++) {
-                                const uint32_t a = w[j], b = a >> 8;
-                                o[4 * j] = as_u32(__hfma2(magic_and<0x000f000fu>(a), sl[i], cl));
-                                o[4 * j + 1] = as_u32(__hfma2(magic_and<0x000f000fu>(b), sl[i], cl));
-                                o[4 * j + 2] = as_u32(__hfma2(magic_and<0x00f000f0u>(a), s16, ch));
-                                o[4 * j + 3] = as_u32(__hfma2(magic_and<0x00f000f0u>(b), s16, ch));
-                            }
+                            kq_unpack4(w + 4 * i, sl[i], sh[i], o);
+                            tmem_st16(dst + 16 * i, o);
                         }
-                        tmem_st32(dst, o);
-                        kq_words8(src + 128 + 32 * hh, w);
+                        kq_words8(src + kq_q6_word<FMT>(r, 8 + 2 * hh), src + kq_q6_word<FMT>(r, 9 + 2 * hh), w);
                         const __half2 m = as_h2(0x64206420u);      // 1024 + 32
                         const int up = 4 - 2 * pp, down = 2 * pp;   // the two bits moved to bits 4 and 5 of their byte
 #pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            const uint32_t lo = w[j] << up, hi = w[j] >> down;
-                            o[4 * j] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(lo), m), sl[j >> 2]));
-                            o[4 * j + 1] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(lo >> 8), m), sl[j >> 2]));
-                            o[4 * j + 2] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(hi), m), sh[j >> 2]));
-                            o[4 * j + 3] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(hi >> 8), m), sh[j >> 2]));
+                        for (int i = 0; i < 2; i++) {
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                const uint32_t lo = w[4 * i + j] << up, hi = w[4 * i + j] >> down;
+                                o[4 * j] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(lo), m), sl[i]));
+                                o[4 * j + 1] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(lo >> 8), m), sl[i]));
+                                o[4 * j + 2] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(hi), m), sh[i]));
+                                o[4 * j + 3] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(hi >> 8), m), sh[i]));
+                            }
+                            tmem_st16(dst + 32 + 16 * i, o);
                         }
-                        tmem_st32(dst + 32, o);
                     }
                     tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) bar_arrive(smem_u32(&misc.a_full[mat][stage & 1]));
+                    if (lane == 0) bar_arrive(smem_u32(&misc.a_full[mat][half]));
                 }
-                fetch();                                           // refills the slot just read (every lane is past its reads: the __syncwarp above)
-                slot = slot == C::kRing - 1 ? 0 : slot + 1;
+                if (lane == 0) bar_arrive(smem_u32(&misc.raw_free[slot]));
+                if (++slot == C::kRing) { slot = 0; sphase ^= 1; }
             }
         }
-        kq_cp_wait<0>();
-    } else if (warp < 12) {
-        regs_down<C::kRegsI>();
-        if (warp == 8) {
+    } else if (warp < 20) {
+        if (warp == 16) {
             // ====================================================================== activations
             if (lane == 0) {
+                tma_prefetch_desc(&maps.q);
                 unsigned it = 0;
                 for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                     const KqTile t = kq_tile(p, tile);
                     const int groups = (t.n + 31) >> 5;
                     for (int s = 0; s < t.nsb; s++, it++) {
                         const int b = it & 1, sb = t.sb0 + s;
-                        kq_wait(smem_u32(&misc.b_free[b]), ((it >> 1) & 1) ^ 1);
+                        bar_wait(smem_u32(&misc.b_free[b]), ((it >> 1) & 1) ^ 1);
                         const uint32_t full = smem_u32(&misc.b_full[b]);
                         bar_expect_tx(full, groups * 32 * (Q6 ? 512 : 544));
                         for (int g = 0; g < groups; g++) {
 #pragma unroll
-                            for (int c = 0; c < 4; c++) tma_load_2d(base + b * C::kB + c * (kKqN * 128) + g * 4096, &qmap, full, sb * 256 + c * 64, t.p0 + 32 * g);
-                            if (!Q6) tma_load_2d(base + C::kOffSums + b * C::kSums + g * 1024, &smap, full, sb * 16, t.p0 + 32 * g);
+                            for (int c = 0; c < 4; c++) tma_load_2d(base + b * C::kB + c * (kKqN * 128) + g * 4096, &maps.q, full, sb * 256 + c * 64, t.p0 + 32 * g);
+                            if (!Q6) tma_load_2d(base + C::kOffSums + b * C::kSums + g * 1024, &maps.sums, full, sb * 16, t.p0 + 32 * g);
                         }
                         const int d = it & 3;
-                        kq_wait(smem_u32(&misc.dx_free[d]), ((it >> 2) & 1) ^ 1);
+                        bar_wait(smem_u32(&misc.dx_free[d]), ((it >> 2) & 1) ^ 1);
                         bar_expect_tx(smem_u32(&misc.dx_full[d]), kKqN * 4);
                         kq_bulk(smem_u32(&misc.dx[d][0]), p.dx + (long)sb * p.dpitch + t.p0, kKqN * 4, smem_u32(&misc.dx_full[d]));
                     }
                 }
             }
             __syncwarp();
-        } else if (warp < 11) {
+        } else if (warp == 19) {
+            // ====================================================================== weights: the blocks of 2 x 128 rows as they lie in memory
+            if (lane == 0) {
+                int slot = 0, sphase = 1;
+                for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+                    const KqTile t = kq_tile(p, tile);
+                    const int row = t.e * p.R + t.row0;
+                    for (int s = 0; s < t.nsb; s++) {
+                        const int sb = t.sb0 + s;
+                        bar_wait(smem_u32(&misc.raw_free[slot]), sphase);
+                        const uint32_t full = smem_u32(&misc.raw_full[slot]);
+                        bar_expect_tx(full, C::kSlot);
+#pragma unroll
+                        for (int mat = 0; mat < 2; mat++) {
+                            const uint32_t dst = base + C::kOffRing + slot * C::kSlot + mat * C::kMat;
+                            const CUtensorMap* m = maps.w[mat];
+                            const int r0 = row + (p.pair ? 0 : 128 * mat);
+                            if (!Q6) tma_load_2d(dst, m, full, sb * C::kRow, r0);
+                            else if (FMT == KQ_Q6K_T4) tma_load_5d(dst, m, full, 0, sb, 0, 0, r0 >> 2);
+                            else {
+                                tma_load_3d(dst, m, full, sb * 128, 0, r0 >> 3);
+                                tma_load_3d(dst + 128 * 128, m + 1, full, sb * 64, 0, r0 >> 3);
+                                tma_load_3d(dst + 128 * 192, m + 2, full, sb * 16, 0, r0 >> 3);
+                            }
+                        }
+                        if (++slot == C::kRing) { slot = 0; sphase ^= 1; }
+                    }
+                }
+            }
+            __syncwarp();
+        } else {
             // ====================================================================== tensor-core issuers (converged warps), one per matrix
-            const int mat = warp - 9;
+            const int mat = warp - 17;
             const uint32_t acc = tmem + mat * kAccCols, a0 = tmem + kColA + mat * 128;
-            unsigned it = 0, stage = 0;
+            unsigned it = 0, uses = 0;
             for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                 const KqTile t = kq_tile(p, tile);
                 const uint32_t idesc = instr_desc(1, 0, 0, 0, 0, 128, (t.n + 15) & ~15);      // f32 += f16 . f16
                 for (int s = 0; s < t.nsb; s++, it++) {
                     const int b = it & 1;
-                    kq_wait(smem_u32(&misc.b_full[b]), (it >> 1) & 1);
-                    kq_wait(smem_u32(&misc.acc_free[mat]), (it & 1) ^ 1);
+                    bar_wait(smem_u32(&misc.b_full[b]), (it >> 1) & 1);
+                    bar_wait(smem_u32(&misc.acc_free[mat]), (it & 1) ^ 1);
                     uint64_t bd = smem_desc(base + b * C::kB, 16, 1024, kLayoutSw128);
 #pragma unroll 1
-                    for (int h = 0; h < C::kStages; h++, stage++) {
-                        kq_wait(smem_u32(&misc.a_full[mat][stage & 1]), (stage >> 1) & 1);
+                    for (int h = 0; h < C::kStages; h++) {
+                        bar_wait(smem_u32(&misc.a_full[mat][h & 1]), uses & 1);
                         tc_fence_after();
                         // (the address field of a descriptor counts 16 bytes, and nothing carries out of it)
-                        mma_f16_ta8(acc, a0 + (stage & 1) * 64, bd, Q6 ? 0 : kKqN * 128 >> 4, idesc, h);      // Q6_K: both terms of the quarter's 64 weights
+                        mma_f16_ta8(acc, a0 + (h & 1) * 64, bd, Q6 ? 0 : kKqN * 128 >> 4, idesc, h);      // Q6_K: both terms of the quarter's 64 weights
                         bd += (Q6 ? 1 : 2) * (kKqN * 128 >> 4);
                         if (!Q6 && h == 0)
                             mma_f16(acc + kKqN, smem_desc(base + C::kOffMins + (mat * 2 + b) * C::kMins, 128, 256, kLayoutNone),
                                     smem_desc(base + C::kOffSums + b * C::kSums, 16, 256, kLayoutSw32), idesc, 0);
-                        mma_commit(smem_u32(&misc.a_free[mat][stage & 1]));
+                        mma_commit(smem_u32(&misc.a_free[mat][h & 1]));
+                        if (h & 1) uses++;
                     }
                     mma_commit(smem_u32(&misc.acc_full[mat]));
                     mma_commit(smem_u32(&misc.b_free[b]));
@@ -484,19 +452,36 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
     } else {
         // ========================================================================== epilogue: a thread owns one weight row and the tile's tokens
         regs_up<C::kRegsE>();
-        const int mat = (warp - 12) >> 2, sp = warp & 3, r = 32 * sp + lane;
+        const int mat = (warp - 20) >> 2, sp = warp & 3, r = 32 * sp + lane;
+        const bool leader = sp == 0;
         const uint32_t tacc = tmem + ((uint32_t)(32 * sp) << 16) + mat * kAccCols;
         unsigned it = 0;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
             const KqTile t = kq_tile(p, tile);
+            const int row = t.row0 + (p.pair ? 0 : 128 * mat) + r;
+            // a Q6_K block's d comes straight from memory, a block ahead
+            const uint16_t* dsrc = nullptr;
+            uint16_t dnext = 0;
+            if (Q6) {
+                const int rc = min(row, p.R - 1);
+                const uint8_t* w = p.w[p.pair ? mat : 0] + (long)t.e * p.expert_bytes;
+                dsrc = reinterpret_cast<const uint16_t*>(FMT == KQ_Q6K_T4 ? w + (long)(rc >> 2) * 4 * p.nblk * SZ_Q6_K + 13L * 64 * p.nblk + (rc & 3) * p.nblk * 2
+                                                                         : w + (long)(rc >> 3) * 8 * p.nblk * SZ_Q6_K + 1664L * p.nblk + (rc & 7) * p.nblk * 2) + t.sb0;
+                dnext = __ldg(dsrc);
+            }
             f32x2 acc[kKqN / 2];
 #pragma unroll
             for (int n = 0; n < kKqN / 2; n++) acc[n] = 0;
             for (int s = 0; s < t.nsb; s++, it++) {
-                kq_wait(smem_u32(&misc.dx_full[it & 3]), (it >> 2) & 1);
-                kq_wait(smem_u32(&misc.acc_full[mat]), it & 1);
+                const uint16_t dcur = dnext;
+                if (Q6 && s + 1 < t.nsb) dnext = __ldg(dsrc + s + 1);
+                if (leader) {
+                    bar_wait(smem_u32(&misc.dx_full[it & 3]), (it >> 2) & 1);
+                    bar_wait(smem_u32(&misc.acc_full[mat]), it & 1);
+                }
+                group_sync(5 + mat);
                 tc_fence_after();
-                const __half2 dm = as_h2(misc.hdr[mat][it & 1][r]);
+                const __half2 dm = as_h2(Q6 ? (uint32_t)dcur : misc.hdr[mat][it & 1][r]);
                 const float dw = __low2float(dm) * C::kScale, dmin = -__high2float(dm);
                 const f32x2 dw2 = pack2(dw, dw), dmin2 = pack2(dmin, dmin);
                 const ulonglong2* dx = reinterpret_cast<const ulonglong2*>(misc.dx[it & 3]);
@@ -507,6 +492,11 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
                         tmem_ld16(tacc + 16 * c, v);
                         if (!Q6) tmem_ld16(tacc + kKqN + 16 * c, m);
                         tmem_wait_ld();
+                        if (16 * c + 16 >= t.n) {      // the last columns are out: the next block may be multiplied while these are scaled
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) bar_arrive(smem_u32(&misc.acc_free[mat]));
+                        }
 #pragma unroll
                         for (int i = 0; i < 4; i++) {
                             const ulonglong2 x = dx[4 * c + i];
@@ -520,15 +510,12 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
                         }
                     }
                 }
-                tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    bar_arrive(smem_u32(&misc.acc_free[mat]));
                     bar_arrive(smem_u32(&misc.hdr_free[mat][it & 1]));
                     bar_arrive(smem_u32(&misc.dx_free[it & 3]));
                 }
             }
-            const int row = t.row0 + (p.pair ? 0 : 128 * mat) + r;
             if (row < p.R) {
                 if (p.y) {
                     const float b = p.bias ? p.bias[row] : 0.f;
@@ -553,7 +540,7 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == 17) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }
@@ -644,22 +631,51 @@ static EncodeTiledFnKq encode_tiled_kq() {
     }();
     return fn;
 }
-// boxes of 32 rows x `cols` fp16 of a row-major matrix
-static int kq_map(CUtensorMap* map, const void* ptr, long width, long rows, int cols, CUtensorMapSwizzle sw) {
+// a tensor map of `rank` dimensions (innermost first) with the given byte strides of dimensions 1 .. rank - 1
+static int kq_map(CUtensorMap* map, CUtensorMapDataType type, const void* ptr, int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box, CUtensorMapSwizzle sw) {
     EncodeTiledFnKq enc = encode_tiled_kq();
     if (!enc) { set_error("kq_gemm: cuTensorMapEncodeTiled is not available from this driver"); return KTB200_ECUDA; }
-    const cuuint64_t gdim[2] = {(cuuint64_t)width, (cuuint64_t)rows};
-    const cuuint64_t gstr[1] = {(cuuint64_t)width * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)cols, 32}, estr[2] = {1, 1};
-    const CUresult cr = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult cr = enc(map, type, rank, const_cast<void*>(ptr), dim, stride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) { set_error("kq_gemm: cuTensorMapEncodeTiled failed (%d)", (int)cr); return KTB200_ECUDA; }
     return KTB200_OK;
 }
+// boxes of 32 rows x `cols` fp16 of a row-major matrix
+static int kq_map_acts(CUtensorMap* map, const void* ptr, long width, long rows, int cols, CUtensorMapSwizzle sw) {
+    const cuuint64_t dim[2] = {(cuuint64_t)width, (cuuint64_t)rows}, stride[1] = {(cuuint64_t)width * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)cols, 32};
+    return kq_map(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ptr, 2, dim, stride, box, sw);
+}
+// one block of 128 rows of a matrix of `rows` rows (all experts') of nblk blocks
+static int kq_map_weights(CUtensorMap* m, KqFmt f, const void* w, long rows, int nblk) {
+    const CUtensorMapDataType u8 = CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    const cuuint64_t nb = (cuuint64_t)nblk;
+    if (!kq_is_q6(f)) {
+        const int bytes = f == KQ_Q4K ? SZ_Q4_K : SZ_Q5_K;
+        const cuuint64_t dim[2] = {nb * bytes, (cuuint64_t)rows}, stride[1] = {nb * bytes};
+        const cuuint32_t box[2] = {(cuuint32_t)bytes, 128};
+        return kq_map(m, u8, w, 2, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+    }
+    if (f == KQ_Q6K_T4) {      // [4-row item][word][row][block][16 bytes]
+        const cuuint64_t dim[5] = {16, nb, 4, 13, (cuuint64_t)rows / 4}, stride[4] = {16, 16 * nb, 64 * nb, 4 * nb * SZ_Q6_K};
+        const cuuint32_t box[5] = {16, 1, 4, 13, 32};
+        return kq_map(m, u8, w, 5, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+    }
+    const int bytes[3] = {128, 64, 16}, off[3] = {0, 1024, 1536};      // 8-row groups: [ql: row][block] | [qh: row][block] | [scales: row][block]
+    const CUtensorMapSwizzle sw[3] = {CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_SWIZZLE_NONE};
+    for (int i = 0; i < 3; i++) {
+        const cuuint64_t dim[3] = {nb * bytes[i], 8, (cuuint64_t)rows / 8}, stride[2] = {nb * bytes[i], 8 * nb * SZ_Q6_K};
+        const cuuint32_t box[3] = {(cuuint32_t)bytes[i], 8, 16};
+        const int rc = kq_map(m + i, u8, reinterpret_cast<const uint8_t*>(w) + (size_t)off[i] * nblk, 3, dim, stride, box, sw[i]);
+        if (rc) return rc;
+    }
+    return KTB200_OK;
+}
 template <int FMT>
-static int kq_launch(const CUtensorMap& qmap, const CUtensorMap& smap, const KqParams& p, int grid, cudaStream_t s) {
+static int kq_launch(const KqMaps& maps, const KqParams& p, int grid, cudaStream_t s) {
     KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kq_smem<FMT>()));
-    kq_gemm_kernel<FMT><<<grid, kKqThreads, kq_smem<FMT>(), s>>>(qmap, smap, p);
+    kq_gemm_kernel<FMT><<<grid, kKqThreads, kq_smem<FMT>(), s>>>(maps, p);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
@@ -670,16 +686,17 @@ int kq_gemm(const KqGemm& g, int device, cudaStream_t s) {
     p.expert_bytes = g.expert_bytes; p.dpitch = g.acts->pitch; p.pair = g.pair; p.R = g.R; p.nblk = g.K / QK_K; p.dx = g.acts->d;
     p.tinfo = g.tinfo; p.n_tiles = g.n_tiles_dev; p.tiles_mul = g.tiles_mul; p.y = g.y; p.hidden_type = g.hidden_type; p.bias = g.bias; p.bsz = g.bsz;
     p.t0 = g.t0; p.T = g.T; p.splits = g.splits; p.rt = (g.R + kKqRows - 1) / kKqRows; p.nt = (g.T + kKqN - 1) / kKqN; p.total = p.rt * p.nt * g.splits;
-    CUtensorMap qmap, smap;
-    int rc = kq_map(&qmap, g.acts->q, g.K, g.acts->rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc == KTB200_OK) rc = kq_map(&smap, g.acts->sums, g.K / 16, g.acts->rows, 16, CU_TENSOR_MAP_SWIZZLE_32B);
+    KqMaps maps;
+    int rc = kq_map_acts(&maps.q, g.acts->q, g.K, g.acts->rows, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc == KTB200_OK) rc = kq_map_acts(&maps.sums, g.acts->sums, g.K / 16, g.acts->rows, 16, CU_TENSOR_MAP_SWIZZLE_32B);
+    for (int i = 0; i < 2 && rc == KTB200_OK; i++) rc = kq_map_weights(maps.w[i], g.fmt, g.w[i], (long)g.experts * g.R, p.nblk);
     if (rc) return rc;
     const int sms = num_sms(device), grid = g.tinfo || p.total > sms ? sms : p.total;
     switch (g.fmt) {
-        case KQ_Q4K: return kq_launch<KQ_Q4K>(qmap, smap, p, grid, s);
-        case KQ_Q5K: return kq_launch<KQ_Q5K>(qmap, smap, p, grid, s);
-        case KQ_Q6K_T4: return kq_launch<KQ_Q6K_T4>(qmap, smap, p, grid, s);
-        case KQ_Q6K_SOA8: return kq_launch<KQ_Q6K_SOA8>(qmap, smap, p, grid, s);
+        case KQ_Q4K: return kq_launch<KQ_Q4K>(maps, p, grid, s);
+        case KQ_Q5K: return kq_launch<KQ_Q5K>(maps, p, grid, s);
+        case KQ_Q6K_T4: return kq_launch<KQ_Q6K_T4>(maps, p, grid, s);
+        case KQ_Q6K_SOA8: return kq_launch<KQ_Q6K_SOA8>(maps, p, grid, s);
         default: set_error("kq_gemm: unsupported weight type"); return KTB200_EINVAL;
     }
 }
@@ -703,7 +720,7 @@ int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_
         int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * K * hb, hidden_type, n, K, nullptr, 1, kq_is_q6(f), a, s);
         if (rc) return rc;
         KqGemm g{};
-        g.fmt = f; g.w[0] = g.w[1] = w; g.R = R; g.K = K; g.acts = &a; g.T = n; g.splits = splits; g.hidden_type = hidden_type; g.bias = bias; g.t0 = t0;
+        g.fmt = f; g.w[0] = g.w[1] = w; g.experts = 1; g.R = R; g.K = K; g.acts = &a; g.T = n; g.splits = splits; g.hidden_type = hidden_type; g.bias = bias; g.t0 = t0;
         void* yc = reinterpret_cast<uint8_t*>(y) + (size_t)t0 * R * hb;
         float* part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(mem.ptr) + act);
         if (splits == 1) { g.y = yc; g.bsz = bsz; }

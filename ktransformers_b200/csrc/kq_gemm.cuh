@@ -39,6 +39,7 @@ struct KqGemm {
     const void* w[2];          // pair: one matrix each; else both are the same matrix, a tile's second 128 rows following its first
     bool pair;
     long expert_bytes;         // bytes between two experts' matrices
+    int experts;
     int R, K;
     const KqActs* acts;
     // experts: device tables made by the caller; a tile is {expert, first row, first activation row (a multiple of 4), tokens}
