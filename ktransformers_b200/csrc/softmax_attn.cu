@@ -770,6 +770,10 @@ __global__ void __launch_bounds__(kMmaRows * 2, 4) window_softmax_attn_mma_kerne
     }
 }
 
+}  // namespace ktb
+#include "softmax_attn_tc.cuh"
+namespace ktb {
+
 // one CTA of 128 threads per map for each (token, head): the parts' weights exp(m_s - m) / l once in shared memory (parts without a key have
 // m = -inf and weigh nothing; the sink joins l), then the columns in parallel, parts in order; two maps are combined and the row normed here
 constexpr int kMergeMaxSplits = 128;
@@ -974,6 +978,11 @@ extern "C" int ktb200_softmax_attn(const ktb200_softmax_attn_params* c, int n_to
     if (tc) {
         using B = __nv_bfloat16;
         const int RH = a.RH = mma_heads_per_tile(heads / kv_heads), row_tile = kMmaRows / maps;
+        // prompt portions: 256 rows per CTA on tcgen05 (its TMA reads whole runs of 64 keys of a page)
+        if (maps == 1 && splits == 1 && dim == 128 && vdim == 128 && 128 % RH == 0 && c->page_size % 64 == 0 && n_tokens >= c->n_seqs * (64 / RH) &&
+            softmax_tc_tiles(RH, n_tokens, c->n_seqs) * (heads / RH) >= kTcMinCtas &&
+            ((reinterpret_cast<uintptr_t>(c->q) | reinterpret_cast<uintptr_t>(c->cache)) & 15) == 0)
+            return launch_softmax_tc(a, n_tokens, (cudaStream_t)stream);
         const dim3 grid(ktb200_softmax_attn_tiles(heads, kv_heads, maps, n_tokens, c->n_seqs), kv_heads * (heads / kv_heads / RH), splits);
         const size_t smem = (((size_t)row_tile + 2 * kMmaKeys) * (maps * dim + kMmaPad) + (size_t)2 * kMmaKeys * (vdim + kMmaPad)) * sizeof(B);
 #define MMA_LAUNCH(DK, DV, MAPS, BIAS)                                                                                             \
