@@ -420,6 +420,13 @@ int ktb200_experts_gate_up_by_expert(const void* x, const int64_t* ids, int top,
                                      void* stream);
 int ktb200_experts_down_by_expert(const void* act, const int64_t* ids, const float* weights, int top, int n_experts, const void* w_down,
                                   float* pair_rows, float* out, int n_tokens, int width, int ff, int staged, int dtype, void* stream);
+/* A prompt portion through un-quantised bf16 experts (csrc/experts_gemm.cu): pairs sorted by expert, two grouped tensor-core GEMMs, the weighted sum in
+ * slot order: out [n_tokens][width] fp32.  w_gate NULL: relu(W_up x)^2.  weights_on_input: a weight multiplies its expert's pre-activations instead
+ * of its output.  width and ff multiples of 8, at most 1024 experts, 16-byte aligned; workspace of the given size. */
+size_t ktb200_experts_prompt_workspace(int n_tokens, int top, int n_experts, int width, int ff);
+int ktb200_experts_prompt(const void* x, const int64_t* ids, const float* weights, int weights_on_input, int top, int n_experts, const void* w_gate,
+                          const void* w_up, const void* w_down, float* out, int n_tokens, int width, int ff, int act_kind, float limit, void* workspace,
+                          void* stream);
 /* ktb200_experts_combine: out[t] = sum_j weights[t][j] rows[place[t * top + j]] (place NULL: row t * top + j), rows of dtype, fp32 sums in slot
  *   order: the last step of a grouped run.  In all of these calls an id at or beyond n_experts names no expert: its pair adds nothing. */
 int ktb200_experts_combine(const void* rows, const int64_t* place, const int64_t* ids, int n_experts, const float* weights, int top, float* out,

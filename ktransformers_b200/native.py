@@ -165,6 +165,8 @@ SEQ_SYMBOLS = {
     "ktb200_experts_down": (_I, [_VP, _VP, _VP, _I, _I, _VP, _VP, _I, _I, _I, _I, _VP]),
     "ktb200_experts_gate_up_by_expert": (_I, [_VP, _VP, _I, _I, _VP, _VP, _VP, _I, _I, _I, _I, _I, _F, _VP, _I, _VP]),
     "ktb200_experts_down_by_expert": (_I, [_VP, _VP, _VP, _I, _I, _VP, _VP, _VP, _I, _I, _I, _I, _I, _VP]),
+    "ktb200_experts_prompt_workspace": (C.c_size_t, [_I, _I, _I, _I, _I]),
+    "ktb200_experts_prompt": (_I, [_VP, _VP, _VP, _I, _I, _I, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _F, _VP, _VP]),
     "ktb200_experts_combine": (_I, [_VP, _VP, _VP, _I, _VP, _I, _VP, _I, _I, _I, _VP]),
     "ktb200_sum_rmsnorm": (_I, [C.POINTER(SumRmsnormParams), _I, _I, _I, _VP]),
     # csrc/seq_mixers.cu

@@ -532,9 +532,9 @@ class KExpertsDense(nn.Module):
     Batches of a few tokens (decode steps of several sequences) take the `_by_expert` kernels: one CTA column per expert
     finds the pairs routed to it and streams each weight row once for two or four of them, with the same per-pair sums.
     From `grouped_min_tokens` tokens on (the threshold of the quantised experts' grouped path) the pairs are sorted by expert
-    and each matrix runs as ONE library grouped GEMM over the per-expert token segments (bf16; fp32 and odd sizes: one GEMM
-    per expert), so an expert's weights are read once per step instead of once per pair; the weighted sum over a token's
-    slots stays fp32 in slot order.
+    and the matrices run as grouped tensor-core GEMMs over the per-expert token segments (bf16: `ktb200_experts_prompt`, activation and fp32
+    output included; rows it does not take: the library's grouped GEMM, or one GEMM per expert), so an expert's weights are read once per
+    128 of its pairs instead of once per pair; the weighted sum over a token's slots stays fp32 in slot order.
     A choice at or beyond `experts` names no expert with weights (an identity expert): it adds nothing on any path.
     The counterpart of KExpertsB200 for checkpoints that ship dense experts (the reference's KExpertsTorch, experts.py:562-678,
     loops over experts in torch)."""
@@ -564,7 +564,7 @@ class KExpertsDense(nn.Module):
                     p.data[e].copy_(loader.load_tensor(f"{prefix}e{e}.{n}", "cpu"))
 
     def grouped_is_device_only(self, dtype) -> bool:
-        """whether the grouped path runs as the library's grouped GEMM, which takes the segment ends on the device (no host read)"""
+        """whether the grouped path takes the segments on the device (no host read)"""
         return dtype == torch.bfloat16 and self.width % 8 == 0 and self.ff % 8 == 0 and hasattr(nn.functional, "grouped_mm")
 
     def small_batches_stay_on_device(self, top: int, dtype, max_tokens: int) -> bool:
@@ -575,17 +575,18 @@ class KExpertsDense(nn.Module):
         return self.grouped_is_device_only(dtype) or per_pair or by_expert
 
     def prefers_grouped(self, T: int, top: int, dtype) -> bool:
-        """Below `grouped_min_tokens`: the by-expert kernels stream an expert's rows once per four of its pairs, about
-        `pairs / (4 experts) + 1/2` passes over all experts' weights at ~5 TB/s; the grouped GEMM path reads them once but
-        costs ~0.3 ms of sorting and small launches.  Taken only when it needs no host read, so that a decode step's
-        launches do not depend on the batch size in a way that graph replay could not follow."""
+        """Below `grouped_min_tokens`: the by-expert kernels stream an expert's rows once for every few of its pairs, measured as 20 us and about
+        `experts present + pairs / 8` experts' weights at 4.5 TB/s; the grouped products stream them once, 30 us and 5.6 TB/s.  Both models are good
+        to a quarter (4-47 tokens on five shapes of 8-128 experts of 3-100 MB: from 24 tokens on 138-144 us against 104 with 32 experts of 13 MB, 471 against
+        166 at 32 tokens with 8 of 100 MB), hence the margin.  Taken only when it needs no host read, so that a decode step's launches do not
+        depend on the batch size in a way that graph replay could not follow."""
         if T >= self.grouped_min_tokens:
             return True
         if not self.grouped_is_device_only(dtype):
             return False
-        all_bytes = (3.0 if self.gated else 2.0) * self.experts * self.ff * self.width * 2
-        passes = T * top / (4.0 * self.experts) + 0.5
-        return (passes - 1.0) * all_bytes / 5e12 > 300e-6
+        expert_bytes, pairs = (3.0 if self.gated else 2.0) * self.ff * self.width * 2, T * top
+        present = self.experts * (1.0 - (1.0 - min(1.0, top / self.experts)) ** T)
+        return 20e-6 + (present + pairs / 8) * expert_bytes / 4.5e12 > 1.35 * (30e-6 + present * expert_bytes / 5.6e12)
 
     def forward(self, x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, on_input: bool = False) -> torch.Tensor:
         """x [T, width], ids [T, top] int64, weights [T, top] fp32 -> [T, width] fp32.  A weight multiplies its expert's output, or with
@@ -628,9 +629,23 @@ class KExpertsDense(nn.Module):
                                                       row_scale.data_ptr() if row_scale is not None else None, TORCH_TO_GGML_HIDDEN[u.dtype], st))
         return out
 
+    def _sorted_gemms(self, x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor) -> bool:
+        """whether a batch runs as this library's grouped GEMMs (csrc/experts_gemm.cu): bf16 rows as they are, whole 16-byte pieces"""
+        mats = (self.up, self.down) + ((self.gate,) if self.gated else ())
+        return (x.dtype == torch.bfloat16 and x.is_cuda and self.width % 8 == 0 and self.ff % 8 == 0 and self.experts <= 1024 and ids.dtype == torch.int64
+                and weights.dtype == torch.float32 and all(t.is_contiguous() for t in (x, ids, weights)) and x.data_ptr() % 16 == 0
+                and all(m.is_contiguous() and m.data_ptr() % 16 == 0 and m.dtype == torch.bfloat16 for m in mats))
+
     def forward_grouped(self, x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, on_input: bool = False) -> torch.Tensor:
         T, top = ids.shape
         F = nn.functional
+        if self._sorted_gemms(x, ids, weights):
+            lib = native.seq_lib()
+            out = torch.empty((T, self.width), dtype=torch.float32, device=x.device)
+            ws = torch.empty(lib.ktb200_experts_prompt_workspace(T, top, self.experts, self.width, self.ff), dtype=torch.uint8, device=x.device)
+            native.check_seq(lib.ktb200_experts_prompt(x.data_ptr(), ids.data_ptr(), weights.data_ptr(), int(on_input), top, self.experts, self.gate.data_ptr() if self.gated else None,
+                                                       self.up.data_ptr(), self.down.data_ptr(), out.data_ptr(), T, self.width, self.ff, self.act, self.limit, ws.data_ptr(), _stream(x.device)))
+            return out
         flat = ids.reshape(-1)
         order = torch.argsort(flat, stable=True)
         # (choices beyond the experts sort behind every segment and are left out of the counts)
