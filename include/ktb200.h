@@ -125,7 +125,8 @@ float* ktb200_moe_intermediate(ktb200_moe* moe);
  * weight: DEVICE ptr, e4m3 bytes [out][in] (16-byte aligned, in % 128 == 0); weight_scale_inv: DEVICE fp32 [ceil(out/128)][in/128].
  * forward: x [qlen][in] -> y [qlen][out] in hidden_type (x is quantised per token and 128 values inside the kernel, exactly like
  * act_quant; rows >= *bsz untouched).  An all-zero 128-block of x yields NaN outputs, as it does in the reference (0 / 0).
- * TMA + tcgen05.mma.kind::f8f6f4 + TMEM; stream-ordered; everything is allocated at create -> CUDA-graph capturable.
+ * TMA + tcgen05.mma.kind::f8f6f4 + TMEM; stream-ordered, CUDA-graph capturable: up to 16 rows use what create allocated, more rows take their
+ * quantised activations' scratch from a stream-ordered pool for the call.
  * ------------------------------------------------------------------------------------------ */
 typedef struct ktb200_fp8_linear ktb200_fp8_linear;
 int ktb200_fp8_linear_create(int in_features, int out_features, const void* weight_e4m3_dev, const float* weight_scale_inv_dev, int hidden_type, int device,
