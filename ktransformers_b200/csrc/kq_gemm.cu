@@ -579,16 +579,23 @@ __global__ void __launch_bounds__(256) kq_quant_kernel(const void* x, int hidden
             if (row >= 0) kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2);
         }
 }
-__global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const float* u, const int* pos, int n, int K, int use_silu, int q6, const KqActs a) {
+// (without pos: rows 0 .. n, each the sum of `splits` parts)
+__global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const float* u, const int* pos, int splits, int n, int K, int use_silu, int q6, const KqActs a) {
     const int lane = threadIdx.x & 31, nblk = K / QK_K;
     const long gw = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gw >= (long)n * nblk) return;
-    const int i = (int)(gw / nblk), b = (int)(gw - (long)i * nblk), row = pos[i];
+    const int i = (int)(gw / nblk), b = (int)(gw - (long)i * nblk), row = pos ? pos[i] : i;
     if (row < 0) return;
     const long o = (long)row * K + (long)b * QK_K + lane * 8;
     const float4 g0 = *reinterpret_cast<const float4*>(g + o), g1 = *reinterpret_cast<const float4*>(g + o + 4);
     const float4 u0 = *reinterpret_cast<const float4*>(u + o), u1 = *reinterpret_cast<const float4*>(u + o + 4);
-    const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uv[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+    for (int p = 1; p < splits; p++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            gv[j] += g[(long)p * n * K + o + j];
+            uv[j] += u[(long)p * n * K + o + j];
+        }
     float v[8], d;
     uint32_t w0, w1;
     int s;
@@ -598,13 +605,14 @@ __global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const
     const int s2 = s + __shfl_xor_sync(0xffffffffu, s, 1);
     kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2);
 }
-// y = sum of the K parts + bias, in the hidden type
-__global__ void __launch_bounds__(256) kq_finish_kernel(const float* part, int splits, int T, int R, void* y, int hidden_type, const float* bias, const int* bsz, int t0) {
+// y = sum of the K parts + bias, in the hidden type (accumulate: y + that sum, rounded first)
+__global__ void __launch_bounds__(256) kq_finish_kernel(const float* part, int splits, int T, int R, void* y, int hidden_type, const float* bias, int accumulate, const int* bsz, int t0) {
     const long i = (long)blockIdx.x * 256 + threadIdx.x, n = (long)(bsz ? max(0, min(T, *bsz - t0)) : T) * R;
     if (i >= n) return;
     float v = part[i];
     for (int s = 1; s < splits; s++) v += part[(long)s * T * R + i];
     if (bias) v += bias[i % R];
+    if (accumulate) v = load_hidden(y, i, hidden_type) + round_hidden(v, hidden_type);
     store_hidden(y, i, hidden_type, v);
 }
 
@@ -614,7 +622,7 @@ int kq_quant(const void* x, int hidden_type, int T, int K, const int* pos, int k
     return KTB200_OK;
 }
 int kq_act_quant(const float* g, const float* u, const int* pos, int n, int K, int use_silu, bool q6, const KqActs& a, cudaStream_t s) {
-    kq_act_quant_kernel<<<(unsigned)(((long)n * (K / QK_K) + 7) / 8), 256, 0, s>>>(g, u, pos, n, K, use_silu, q6, a);
+    kq_act_quant_kernel<<<(unsigned)(((long)n * (K / QK_K) + 7) / 8), 256, 0, s>>>(g, u, pos, 1, n, K, use_silu, q6, a);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
@@ -701,6 +709,12 @@ int kq_gemm(const KqGemm& g, int device, cudaStream_t s) {
     }
 }
 
+// K in parts when the tiles leave SMs idle, two blocks or more each
+static int kq_splits(int tiles, int nblk, int sms) {
+    const int n = sms / tiles < nblk / 2 ? sms / tiles : nblk / 2;
+    return n < 1 ? 1 : n;
+}
+
 int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_type, int T, void* y, const float* bias, const int* bsz, int device, cudaStream_t s) {
     const KqFmt f = kq_fmt(fmt);
     if (f == KQ_NONE || (uintptr_t)w % 16) return 1;
@@ -709,10 +723,7 @@ int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_
     for (int t0 = 0; t0 < T; t0 += kChunk) {
         const int n = T - t0 < kChunk ? T - t0 : kChunk, sms = num_sms(device);
         const int tiles = ((R + kKqRows - 1) / kKqRows) * ((n + kKqN - 1) / kKqN), nblk = K / QK_K;
-        // K in parts when the tiles leave SMs idle, two blocks or more each
-        int splits = sms / tiles;
-        if (splits > nblk / 2) splits = nblk / 2;
-        if (splits < 1) splits = 1;
+        const int splits = kq_splits(tiles, nblk, sms);
         ScratchBlock mem(s);
         const size_t act = (KqActs::bytes(n, K) + 255) / 256 * 256;
         KTB_CUDA_CHECK(mem.take(device, act + (splits > 1 ? (size_t)splits * n * R * 4 : 0)));
@@ -728,9 +739,48 @@ int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_
         rc = kq_gemm(g, device, s);
         if (rc) return rc;
         if (splits > 1) {
-            kq_finish_kernel<<<(unsigned)(((long)n * R + 255) / 256), 256, 0, s>>>(part, splits, n, R, yc, hidden_type, bias, bsz, t0);
+            kq_finish_kernel<<<(unsigned)(((long)n * R + 255) / 256), 256, 0, s>>>(part, splits, n, R, yc, hidden_type, bias, 0, bsz, t0);
             KTB_LAUNCH_CHECK();
         }
+    }
+    return KTB200_OK;
+}
+
+int kq_mlp(const ktb200_mlp* m, const void* x, int T, void* y, int accumulate, const int* bsz, cudaStream_t s) {
+    const KqFmt f[3] = {kq_fmt(pick_fmt(m->gate_type, m->gu_soa)), kq_fmt(pick_fmt(m->up_type, m->gu_soa)), kq_fmt(pick_fmt(m->down_type, m->down_layout))};
+    const void* w[3] = {m->gate, m->up, m->down};
+    for (int i = 0; i < 3; i++)
+        if (f[i] == KQ_NONE || (uintptr_t)w[i] % 16) return 1;
+    if (kq_is_q6(f[0]) != kq_is_q6(f[1])) return 1;      // (gate and up read the same activations)
+    constexpr int kChunk = 1024;      // rows per pass: bounds the scratch
+    const int H = m->H, I = m->I, dev = m->device, sms = num_sms(dev);
+    const size_t hb = type_size(m->hidden_type);
+    for (int t0 = 0; t0 < T; t0 += kChunk) {
+        const int n = T - t0 < kChunk ? T - t0 : kChunk, nt = (n + kKqN - 1) / kKqN;
+        const int su = kq_splits((I + kKqRows - 1) / kKqRows * nt, H / QK_K, sms), sd = kq_splits((H + kKqRows - 1) / kKqRows * nt, I / QK_K, sms);
+        auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+        const size_t n_x = up(KqActs::bytes(n, H)), n_a = up(KqActs::bytes(n, I)), n_g = up((size_t)su * n * I * 4), n_d = up((size_t)sd * n * H * 4);
+        ScratchBlock mem(s);
+        KTB_CUDA_CHECK(mem.take(dev, n_x + n_a + 2 * n_g + n_d));
+        uint8_t* at = reinterpret_cast<uint8_t*>(mem.ptr);
+        const KqActs xa(at, n, H), aa(at + n_x, n, I);
+        float *gu[2] = {reinterpret_cast<float*>(at + n_x + n_a), reinterpret_cast<float*>(at + n_x + n_a + n_g)}, *part = reinterpret_cast<float*>(at + n_x + n_a + 2 * n_g);
+        int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * H * hb, m->hidden_type, n, H, nullptr, 1, kq_is_q6(f[0]), xa, s);
+        if (rc) return rc;
+        KqGemm g{};
+        g.experts = 1; g.R = I; g.K = H; g.acts = &xa; g.T = n; g.splits = su;
+        for (int i = 0; i < 2; i++) {
+            g.fmt = f[i]; g.w[0] = g.w[1] = w[i]; g.out[0] = g.out[1] = gu[i];
+            rc = kq_gemm(g, dev, s);
+            if (rc) return rc;
+        }
+        kq_act_quant_kernel<<<(unsigned)(((long)n * (I / QK_K) + 7) / 8), 256, 0, s>>>(gu[0], gu[1], nullptr, su, n, I, 1, kq_is_q6(f[2]), aa);
+        KTB_LAUNCH_CHECK();
+        g.fmt = f[2]; g.w[0] = g.w[1] = w[2]; g.R = H; g.K = I; g.acts = &aa; g.splits = sd; g.out[0] = g.out[1] = part;
+        rc = kq_gemm(g, dev, s);
+        if (rc) return rc;
+        kq_finish_kernel<<<(unsigned)(((long)n * H + 255) / 256), 256, 0, s>>>(part, sd, n, H, reinterpret_cast<uint8_t*>(y) + (size_t)t0 * H * hb, m->hidden_type, nullptr, accumulate, bsz, t0);
+        KTB_LAUNCH_CHECK();
     }
     return KTB200_OK;
 }

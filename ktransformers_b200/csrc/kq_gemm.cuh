@@ -64,5 +64,7 @@ int kq_act_quant(const float* g, const float* u, const int* pos, int n, int K, i
 
 // y = x . W^T for a batch of T rows of one matrix.  Returns 1 when the shape does not suit it.
 int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_type, int T, void* y, const float* bias, const int* bsz, int device, cudaStream_t s);
+// y (+)= W_down (silu(W_gate x) * W_up x) for a batch of T rows.  Returns 1 when the matrices' layouts do not suit it.
+int kq_mlp(const ktb200_mlp* m, const void* x, int T, void* y, int accumulate, const int* bsz, cudaStream_t s);
 
 }  // namespace ktb

@@ -127,3 +127,31 @@ def test_experts_of_a_prompt_at_tile_edges(gu, down, H, I, T):
     assert (got.double() - want).norm() <= 1e-3 * want.norm()
     assert (got.double() - want).abs().max() <= 2e-2 * want.abs().max()
     m.close()
+
+
+# an MLP of a prompt portion against the CPU oracle (its bounds are those of the decode kernels: an activation whose rounding falls to the other side moves a
+# quantised value by one step), with the rounded sum of `accumulate` and a device-side batch size
+@pytest.mark.parametrize("gate,up,down,H,I,T", [(Q4_K, Q4_K, Q6_K, 512, 256, 9), (Q4_K, Q5_K, Q4_K, 1024, 768, 64), (Q6_K, Q6_K, Q6_K, 768, 512, 65), (Q5_K, Q5_K, Q5_K, 256, 1280, 130),
+                                                (Q4_K, Q4_K, Q6_K, 2048, 512, 1100)])
+@pytest.mark.parametrize("hid", [F32, BF16])
+def test_mlp_of_a_prompt(gate, up, down, H, I, T, hid):
+    g, u, d = (synth_blocks(t, n, seed=i + 3) for i, (t, n) in enumerate(((gate, I * H), (up, I * H), (down, H * I))))
+    rnd = torch.Generator().manual_seed(T)
+    x, y0 = (torch.randn(T, H, generator=rnd) / 100).to(TORCH[hid]), torch.randn(T, H, generator=rnd).to(TORCH[hid])
+    host = lambda t: (t.view(torch.int16).numpy().view("uint16") if hid == BF16 else t.numpy())
+    want = torch.from_numpy(Oracle().mlp_forward(H, I, g.cpu().numpy(), u.cpu().numpy(), d.cpu().numpy(), gate, up, down, hid, host(x)).copy().view("int16" if hid == BF16 else "float32"))
+    want = want.view(TORCH[hid]).view(T, H)
+    lib, h, w = native.lib(), C.c_void_p(), [t.cuda() for t in (g, u, d)]
+    native.check(lib.ktb200_mlp_create(H, I, *[t.data_ptr() for t in w], gate, up, down, hid, T, 0, C.byref(h)))
+    native.check(lib.ktb200_mlp_load_weights(h, _stream()))
+    xd, live = x.cuda(), torch.tensor([T - 5], dtype=torch.int32, device="cuda")
+    for accumulate in (0, 1):
+        y = y0.cuda()
+        native.check(lib.ktb200_mlp_forward(h, T, xd.data_ptr(), y.data_ptr(), accumulate, live.data_ptr(), _stream()))
+        got, ref = y.cpu(), (y0 + want if accumulate else want)
+        assert torch.equal(got[T - 5:], y0[T - 5:])
+        diff, size = (got[:T - 5].double() - ref[:T - 5].double()).abs(), want.double().abs().max()
+        # bf16: the MLP's rows are rounded, then their sum with what was there; each may fall to the other side, one unit (at most 2^-7) of either
+        units = 2.0 ** -7 * (ref.double().abs() + want.double().abs())[:T - 5] if hid == BF16 else 0
+        assert (diff <= units + 1e-3 * size).all(), (diff / size).max().item()
+    lib.ktb200_mlp_destroy(h)
