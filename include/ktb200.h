@@ -340,7 +340,8 @@ int ktb200_mla_prep(const void* q_dev, int num_heads, int qk_nope_head_dim, cons
 
 /* ktb200_mla_prep for one new token per sequence, from the positions themselves (int64, `position_stride` elements apart): cos / sin of
  * position * inv_freq[32], the cache row of `cache_position` (one for all sequences) in the static cache whose sequence b owns pages
- * [b * max_pages, (b + 1) * max_pages), and kv_len_out[b] = position + 1. */
+ * [b * max_pages, (b + 1) * max_pages), and kv_len_out[b] = position + 1,
+ * at most max_pages * page_size.  kv_len_out has `batch` elements: the caller checks that. */
 int ktb200_mla_step_prep(const void* q_dev, int num_heads, int qk_nope_head_dim, const void* kv_a_out_dev, const void* kv_a_norm_weight_dev, float eps,
                          const float* inv_freq_dev, const long long* positions_dev, long position_stride, const long long* cache_position_dev, void* kv_cache_dev,
                          int page_size, int max_pages, void* q_pe_out_dev, int* kv_len_out_dev, int batch, void* stream);

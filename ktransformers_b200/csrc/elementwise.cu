@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) mla_step_prep_kernel(const __nv_bfloat16*
         }
         return;
     }
-    if (threadIdx.x == 0) kv_len_out[b] = (int)at + 1;
+    if (threadIdx.x == 0) kv_len_out[b] = (int)min(at + 1, (long long)max_pages * page_size);      // (no row lies behind the cache's last)
     const __nv_bfloat16* row = kva + b * (LAT + R);
     const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + 2 * threadIdx.x));
     const float inv = rsqrtf(block_sum(v.x * v.x + v.y * v.y, red) / (float)LAT + eps);

@@ -53,6 +53,14 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         bsz, heads, nope = x.shape[0], self.num_heads, self.qk_nope_head_dim
         if tuple(position_ids.shape) != (bsz, 1) or cache_position.numel() != 1 or cache.max_batch_size < bsz or rot.inv_freq.dtype != torch.float32 or nope % 2:
             return None
+        w = self.mla_wrapper
+        if w is None:
+            w = self.mla_wrapper = MLAWrapperSingleton.get_instance(str(x.device), bsz, cache.max_pages * bsz, use_cuda_graph=True)
+        # the prep kernel writes `bsz` lengths as they come: a wrapper made for fewer sequences or pages (the device's wrapper keeps its first caller's
+        # sizes) is left to the path below, whose copies check the shapes
+        lens = w.kv_len_arr_buf
+        if lens.numel() < bsz or lens.dtype != torch.int32 or lens.device != x.device or not lens.is_contiguous() or w.max_pages < cache.max_pages:
+            return None
         lib, stream = native.lib(), torch.cuda.current_stream(x.device).cuda_stream
         if self.q_lora_rank is None:
             q = self.q_proj(x)
@@ -70,9 +78,6 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
             return None
         inv_freq = rot.inv_freq.to(x.device)
         kv = cache.key_cache[self.layer_idx]
-        w = self.mla_wrapper
-        if w is None:
-            w = self.mla_wrapper = MLAWrapperSingleton.get_instance(str(x.device), bsz, cache.max_pages * bsz, use_cuda_graph=True)
         if w.need_plan:
             indptr = torch.arange(0, bsz + 1, dtype=torch.int32, device=x.device) * cache.max_pages
             w.plan(None, indptr, cache.page_table_list[self.layer_idx].reshape(-1), (position_ids[:, 0] + 1).to(torch.int32), None, heads, 512, 64, cache.page_size, self.softmax_scale, bf16, kv.dtype)
@@ -81,7 +86,7 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         q_abs = torch.empty((bsz, heads, 512), dtype=bf16, device=x.device)
         native.check(lib.ktb200_mla_step_prep(q.data_ptr(), heads, nope, kva.data_ptr(), kv_norm.weight.data_ptr(), float(kv_norm.variance_epsilon), inv_freq.data_ptr(),
                                               position_ids.data_ptr(), position_ids.stride(0), cache_position.data_ptr(), kv.data_ptr(), cache.page_size, cache.max_pages, q_pe.data_ptr(),
-                                              w.kv_len_arr_buf.data_ptr(), bsz, stream))
+                                              lens.data_ptr(), bsz, stream))
         native.check(lib.ktb200_mla_absorb_q(q.data_ptr(), nope + 64, heads * (nope + 64), q_absorb.data_ptr(), heads, nope, 512, q_abs.data_ptr(), bsz, stream))
         if not torch.cuda.is_current_stream_capturing():
             cache.past_tokens[self.layer_idx] += 1

@@ -54,6 +54,9 @@ class MLAWrapper:
     def run(self, q_nope, q_pe, ckv, k_pe, return_lse=False):
         assert not self.need_plan, "plan() before run()"
         B = q_nope.shape[0]
+        # the kernel reads a page-table row and a length for every query row, and num_heads heads of each
+        if B > self.max_batch_size or q_nope.numel() != B * self.num_heads * 512 or q_pe.numel() != B * self.num_heads * 64:
+            raise ValueError(f"run: queries {tuple(q_nope.shape)} / {tuple(q_pe.shape)} for a wrapper of {self.max_batch_size} sequences, planned for {self.num_heads} heads of 512 + 64")
         # the two views must alias one [pages, page, 576] buffer
         cache_ptr = ckv.data_ptr()
         assert ckv.stride(-1) == 1 and k_pe.data_ptr() == cache_ptr + 512 * ckv.element_size() and \

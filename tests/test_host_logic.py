@@ -386,3 +386,14 @@ def test_hybrid_safetensors_serve_the_gguf_loader_surface(tmp_path):
         ld.load_gguf_tensor("model.layers.1.mlp.shared_experts.up_proj.weight")
     with pytest.raises(ValueError):
         ld.load_experts("model.layers.7.mlp.experts")
+
+
+@pytest.mark.parametrize("q,q_pe", [((2, 16, 512), (2, 16, 64)), ((1, 8, 512), (1, 8, 64)), ((1, 16, 512), (1, 8, 64))])
+def test_mla_wrapper_refuses_queries_it_has_no_rows_for(q, q_pe):
+    """more sequences than the wrapper was made for, or fewer heads than it was planned for: refused on the host, before the library is called"""
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapper
+    w = MLAWrapper(1, 4, device="cpu")
+    w.need_plan, w.num_heads, w.page_size, w.sm_scale, w.workspace = False, 16, 64, 1.0, torch.empty(0, dtype=torch.uint8)
+    kv = torch.zeros(4, 64, 576, dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="1 sequences, planned for 16 heads"):
+        w.run(torch.zeros(q, dtype=torch.bfloat16), torch.zeros(q_pe, dtype=torch.bfloat16), kv[..., :512], kv[..., 512:])

@@ -44,3 +44,37 @@ def test_step_equals_the_module_path(bsz, heads, q_rank, pos):
     assert torch.equal(lens[0], lens[1]) and (lens[0] == pos + 1).all()
     assert ((rows[0] - rows[1]).abs() <= 2.0 ** -6 * rows[1].abs() + 2.0 ** -7).all()
     assert (outs[0] - outs[1]).abs().max() <= 2.0 ** -6 * outs[1].abs().max()
+
+
+def test_step_beyond_its_wrapper_is_refused(monkeypatch):
+    """The attention's wrapper keeps the sizes of its first caller.  A step of two sequences on one made for one raises, before the prep kernel
+    could write two lengths into one place (here that kernel and the attention are replaced by a failure: neither may be reached)."""
+    from ktransformers_b200 import native
+    from ktransformers_b200.models.custom_cache import StaticCache
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3Config, DeepseekV3RotaryEmbedding
+    from ktransformers_b200.operators.attention import KDeepseekV2Attention
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapperSingleton
+
+    real = native.lib()
+
+    class Watched:
+        def __getattr__(self, name):
+            assert name not in ("ktb200_mla_step_prep", "ktb200_mla_decode"), name
+            return getattr(real, name)
+
+    monkeypatch.setattr(MLAWrapperSingleton, "wrappers", {})
+    cfg = DeepseekV3Config(hidden_size=512, num_attention_heads=16, q_lora_rank=64, num_hidden_layers=1)
+    plain = DeepseekV3Attention(cfg, layer_idx=0).to(device="cuda", dtype=torch.bfloat16)
+    plain.rotary_emb = DeepseekV3RotaryEmbedding(64).to("cuda")
+    for bsz in (1, 2):
+        op = KDeepseekV2Attention("blk.0.self_attn", None, cfg, plain, "cuda", "cuda")
+        cache = StaticCache(cfg, max_batch_size=bsz, max_cache_len=128, device="cuda")
+        step = lambda: op(torch.randn(bsz, 1, 512, device="cuda").to(torch.bfloat16), position_ids=torch.zeros((bsz, 1), dtype=torch.int64, device="cuda"), past_key_value=cache,
+                          cache_position=torch.zeros(1, dtype=torch.int64, device="cuda"))
+        with torch.no_grad():
+            if bsz == 1:
+                step()
+            else:
+                monkeypatch.setattr(native, "lib", lambda: Watched())
+                with pytest.raises((RuntimeError, ValueError)):
+                    step()
