@@ -16,6 +16,7 @@
 #pragma once
 #include <cuda.h>
 
+#include "key_runs.h"
 #include "umma.cuh"
 
 namespace ktb {
@@ -111,8 +112,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
                 const int st = j & 1, ph = ((j >> 1) & 1) ^ 1;
                 int row[2];
 #pragma unroll
-                for (int i = 0; i < 2; i++) {      // (keys behind max_pos may name a page that is not this sequence's: they are masked, and their values zeroed)
-                    const int kp = (t0 + j) * kTcKeys + 64 * i;
+                for (int i = 0; i < 2; i++) {      // (keys outside [lo, max_pos] that come along are masked, and their values zeroed)
+                    const int kp = key_run((t0 + j) * kTcKeys, i, lo, max_pos);
                     row[i] = pt[(kp / a.page_size) % a.max_pages] * a.page_size + kp % a.page_size;
                 }
                 const uint32_t kf = smem_u32(&misc.k_full[st]), vf = smem_u32(&misc.v_full[st]);
@@ -341,7 +342,7 @@ static int launch_softmax_tc(const SmAttn& a, int n_tokens, cudaStream_t s) {
     const cuuint32_t estr[3] = {1, 1, 1};
     const cuuint64_t qd[3] = {128, (cuuint64_t)a.H, (cuuint64_t)n_tokens}, qs[2] = {256, (cuuint64_t)a.H * 256};
     const cuuint32_t qb[3] = {64, (cuuint32_t)a.RH, (cuuint32_t)(128 / a.RH)};
-    // (rows are named by the page table, which bounds them: the map itself does not know how many pages there are)
+    // (rows come from the page table's columns of pages that hold a visible key, which bounds them: the map itself does not know how many pages there are)
     const cuuint64_t kd[2] = {(cuuint64_t)a.G * 256, 1u << 30}, ks[1] = {(cuuint64_t)a.G * 512};
     const cuuint32_t kb[2] = {64, 64};
     CUresult cr = enc(&qmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(a.q), qd, qs, qb, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,

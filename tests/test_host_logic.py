@@ -397,3 +397,23 @@ def test_mla_wrapper_refuses_queries_it_has_no_rows_for(q, q_pe):
     kv = torch.zeros(4, 64, 576, dtype=torch.bfloat16)
     with pytest.raises(ValueError, match="1 sequences, planned for 16 heads"):
         w.run(torch.zeros(q, dtype=torch.bfloat16), torch.zeros(q_pe, dtype=torch.bfloat16), kv[..., :512], kv[..., 512:])
+
+
+def test_prompt_attention_looks_up_only_pages_with_visible_keys(tmp_path):
+    """csrc/key_runs.h as the prompt attention's copies use it: every run of 64 keys that is copied holds a visible key, and every visible key is
+    copied to its own place"""
+    import ctypes
+    import subprocess
+    src = tmp_path / "runs.cpp"
+    src.write_text('#include "key_runs.h"\nextern "C" int run(int k0, int i, int lo, int hi) { return ktb::key_run(k0, i, lo, hi); }\n')
+    subprocess.check_call(["g++", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "ktransformers_b200", "csrc"), str(src), "-o", str(tmp_path / "runs.so")])
+    run = ctypes.CDLL(str(tmp_path / "runs.so")).run
+    edges = [0, 1, 62, 63, 64, 65, 127, 128, 129, 191, 192, 255, 256, 300, 319, 320]
+    for lo in edges:
+        for hi in (e for e in edges if e >= lo):
+            for k0 in range(lo // 128 * 128, hi + 1, 128):
+                for i in (0, 1):
+                    k = run(k0, i, lo, hi)
+                    assert k % 64 == 0 and k + 63 >= lo and k <= hi, (lo, hi, k0, i, k)
+                    if any(lo <= x <= hi for x in range(k0 + 64 * i, k0 + 64 * i + 64)):
+                        assert k == k0 + 64 * i
