@@ -430,7 +430,8 @@ int ktb200_experts_prompt(const void* x, const int64_t* ids, const float* weight
                           const void* w_up, const void* w_down, float* out, int n_tokens, int width, int ff, int act_kind, float limit, void* workspace,
                           void* stream);
 /* ktb200_experts_combine: out[t] = sum_j weights[t][j] rows[place[t * top + j]] (place NULL: row t * top + j), rows of dtype, fp32 sums in slot
- *   order: the last step of a grouped run.  In all of these calls an id at or beyond n_experts names no expert: its pair adds nothing. */
+ *   order: the last step of a grouped run.  In all of these calls an id at or beyond n_experts names no expert: its pair adds nothing;
+ *   in ktb200_experts_prompt and here a negative one neither. */
 int ktb200_experts_combine(const void* rows, const int64_t* place, const int64_t* ids, int n_experts, const float* weights, int top, float* out,
                            int n_tokens, int width, int dtype, void* stream);
 /* w_gate == NULL in the four calls above: experts of two matrices, act = relu(W_up x)^2.  Otherwise act_kind picks what becomes of

@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(256) experts_down_by_expert_kernel(const T* __
     }
 }
 
-// out[t][d] = sum_j w[t][j] * y[row(t, j)][d], fp32, slot order; row = place[t * top + j] (place == nullptr: t * top + j); ids at or beyond n_experts
+// out[t][d] = sum_j w[t][j] * y[row(t, j)][d], fp32, slot order; row = place[t * top + j] (place == nullptr: t * top + j); negative ids and those at or beyond n_experts
 // have no row.  VEC columns per thread.
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) experts_combine_kernel(const T* __restrict__ y, const int64_t* __restrict__ place, const int64_t* __restrict__ ids, int n_experts,
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(256) experts_combine_kernel(const T* __restric
         for (int e = 0; e < VEC; e++) acc[e] = 0.f;
         for (int j = 0; j < top; j++) {
             const long p = t * top + j;
-            if (ids[p] >= n_experts) continue;
+            if (ids[p] < 0 || ids[p] >= n_experts) continue;      // (its row was never written)
             const float w = wts ? wts[p] : 1.0f;
             const T* row = y + (place ? place[p] : p) * D + d;
             if (VEC == 4) {

@@ -43,3 +43,20 @@ def test_prompt_experts(T, width, ff, E, top, kind):
             want.index_add_(0, t, o * (a @ op.down[e].double().T))
             room.index_add_(0, t, o * (a.abs() @ op.down[e].double().abs().T))
         assert ((got - want).abs() <= 2.0 ** -8 * room + 1e-6).all(), ((got - want).abs() / (room + 1e-6)).max().item()
+
+
+def test_negative_ids_name_no_expert():
+    """as those at or beyond the experts: the same bits"""
+    from ktransformers_b200.operators.experts import KExpertsDense
+    T, width, ff, E, top = 70, 256, 136, 4, 3
+    g = torch.Generator(device="cuda").manual_seed(7)
+    op = KExpertsDense(width, ff, E)
+    for p in (op.gate, op.up, op.down):
+        p.data.copy_(torch.randn(p.shape, generator=g, device="cuda") * 0.1)
+    x, w = torch.randn((T, width), generator=g, device="cuda").to(torch.bfloat16), torch.rand((T, top), generator=g, device="cuda") + 0.5
+    ids = torch.stack([torch.randperm(E, generator=g, device="cuda")[:top] for _ in range(T)])
+    ids[::3, 1] = E + 9
+    ids[5] = E
+    want = op.forward_grouped(x, ids, w)
+    assert (want[5] == 0).all()
+    assert torch.equal(op.forward_grouped(x, torch.where(ids >= E, E - 1 - ids, ids), w), want)      # -1 and -10
