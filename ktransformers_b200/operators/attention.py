@@ -21,6 +21,13 @@ from .base_operator import BaseInjectedModule
 from .flashinfer_wrapper import MLAWrapperSingleton
 
 
+def _is_plain(module, cls) -> bool:
+    """whether calling `module` is calling cls.forward and nothing else: no subclass, no forward of its own, no hooks that want to see the call"""
+    m = torch.nn.modules.module
+    return (type(module) is cls and "forward" not in vars(module) and not module._forward_hooks and not module._forward_pre_hooks
+            and not m._global_forward_hooks and not m._global_forward_pre_hooks)
+
+
 class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
     def __init__(self, key, gguf_loader, config, orig_module, prefill_device: str = "cuda", generate_device: str = "cuda",
                  chunck_size: int = 1000, absorb_for_prefill: bool = False, **kwargs):
@@ -44,14 +51,14 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         module-by-module path below takes.  (The reference's decode branch: archive/ktransformers/operators/attention.py:395-478.)"""
         rot, kv_norm, x = self.rotary_emb, self.kv_a_layernorm, hidden_states
         bf16 = torch.bfloat16
-        if not (x.dtype == bf16 and x.is_cuda and type(rot) is DeepseekV3RotaryEmbedding and type(kv_norm) is DeepseekV3RMSNorm and type(cache) is StaticCache
+        if not (x.dtype == bf16 and x.is_cuda and _is_plain(rot, DeepseekV3RotaryEmbedding) and _is_plain(kv_norm, DeepseekV3RMSNorm) and type(cache) is StaticCache
                 and kv_norm.weight.dtype == bf16 and kv_norm.weight.device == x.device and self.kv_lora_rank == 512 and self.qk_rope_head_dim == 64):
             return None
         for t in (position_ids, cache_position):
             if t is None or t.dtype != torch.int64 or t.device != x.device:
                 return None
         bsz, heads, nope = x.shape[0], self.num_heads, self.qk_nope_head_dim
-        if tuple(position_ids.shape) != (bsz, 1) or cache_position.numel() != 1 or cache.max_batch_size < bsz or rot.inv_freq.dtype != torch.float32 or nope % 2:
+        if tuple(position_ids.shape) != (bsz, 1) or cache_position.numel() != 1 or cache.max_batch_size < bsz or rot.inv_freq.dtype != torch.float32 or rot.inv_freq.numel() != 32 or nope % 2:
             return None
         w = self.mla_wrapper
         if w is None:
@@ -66,7 +73,7 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
             q = self.q_proj(x)
         else:
             qa, norm = self.q_a_proj(x), self.q_a_layernorm
-            if type(norm) is DeepseekV3RMSNorm and norm.weight.dtype == bf16 == qa.dtype and qa.is_contiguous() and self.q_lora_rank % 2 == 0 and self.q_lora_rank <= 8192:
+            if _is_plain(norm, DeepseekV3RMSNorm) and norm.weight.dtype == bf16 == qa.dtype and qa.is_contiguous() and self.q_lora_rank % 2 == 0 and self.q_lora_rank <= 8192:
                 qn = torch.empty_like(qa)
                 native.check(lib.ktb200_add_rmsnorm(qa.data_ptr(), None, norm.weight.data_ptr(), float(norm.variance_epsilon), qn.data_ptr(), bsz, self.q_lora_rank, stream))
             else:

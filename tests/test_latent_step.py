@@ -78,3 +78,25 @@ def test_step_beyond_its_wrapper_is_refused(monkeypatch):
                 monkeypatch.setattr(native, "lib", lambda: Watched())
                 with pytest.raises((RuntimeError, ValueError)):
                     step()
+
+
+def test_hooks_of_the_modules_between_the_projections_still_run():
+    from ktransformers_b200.models.custom_cache import StaticCache
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3Config, DeepseekV3RotaryEmbedding
+    from ktransformers_b200.operators.attention import KDeepseekV2Attention
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapper
+    cfg = DeepseekV3Config(hidden_size=512, num_attention_heads=16, q_lora_rank=64, num_hidden_layers=1)
+    plain = DeepseekV3Attention(cfg, layer_idx=0).to(device="cuda", dtype=torch.bfloat16)
+    plain.rotary_emb = DeepseekV3RotaryEmbedding(64).to("cuda")
+    op = KDeepseekV2Attention("blk.0.self_attn", None, cfg, plain, "cuda", "cuda")
+    cache = StaticCache(cfg, max_batch_size=1, max_cache_len=64, device="cuda")
+    op.mla_wrapper = MLAWrapper(1, cache.max_pages)
+    for name in ("rotary_emb", "kv_a_layernorm", "q_a_layernorm"):
+        for register in ("register_forward_hook", "register_forward_pre_hook"):
+            seen = []
+            handle = getattr(getattr(plain, name), register)(lambda *a: seen.append(name))
+            with torch.no_grad():
+                op(torch.randn(1, 1, 512, device="cuda").to(torch.bfloat16), position_ids=torch.zeros((1, 1), dtype=torch.int64, device="cuda"), past_key_value=cache,
+                   cache_position=torch.zeros(1, dtype=torch.int64, device="cuda"))
+            handle.remove()
+            assert seen == [name], (name, register)
