@@ -43,6 +43,7 @@ void count_launch(int n = 1);
 int num_sms(int device);
 // stream-ordered scratch from a bounded pool (runtime.cu); ScratchBlock gives it back behind the work already queued on the stream
 cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out);
+void scratch_prepare(int device);      // when a handle is created: its calls may then be captured from the first on
 struct ScratchBlock {
     void* ptr = nullptr;
     cudaStream_t stream;

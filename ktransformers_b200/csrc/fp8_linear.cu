@@ -518,6 +518,7 @@ int ktb200_fp8_linear_create(int in_features, int out_features, const void* weig
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) { set_error("fp8_linear: cuTensorMapEncodeTiled failed (%d)", (int)cr); delete l; return KTB200_ECUDA; }
     l->ws = nullptr; l->tickets = nullptr; l->xq = nullptr; l->xs = nullptr;
+    scratch_prepare(device);
     cudaError_t e = cudaMalloc(&l->ws, (size_t)kFT * out_features * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(l->ws, 0, (size_t)kFT * out_features * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&l->tickets, (size_t)l->row_tiles * sizeof(unsigned));

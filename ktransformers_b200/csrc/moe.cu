@@ -516,6 +516,7 @@ int ktb200_moe_create(const ktb200_moe_config* c, int device, ktb200_moe** out) 
     const size_t slots = (size_t)c->group_max_len * c->routed_expert_num;
     const size_t hid = (size_t)c->group_max_len * c->hidden_size * type_size(c->hidden_type);
     // +1 slot per token: the optionally fused shared expert (ktb200_moe_forward_shared)
+    scratch_prepare(device);
     cudaError_t e = cudaMalloc(&m->inter, (slots + c->group_max_len) * c->intermediate_size * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&m->ids_d, slots * sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMalloc(&m->w_d, slots * sizeof(float));
@@ -736,6 +737,7 @@ int ktb200_linear_create(int in_size, int out_size, const void* proj, int proj_t
     if (!l) return KTB200_ENOMEM;
     l->in_size = in_size; l->out_size = out_size; l->proj = proj; l->proj_type = proj_type; l->hidden_type = hidden_type;
     l->group_max_len = group_max_len; l->device = device; l->loaded = false; l->soa = false;
+    scratch_prepare(device);
     *out = l;
     return KTB200_OK;
 }
@@ -793,6 +795,7 @@ int ktb200_mlp_create(int H, int I, const void* gate, const void* up, const void
         delete m;
         return KTB200_ENOMEM;
     }
+    scratch_prepare(device);
     *out = m;
     return KTB200_OK;
 }

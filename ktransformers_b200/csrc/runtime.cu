@@ -39,27 +39,42 @@ int num_sms(int device) {
 // Scratch of one call, taken and given back in stream order from a pool of this library's own (one per device): safe for any number of
 // threads and streams, and under stream capture (the graph then owns the memory).  The pool keeps at most kScratchKeep bytes between
 // calls, so that a prompt's layers do not pay for mapping memory each; what exceeds it goes back to the driver at the next synchronisation.
+// A stream capture allows neither call that makes a pool (outside relaxed capture mode), so the handles whose calls take scratch have it made when they are.
 constexpr unsigned long long kScratchKeep = 1ull << 30;
-cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out) {
+static cudaError_t scratch_pool(int device, cudaMemPool_t* out) {
     static std::mutex mu;
     static cudaMemPool_t pools[64] = {};
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!pools[device]) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = device;
-            const cudaError_t e = cudaMemPoolCreate(&pools[device], &props);
-            if (e != cudaSuccess) { pools[device] = nullptr; return e; }
-            unsigned long long keep = kScratchKeep;
-            cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep);
-        }
-        pool = pools[device];
+    std::lock_guard<std::mutex> lock(mu);
+    if (!pools[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaMemPoolCreate(&pools[device], &props);
+        unsigned long long keep = kScratchKeep;
+        if (e == cudaSuccess) cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) { pools[device] = nullptr; return e; }
     }
-    return cudaMallocFromPoolAsync(out, bytes, pool, stream);
+    *out = pools[device];
+    return cudaSuccess;
+}
+void scratch_prepare(int device) {
+    cudaMemPool_t pool;
+    if (scratch_pool(device, &pool) != cudaSuccess) cudaGetLastError();      // (tried again, and reported, by the first call that needs it)
+}
+cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out) {
+    cudaMemPool_t pool;
+    cudaError_t e = scratch_pool(device, &pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(out, bytes, pool, stream);
+    if (e != cudaSuccess) {      // the caller reports it: it must not turn up again at somebody's next launch
+        *out = nullptr;
+        cudaGetLastError();
+    }
+    return e;
 }
 
 }  // namespace ktb
