@@ -10,7 +10,7 @@
 //     grid = (ceil(N / 128) row tiles, K splits), two CTAs per SM; 192 threads: warp 0 TMA producer (4-stage ring), warp 1 issuer,
 //     warps 2-5 quantise x for the CTA's K range while the first weight boxes are in flight, then run the epilogue.
 // K splits add their fp32 partial sums with atomics into a zeroed workspace; the last CTA of a row tile converts and re-zeroes.
-// Batches of more than kFT tokens take fp8_gemm_kernel below: tokens on the MMA's rows, so that the weights are read once per 128 of them.
+// Most batches of more than kFT tokens take fp8_gemm_kernel below: tokens on the MMA's rows, so that the weights are read once per 128 of them.
 #include <cuda.h>
 #include <cuda_fp8.h>
 
@@ -434,6 +434,15 @@ struct ktb200_fp8_linear {
 };
 
 namespace ktb {
+// Whether a batch of more than kFT tokens is still faster in passes of kFT.  The GEMM has no K splits, so a matrix of few rows is one serial chain of
+// K / 128 steps a tile: measured 10 us + 0.48 us a step and round of tiles (7168 -> 576: 35-39 us, 16384 -> 64: 76, 18432 -> 1536: 75); a pass takes 17.5 us
+// + 1 us per 2.9 MB of weights, a last one of a few tokens less (7168 -> 576: 28 us at 17 tokens, 36 at 24, 40 at 32, 58 at 48).
+static bool fp8_passes_win(const ktb200_fp8_linear* l, int T, int sms) {
+    if (T > 64) return false;
+    const int rest = T % kFT, rounds = ((l->N + 63) / 64 + sms - 1) / sms;      // (few tiles: 64 weight rows each)
+    const float pass = 17.5f + (float)l->N * l->K / 2.9e6f, last = rest == 0 ? 0.f : rest <= 2 ? -10.f : rest <= 8 ? -4.f : 0.f;
+    return (T + kFT - 1) / kFT * pass + last < 10.f + 0.48f * l->nkb * rounds;
+}
 // one box of `rows` x 128 bytes of a row-major byte matrix [n][K]
 static int fp8_map(CUtensorMap* map, const void* ptr, int K, int n, int rows) {
     const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)n};
@@ -543,7 +552,7 @@ int ktb200_fp8_linear_forward(ktb200_fp8_linear* l, int qlen, const void* x, voi
     if (!l || !x || !y) { set_error("fp8_linear: null pointer"); return KTB200_EINVAL; }
     if (qlen <= 0) return KTB200_OK;
     DeviceGuard g(l->device);
-    if (qlen > kFT) return fp8_forward_gemm(l, qlen, x, y, bsz, (cudaStream_t)stream);
+    if (qlen > kFT && !fp8_passes_win(l, qlen, num_sms(l->device))) return fp8_forward_gemm(l, qlen, x, y, bsz, (cudaStream_t)stream);
     const size_t hb = type_size(l->hidden_type);
     for (int t0 = 0; t0 < qlen; t0 += kFT) {
         Fp8Params p{};

@@ -155,3 +155,37 @@ def test_mlp_of_a_prompt(gate, up, down, H, I, T, hid):
         units = 2.0 ** -7 * (ref.double().abs() + want.double().abs())[:T - 5] if hid == BF16 else 0
         assert (diff <= units + 1e-3 * size).all(), (diff / size).max().item()
     lib.ktb200_mlp_destroy(h)
+
+
+# matrices so small that the launches of the GEMM cost more than the row kernels (the FP8 passes) take: (path, K, R or N, rows, launches)
+@pytest.mark.parametrize("kind,K,R,T,launches", [("fp8", 7168, 576, 24, 4), ("fp8", 7168, 576, 25, 2), ("fp8", 16384, 72, 48, 6), ("fp8", 512, 512, 17, 2)])
+def test_small_matrices_keep_the_kernels_of_few_rows(kind, K, R, T, launches):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, K), generator=g, device="cuda").to(torch.bfloat16)
+    lib, h = native.lib(), C.c_void_p()
+    out = K if kind == "mlp" else R
+    if kind == "fp8":
+        w, ws = (torch.randn((R, K), generator=g, device="cuda") * 50).to(torch.float8_e4m3fn), torch.rand(((R + 127) // 128, K // 128), generator=g, device="cuda")
+        native.check(lib.ktb200_fp8_linear_create(K, R, w.data_ptr(), ws.data_ptr(), BF16, 0, C.byref(h)))
+        run = lambda x, y: lib.ktb200_fp8_linear_forward(h, x.shape[0], x.data_ptr(), y.data_ptr(), None, _stream())
+    elif kind == "mlp":
+        keep = [synth_blocks(t, R * K, "cuda", i) for i, t in enumerate((Q4_K, Q4_K, Q6_K))]
+        native.check(lib.ktb200_mlp_create(K, R, *[t.data_ptr() for t in keep], Q4_K, Q4_K, Q6_K, BF16, T, 0, C.byref(h)))
+        native.check(lib.ktb200_mlp_load_weights(h, _stream()))
+        run = lambda x, y: lib.ktb200_mlp_forward(h, x.shape[0], x.data_ptr(), y.data_ptr(), 0, None, _stream())
+    else:
+        q = Q6_K if kind == "q6" else Q4_K
+        keep = synth_blocks(q, R * K, "cuda", 1)
+        native.check(lib.ktb200_linear_create(K, R, keep.data_ptr(), q, BF16, T, 0, C.byref(h)))
+        native.check(lib.ktb200_linear_load_weights(h, _stream()))
+        run = lambda x, y: lib.ktb200_linear_forward(h, x.shape[0], x.data_ptr(), y.data_ptr(), None, None, _stream())
+    y, few = (torch.zeros((T, out), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    n0 = native.launch_count()
+    native.check(run(x, y))
+    assert native.launch_count() - n0 == launches
+    for t in range(0, T, 8):
+        native.check(run(x[t:t + 8], few[t:t + 8]))
+    # the same sums in another order: a value at the edge of two bf16 steps falls to the other; an activation of the MLP at the edge of two int8 steps moves a row by 1e-3
+    size = few.double().abs().max()
+    assert ((y.double() - few.double()).abs() <= 2.0 ** -7 * few.double().abs() + (1e-3 if kind == "mlp" else 4e-6) * size).all()
+    (lib.ktb200_fp8_linear_destroy if kind == "fp8" else lib.ktb200_mlp_destroy if kind == "mlp" else lib.ktb200_linear_destroy)(h)
