@@ -723,9 +723,16 @@ struct ktb200_linear {
     bool loaded, soa;
 };
 
-// rows from which a linear runs as a tensor-core GEMM (kq_gemm.cu): the row kernels keep up to 8 rows of activations on the SM and read the weights
-// once for them; beyond, once more for every row
-constexpr int kLinearGemmMin = 9;
+// Whether a linear of T rows runs as a tensor-core GEMM (kq_gemm.cu).  The row kernels keep up to 8 rows of activations on the SM and read the weights once for
+// them; beyond, once more for every row.  The GEMM's two or three launches take 19-25 us however small the matrix is, and small ones are done by then: the row kernels
+// take about 8 us and, per row, R (500 + 0.35 K) 1e-6 us (512 -> 512: 14 us at 16 rows, 18 at 32, 30 at 64 against 21-25), of Q6_K 1.7 times that;
+// the bulk-copy form (Q4_K from 16 blocks on) at least 1.3 us a row (4096 -> 64: 22 us at 12 rows, 27 at 16 against 23).
+static bool linear_as_gemm(FmtId f, int R, int K, int T) {
+    if (T <= 8 || kq_fmt(f) == KQ_NONE) return false;
+    if (f == FMT_Q4K && K >= 16 * QK_K && T > 11) return true;
+    const double rows = (double)T * R * (500.0 + 0.35 * K) * (kq_is_q6(kq_fmt(f)) ? 1.7 : 1.0);
+    return rows > 12.5e6 + 3e3 * (K < 1024 ? K : 1024);
+}
 
 int ktb200_linear_create(int in_size, int out_size, const void* proj, int proj_type, int hidden_type, int group_max_len,
                          int device, ktb200_linear** out) {
@@ -764,7 +771,7 @@ int ktb200_linear_forward(ktb200_linear* l, int qlen, const void* input, void* o
     if (!input || !output) { set_error("forward: null pointer"); return KTB200_EINVAL; }
     DeviceGuard g(l->device);
     const FmtId fmt = pick_fmt(l->proj_type, l->soa);
-    if (qlen >= kLinearGemmMin) {
+    if (linear_as_gemm(fmt, l->out_size, l->in_size, qlen)) {
         const int rc = kq_linear(fmt, l->proj, l->out_size, l->in_size, input, l->hidden_type, qlen, output, bias, bsz, l->device, (cudaStream_t)stream);
         if (rc != 1) return rc;
     }
@@ -830,9 +837,15 @@ int ktb200_mlp_load_weights(ktb200_mlp* m, void* stream) {
     m->loaded = true;
     return KTB200_OK;
 }
-// rows from which an MLP runs as tensor-core GEMMs (kq_mlp), the row kernels' 8 rows plus one as for the linears: 7168 x 2048, Q4_K and Q6_K, 9 rows 72 us
-// against 87, 1024 rows 287 us against 7.9 ms; 7168 x 18432, 9 rows 129 us against 519, 1024 rows 1.8 ms against 42
-constexpr int kMlpGemmMin = 9;
+// Rows from which an MLP runs as tensor-core GEMMs (kq_mlp).  Its six launches take 45-65 us however small the matrices are; the row kernels' time grows
+// with the rows: 7168 x 2048, Q4_K and Q6_K, 9 rows 72 us against 87, 1024 rows 287 us against 7.9 ms, but 1024 x 1024 60 us against 54 at 16 rows and 69 at 20, 512 x 512 60
+// against 50 and 60, 1024 x 256 57 against 34 and 40.  The lines lie where the two met, by H * I in units of 256 x 256, times 1.6 for Q6_K gates and 0.5 for Q5_K.
+// Small ones differ by the down kernel: the bulk-copy form (Q4_K; Q6_K from 512 columns on) takes about 2 us a row however short the rows are, the others 0.3-1.
+static int mlp_gemm_min(const ktb200_mlp* m) {
+    const double n = (double)m->H * m->I / 65536 * (m->gate_type == KTB200_TYPE_Q6_K ? 1.6 : m->gate_type == KTB200_TYPE_Q5_K ? 0.5 : 1.0);
+    const bool bulk = m->down_type == KTB200_TYPE_Q4_K || (m->down_type == KTB200_TYPE_Q6_K && m->I >= 512);
+    return n > 40 ? 9 : n > 20 ? 11 : n > 10 ? 16 : bulk ? 18 : n > 5 ? 20 : 40;
+}
 
 int ktb200_mlp_forward(ktb200_mlp* m, int qlen, const void* input, void* output, int accumulate, const int* bsz, void* stream) {
     if (!m) { set_error("null handle"); return KTB200_EINVAL; }
@@ -841,7 +854,7 @@ int ktb200_mlp_forward(ktb200_mlp* m, int qlen, const void* input, void* output,
     if (qlen > m->group_max_len) { set_error("forward: qlen=%d exceeds group_max_len=%d", qlen, m->group_max_len); return KTB200_EINVAL; }
     DeviceGuard g(m->device);
     cudaStream_t s = (cudaStream_t)stream;
-    if (qlen >= kMlpGemmMin && input && output) {
+    if (qlen >= mlp_gemm_min(m) && input && output) {
         const int rc = kq_mlp(m, input, qlen, output, accumulate, bsz, s);
         if (rc != 1) return rc;
     }

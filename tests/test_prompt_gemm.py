@@ -158,7 +158,9 @@ def test_mlp_of_a_prompt(gate, up, down, H, I, T, hid):
 
 
 # matrices so small that the launches of the GEMM cost more than the row kernels (the FP8 passes) take: (path, K, R or N, rows, launches)
-@pytest.mark.parametrize("kind,K,R,T,launches", [("fp8", 7168, 576, 24, 4), ("fp8", 7168, 576, 25, 2), ("fp8", 16384, 72, 48, 6), ("fp8", 512, 512, 17, 2)])
+@pytest.mark.parametrize("kind,K,R,T,launches", [("linear", 512, 512, 32, 1), ("linear", 512, 512, 41, 2), ("linear", 4096, 64, 11, 1), ("linear", 4096, 64, 12, 3), ("q6", 512, 512, 20, 1),
+                                                 ("q6", 512, 512, 24, 2), ("fp8", 7168, 576, 24, 4), ("fp8", 7168, 576, 25, 2), ("fp8", 16384, 72, 48, 6), ("fp8", 512, 512, 17, 2),
+                                                 ("mlp", 512, 512, 17, 2), ("mlp", 512, 512, 18, 6), ("mlp", 512, 256, 39, 2), ("mlp", 512, 256, 40, 6)])
 def test_small_matrices_keep_the_kernels_of_few_rows(kind, K, R, T, launches):
     g = torch.Generator(device="cuda").manual_seed(T)
     x = torch.randn((T, K), generator=g, device="cuda").to(torch.bfloat16)
