@@ -575,6 +575,8 @@ int ktb200_softmax_attn(const ktb200_softmax_attn_params* params, int n_tokens, 
 size_t ktb200_softmax_attn_workspace(int n_tokens, int heads, int maps, int vdim, int splits, int tensor_cores);
 int ktb200_softmax_attn_uses_tensor_cores(int heads, int kv_heads, int maps, int dim, int vdim, int dtype);
 int ktb200_softmax_attn_tiles(int heads, int kv_heads, int maps, int n_tokens, int n_seqs);
+/* whether a tensor-core call runs the 256-row tiles on tcgen05 (csrc/softmax_attn_tc.cuh) */
+int ktb200_softmax_attn_prompt_tiles(const ktb200_softmax_attn_params* params, int n_tokens, int splits);
 
 /* Mamba-2 (csrc/ssd.cu): proj rows hold [x heads*vdim | B groups*state_size | C groups*state_size] at xbc_off and one step logit per head at
  * dt_off; conv_w [channels][taps] (last column = current token), conv_b [channels]; state rows [S heads*state_size*vdim | filter inputs

@@ -956,6 +956,16 @@ extern "C" int ktb200_window_softmax_attn_uses_tensor_cores(int heads, int kv_he
 }
 extern "C" int ktb200_window_softmax_attn_tiles(int heads, int kv_heads, int n_tokens, int n_seqs) { return ktb200_softmax_attn_tiles(heads, kv_heads, 1, n_tokens, n_seqs); }
 
+/* Whether a tensor-core call runs 256-row tiles on tcgen05 (their TMA reads whole runs of 64 keys of a page): portions of half a row tile's tokens on average, and
+ * enough CTAs.  In a step that mixes a prompt with decoded tokens a short portion leaves most of its tile empty, and the step still gains: 64 heads over 8, 1900
+ * tokens beside 16 (100) single ones at 1124 keys 472 -> 132 us (593 -> 308) against the 64-row tiles, at 8292 keys 1024 -> 267 (1715 -> 1196). */
+extern "C" int ktb200_softmax_attn_prompt_tiles(const ktb200_softmax_attn_params* c, int n_tokens, int splits) {
+    const int RH = mma_heads_per_tile(c->heads / c->kv_heads);
+    if (c->maps != 1 || splits != 1 || c->dim != 128 || c->vdim != 128 || 128 % RH || c->page_size % 64 || ((reinterpret_cast<uintptr_t>(c->q) | reinterpret_cast<uintptr_t>(c->cache)) & 15)) return 0;
+    const int tiles = softmax_tc_tiles(RH, n_tokens, c->n_seqs);
+    return n_tokens >= c->n_seqs * (64 / RH) && tiles * (c->heads / RH) >= kTcMinCtas && tiles <= 65535;
+}
+
 extern "C" int ktb200_softmax_attn(const ktb200_softmax_attn_params* c, int n_tokens, int splits, float* workspace, int dtype, int allow_tensor_cores, void* stream) {
     if (!c || !c->q || !c->pos || !c->slot || !c->page_table || !c->cache || !c->out || c->heads <= 0 || c->kv_heads <= 0 || c->heads % c->kv_heads || c->maps < 1 || c->maps > 2 ||
         c->dim <= 0 || c->vdim <= 0 || c->vdim > 32 * kSmMaxCols || (c->maps == 2 && !c->lambda) || (c->dist_r1 && !c->dist_r2) || splits < 1 || c->page_size <= 0 || c->max_pages <= 0 ||
@@ -978,11 +988,7 @@ extern "C" int ktb200_softmax_attn(const ktb200_softmax_attn_params* c, int n_to
     if (tc) {
         using B = __nv_bfloat16;
         const int RH = a.RH = mma_heads_per_tile(heads / kv_heads), row_tile = kMmaRows / maps;
-        // prompt portions: 256 rows per CTA on tcgen05 (its TMA reads whole runs of 64 keys of a page)
-        if (maps == 1 && splits == 1 && dim == 128 && vdim == 128 && 128 % RH == 0 && c->page_size % 64 == 0 && n_tokens >= c->n_seqs * (64 / RH) &&
-            softmax_tc_tiles(RH, n_tokens, c->n_seqs) * (heads / RH) >= kTcMinCtas &&
-            ((reinterpret_cast<uintptr_t>(c->q) | reinterpret_cast<uintptr_t>(c->cache)) & 15) == 0)
-            return launch_softmax_tc(a, n_tokens, (cudaStream_t)stream);
+        if (ktb200_softmax_attn_prompt_tiles(c, n_tokens, splits)) return launch_softmax_tc(a, n_tokens, (cudaStream_t)stream);
         const dim3 grid(ktb200_softmax_attn_tiles(heads, kv_heads, maps, n_tokens, c->n_seqs), kv_heads * (heads / kv_heads / RH), splits);
         const size_t smem = (((size_t)row_tile + 2 * kMmaKeys) * (maps * dim + kMmaPad) + (size_t)2 * kMmaKeys * (vdim + kMmaPad)) * sizeof(B);
 #define MMA_LAUNCH(DK, DV, MAPS, BIAS)                                                                                             \

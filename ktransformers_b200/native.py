@@ -195,6 +195,7 @@ SEQ_SYMBOLS = {
     "ktb200_softmax_attn_workspace": (C.c_size_t, [_I, _I, _I, _I, _I, _I]),
     "ktb200_softmax_attn_uses_tensor_cores": (_I, [_I, _I, _I, _I, _I, _I]),
     "ktb200_softmax_attn_tiles": (_I, [_I, _I, _I, _I, _I]),
+    "ktb200_softmax_attn_prompt_tiles": (_I, [C.POINTER(SoftmaxAttnParams), _I, _I]),
     # csrc/retention.cu, csrc/selective_scan.cu
     "ktb200_turn_table": (_I, [_VP, _VP, _I, _VP, _I, _VP]),
     "ktb200_retention_chunk_supported": (_I, [_I, _I, _I]),

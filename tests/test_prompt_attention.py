@@ -77,3 +77,31 @@ def test_prompt_portions(heads, kv_heads, portions, opts):
             want = want * torch.sigmoid(gate[mine].double())
         err = (o[mine].double() - want).abs()
         assert (err <= 2.0 ** -8 * want.abs() + 6 * 2.0 ** -9 * reach.reshape(want.shape) + 1e-6).all(), err.max().item()
+
+
+
+# steps that mix portions of every length run the 256-row tiles as a whole (a portion of one token among them); few short portions, and keys cut into parts, do not
+@pytest.mark.parametrize("heads,kv_heads,portions,opts,tiles", [
+    (64, 8, [(0, 128)], {}, 1),
+    (64, 8, [(5, 300), (1000, 1), (70, 15), (200, 16)], {"sink": 1, "gate": 1}, 1),
+    (64, 8, [(3, 10), (100, 12), (0, 15), (64, 9)], {}, 1),
+    (32, 8, [(77, 1), (129, 513), (900, 33), (64, 31)], {"window": 100}, 1),
+    (16, 16, [(200, 600), (5, 127), (9, 128)], {"chunk": 192, "head_scale": 1}, 1),
+    (64, 4, [(100, 8), (511, 7), (64, 333), (0, 1)], {"softcap": 20.0, "bias": 1, "out_scale": 0.5}, 1),
+    (16, 8, [(0, 100)], {}, 0),
+    (64, 8, [(900, 1)] * 4, {}, 0),
+    (64, 8, [(900, 7)], {}, 0),
+])
+def test_steps_of_mixed_portions(monkeypatch, heads, kv_heads, portions, opts, tiles):
+    from ktransformers_b200 import native
+    real, seen = native.seq_lib(), []
+
+    class Watched:
+        def __getattr__(self, name):
+            if name != "ktb200_softmax_attn":
+                return getattr(real, name)
+            return lambda a, T, splits, *rest: seen.append(real.ktb200_softmax_attn_prompt_tiles(a, T, splits)) or real.ktb200_softmax_attn(a, T, splits, *rest)
+
+    monkeypatch.setattr(native, "seq_lib", lambda **kw: Watched())
+    test_prompt_portions(heads, kv_heads, portions, opts)
+    assert seen == [tiles]
