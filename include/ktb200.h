@@ -319,8 +319,6 @@ size_t ktb200_mla_workspace_bytes(int batch, int num_heads, int max_splits);
 int ktb200_mla_decode(const ktb200_mla_params* p, void* stream);
 /* Diagnostics: while non-NULL, one CTA of ktb200_mla_decode dumps the raw scores of its first tile (>= 2048 floats). */
 void ktb200_debug_mla(float* debug_dev);
-/* Debug aid of an earlier grouped (prefill) expert GEMM; nothing is written any more. */
-void ktb200_debug_grouped(long long* trace_dev);
 
 /* ------------------------------------------------------------------------------------------
  * The memory-bound steps between the projections of a DeepSeek decode layer (bf16), fused:

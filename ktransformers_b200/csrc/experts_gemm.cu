@@ -253,19 +253,8 @@ __global__ void __launch_bounds__(kEgThreads, 1) eg_gemm_kernel(const __grid_con
     }
 }
 
-typedef CUresult (*EncodeTiledFnEg)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                    CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFnEg encode_tiled_eg() {
-    static EncodeTiledFnEg fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-        return (EncodeTiledFnEg)f;
-    }();
-    return fn;
-}
 static int eg_map(CUtensorMap* map, const void* ptr, long cols, long rows, int box_rows) {      // boxes of so many rows x 64 bf16
-    EncodeTiledFnEg enc = encode_tiled_eg();
+    EncodeTiledFn enc = encode_tiled();
     if (!enc) { set_error("experts_prompt: cuTensorMapEncodeTiled is not available from this driver"); return KTB200_ECUDA; }
     const cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, stride[1] = {(cuuint64_t)cols * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, estr[2] = {1, 1};

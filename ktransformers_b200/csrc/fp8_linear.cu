@@ -409,17 +409,6 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
     }
 }
 
-typedef CUresult (*EncodeTiledFn8)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn8 encode_tiled8() {
-    static EncodeTiledFn8 fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-        return (EncodeTiledFn8)f;
-    }();
-    return fn;
-}
 }  // namespace ktb
 
 struct ktb200_fp8_linear {
@@ -448,7 +437,7 @@ static int fp8_map(CUtensorMap* map, const void* ptr, int K, int n, int rows) {
     const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)n};
     const cuuint64_t gstr[1] = {(cuuint64_t)K};
     const cuuint32_t box[2] = {128, (cuuint32_t)rows}, estr[2] = {1, 1};
-    const CUresult cr = encode_tiled8()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult cr = encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) { set_error("fp8_linear: cuTensorMapEncodeTiled failed (%d)", (int)cr); return KTB200_ECUDA; }
     return KTB200_OK;
@@ -506,7 +495,7 @@ int ktb200_fp8_linear_create(int in_features, int out_features, const void* weig
     if ((uintptr_t)weight_e4m3 & 15) { set_error("fp8_linear: weight must be 16-byte aligned"); return KTB200_EINVAL; }
     DeviceGuard g(device);
     if (!g.ok) { set_error("cudaSetDevice(%d) failed", device); return KTB200_ECUDA; }
-    EncodeTiledFn8 enc = encode_tiled8();
+    EncodeTiledFn enc = encode_tiled();
     if (!enc) { set_error("fp8_linear: cuTensorMapEncodeTiled is not available from this driver"); return KTB200_ECUDA; }
     ktb200_fp8_linear* l = new (std::nothrow) ktb200_fp8_linear();
     if (!l) return KTB200_ENOMEM;

@@ -84,9 +84,6 @@ template <int N>
 __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
 __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3, int c4) {
     asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(c1),
                  "r"(c2), "r"(c3), "r"(c4)
@@ -142,28 +139,6 @@ __device__ __forceinline__ __half2 magic_and(uint32_t a) {
     uint32_t d;
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(MASK), "r"(kMagic));
     return as_h2(d);
-}
-// packed fp32: two products or fused multiply-adds per instruction, each rounded as the scalar one
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ f32x2 pack2(uint32_t lo, uint32_t hi) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
-    return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
 }
 __device__ __forceinline__ float half_of(f32x2 v, int hi) { return __uint_as_float((uint32_t)(hi ? v >> 32 : v)); }
 __device__ __forceinline__ __half2 h2_of(int small) { return __hsub2(as_h2(kMagic | (uint32_t)small * 0x10001u), as_h2(kMagic)); }      // 0 <= small < 1024
@@ -628,20 +603,9 @@ int kq_act_quant(const float* g, const float* u, const int* pos, int n, int K, i
 }
 
 // ---------------------------------------------------------------------------------------------------------------- launch
-typedef CUresult (*EncodeTiledFnKq)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                    CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFnKq encode_tiled_kq() {
-    static EncodeTiledFnKq fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-        return (EncodeTiledFnKq)f;
-    }();
-    return fn;
-}
 // a tensor map of `rank` dimensions (innermost first) with the given byte strides of dimensions 1 .. rank - 1
 static int kq_map(CUtensorMap* map, CUtensorMapDataType type, const void* ptr, int rank, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box, CUtensorMapSwizzle sw) {
-    EncodeTiledFnKq enc = encode_tiled_kq();
+    EncodeTiledFn enc = encode_tiled();
     if (!enc) { set_error("kq_gemm: cuTensorMapEncodeTiled is not available from this driver"); return KTB200_ECUDA; }
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUresult cr = enc(map, type, rank, const_cast<void*>(ptr), dim, stride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -495,20 +495,6 @@ static int pick_splits(int batch, int num_heads, int max_kv_tiles, int device) {
     return s;
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (libktb200.so links libcudart only)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-        return (EncodeTiledFn)f;
-    }();
-    return fn;
-}
-
 static float* g_mla_debug = nullptr;
 
 }  // namespace ktb

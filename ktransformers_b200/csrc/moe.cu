@@ -578,8 +578,6 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
 }
 // qlen from which the per-expert tensor-core GEMMs (grouped.cu) replace the per-pair GEMV kernels: the reference makes the
 // same split between MOE::forward_one and MOE::forward_many (moe.cpp:367-377, threshold group_min_len)
-// (kept for callers that look it up: the kernel whose stamps it asked for is gone)
-void ktb200_debug_grouped(long long*) {}
 static int grouped_min_qlen() {
     static const int v = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : 48; }();
     return v;

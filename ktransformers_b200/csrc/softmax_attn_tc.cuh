@@ -36,26 +36,6 @@ __device__ __forceinline__ float tc_ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ unsigned long long tc_pack(float a, float b) {
-    unsigned long long d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-    return d;
-}
-__device__ __forceinline__ void tc_unpack(unsigned long long v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ unsigned long long tc_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long tc_add2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ void tc_load_3d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(m), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-
 __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kvmap, const SmAttn a) {
     using namespace umma;
     extern __shared__ __align__(16) uint8_t tc_smem[];
@@ -106,7 +86,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
 #pragma unroll
             for (int t = 0; t < 2; t++)
 #pragma unroll
-                for (int c = 0; c < 2; c++) tc_load_3d(base + t * kTcTile + c * (kTcTile / 2), &qmap, qf, 64 * c, h0, tok0 + t * TOKS);
+                for (int c = 0; c < 2; c++) tma_load_3d(base + t * kTcTile + c * (kTcTile / 2), &qmap, qf, 64 * c, h0, tok0 + t * TOKS);
             const int* pt = a.page_table + (long)a.slot[tok0] * a.max_pages;
             for (int j = 0; j < n; j++) {
                 const int st = j & 1, ph = ((j >> 1) & 1) ^ 1;
@@ -249,20 +229,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
                 }
             }
             const float u = m_ref == -INFINITY ? 0.f : m_ref;
-            const unsigned long long c2 = tc_pack(c, c), nu2 = tc_pack(-u, -u);
-            unsigned long long sum[2] = {0, 0};
+            const f32x2 c2 = pack2(c, c), nu2 = pack2(-u, -u);
+            f32x2 sum[2] = {0, 0};
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 uint32_t pk[32];
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
                     float e0, e1;
-                    tc_unpack(tc_fma2(tc_pack(s[64 * q + 2 * i], s[64 * q + 2 * i + 1]), c2, nu2), e0, e1);
+                    unpack2(fma2(pack2(s[64 * q + 2 * i], s[64 * q + 2 * i + 1]), c2, nu2), e0, e1);
                     e0 = tc_ex2(e0);
                     e1 = tc_ex2(e1);
                     pk[i] = pack_bf16(e0, e1);
                     // the sum is of the weights as they are used: what rounding takes from a weight it takes from its share of the sum too
-                    sum[i & 1] = tc_add2(sum[i & 1], tc_pack(__uint_as_float(pk[i] << 16), __uint_as_float(pk[i] & 0xffff0000u)));
+                    sum[i & 1] = add2(sum[i & 1], pack2(__uint_as_float(pk[i] << 16), __uint_as_float(pk[i] & 0xffff0000u)));
                 }
                 tmem_st32(ts + 32 * q, pk);
             }
@@ -271,8 +251,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
             __syncwarp();
             if (lane == 0) bar_arrive(smem_u32(&misc.p_full[t]));
             float a0, a1, a2, a3;
-            tc_unpack(sum[0], a0, a1);
-            tc_unpack(sum[1], a2, a3);
+            unpack2(sum[0], a0, a1);
+            unpack2(sum[1], a2, a3);
             l += (a0 + a1) + (a2 + a3);
         }
         bar_wait(smem_u32(&misc.o_done[t]), 0);
@@ -320,23 +300,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
     }
 }
 
-typedef CUresult (*EncodeTiledFnTc)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                    CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFnTc encode_tiled_tc() {
-    static EncodeTiledFnTc fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-        return (EncodeTiledFnTc)f;
-    }();
-    return fn;
-}
-
 // CTAs of softmax_attn_tc_kernel per key/value head and head block (an upper bound)
 static int softmax_tc_tiles(int RH, int n_tokens, int n_seqs) { return n_seqs + n_tokens / (2 * (128 / RH)); }
 
 static int launch_softmax_tc(const SmAttn& a, int n_tokens, cudaStream_t s) {
-    EncodeTiledFnTc enc = encode_tiled_tc();
+    umma::EncodeTiledFn enc = umma::encode_tiled();
     if (!enc) { set_error("softmax_attn: cuTensorMapEncodeTiled is not available from this driver"); return KTB200_ECUDA; }
     CUtensorMap qmap, kvmap;
     const cuuint32_t estr[3] = {1, 1, 1};
