@@ -124,14 +124,14 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
         grp_scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids_c, n, k, c.expert_id_offset, E, bsz, t0, cursor, pos);
         grp_tiles_kernel<<<(ub_gu + 255) / 256, 256, 0, s>>>(nt_prefix, offsets, counts, E, I / 128, 128, tinfo_gu);
         grp_tiles_kernel<<<(ub_d + 255) / 256, 256, 0, s>>>(nt_prefix, offsets, counts, E, H / kKqRows, kKqRows, tinfo_d);
-        int rc = kq_quant(x_c, c.hidden_type, T, H, pos, k, kq_is_q6(fg), xa, s);
+        int rc = kq_quant(x_c, c.hidden_type, T, H, pos, k, kq_is_q6(fg), kq_limit(fg), xa, s);
         if (rc) return rc;
         KqGemm gp{};
         gp.fmt = fg; gp.w[0] = c.gate_proj; gp.w[1] = c.up_proj; gp.pair = true; gp.expert_bytes = (long)I * row_bytes(H, c.gate_type); gp.experts = E; gp.R = I; gp.K = H; gp.acts = &xa;
         gp.tinfo = tinfo_gu; gp.n_tiles_dev = nt_prefix + E; gp.tiles_mul = I / 128; gp.splits = 1; gp.out[0] = g; gp.out[1] = u;
         rc = kq_gemm(gp, dev, s);
         if (rc) return rc;
-        rc = kq_act_quant(g, u, pos, n, I, c.use_silu, kq_is_q6(fd), aa, s);
+        rc = kq_act_quant(g, u, pos, n, I, c.use_silu, kq_is_q6(fd), kq_limit(fd), aa, s);
         if (rc) return rc;
         KqGemm gd{};
         gd.fmt = fd; gd.w[0] = gd.w[1] = c.down_proj; gd.expert_bytes = (long)H * row_bytes(I, c.down_type); gd.experts = E; gd.R = H; gd.K = I; gd.acts = &aa;

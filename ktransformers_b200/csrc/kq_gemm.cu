@@ -4,9 +4,15 @@
 //
 // Arithmetic: the reference's dot of a 256-block is an exact integer, sum_j sc_j * sum_i q_ij * x8_ij, scaled in fp32.  Here a weight enters the
 // tensor core as the fp16 integer sc * q (Q4_K: at most 63 * 15; Q5_K: 63 * 31, halved; Q6_K: two terms, sc * (low four bits) and
-// sc * (16 * high two bits - 32), both quartered), an activation as the fp16 integer x8; the products are exact, the fp32 accumulator of a
-// 256-block holds integers (or halves, quarters) that stay below 2^24 short of inputs built for it, and the epilogue applies
+// sc * (16 * high two bits - 32), both quartered), an activation as the fp16 integer x8; the products are exact, and the epilogue applies
 // dx * (d * isum - dmin * msum) once per block in fp32, the decode kernels' formula; msum (minima x 16-value activation sums) is one K = 16 MMA.
+// The fp32 accumulator of a 256-block holds integers (or halves, quarters), exact while they stay within 2^24 of their unit.  A full block can reach 31, 63 and
+// 133 million (Q4_K, Q5_K, Q6_K), and an ordinary Q5_K block under activations of one sign and size 20 million, of which the minima then take most away again.  So a block
+// of activations that might get there (kq_limit in kq_gemm.cuh, marked by the quantiser) is summed stage by stage: each stage's 128 values (Q6_K: 64), at most
+// 16 (Q4_K), 32 (Q5_K) or 33 million, go to columns of their own and the epilogue adds them to the accumulator, which then holds isum rounded once, like an int32 sum.
+// A tile's other rows come out the same bits either way.  Measured against 64 bits (fp32 linears, K = 7168, 2-norm of 64 x 1024): activations 1 + 0.01 n on Q5_K
+// 24.8e-7 with one accumulator, 7.0e-7 like this, 7.6e-7 in the row kernels (int32); all weights and activations at their largest Q4_K 2.5e-7, 0.3e-7, 0.4e-7, Q5_K 4.8e-7,
+// 1.3e-7 (a stage's sum may pass 2^24 by one bit), 0.3e-7, Q6_K 7.7e-7, 0.3e-7, 0.3e-7.
 //
 // What bounds it: an expert's weights are read from HBM once per 64 of its tokens (1024 tokens of 256 experts: about once), so the routed
 // experts are HBM-bound, and the work per weight has to stay under what an SM has per weight byte that arrives (24 B per cycle):
@@ -22,9 +28,12 @@
 //      groups 5 / 6 epilogue of matrix 0 / 1.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
 //      warps took a third of the issue slots, and the four roles' code is kept in rolled loops: unrolled it overran the instruction cache (10,000
 //      cycles for a block of two matrices; now 3,400; HBM brings one every 1,550).  What is left is the chain product -> drain -> product of
-//      a matrix beside producers that issue ~8,000 instructions per block; measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 6556 us with one
-//      int32 accumulator per 32 values and operands through shared memory, 2500 us; Q4_K linear 777 x 1536 -> 24576 172 us (345 TFLOP/s).
+//      a matrix beside producers that issue ~8,000 instructions per block; measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 6.6 ms with one
+//      int32 accumulator per 32 values and operands through shared memory, 2.9 ms (the operator's call); Q4_K linear 777 x 1536 -> 24576 180 us (326 TFLOP/s).
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
+#include <algorithm>
+#include <atomic>
+
 #include <cuda_fp16.h>
 
 #include "act_quant.cuh"
@@ -51,7 +60,7 @@ struct KqCfg {
 };
 struct KqMisc {
     unsigned long long b_full[2], b_free[2], dx_full[4], dx_free[4], raw_full[3], raw_free[3], a_full[2][2], a_free[2][2], acc_full[2], acc_free[2], hdr_free[2][2];
-    uint32_t tmem_base, pad[3];
+    uint32_t tmem_base, marked[2], pad;      // marked: whether the matrix's block is summed stage by stage
     float dx[4][kKqN];
     uint32_t hdr[2][2][128];      // Q4_K, Q5_K: half2 (d, dmin) of a row's block
 };
@@ -65,6 +74,9 @@ struct KqParams {
     long expert_bytes, dpitch;
     int pair, R, nblk, T, rt, nt, splits, total, tiles_mul, hidden_type, t0;
     const float* dx;
+    const uint8_t* marks;
+    const unsigned long long* any;
+    unsigned long long id;
     const int4* tinfo;
     const int* n_tiles;
     float* out[2];
@@ -130,6 +142,18 @@ __device__ __forceinline__ void mma_f16_ta8(uint32_t tmem_d, uint32_t tmem_a, ui
         "r"(tmem_a), "l"(desc_b), "l"(next), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// the elected lane of a converged warp leaves `value` for those who wait for `bar`, and arrives there
+__device__ __forceinline__ void kq_tell(uint32_t at, uint32_t value, uint32_t bar) {
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        ".reg .b32 r;\n"
+        "elect.sync r|q, 0xffffffff;\n"
+        "@q st.shared.b32 [%0], %1;\n"
+        "@q mbarrier.arrive.shared::cta.b64 _, [%2];\n"
+        "}\n" ::"r"(at), "r"(value), "r"(bar)
+        : "memory");
+}
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 constexpr uint32_t kMagic = 0x64006400u;      // fp16 1024, 1024: a small integer or-ed into the mantissa adds itself
@@ -171,6 +195,14 @@ __device__ __forceinline__ KqTile kq_tile(const KqParams& p, int tile) {
     return t;
 }
 
+// four rows a lane of the marks of block sb of rows p0 .. p0 + n: not 0 in some lane where the block has to be summed stage by stage
+__device__ __forceinline__ uint32_t kq_mark(const KqParams& p, int sb, int p0, int n, int lane) {
+    const int left = n - 4 * lane;
+    if (left <= 0) return 0;
+    const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p.marks + (long)sb * p.dpitch + p0) + lane);
+    return left < 4 ? w & ((1u << (8 * left)) - 1) : w;
+}
+
 // 16 columns (32 weights of a row) of an operand stage from 4 words of quants; sl / sh: scales of the low / high nibbles' values
 __device__ __forceinline__ void kq_unpack4(const uint32_t* w, __half2 sl, __half2 sh, uint32_t (&o)[16]) {
     const __half2 cl = __hmul2(sl, __float2half2_rn(-1024.f)), s16 = __hmul2(sh, __float2half2_rn(1.f / 16.f)), ch = __hmul2(sh, __float2half2_rn(-64.f));
@@ -209,34 +241,12 @@ __device__ __forceinline__ int kq_q6_word(int r, int c) {
 }
 struct KqMaps { CUtensorMap q, sums, w[2][3]; };      // activations, their sums; weights of matrix 0 / 1 (Q6_K in 8-row groups: ql, qh, scales)
 
-template <int FMT>
-__global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_constant__ KqMaps maps, const KqParams p) {
+template <int FMT, bool MARKS>
+__device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, uint8_t* smem, KqMisc& misc, uint32_t base, uint32_t tmem, int total) {
     using C = KqCfg<FMT>;
     constexpr bool Q6 = C::kQ6;
-    constexpr int kAccCols = Q6 ? kKqN : 2 * kKqN, kColA = 2 * kAccCols;      // per matrix: accumulator (and minima); then the operand stages
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t raw = smem_u32(smem_raw);
-    const uint32_t base = (raw + 1023u) & ~1023u;
-    uint8_t* smem = smem_raw + (base - raw);
-    KqMisc& misc = *reinterpret_cast<KqMisc*>(smem + C::kOffMisc);
+    constexpr int kAccCols = 2 * kKqN, kColA = 2 * kAccCols;      // per matrix: accumulator, minima or the sum of one stage; then the operand stages
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) {
-        for (int i = 0; i < 2; i++) {
-            bar_init(smem_u32(&misc.b_full[i]), 1); bar_init(smem_u32(&misc.b_free[i]), 2);
-            bar_init(smem_u32(&misc.acc_full[i]), 1); bar_init(smem_u32(&misc.acc_free[i]), 4);
-            for (int j = 0; j < 2; j++) { bar_init(smem_u32(&misc.a_full[i][j]), 4); bar_init(smem_u32(&misc.a_free[i][j]), 1); bar_init(smem_u32(&misc.hdr_free[i][j]), 4); }
-        }
-        for (int i = 0; i < 4; i++) { bar_init(smem_u32(&misc.dx_full[i]), 1); bar_init(smem_u32(&misc.dx_free[i]), 8); }
-        for (int i = 0; i < C::kRing; i++) { bar_init(smem_u32(&misc.raw_full[i]), 1); bar_init(smem_u32(&misc.raw_free[i]), 16); }
-        bar_fence_init();
-    }
-    if (warp == 17) tmem_alloc(smem_u32(&misc.tmem_base), 512);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = misc.tmem_base;
-    const int total = p.n_tiles ? *p.n_tiles * p.tiles_mul : p.total;
-
     if (warp < 16) {
         // ========================================================================== producers
         regs_down<C::kRegsP>();
@@ -397,29 +407,55 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
             // ====================================================================== tensor-core issuers (converged warps), one per matrix
             const int mat = warp - 17;
             const uint32_t acc = tmem + mat * kAccCols, a0 = tmem + kColA + mat * 128;
-            unsigned it = 0, uses = 0;
+            unsigned it = 0, uses = 0, fills = 0;      // blocks, stages / 2, and accumulators handed to the epilogue so far
             for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                 const KqTile t = kq_tile(p, tile);
                 const uint32_t idesc = instr_desc(1, 0, 0, 0, 0, 128, (t.n + 15) & ~15);      // f32 += f16 . f16
                 for (int s = 0; s < t.nsb; s++, it++) {
                     const int b = it & 1;
+                    const bool marked = MARKS && __any_sync(0xffffffffu, kq_mark(p, t.sb0 + s, t.p0, t.n, lane));
+                    // the accumulator is the epilogue's until it gives it back
+                    auto taken = [&] { bar_wait(smem_u32(&misc.acc_free[mat]), (fills & 1) ^ 1); };
+                    auto give = [&] {
+                        mma_commit(smem_u32(&misc.acc_full[mat]));
+                        if (MARKS) kq_tell(smem_u32(&misc.marked[mat]), marked, smem_u32(&misc.acc_full[mat]));
+                        fills++;
+                    };
                     bar_wait(smem_u32(&misc.b_full[b]), (it >> 1) & 1);
-                    bar_wait(smem_u32(&misc.acc_free[mat]), (it & 1) ^ 1);
-                    uint64_t bd = smem_desc(base + b * C::kB, 16, 1024, kLayoutSw128);
+                    taken();
+                    uint64_t bd = smem_desc(base + b * C::kB, 16, 1024, kLayoutSw128);      // (the address field counts 16 bytes, and nothing carries out of it)
+                    const uint64_t md = smem_desc(base + C::kOffMins + (mat * 2 + b) * C::kMins, 128, 256, kLayoutNone), sd = smem_desc(base + C::kOffSums + b * C::kSums, 16, 256, kLayoutSw32);
+                    constexpr uint64_t kStep = kKqN * 128 >> 4;      // Q6_K: both terms of a quarter's 64 weights meet one tile of activations
+                    if (!marked) {
 #pragma unroll 1
-                    for (int h = 0; h < C::kStages; h++) {
-                        bar_wait(smem_u32(&misc.a_full[mat][h & 1]), uses & 1);
-                        tc_fence_after();
-                        // (the address field of a descriptor counts 16 bytes, and nothing carries out of it)
-                        mma_f16_ta8(acc, a0 + (h & 1) * 64, bd, Q6 ? 0 : kKqN * 128 >> 4, idesc, h);      // Q6_K: both terms of the quarter's 64 weights
-                        bd += (Q6 ? 1 : 2) * (kKqN * 128 >> 4);
-                        if (!Q6 && h == 0)
-                            mma_f16(acc + kKqN, smem_desc(base + C::kOffMins + (mat * 2 + b) * C::kMins, 128, 256, kLayoutNone),
-                                    smem_desc(base + C::kOffSums + b * C::kSums, 16, 256, kLayoutSw32), idesc, 0);
-                        mma_commit(smem_u32(&misc.a_free[mat][h & 1]));
-                        if (h & 1) uses++;
+                        for (int h = 0; h < C::kStages; h++) {
+                            bar_wait(smem_u32(&misc.a_full[mat][h & 1]), uses & 1);
+                            tc_fence_after();
+                            mma_f16_ta8(acc, a0 + (h & 1) * 64, bd, Q6 ? 0 : kStep, idesc, h);
+                            bd += (Q6 ? 1 : 2) * kStep;
+                            if (!Q6 && h == 0) mma_f16(acc + kKqN, md, sd, idesc, 0);
+                            mma_commit(smem_u32(&misc.a_free[mat][h & 1]));
+                            if (h & 1) uses++;
+                        }
+                    } else {      // the first stage's sum in the accumulator, each other one behind it, where the epilogue adds it; the minima's product last
+#pragma unroll 1
+                        for (int h = 0; h < C::kStages; h++) {
+                            bar_wait(smem_u32(&misc.a_full[mat][h & 1]), uses & 1);
+                            if (h > 1) taken();
+                            tc_fence_after();
+                            mma_f16_ta8(acc + (h ? kKqN : 0), a0 + (h & 1) * 64, bd, Q6 ? 0 : kStep, idesc, 0);
+                            bd += (Q6 ? 1 : 2) * kStep;
+                            mma_commit(smem_u32(&misc.a_free[mat][h & 1]));
+                            if (h & 1) uses++;
+                            if (h && h < C::kStages - Q6) give();
+                        }
+                        if (!Q6) {
+                            taken();
+                            tc_fence_after();
+                            mma_f16(acc + kKqN, md, sd, idesc, 0);
+                        }
                     }
-                    mma_commit(smem_u32(&misc.acc_full[mat]));
+                    give();
                     mma_commit(smem_u32(&misc.b_free[b]));
                 }
             }
@@ -430,7 +466,7 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
         const int mat = (warp - 20) >> 2, sp = warp & 3, r = 32 * sp + lane;
         const bool leader = sp == 0;
         const uint32_t tacc = tmem + ((uint32_t)(32 * sp) << 16) + mat * kAccCols;
-        unsigned it = 0;
+        unsigned it = 0, fills = 0;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
             const KqTile t = kq_tile(p, tile);
             const int row = t.row0 + (p.pair ? 0 : 128 * mat) + r;
@@ -450,12 +486,36 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
             for (int s = 0; s < t.nsb; s++, it++) {
                 const uint16_t dcur = dnext;
                 if (Q6 && s + 1 < t.nsb) dnext = __ldg(dsrc + s + 1);
-                if (leader) {
-                    bar_wait(smem_u32(&misc.dx_full[it & 3]), (it >> 2) & 1);
-                    bar_wait(smem_u32(&misc.acc_full[mat]), it & 1);
+                if (leader) bar_wait(smem_u32(&misc.dx_full[it & 3]), (it >> 2) & 1);
+                auto sums = [&] {
+                    if (leader) bar_wait(smem_u32(&misc.acc_full[mat]), fills & 1);
+                    fills++;
+                    group_sync(5 + mat);
+                    tc_fence_after();
+                };
+                sums();
+                if (MARKS && misc.marked[mat]) {      // a stage's sum, in the columns behind the accumulator, joins it here
+#pragma unroll 1
+                    for (int h = 1;; h++) {
+#pragma unroll 1
+                        for (int c = 0; c < t.n; c += 16) {
+                            uint32_t v[16], m[16];
+                            tmem_ld16(tacc + c, v);
+                            tmem_ld16(tacc + kKqN + c, m);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 16; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) + __uint_as_float(m[i]));
+                            tmem_st16(tacc + c, v);
+                        }
+                        tmem_wait_st();
+                        if (Q6 && h + 1 == C::kStages) break;      // nothing follows the last stage
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(smem_u32(&misc.acc_free[mat]));
+                        sums();
+                        if (!Q6) break;                            // that was the minima's product
+                    }
                 }
-                group_sync(5 + mat);
-                tc_fence_after();
                 const __half2 dm = as_h2(Q6 ? (uint32_t)dcur : misc.hdr[mat][it & 1][r]);
                 const float dw = __low2float(dm) * C::kScale, dmin = -__high2float(dm);
                 const f32x2 dw2 = pack2(dw, dw), dmin2 = pack2(dmin, dmin);
@@ -513,6 +573,35 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
             }
         }
     }
+}
+
+template <int FMT, bool MARKS>
+__device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
+    using C = KqCfg<FMT>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t* smem = smem_raw + (base - raw);
+    KqMisc& misc = *reinterpret_cast<KqMisc*>(smem + C::kOffMisc);
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int total = p.n_tiles ? *p.n_tiles * p.tiles_mul : p.total;
+    if (tid == 0) {
+        for (int i = 0; i < 2; i++) {
+            bar_init(smem_u32(&misc.b_full[i]), 1); bar_init(smem_u32(&misc.b_free[i]), 2);
+            bar_init(smem_u32(&misc.acc_full[i]), MARKS ? 2 : 1); bar_init(smem_u32(&misc.acc_free[i]), 4);
+            for (int j = 0; j < 2; j++) { bar_init(smem_u32(&misc.a_full[i][j]), 4); bar_init(smem_u32(&misc.a_free[i][j]), 1); bar_init(smem_u32(&misc.hdr_free[i][j]), 4); }
+        }
+        for (int i = 0; i < 4; i++) { bar_init(smem_u32(&misc.dx_full[i]), 1); bar_init(smem_u32(&misc.dx_free[i]), 8); }
+        for (int i = 0; i < C::kRing; i++) { bar_init(smem_u32(&misc.raw_full[i]), 1); bar_init(smem_u32(&misc.raw_free[i]), 16); }
+        bar_fence_init();
+    }
+    if (warp == 17) tmem_alloc(smem_u32(&misc.tmem_base), 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = misc.tmem_base;
+
+    kq_roles<FMT, MARKS>(maps, p, smem, misc, base, tmem, total);
     tc_fence_before();
     __syncthreads();
     if (warp == 17) {
@@ -521,8 +610,24 @@ __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_con
     }
 }
 
+template <int FMT>
+__device__ __noinline__ void kq_body_marked(const KqMaps& maps, const KqParams& p) { kq_body<FMT, true>(maps, p); }
+// The form for activations with marked blocks is a function apart, and the quantiser's word says which one a call needs: in one form the calls without marks took 6-10 % longer
+// (777 x 1536 -> 24576 177 -> 194 us: a block's hand-overs wait for its mark, an MMA whose operand depends on it waits for that to be made uniform), as two inlined forms 10 %
+// (spills), like this 3 % (long ones; registers) and short ones nothing.  As two launches, one of which ends at once, 1 % and 2-4 %, but 6 us more for short ones.
+template <int FMT>
+__global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_constant__ KqMaps maps, const __grid_constant__ KqParams p) {
+    if (*p.any == p.id) kq_body_marked<FMT>(maps, p);
+    else kq_body<FMT, false>(maps, p);
+}
+
 // ---------------------------------------------------------------------------------------------------------------- activations
-__device__ __forceinline__ void kq_store_block(const KqActs& a, long row, int b, int K, int lane, bool q6, uint32_t w0, uint32_t w1, float d, int s2) {
+// whether a block is beyond its limit (kq_limit); s: the lane's sum of quants
+__device__ __forceinline__ bool kq_beyond(uint32_t w0, uint32_t w1, int s, bool q6, int limit) {
+    const int size = __reduce_add_sync(0xffffffffu, __dp4a((int)__vabs4(w0), 0x01010101, __dp4a((int)__vabs4(w1), 0x01010101, 0)));
+    return (q6 ? 2 * size : size + abs(__reduce_add_sync(0xffffffffu, s))) > limit;
+}
+__device__ __forceinline__ void kq_store_block(const KqActs& a, long row, int b, int K, int lane, bool q6, uint32_t w0, uint32_t w1, float d, int s2, bool beyond) {
     const uint32_t w[2] = {w0, w1};
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -533,10 +638,14 @@ __device__ __forceinline__ void kq_store_block(const KqActs& a, long row, int b,
             make_uint2(as_u32(__halves2half2(v[0], v[2])), as_u32(__halves2half2(v[1], v[3])));
     }
     if (!q6 && (lane & 1) == 0) a.sums[row * (K / 16) + b * 16 + (lane >> 1)] = __int2half_rn((int)(int16_t)s2);
-    if (lane == 0) a.d[(long)b * a.pitch + row] = d;
+    if (lane == 0) {
+        a.d[(long)b * a.pitch + row] = d;
+        a.marks[(long)b * a.pitch + row] = beyond;
+        if (beyond) *a.any = a.id;
+    }
 }
 // one warp per (token, 256-block): quantised once, stored for every row the token has
-__global__ void __launch_bounds__(256) kq_quant_kernel(const void* x, int hidden_type, int T, int K, const int* pos, int k, int q6, const KqActs a) {
+__global__ void __launch_bounds__(256) kq_quant_kernel(const void* x, int hidden_type, int T, int K, const int* pos, int k, int q6, int limit, const KqActs a) {
     const int lane = threadIdx.x & 31, nblk = K / QK_K;
     const long gw = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gw >= (long)T * nblk) return;
@@ -547,15 +656,16 @@ __global__ void __launch_bounds__(256) kq_quant_kernel(const void* x, int hidden
     load_block8(x, (long)t * K + (long)b * QK_K + lane * 8, hidden_type, v);
     warp_q8k_words(v, w0, w1, d, s);
     const int s2 = s + __shfl_xor_sync(0xffffffffu, s, 1);
-    if (!pos) kq_store_block(a, t, b, K, lane, q6, w0, w1, d, s2);
+    const bool beyond = kq_beyond(w0, w1, s, q6, limit);
+    if (!pos) kq_store_block(a, t, b, K, lane, q6, w0, w1, d, s2, beyond);
     else
         for (int j = 0; j < k; j++) {
             const int row = pos[t * k + j];
-            if (row >= 0) kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2);
+            if (row >= 0) kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2, beyond);
         }
 }
 // (without pos: rows 0 .. n, each the sum of `splits` parts)
-__global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const float* u, const int* pos, int splits, int n, int K, int use_silu, int q6, const KqActs a) {
+__global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const float* u, const int* pos, int splits, int n, int K, int use_silu, int q6, int limit, const KqActs a) {
     const int lane = threadIdx.x & 31, nblk = K / QK_K;
     const long gw = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gw >= (long)n * nblk) return;
@@ -578,7 +688,8 @@ __global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const
     for (int j = 0; j < 8; j++) v[j] = (use_silu ? act_silu(gv[j]) : act_relu(gv[j])) * uv[j];
     warp_q8k_words(v, w0, w1, d, s);
     const int s2 = s + __shfl_xor_sync(0xffffffffu, s, 1);
-    kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2);
+    const bool beyond = kq_beyond(w0, w1, s, q6, limit);
+    kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2, beyond);
 }
 // y = sum of the K parts + bias, in the hidden type (accumulate: y + that sum, rounded first)
 __global__ void __launch_bounds__(256) kq_finish_kernel(const float* part, int splits, int T, int R, void* y, int hidden_type, const float* bias, int accumulate, const int* bsz, int t0) {
@@ -591,13 +702,18 @@ __global__ void __launch_bounds__(256) kq_finish_kernel(const float* part, int s
     store_hidden(y, i, hidden_type, v);
 }
 
-int kq_quant(const void* x, int hidden_type, int T, int K, const int* pos, int k, bool q6, const KqActs& a, cudaStream_t s) {
-    kq_quant_kernel<<<(unsigned)(((long)T * (K / QK_K) + 7) / 8), 256, 0, s>>>(x, hidden_type, T, K, pos, k, q6, a);
+unsigned long long kq_next_id() {
+    static std::atomic<unsigned long long> next{0x6b715f6964000001ull};
+    return next.fetch_add(1, std::memory_order_relaxed);
+}
+
+int kq_quant(const void* x, int hidden_type, int T, int K, const int* pos, int k, bool q6, int limit, const KqActs& a, cudaStream_t s) {
+    kq_quant_kernel<<<(unsigned)(((long)T * (K / QK_K) + 7) / 8), 256, 0, s>>>(x, hidden_type, T, K, pos, k, q6, limit, a);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
-int kq_act_quant(const float* g, const float* u, const int* pos, int n, int K, int use_silu, bool q6, const KqActs& a, cudaStream_t s) {
-    kq_act_quant_kernel<<<(unsigned)(((long)n * (K / QK_K) + 7) / 8), 256, 0, s>>>(g, u, pos, 1, n, K, use_silu, q6, a);
+int kq_act_quant(const float* g, const float* u, const int* pos, int n, int K, int use_silu, bool q6, int limit, const KqActs& a, cudaStream_t s) {
+    kq_act_quant_kernel<<<(unsigned)(((long)n * (K / QK_K) + 7) / 8), 256, 0, s>>>(g, u, pos, 1, n, K, use_silu, q6, limit, a);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
@@ -655,7 +771,7 @@ static int kq_launch(const KqMaps& maps, const KqParams& p, int grid, cudaStream
 int kq_gemm(const KqGemm& g, int device, cudaStream_t s) {
     KqParams p{};
     for (int i = 0; i < 2; i++) { p.w[i] = reinterpret_cast<const uint8_t*>(g.w[i]); p.out[i] = g.out[i]; }
-    p.expert_bytes = g.expert_bytes; p.dpitch = g.acts->pitch; p.pair = g.pair; p.R = g.R; p.nblk = g.K / QK_K; p.dx = g.acts->d;
+    p.expert_bytes = g.expert_bytes; p.dpitch = g.acts->pitch; p.pair = g.pair; p.R = g.R; p.nblk = g.K / QK_K; p.dx = g.acts->d; p.marks = g.acts->marks; p.any = g.acts->any; p.id = g.acts->id;
     p.tinfo = g.tinfo; p.n_tiles = g.n_tiles_dev; p.tiles_mul = g.tiles_mul; p.y = g.y; p.hidden_type = g.hidden_type; p.bias = g.bias; p.bsz = g.bsz;
     p.t0 = g.t0; p.T = g.T; p.splits = g.splits; p.rt = (g.R + kKqRows - 1) / kKqRows; p.nt = (g.T + kKqN - 1) / kKqN; p.total = p.rt * p.nt * g.splits;
     KqMaps maps;
@@ -692,7 +808,7 @@ int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_
         const size_t act = (KqActs::bytes(n, K) + 255) / 256 * 256;
         KTB_CUDA_CHECK(mem.take(device, act + (splits > 1 ? (size_t)splits * n * R * 4 : 0)));
         const KqActs a(mem.ptr, n, K);
-        int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * K * hb, hidden_type, n, K, nullptr, 1, kq_is_q6(f), a, s);
+        int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * K * hb, hidden_type, n, K, nullptr, 1, kq_is_q6(f), kq_limit(f), a, s);
         if (rc) return rc;
         KqGemm g{};
         g.fmt = f; g.w[0] = g.w[1] = w; g.experts = 1; g.R = R; g.K = K; g.acts = &a; g.T = n; g.splits = splits; g.hidden_type = hidden_type; g.bias = bias; g.t0 = t0;
@@ -729,7 +845,7 @@ int kq_mlp(const ktb200_mlp* m, const void* x, int T, void* y, int accumulate, c
         uint8_t* at = reinterpret_cast<uint8_t*>(mem.ptr);
         const KqActs xa(at, n, H), aa(at + n_x, n, I);
         float *gu[2] = {reinterpret_cast<float*>(at + n_x + n_a), reinterpret_cast<float*>(at + n_x + n_a + n_g)}, *part = reinterpret_cast<float*>(at + n_x + n_a + 2 * n_g);
-        int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * H * hb, m->hidden_type, n, H, nullptr, 1, kq_is_q6(f[0]), xa, s);
+        int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * H * hb, m->hidden_type, n, H, nullptr, 1, kq_is_q6(f[0]), std::min(kq_limit(f[0]), kq_limit(f[1])), xa, s);
         if (rc) return rc;
         KqGemm g{};
         g.experts = 1; g.R = I; g.K = H; g.acts = &xa; g.T = n; g.splits = su;
@@ -738,7 +854,7 @@ int kq_mlp(const ktb200_mlp* m, const void* x, int T, void* y, int accumulate, c
             rc = kq_gemm(g, dev, s);
             if (rc) return rc;
         }
-        kq_act_quant_kernel<<<(unsigned)(((long)n * (I / QK_K) + 7) / 8), 256, 0, s>>>(gu[0], gu[1], nullptr, su, n, I, 1, kq_is_q6(f[2]), aa);
+        kq_act_quant_kernel<<<(unsigned)(((long)n * (I / QK_K) + 7) / 8), 256, 0, s>>>(gu[0], gu[1], nullptr, su, n, I, 1, kq_is_q6(f[2]), kq_limit(f[2]), aa);
         KTB_LAUNCH_CHECK();
         g.fmt = f[2]; g.w[0] = g.w[1] = w[2]; g.R = H; g.K = I; g.acts = &aa; g.splits = sd; g.out[0] = g.out[1] = part;
         rc = kq_gemm(g, dev, s);

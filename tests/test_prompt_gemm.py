@@ -157,6 +157,49 @@ def test_mlp_of_a_prompt(gate, up, down, H, I, T, hid):
     lib.ktb200_mlp_destroy(h)
 
 
+# Activations of one sign and about one size: an ordinary Q5_K block then sums to about 20 million, beyond the 2^24 of an fp32 accumulator, and its minima take most of
+# it away again; and blocks at the largest sums their format has.  The decode kernels, 8 rows at a time, round a block's sum once: the prompt's may not be further
+# from 64 bits than they are, or than two units of fp32.  Rows in between are ordinary ones (marked and other blocks beside each other), and the order of the rows must not matter
+@pytest.mark.parametrize("type", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,R,T", [(256, 3000, 9), (512, 520, 65), (7168, 1024, 130), (4096, 20000, 320)])
+@pytest.mark.parametrize("weights", ["ordinary", "largest"])
+def test_k_quant_sums_beyond_an_fp32_accumulator(type, K, R, T, weights):
+    b = synth_blocks(type, R * K, "cuda", T + K).view(R * K // 256, -1)
+    if weights == "largest":
+        b[:, 4 if type != Q6_K else 0:208] = 255      # (d and dmin of the first, d of the second lie outside)
+        if type == Q6_K:
+            b[:, 192:208] = 127
+        b[::7, 20:60] = 170
+    elif type != Q6_K:       # minima like the scales times the middle quant: values about 0
+        b[:, 8:12] = b[:, 4:8]
+        b[:, 12:16] = (b[:, 12:16] & 15) * 17
+        d = b[:, 0:2].contiguous().view(torch.float16).float()
+        b[:, 2:4] = (d * (7.5 if type == Q4_K else 15.5)).to(torch.float16).view(torch.uint8)
+    blocks = b.reshape(-1)
+    dense = torch.from_numpy(Oracle().to_float(blocks.cpu().numpy(), type, R * K)).cuda().view(R, K)
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x = torch.randn((T, K), generator=g, device="cuda")
+    flat = torch.arange(T, device="cuda") % 3 != 1
+    x[flat] = 1 + 0.01 * x[flat]
+    lib, h = native.lib(), C.c_void_p()
+    native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), type, F32, T, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, _stream()))
+
+    def call(x):
+        y = torch.zeros((x.shape[0], R), device="cuda")
+        native.check(lib.ktb200_linear_forward(h, x.shape[0], x.data_ptr(), y.data_ptr(), None, None, _stream()))
+        return y
+
+    want = _q8(x) @ dense.double().T
+    y, rows = call(x), torch.cat([call(x[t:t + 8].contiguous()) for t in range(0, T, 8)])
+    for part in (flat, ~flat):
+        off, off_rows = (((v[part].double() - want[part]).norm() / want[part].norm()).item() for v in (y, rows))
+        assert off <= max(1.1 * off_rows, 2.0 ** -23), (off, off_rows)
+    order = torch.randperm(T, generator=g, device="cuda")
+    assert torch.equal(call(x[order].contiguous()), y[order])
+    lib.ktb200_linear_destroy(h)
+
+
 # matrices so small that the launches of the GEMM cost more than the row kernels (the FP8 passes) take: (path, K, R or N, rows, launches)
 @pytest.mark.parametrize("kind,K,R,T,launches", [("linear", 512, 512, 32, 1), ("linear", 512, 512, 41, 2), ("linear", 4096, 64, 11, 1), ("linear", 4096, 64, 12, 3), ("q6", 512, 512, 20, 1),
                                                  ("q6", 512, 512, 24, 2), ("fp8", 7168, 576, 24, 4), ("fp8", 7168, 576, 25, 2), ("fp8", 16384, 72, 48, 6), ("fp8", 512, 512, 17, 2),
@@ -191,3 +234,20 @@ def test_small_matrices_keep_the_kernels_of_few_rows(kind, K, R, T, launches):
     size = few.double().abs().max()
     assert ((y.double() - few.double()).abs() <= 2.0 ** -7 * few.double().abs() + (1e-3 if kind == "mlp" else 4e-6) * size).all()
     (lib.ktb200_fp8_linear_destroy if kind == "fp8" else lib.ktb200_mlp_destroy if kind == "mlp" else lib.ktb200_linear_destroy)(h)
+
+
+# the same through routed experts: rows in between with marked blocks, against the per-pair kernels (8 tokens at a time)
+@pytest.mark.parametrize("gu,down", [(Q4_K, Q6_K), (Q5_K, Q5_K), (Q6_K, Q4_K)])
+def test_experts_with_flat_activations(gu, down):
+    import gpu_util as G
+    E, k, H, I, T = 4, 2, 1024, 512, 200
+    w = synth_blocks(gu, E * I * H, "cuda", 1), synth_blocks(gu, E * I * H, "cuda", 2), synth_blocks(down, E * H * I, "cuda", 3)
+    gen = torch.Generator().manual_seed(T)
+    x = torch.randn((T, H), generator=gen) / 10
+    x[::3] = 0.1 + 0.001 * x[::3]
+    ids, wt = torch.stack([torch.randperm(E, generator=gen)[:k] for _ in range(T)]).numpy(), torch.rand((T, k), generator=gen).numpy()
+    m = G.Moe(E, k, H, I, *w, gu, gu, down, F32, max_tokens=T)
+    got = torch.from_numpy(m.forward(ids, wt, x.numpy()))
+    want = torch.cat([torch.from_numpy(m.forward(ids[t:t + 8], wt[t:t + 8], x[t:t + 8].numpy())) for t in range(0, T, 8)])
+    assert torch.isfinite(got).all() and (got - want).norm() <= 1e-3 * want.norm()
+    m.close()
