@@ -33,6 +33,7 @@
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
 #include <algorithm>
 #include <atomic>
+#include <climits>
 
 #include <cuda_fp16.h>
 
@@ -691,12 +692,14 @@ __global__ void __launch_bounds__(256) kq_act_quant_kernel(const float* g, const
     const bool beyond = kq_beyond(w0, w1, s, q6, limit);
     kq_store_block(a, row, b, K, lane, q6, w0, w1, d, s2, beyond);
 }
-// y = sum of the K parts + bias, in the hidden type (accumulate: y + that sum, rounded first)
+// y = sum of the K parts + bias, in the hidden type (accumulate: y + that sum, rounded first).  The parts are added in 64 bits: the launch is bound by their bytes, and
+// a chain of 32 in fp32 was half of the error of a long row (K = 16384)
 __global__ void __launch_bounds__(256) kq_finish_kernel(const float* part, int splits, int T, int R, void* y, int hidden_type, const float* bias, int accumulate, const int* bsz, int t0) {
     const long i = (long)blockIdx.x * 256 + threadIdx.x, n = (long)(bsz ? max(0, min(T, *bsz - t0)) : T) * R;
     if (i >= n) return;
-    float v = part[i];
-    for (int s = 1; s < splits; s++) v += part[(long)s * T * R + i];
+    double sum = part[i];
+    for (int s = 1; s < splits; s++) sum += part[(long)s * T * R + i];
+    float v = (float)sum;
     if (bias) v += bias[i % R];
     if (accumulate) v = load_hidden(y, i, hidden_type) + round_hidden(v, hidden_type);
     store_hidden(y, i, hidden_type, v);
@@ -795,15 +798,24 @@ static int kq_splits(int tiles, int nblk, int sms) {
     return n < 1 ? 1 : n;
 }
 
+// fp32 results, where the order of a long fp32 chain shows: parts of at most kKqChain blocks
+constexpr int kKqChain = 10;
+static int kq_splits_of(int tiles, int nblk, int sms, int hidden_type) {
+    const int n = kq_splits(tiles, nblk, sms);
+    return hidden_type == KTB200_TYPE_F32 ? std::max(n, (nblk + kKqChain - 1) / kKqChain) : n;
+}
+
 int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_type, int T, void* y, const float* bias, const int* bsz, int device, cudaStream_t s) {
     const KqFmt f = kq_fmt(fmt);
     if (f == KQ_NONE || (uintptr_t)w % 16) return 1;
-    constexpr int kChunk = 4096;      // rows per pass: bounds the scratch
+    // rows per pass: bounds the scratch (fp32 results in parts: to 256 MB of those)
+    const int nparts = kq_splits_of(INT_MAX, K / QK_K, 1, hidden_type);
+    const int chunk = nparts == 1 ? 4096 : std::max(256L, std::min(4096L, (1L << 26) / ((long)nparts * R) / kKqN * kKqN));
     const size_t hb = type_size(hidden_type);
-    for (int t0 = 0; t0 < T; t0 += kChunk) {
-        const int n = T - t0 < kChunk ? T - t0 : kChunk, sms = num_sms(device);
+    for (int t0 = 0; t0 < T; t0 += chunk) {
+        const int n = T - t0 < chunk ? T - t0 : chunk, sms = num_sms(device);
         const int tiles = ((R + kKqRows - 1) / kKqRows) * ((n + kKqN - 1) / kKqN), nblk = K / QK_K;
-        const int splits = kq_splits(tiles, nblk, sms);
+        const int splits = kq_splits_of(tiles, nblk, sms, hidden_type);
         ScratchBlock mem(s);
         const size_t act = (KqActs::bytes(n, K) + 255) / 256 * 256;
         KTB_CUDA_CHECK(mem.take(device, act + (splits > 1 ? (size_t)splits * n * R * 4 : 0)));
@@ -837,7 +849,7 @@ int kq_mlp(const ktb200_mlp* m, const void* x, int T, void* y, int accumulate, c
     const size_t hb = type_size(m->hidden_type);
     for (int t0 = 0; t0 < T; t0 += kChunk) {
         const int n = T - t0 < kChunk ? T - t0 : kChunk, nt = (n + kKqN - 1) / kKqN;
-        const int su = kq_splits((I + kKqRows - 1) / kKqRows * nt, H / QK_K, sms), sd = kq_splits((H + kKqRows - 1) / kKqRows * nt, I / QK_K, sms);
+        const int su = kq_splits((I + kKqRows - 1) / kKqRows * nt, H / QK_K, sms), sd = kq_splits_of((H + kKqRows - 1) / kKqRows * nt, I / QK_K, sms, m->hidden_type);
         auto up = [](size_t b) { return (b + 255) / 256 * 256; };
         const size_t n_x = up(KqActs::bytes(n, H)), n_a = up(KqActs::bytes(n, I)), n_g = up((size_t)su * n * I * 4), n_d = up((size_t)sd * n * H * 4);
         ScratchBlock mem(s);

@@ -251,3 +251,25 @@ def test_experts_with_flat_activations(gu, down):
     want = torch.cat([torch.from_numpy(m.forward(ids[t:t + 8], wt[t:t + 8], x[t:t + 8].numpy())) for t in range(0, T, 8)])
     assert torch.isfinite(got).all() and (got - want).norm() <= 1e-3 * want.norm()
     m.close()
+
+
+# fp32 results of long rows: no further from 64 bits than the row kernels, whose lanes add short chains of blocks (parts, and many tiles without parts of their own)
+@pytest.mark.parametrize("type", [Q4_K, Q6_K])
+@pytest.mark.parametrize("K,R,T", [(16384, 256, 64), (4096, 8192, 260)])
+def test_k_quant_long_rows_in_fp32(type, K, R, T):
+    blocks = synth_blocks(type, R * K, "cuda", K)
+    dense = torch.from_numpy(Oracle().to_float(blocks.cpu().numpy(), type, R * K)).cuda().view(R, K)
+    x = torch.randn((T, K), generator=torch.Generator(device="cuda").manual_seed(R), device="cuda")
+    lib, h = native.lib(), C.c_void_p()
+    native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), type, F32, T, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, _stream()))
+
+    def call(x):
+        y = torch.zeros((x.shape[0], R), device="cuda")
+        native.check(lib.ktb200_linear_forward(h, x.shape[0], x.data_ptr(), y.data_ptr(), None, None, _stream()))
+        return y
+
+    want = _q8(x) @ dense.double().T
+    off, off_rows = ((v.double() - want).norm().item() for v in (call(x), torch.cat([call(x[t:t + 8].contiguous()) for t in range(0, T, 8)])))
+    assert off <= 1.05 * off_rows, (off, off_rows)
+    lib.ktb200_linear_destroy(h)
