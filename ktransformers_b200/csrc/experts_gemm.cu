@@ -5,7 +5,7 @@
 // activation is applied to the fp32 sums in the epilogue and the pre-activations never reach memory; y stays fp32 up to the weighted sum.
 // Bounds: each expert's weights once per 128 of its pairs from HBM or L2 (48 KB a stage for 512 cycles of the tensor pipe), so at 100-300 pairs per expert the
 // second row tile's reading from L2 shows.  1000 tokens, 32 experts of 1024 x 2048, 4 choices (403 MB of weights, 62 us at 6.5 TB/s): 253 us as library GEMMs
-// with sorting and elementwise launches between them, 146 us like this (shares: products 48 and 31 %, weighted sum 8, sort 7, gather 5); 128 tokens,
+// with sorting and elementwise launches between them, 148 us like this (shares: products 48 and 31 %, weighted sum 8, sort 7, gather 5); 128 tokens,
 // 64 experts of 1536 x 4096, 6 choices (2.4 GB): 640 -> 434 us, 5.6 TB/s; 47 tokens, 8 experts of 4096 x 4096: 298 -> 172 us.
 //     kernel: warp 0 TMA (4 stages of 16 + 32 KB, 128-byte swizzle; of the 128 rows only pieces of 32 that the tile has), warp 1 issuer, warps 2-9
 //     epilogue; two accumulators of 256 columns, so that a tile's epilogue runs beside the next tile's products.  The launches are chained (programmatic

@@ -1,4 +1,4 @@
-"""Launches the kernels tools/gpu_profile_r02.sh captures with ncu: MLA decode (ctx 32768) and the o_proj-shaped dense linear."""
+"""Launches kernels to be captured with ncu: MLA decode (ctx 32768) and the o_proj-shaped dense linear."""
 import ctypes as C
 import os
 import sys
