@@ -15,8 +15,7 @@ namespace ktb {
 
 // tile table: tile -> {expert, first weight row, first sorted position, tokens}, token tile fastest so that CTAs running side by side share the
 // weight tile through L2.  One thread per tile; tiles beyond the data-dependent total are left alone.
-__global__ void grp_tiles_kernel(const int* nt_prefix, const int* offsets, const int* counts, int E, int MT, int rows, int4* tinfo) {
-    const int tile = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void grp_tile(int tile, const int* nt_prefix, const int* offsets, const int* counts, int E, int MT, int rows, int4* tinfo) {
     if (tile >= nt_prefix[E] * MT) return;
     int lo = 0, hi = E;
     while (hi - lo > 1) {
@@ -57,13 +56,20 @@ __global__ void __launch_bounds__(1024) grp_scan_kernel(const int* counts, int E
         if (e == E - 1) nt_prefix[E] = v.y;
     }
 }
-__global__ void grp_scatter_kernel(const int64_t* ids, int npairs, int k, int id_offset, int n_local, const int* bsz, int t0, int* cursor, int* pos) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npairs) return;
-    const long e = (long)ids[i] - id_offset;
-    if ((bsz && t0 + i / k >= *bsz) || e < 0 || e >= n_local) { pos[i] = -1; return; }
-    const int s = atomicAdd(cursor + e, 1);   // order inside an expert is irrelevant: every pair's result is independent
-    pos[i] = s;
+// what the offsets are for, in one launch: a thread per pair (its place), then a thread per tile of gate and up, then of down
+__global__ void grp_place_kernel(const int64_t* ids, int npairs, int k, int id_offset, int n_local, const int* bsz, int t0, int* cursor, int* pos, const int* nt_prefix, const int* offsets,
+                                 const int* counts, int mt_gu, int ub_gu, int4* tinfo_gu, int mt_d, int rows_d, int4* tinfo_d) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < npairs) {
+        const long e = (long)ids[i] - id_offset;
+        if ((bsz && t0 + i / k >= *bsz) || e < 0 || e >= n_local) { pos[i] = -1; return; }
+        const int s = atomicAdd(cursor + e, 1);   // order inside an expert is irrelevant: every pair's result is independent
+        pos[i] = s;
+        return;
+    }
+    i -= npairs;
+    if (i < ub_gu) grp_tile(i, nt_prefix, offsets, counts, n_local, mt_gu, 128, tinfo_gu);
+    else grp_tile(i - ub_gu, nt_prefix, offsets, counts, n_local, mt_d, rows_d, tinfo_d);
 }
 // out[t] = sum_j w[t][j] * down[pos[t][j]] in expert_ids order, one FMA per expert (moe.cpp:340-358), rounded like from_float
 __global__ void __launch_bounds__(256) grp_combine_kernel(const float* dd, const int* pos, const float* weights, int T, int k, int H, const int* bsz, int t0, void* out,
@@ -121,9 +127,8 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
         KTB_CUDA_CHECK(cudaMemsetAsync(counts, 0, (size_t)E * sizeof(int), s));
         grp_count_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids_c, n, k, c.expert_id_offset, E, bsz, t0, counts);
         grp_scan_kernel<<<1, 1024, 0, s>>>(counts, E, offsets, nt_prefix, cursor);
-        grp_scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(ids_c, n, k, c.expert_id_offset, E, bsz, t0, cursor, pos);
-        grp_tiles_kernel<<<(ub_gu + 255) / 256, 256, 0, s>>>(nt_prefix, offsets, counts, E, I / 128, 128, tinfo_gu);
-        grp_tiles_kernel<<<(ub_d + 255) / 256, 256, 0, s>>>(nt_prefix, offsets, counts, E, H / kKqRows, kKqRows, tinfo_d);
+        grp_place_kernel<<<(n + ub_gu + ub_d + 255) / 256, 256, 0, s>>>(ids_c, n, k, c.expert_id_offset, E, bsz, t0, cursor, pos, nt_prefix, offsets, counts, I / 128, ub_gu, tinfo_gu,
+                                                                        H / kKqRows, kKqRows, tinfo_d);
         int rc = kq_quant(x_c, c.hidden_type, T, H, pos, k, kq_is_q6(fg), kq_limit(fg), xa, s);
         if (rc) return rc;
         KqGemm gp{};
@@ -140,7 +145,7 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
         if (rc) return rc;
         grp_combine_kernel<<<dim3((H + 255) / 256, T), 256, 0, s>>>(dd, pos, weights + (size_t)t0 * k, T, k, H, bsz, t0, o_c, c.hidden_type);
         KTB_LAUNCH_CHECK();
-        count_launch(5);      // 10 launches per chunk: the 4 that kq_* and the 1 that the check counts, and the 5 bookkeeping kernels
+        count_launch(3);      // 10 launches per chunk: the 6 that kq_* and the 1 that the check counts, and the 3 bookkeeping kernels
     }
     return KTB200_OK;
 }

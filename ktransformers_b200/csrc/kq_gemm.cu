@@ -613,13 +613,24 @@ __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
 
 template <int FMT>
 __device__ __noinline__ void kq_body_marked(const KqMaps& maps, const KqParams& p) { kq_body<FMT, true>(maps, p); }
-// The form for activations with marked blocks is a function apart, and the quantiser's word says which one a call needs: in one form the calls without marks took 6-10 % longer
-// (777 x 1536 -> 24576 177 -> 194 us: a block's hand-overs wait for its mark, an MMA whose operand depends on it waits for that to be made uniform), as two inlined forms 10 %
-// (spills), like this 3 % (long ones; registers) and short ones nothing.  As two launches, one of which ends at once, 1 % and 2-4 %, but 6 us more for short ones.
-template <int FMT>
+// The form for activations with marked blocks is apart from the other, and the quantiser's word says which one a call needs: in one form the calls without marks took 6-10 %
+// longer (777 x 1536 -> 24576 177 -> 194 us: a block's hand-overs wait for its mark, an MMA whose operand depends on it waits for that to be made uniform).
+//   KQ_BOTH             one launch, the marked form as a function: costs the other one 3-4 % (registers), and nothing where launches bound a call (512 -> 512, 64 rows: 25 us)
+//   KQ_PLAIN, KQ_MARKED two launches, of which one ends at once; the second starts beside the first.  6 us more for short calls, 1 % for long ones (1024 tokens through the
+//                       routed experts 2920 us against 3013 with KQ_BOTH, 2893 without marks): experts, and from kPairBlocks blocks of a tile per CTA on
+enum KqForms { KQ_PLAIN, KQ_MARKED, KQ_BOTH };
+constexpr int kPairBlocks = 40;
+template <int FMT, KqForms FORMS>
 __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_constant__ KqMaps maps, const __grid_constant__ KqParams p) {
-    if (*p.any == p.id) kq_body_marked<FMT>(maps, p);
-    else kq_body<FMT, false>(maps, p);
+    const bool marks = *p.any == p.id;
+    if (FORMS == KQ_BOTH) {
+        if (marks) kq_body_marked<FMT>(maps, p);
+        else kq_body<FMT, false>(maps, p);
+    } else {
+        if (FORMS == KQ_PLAIN) griddep_launch_dependents();
+        if (marks == (FORMS == KQ_MARKED)) kq_body<FMT, FORMS == KQ_MARKED>(maps, p);
+        if (FORMS == KQ_MARKED) griddep_wait();      // (what follows it in the stream follows both)
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------------- activations
@@ -765,8 +776,18 @@ static int kq_map_weights(CUtensorMap* m, KqFmt f, const void* w, long rows, int
 }
 template <int FMT>
 static int kq_launch(const KqMaps& maps, const KqParams& p, int grid, cudaStream_t s) {
-    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kq_smem<FMT>()));
-    kq_gemm_kernel<FMT><<<grid, kKqThreads, kq_smem<FMT>(), s>>>(maps, p);
+    constexpr int smem = kq_smem<FMT>();
+    if (!p.tinfo && (long)p.total * ((p.nblk + p.splits - 1) / p.splits) < (long)kPairBlocks * grid) {
+        KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_BOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kq_gemm_kernel<FMT, KQ_BOTH><<<grid, kKqThreads, smem, s>>>(maps, p);
+        KTB_LAUNCH_CHECK();
+        return KTB200_OK;
+    }
+    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_MARKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kq_gemm_kernel<FMT, KQ_PLAIN><<<grid, kKqThreads, smem, s>>>(maps, p);
+    KTB_LAUNCH_CHECK();
+    KTB_CUDA_CHECK(launch_pdl(kq_gemm_kernel<FMT, KQ_MARKED>, dim3(grid), dim3(kKqThreads), (size_t)smem, s, maps, p));
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
