@@ -27,7 +27,7 @@
 //      raw blocks from a TMA ring -> registers -> TMEM; warp 16 TMA of activations, 17 / 18 MMA issuers of matrix 0 / 1, 19 TMA of weights;
 //      groups 5 / 6 epilogue of matrix 0 / 1.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
 //      warps took a third of the issue slots, and the four roles' code is kept in rolled loops: unrolled it overran the instruction cache (10,000
-//      cycles for a block of two matrices; now 3,400; HBM brings one every 1,550).  What is left is the chain product -> drain -> product of
+//      cycles for a block of two matrices; now 3,800 at 48 tokens a tile, profiles/prompt_kernels.md; HBM brings one every 1,550).  What is left is the chain product -> drain -> product of
 //      a matrix beside producers that issue ~8,000 instructions per block; measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 6.6 ms with one
 //      int32 accumulator per 32 values and operands through shared memory, 2.9 ms (the operator's call); Q4_K linear 777 x 1536 -> 24576 180 us (326 TFLOP/s).
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
