@@ -19,7 +19,8 @@
 //   * the weights go registers -> tensor memory (tcgen05.st, a thread = a weight row = a lane) and never to shared memory as operands.  Through
 //     shared memory, 2 B per weight written and 2 B read by the MMA would take 128 B per cycle to 21 weights per cycle, half of what HBM brings;
 //     and an MMA of 128 x 64 x 16 runs in 32 cycles with A in tensor memory against 48 with A in shared memory (measured; N = 32: 17 and 40).
-//   * nibbles become fp16 by or-ing them into the mantissa of 1024 and one fused multiply-add with (sc, -1024 sc): 9 instructions for 8
+//   * nibbles become fp16 by or-ing them into the mantissa of 1024 and one fused multiply-add with (sc, -1024 sc), Q6_K's upper two bits into that of 4 or 16
+//     (fewer shifts, and the offset is a product of 11 bits): 9 and 11 instructions for 8
 //     weights.  The pairs come out as (0, 2), (1, 3) of four; the activations are stored in that order (kq_pos4).
 //   * a scale per 256-block needs the accumulator drained per 256-block: two matrices of 128 rows per CTA (gate and up of the same experts, or
 //     256 rows of one) take turns, one drained while the other multiplies, and share the activation tiles.
@@ -27,9 +28,13 @@
 //      raw blocks from a TMA ring -> registers -> TMEM; warp 16 TMA of activations, 17 / 18 MMA issuers of matrix 0 / 1, 19 TMA of weights;
 //      groups 5 / 6 epilogue of matrix 0 / 1.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
 //      warps took a third of the issue slots, and the four roles' code is kept in rolled loops: unrolled it overran the instruction cache (10,000
-//      cycles for a block of two matrices; now 3,800 at 48 tokens a tile, profiles/prompt_kernels.md; HBM brings one every 1,550).  What is left is the chain product -> drain -> product of
-//      a matrix beside producers that issue ~8,000 instructions per block; measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 6.6 ms with one
-//      int32 accumulator per 32 values and operands through shared memory, 2.9 ms (the operator's call); Q4_K linear 777 x 1536 -> 24576 180 us (326 TFLOP/s).
+//      cycles for a block of two matrices).  The warp's number and what the tiles say come through a shuffle, so that the compiler knows them to be the same in all
+//      lanes and keeps a role's state, its branches and the MMAs' operands off the vector pipes (the other roles' share of the issue slots is what an issuer or
+//      an epilogue warp waits for: 157 -> 129 us for the linear below, 2,782 -> 2,600 for the experts; 268 -> 69 branch instructions a block).
+//      A block of two matrices takes 3,150 cycles at 64 tokens a tile (3,440 before), 1,970 at 16 (2,480); HBM brings one every 1,550.  Of the 3,150 the drain of an accumulator is
+//      1,500 (producers issue beside it; 660 alone), the eight MMAs of either stage 600, the rest hand-overs.  Draining in two halves of the tokens, so that one is multiplied
+//      while the other is drained, was slower (140 us, 2,770), and so were both matrices' drains in one thread (244) and other orders of the roles (165).
+//      Measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 2,950 -> 2,640 us (the operator's call); Q4_K linear 777 x 1536 -> 24576 182 -> 129 us (455 TFLOP/s).
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
 #include <algorithm>
 #include <atomic>
@@ -165,20 +170,40 @@ __device__ __forceinline__ __half2 magic_and(uint32_t a) {
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(MASK), "r"(kMagic));
     return as_h2(d);
 }
+template <uint32_t MASK, uint32_t BASE>
+__device__ __forceinline__ __half2 bits_in(uint32_t a) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(MASK), "r"(BASE));
+    return as_h2(d);
+}
+__device__ __forceinline__ __half2 bits_at8(uint32_t a) { return bits_in<0x03000300u, 0x44004400u>(a); }      // 4 + the two bits at 8
+__device__ __forceinline__ __half2 bits_at6(uint32_t a) { return bits_in<0x00c000c0u, 0x4c004c00u>(a); }      // 16 + the two bits at 6
 __device__ __forceinline__ float half_of(f32x2 v, int hi) { return __uint_as_float((uint32_t)(hi ? v >> 32 : v)); }
-__device__ __forceinline__ __half2 h2_of(int small) { return __hsub2(as_h2(kMagic | (uint32_t)small * 0x10001u), as_h2(kMagic)); }      // 0 <= small < 1024
+// byte I of w, 0 .. 255, in both halves as an fp16 integer less BIAS: one byte permutation puts it into the mantissa of 1024
+template <int I, int BIAS = 0>
+__device__ __forceinline__ __half2 h2_byte(uint32_t w) {
+    return __hsub2(as_h2(__byte_perm(w, kMagic, 0x5050u | I * 0x0101u)), as_h2(kMagic + BIAS * 0x10001u));
+}
 
 // the 6-bit scales and minima of a Q4_K / Q5_K header (words 1-3 of the block) as bytes: sub-blocks 0-3 | 4-7 (get_scale_min_k4)
-struct KqScales { uint32_t sc[2], mn[2]; };
-__device__ __forceinline__ KqScales kq_scales(uint32_t w0, uint32_t w1, uint32_t w2) {
-    KqScales k;
-    k.sc[0] = w0 & 0x3f3f3f3fu;
-    k.mn[0] = w1 & 0x3f3f3f3fu;
-    k.sc[1] = (w2 & 0x0f0f0f0fu) | ((w0 >> 2) & 0x30303030u);
-    k.mn[1] = ((w2 >> 4) & 0x0f0f0f0fu) | ((w1 >> 2) & 0x30303030u);
-    return k;
+template <int H>      // four scales or minima as bytes: sub-blocks 0-3 (w: word 0 or 1) or 4-7 (top: word 2's low or high nibbles)
+__device__ __forceinline__ uint32_t kq_six(uint32_t w, uint32_t top) {
+    return H ? (top & 0x0f0f0f0fu) | ((w >> 2) & 0x30303030u) : w & 0x3f3f3f3fu;
 }
 __device__ __forceinline__ int byte_of(uint32_t w, int i) { return (int)((w >> (8 * i)) & 0xffu); }
+
+// two values in a 16-bit type; bf16 as ggml rounds it (subnormals to zero; NaN keeps its upper bits), without branches where there is no NaN or infinity
+__device__ __forceinline__ uint32_t kq_pack16(float a, float b, bool bf16) {
+    if (!bf16) return as_u32(__floats2half2_rn(a, b));
+    float z, fa, fb;
+    asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(fa) : "f"(a));
+    asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(fb) : "f"(b));
+    z = fmaf(a, 0.f, b * 0.f);
+    if (z != z) return (uint32_t)f32_to_bf16_ggml(a) | (uint32_t)f32_to_bf16_ggml(b) << 16;
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(fb), "f"(fa));
+    return d;
+}
 
 struct KqTile { int e, row0, p0, n, sb0, nsb, split; };
 __device__ __forceinline__ KqTile kq_tile(const KqParams& p, int tile) {
@@ -193,6 +218,8 @@ __device__ __forceinline__ KqTile kq_tile(const KqParams& p, int tile) {
         t.sb0 = (int)((long)p.nblk * t.split / p.splits);
         t.nsb = (int)((long)p.nblk * (t.split + 1) / p.splits) - t.sb0;
     }
+    t.e = __shfl_sync(0xffffffffu, t.e, 0); t.row0 = __shfl_sync(0xffffffffu, t.row0, 0); t.p0 = __shfl_sync(0xffffffffu, t.p0, 0); t.n = __shfl_sync(0xffffffffu, t.n, 0);
+    t.sb0 = __shfl_sync(0xffffffffu, t.sb0, 0); t.nsb = __shfl_sync(0xffffffffu, t.nsb, 0);
     return t;
 }
 
@@ -247,7 +274,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
     using C = KqCfg<FMT>;
     constexpr bool Q6 = C::kQ6;
     constexpr int kAccCols = 2 * kKqN, kColA = 2 * kAccCols;      // per matrix: accumulator, minima or the sum of one stage; then the operand stages
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // (known to be uniform: see above)
     if (warp < 16) {
         // ========================================================================== producers
         regs_down<C::kRegsP>();
@@ -273,16 +300,16 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                     if (!Q6) {
                         src += r * C::kRow;
                         const uint4 head = *reinterpret_cast<const uint4*>(src);
-                        const KqScales k = kq_scales(head.y, head.z, head.w);
-                        uint32_t sc = h ? k.sc[1] : k.sc[0];
-#pragma unroll 1
-                        for (int part = 0; part < 2; part++, sc >>= 16) {      // chunk c = 2h + part: low nibbles are sub-block 2c, high nibbles sub-block 2c + 1
+                        const uint32_t sc = h ? kq_six<1>(head.y, head.w) : kq_six<0>(head.y, 0);
+#pragma unroll
+                        for (int part = 0; part < 2; part++) {      // chunk c = 2h + part: low nibbles are sub-block 2c, high nibbles sub-block 2c + 1
+                            const __half2 sl = part ? h2_byte<2>(sc) : h2_byte<0>(sc), sh = part ? h2_byte<3>(sc) : h2_byte<1>(sc);
                             const uint8_t* q = src + C::kRow - 128 + 32 * (2 * h + part);
                             kq_words8(q, q + 16, w);
                             if (FMT == KQ_Q4K) {
 #pragma unroll
                                 for (int i = 0; i < 2; i++) {
-                                    kq_unpack4(w + 4 * i, h2_of(sc & 0xff), h2_of((sc >> 8) & 0xff), o);
+                                    kq_unpack4(w + 4 * i, sl, sh, o);
                                     tmem_st16(dst + 32 * part + 16 * i, o);
                                 }
                             } else {
@@ -290,7 +317,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                                 kq_words8(src + 16, src + 32, qh);
 #pragma unroll
                                 for (int i = 0; i < 2; i++) {
-                                    kq_unpack5(w + 4 * i, qh + 4 * i, 2 * (2 * h + part), h2_of(sc & 0xff), h2_of((sc >> 8) & 0xff), o);
+                                    kq_unpack5(w + 4 * i, qh + 4 * i, 2 * (2 * h + part), sl, sh, o);
                                     tmem_st16(dst + 32 * part + 16 * i, o);
                                 }
                             }
@@ -299,41 +326,52 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                             misc.hdr[mat][it & 1][r] = head.x;
                             uint8_t* m = smem + C::kOffMins + (mat * 2 + (it & 1)) * C::kMins + (r >> 3) * 256 + (r & 7) * 16;      // K-major core matrices of 8 rows x 16 bytes
 #pragma unroll
-                            for (int i = 0; i < 2; i++)
-                                *reinterpret_cast<uint4*>(m + i * 128) = make_uint4(as_u32(h2_of(byte_of(k.mn[i], 0))), as_u32(h2_of(byte_of(k.mn[i], 1))), as_u32(h2_of(byte_of(k.mn[i], 2))),
-                                                                                    as_u32(h2_of(byte_of(k.mn[i], 3))));
+                            for (int i = 0; i < 2; i++) {
+                                const uint32_t mn = i ? kq_six<1>(head.z, head.w >> 4) : kq_six<0>(head.z, 0);
+                                *reinterpret_cast<uint4*>(m + i * 128) = make_uint4(as_u32(h2_byte<0>(mn)), as_u32(h2_byte<1>(mn)), as_u32(h2_byte<2>(mn)), as_u32(h2_byte<3>(mn)));
+                            }
                             fence_async_smem();
                         }
                     } else {
                         // quarter (hh, pp) of the block: elements 128 hh + 32 pp + l (ql low nibbles, qh bits 2 pp) and + 64 (high nibbles, bits 4 + 2 pp), l < 32;
                         // first 32 columns sc * low four bits / 4, last 32 columns sc * (16 * high two bits - 32) / 4; a scale per 16 elements
                         const int hh = h >> 1, pp = h & 1;
-                        const uint2 sc = *reinterpret_cast<const uint2*>(src + kq_q6_word<FMT>(r, 12) + 8 * hh);
+                        const uint2 s8 = *reinterpret_cast<const uint2*>(src + kq_q6_word<FMT>(r, 12) + 8 * hh);
+                        const uint32_t pair = __byte_perm(s8.x, s8.y, pp ? 0x7632 : 0x5410) ^ 0x80808080u;      // scales of (low, i = 0), (low, 1), (high, 0), (high, 1), plus 128
+                        const __half2 sl[2] = {h2_byte<0, 128>(pair), h2_byte<1, 128>(pair)}, sh[2] = {h2_byte<2, 128>(pair), h2_byte<3, 128>(pair)};
                         const __half2 quarter = __float2half2_rn(0.25f);
-                        __half2 sl[2], sh[2];
-#pragma unroll
-                        for (int i = 0; i < 2; i++) {
-                            sl[i] = __hmul2(__half2half2(__int2half_rn((int)(int8_t)((sc.x >> (16 * pp + 8 * i)) & 0xff))), quarter);
-                            sh[i] = __hmul2(__half2half2(__int2half_rn((int)(int8_t)((sc.y >> (16 * pp + 8 * i)) & 0xff))), quarter);
-                        }
                         kq_words8(src + kq_q6_word<FMT>(r, 2 * h), src + kq_q6_word<FMT>(r, 2 * h + 1), w);
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
-                            kq_unpack4(w + 4 * i, sl[i], sh[i], o);
+                            kq_unpack4(w + 4 * i, __hmul2(sl[i], quarter), __hmul2(sh[i], quarter), o);
                             tmem_st16(dst + 16 * i, o);
                         }
                         kq_words8(src + kq_q6_word<FMT>(r, 8 + 2 * hh), src + kq_q6_word<FMT>(r, 9 + 2 * hh), w);
-                        const __half2 m = as_h2(0x64206420u);      // 1024 + 32
-                        const int up = 4 - 2 * pp, down = 2 * pp;   // the two bits moved to bits 4 and 5 of their byte
+                        // 4 sc (b - 2) for the two bits b: in the top mantissa bits of 4 they add b, two places lower in 16 too; 4 sc times that, less 24 sc or 72 sc (exact:
+                        // 9 * 128 has 11 bits).  Bits 0-1 of the even bytes go up by 6, of the odd ones stay; 2-3: 4 up, 4 down; 4-5: 4 up, 4 down; 6-7 stay, 6 down
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
+                            const __half2 l4 = __hmul2(sl[i], __float2half2_rn(4.f)), h4 = __hmul2(sh[i], __float2half2_rn(4.f));
+                            const __half2 l24 = __hmul2(sl[i], __float2half2_rn(-24.f)), l72 = __hmul2(sl[i], __float2half2_rn(-72.f));
+                            const __half2 h24 = __hmul2(sh[i], __float2half2_rn(-24.f)), h72 = __hmul2(sh[i], __float2half2_rn(-72.f));
+                            if (pp == 0) {
 #pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                const uint32_t lo = w[4 * i + j] << up, hi = w[4 * i + j] >> down;
-                                o[4 * j] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(lo), m), sl[i]));
-                                o[4 * j + 1] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(lo >> 8), m), sl[i]));
-                                o[4 * j + 2] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(hi), m), sh[i]));
-                                o[4 * j + 3] = as_u32(__hmul2(__hsub2(magic_and<0x00300030u>(hi >> 8), m), sh[i]));
+                                for (int j = 0; j < 4; j++) {
+                                    const uint32_t a = w[4 * i + j];
+                                    o[4 * j] = as_u32(__hfma2(bits_at6(a << 6), l4, l72));
+                                    o[4 * j + 1] = as_u32(__hfma2(bits_at8(a), l4, l24));
+                                    o[4 * j + 2] = as_u32(__hfma2(bits_at8(a << 4), h4, h24));
+                                    o[4 * j + 3] = as_u32(__hfma2(bits_at8(a >> 4), h4, h24));
+                                }
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 4; j++) {
+                                    const uint32_t a = w[4 * i + j];
+                                    o[4 * j] = as_u32(__hfma2(bits_at6(a << 4), l4, l72));
+                                    o[4 * j + 1] = as_u32(__hfma2(bits_at6(a >> 4), l4, l72));
+                                    o[4 * j + 2] = as_u32(__hfma2(bits_at6(a), h4, h72));
+                                    o[4 * j + 3] = as_u32(__hfma2(bits_at8(a >> 6), h4, h24));
+                                }
                             }
                             tmem_st16(dst + 32 + 16 * i, o);
                         }
@@ -350,8 +388,9 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
     } else if (warp < 20) {
         if (warp == 16) {
             // ====================================================================== activations
-            if (lane == 0) {
-                tma_prefetch_desc(&maps.q);
+            const bool one = lane == 0;
+            if (one) tma_prefetch_desc(&maps.q);
+            {
                 unsigned it = 0;
                 for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                     const KqTile t = kq_tile(p, tile);
@@ -359,24 +398,30 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                     for (int s = 0; s < t.nsb; s++, it++) {
                         const int b = it & 1, sb = t.sb0 + s;
                         bar_wait(smem_u32(&misc.b_free[b]), ((it >> 1) & 1) ^ 1);
-                        const uint32_t full = smem_u32(&misc.b_full[b]);
-                        bar_expect_tx(full, groups * 32 * (Q6 ? 512 : 544));
-                        for (int g = 0; g < groups; g++) {
-#pragma unroll
-                            for (int c = 0; c < 4; c++) tma_load_2d(base + b * C::kB + c * (kKqN * 128) + g * 4096, &maps.q, full, sb * 256 + c * 64, t.p0 + 32 * g);
-                            if (!Q6) tma_load_2d(base + C::kOffSums + b * C::kSums + g * 1024, &maps.sums, full, sb * 16, t.p0 + 32 * g);
-                        }
                         const int d = it & 3;
+                        if (one) {
+                            const uint32_t full = smem_u32(&misc.b_full[b]);
+                            bar_expect_tx(full, groups * 32 * (Q6 ? 512 : 544));
+                            for (int g = 0; g < groups; g++) {
+#pragma unroll
+                                for (int c = 0; c < 4; c++) tma_load_2d(base + b * C::kB + c * (kKqN * 128) + g * 4096, &maps.q, full, sb * 256 + c * 64, t.p0 + 32 * g);
+                                if (!Q6) tma_load_2d(base + C::kOffSums + b * C::kSums + g * 1024, &maps.sums, full, sb * 16, t.p0 + 32 * g);
+                            }
+                        }
                         bar_wait(smem_u32(&misc.dx_free[d]), ((it >> 2) & 1) ^ 1);
-                        bar_expect_tx(smem_u32(&misc.dx_full[d]), kKqN * 4);
-                        kq_bulk(smem_u32(&misc.dx[d][0]), p.dx + (long)sb * p.dpitch + t.p0, kKqN * 4, smem_u32(&misc.dx_full[d]));
+                        if (one) {
+                            bar_expect_tx(smem_u32(&misc.dx_full[d]), kKqN * 4);
+                            kq_bulk(smem_u32(&misc.dx[d][0]), p.dx + (long)sb * p.dpitch + t.p0, kKqN * 4, smem_u32(&misc.dx_full[d]));
+                        }
+                        __syncwarp();
                     }
                 }
             }
             __syncwarp();
         } else if (warp == 19) {
             // ====================================================================== weights: the blocks of 2 x 128 rows as they lie in memory
-            if (lane == 0) {
+            const bool one = lane == 0;
+            {
                 int slot = 0, sphase = 1;
                 for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
                     const KqTile t = kq_tile(p, tile);
@@ -384,21 +429,24 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                     for (int s = 0; s < t.nsb; s++) {
                         const int sb = t.sb0 + s;
                         bar_wait(smem_u32(&misc.raw_free[slot]), sphase);
-                        const uint32_t full = smem_u32(&misc.raw_full[slot]);
-                        bar_expect_tx(full, C::kSlot);
+                        if (one) {
+                            const uint32_t full = smem_u32(&misc.raw_full[slot]);
+                            bar_expect_tx(full, C::kSlot);
 #pragma unroll
-                        for (int mat = 0; mat < 2; mat++) {
-                            const uint32_t dst = base + C::kOffRing + slot * C::kSlot + mat * C::kMat;
-                            const CUtensorMap* m = maps.w[mat];
-                            const int r0 = row + (p.pair ? 0 : 128 * mat);
-                            if (!Q6) tma_load_2d(dst, m, full, sb * C::kRow, r0);
-                            else if (FMT == KQ_Q6K_T4) tma_load_5d(dst, m, full, 0, sb, 0, 0, r0 >> 2);
-                            else {
-                                tma_load_3d(dst, m, full, sb * 128, 0, r0 >> 3);
-                                tma_load_3d(dst + 128 * 128, m + 1, full, sb * 64, 0, r0 >> 3);
-                                tma_load_3d(dst + 128 * 192, m + 2, full, sb * 16, 0, r0 >> 3);
+                            for (int mat = 0; mat < 2; mat++) {
+                                const uint32_t dst = base + C::kOffRing + slot * C::kSlot + mat * C::kMat;
+                                const CUtensorMap* m = maps.w[mat];
+                                const int r0 = row + (p.pair ? 0 : 128 * mat);
+                                if (!Q6) tma_load_2d(dst, m, full, sb * C::kRow, r0);
+                                else if (FMT == KQ_Q6K_T4) tma_load_5d(dst, m, full, 0, sb, 0, 0, r0 >> 2);
+                                else {
+                                    tma_load_3d(dst, m, full, sb * 128, 0, r0 >> 3);
+                                    tma_load_3d(dst + 128 * 128, m + 1, full, sb * 64, 0, r0 >> 3);
+                                    tma_load_3d(dst + 128 * 192, m + 2, full, sb * 16, 0, r0 >> 3);
+                                }
                             }
                         }
+                        __syncwarp();
                         if (++slot == C::kRing) { slot = 0; sphase ^= 1; }
                     }
                 }
@@ -552,25 +600,33 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                     bar_arrive(smem_u32(&misc.dx_free[it & 3]));
                 }
             }
-            if (row < p.R) {
-                if (p.y) {
-                    const float b = p.bias ? p.bias[row] : 0.f;
-                    const int n = p.bsz ? min(t.n, *p.bsz - p.t0 - t.p0) : t.n;
-                    const long at = (long)t.p0 * p.R + row;
-                    auto put = [&](int type) {
+            // eight tokens at a time in a rolled loop, the sums moving down to its registers, and no branch per value: with ggml's rounding in branches a tile's output took
+            // 11,000 cycles, half of a tile of 6 blocks; now 5,500
+            int left = t.n;
+            if (p.y && p.bsz) left = min(left, *p.bsz - p.t0 - t.p0);
+            if (row >= p.R) left = 0;
+            const float bias = p.y && p.bias && left > 0 ? p.bias[row] : 0.f;
+            const int type = p.y ? p.hidden_type : KTB200_TYPE_F32;
+            const long first = ((long)t.split * p.T + t.p0) * p.R;
+            uint8_t* const out = reinterpret_cast<uint8_t*>(p.y ? p.y : p.out[mat]) + (type == KTB200_TYPE_F32 ? 4 : 2) * first;
+            uint32_t at = (uint32_t)row;
+#pragma unroll 1
+            for (; left > 0; left -= 8) {
+                if (type == KTB200_TYPE_F32) {
 #pragma unroll
-                        for (int i = 0; i < kKqN; i++)
-                            if (i < n) store_hidden(p.y, at + (long)i * p.R, type, half_of(acc[i >> 1], i & 1) + b);
-                    };
-                    if (p.hidden_type == KTB200_TYPE_BF16) put(KTB200_TYPE_BF16);
-                    else if (p.hidden_type == KTB200_TYPE_F16) put(KTB200_TYPE_F16);
-                    else put(KTB200_TYPE_F32);
+                    for (int i = 0; i < 8; i++)
+                        if (i < left) reinterpret_cast<float*>(out)[at + (uint32_t)(i * p.R)] = half_of(acc[i >> 1], i & 1) + bias;
                 } else {
-                    float* out = p.out[mat] + ((long)t.split * p.T + t.p0) * p.R + row;
 #pragma unroll
-                    for (int i = 0; i < kKqN; i++)
-                        if (i < t.n) out[(long)i * p.R] = half_of(acc[i >> 1], i & 1);
+                    for (int i = 0; i < 8; i += 2) {
+                        const uint32_t v = kq_pack16(half_of(acc[i >> 1], 0) + bias, half_of(acc[i >> 1], 1) + bias, type == KTB200_TYPE_BF16);
+                        if (i < left) reinterpret_cast<uint16_t*>(out)[at + (uint32_t)(i * p.R)] = (uint16_t)v;
+                        if (i + 1 < left) reinterpret_cast<uint16_t*>(out)[at + (uint32_t)((i + 1) * p.R)] = (uint16_t)(v >> 16);
+                    }
                 }
+                at += 8u * p.R;
+#pragma unroll
+                for (int n = 0; n + 4 < kKqN / 2; n++) acc[n] = acc[n + 4];
             }
         }
     }
@@ -584,7 +640,7 @@ __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
     KqMisc& misc = *reinterpret_cast<KqMisc*>(smem + C::kOffMisc);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int total = p.n_tiles ? *p.n_tiles * p.tiles_mul : p.total;
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
@@ -600,7 +656,7 @@ __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = misc.tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, misc.tmem_base, 0);
 
     kq_roles<FMT, MARKS>(maps, p, smem, misc, base, tmem, total);
     tc_fence_before();

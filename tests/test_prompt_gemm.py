@@ -94,6 +94,34 @@ def test_k_quant_prompt_batches(type, T, K, R, hid):
     lib.ktb200_linear_destroy(h)
 
 
+# results that are infinite, not numbers or subnormal leave as ggml rounds fp32 to bf16 (subnormals to zero, a NaN keeps its upper bits): the same sums in fp32, rounded here.
+# 17 and 70 tokens: a partly filled group of eight at a tile's end, in the first tile and in a second; 1538 rows: two in the last tile
+@pytest.mark.parametrize("T", [17, 70])
+def test_k_quant_prompt_batches_round_special_results(T):
+    K, R = 256, 1538
+    blocks = synth_blocks(Q4_K, R * K, "cuda", T).view(R, 144)
+    d = blocks[:, 0:2].view(torch.int16)
+    d[0], d[1], d[2], d[R - 2], d[R - 1] = 0x7c00, 0x7e01, 1, 0x7c00, 1        # infinity, NaN, the smallest subnormal scale
+    blocks[torch.tensor([2, R - 1]), 2:4] = 0
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, K), generator=g, device="cuda").bfloat16()
+    x[3], x[T - 1] = x[3] * 2.0 ** -112, x[T - 1] * 2.0 ** -112
+    lib, ys = native.lib(), {}
+    for hid in (F32, BF16):
+        h, xt = C.c_void_p(), x.to(TORCH[hid])
+        y = ys[hid] = torch.zeros((T, R), dtype=TORCH[hid], device="cuda")
+        native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), Q4_K, hid, T, 0, C.byref(h)))
+        native.check(lib.ktb200_linear_load_weights(h, _stream()))
+        native.check(lib.ktb200_linear_forward(h, T, xt.data_ptr(), y.data_ptr(), None, None, _stream()))
+        torch.cuda.synchronize()
+        lib.ktb200_linear_destroy(h)
+    i = ys[F32].view(torch.int32).long() & 0xffffffff
+    size = i & 0x7fffffff
+    want = torch.where(size > 0x7f800000, (i >> 16) | 64, torch.where(size < 0x00800000, (i >> 31) << 15, (i + 0x7fff + ((i >> 16) & 1)) >> 16))
+    assert (size > 0x7f800000).any() and (size == 0x7f800000).any() and ((size > 0) & (size < 0x00800000)).any()
+    assert torch.equal(ys[BF16].view(torch.int16).long() & 0xffff, want)
+
+
 # experts with no token, one token, 64, 65 and all tokens; an expert named twice by a token and ids beyond the experts; gate and up of one
 # 128-row tile and of several; down in both layouts
 @pytest.mark.parametrize("gu,down,H,I,T", [(Q4_K, Q6_K, 256, 256, 48), (Q4_K, Q4_K, 512, 256, 131), (Q4_K, Q6_K, 1024, 768, 200), (Q4_K, Q6_K, 2048, 512, 1100), (Q5_K, Q5_K, 768, 512, 100),
