@@ -24,17 +24,20 @@
 //     weights.  The pairs come out as (0, 2), (1, 3) of four; the activations are stored in that order (kq_pos4).
 //   * a scale per 256-block needs the accumulator drained per 256-block: two matrices of 128 rows per CTA (gate and up of the same experts, or
 //     256 rows of one) take turns, one drained while the other multiplies, and share the activation tiles.
-// CTA: 28 warps in 7 groups of 4.  Groups 0-3 producers: (matrix 0, first operand stage), (matrix 1, first), (0, second), (1, second), a warp = 32 rows:
+// CTA: 28 warps in 7 groups of 4.  Groups 0-3 producers: (matrix 0, first operand stage), (matrix 1, first), (0, second), (1, second), a warp = 32 rows, a stage in
+//      two parts of 32 columns that are filled, multiplied and given back by themselves (whole stages: 129 us for the linear below, 2,640 for the experts):
 //      raw blocks from a TMA ring -> registers -> TMEM; warp 16 TMA of activations, 17 / 18 MMA issuers of matrix 0 / 1, 19 TMA of weights;
 //      groups 5 / 6 epilogue of matrix 0 / 1.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
 //      warps took a third of the issue slots, and the four roles' code is kept in rolled loops: unrolled it overran the instruction cache (10,000
 //      cycles for a block of two matrices).  The warp's number and what the tiles say come through a shuffle, so that the compiler knows them to be the same in all
 //      lanes and keeps a role's state, its branches and the MMAs' operands off the vector pipes (the other roles' share of the issue slots is what an issuer or
 //      an epilogue warp waits for: 157 -> 129 us for the linear below, 2,782 -> 2,600 for the experts; 268 -> 69 branch instructions a block).
-//      A block of two matrices takes 3,150 cycles at 64 tokens a tile (3,440 before), 1,970 at 16 (2,480); HBM brings one every 1,550.  Of the 3,150 the drain of an accumulator is
+//      A block of two matrices takes 3,100 cycles at 64 tokens a tile (3,440 before), 1,890 at 16 (2,480; Q6_K 3,570, 4,120); HBM brings one every 1,550 (Q6_K 2,270).  Of the 3,150 the drain of an accumulator is
 //      1,500 (producers issue beside it; 660 alone), the eight MMAs of either stage 600, the rest hand-overs.  Draining in two halves of the tokens, so that one is multiplied
 //      while the other is drained, was slower (140 us, 2,770), and so were both matrices' drains in one thread (244) and other orders of the roles (165).
-//      Measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 2,950 -> 2,640 us (the operator's call); Q4_K linear 777 x 1536 -> 24576 182 -> 129 us (455 TFLOP/s).
+//      At 16 tokens the schedulers issue three instructions of four possible ones a cycle, nearly all of them the producers'; their share of polls and address arithmetic is small
+//      (every producer warp polling for itself, barrier addresses in registers: within 1 %).
+//      Measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 2,910 -> 2,540 us (the operator's call); Q4_K linear 777 x 1536 -> 24576 180 -> 126 us (466 TFLOP/s).
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
 #include <algorithm>
 #include <atomic>
@@ -65,7 +68,7 @@ struct KqCfg {
     static constexpr int kOffSums = kOffMins + 4 * kMins, kSums = kQ6 ? 0 : kKqN * 32, kOffMisc = kOffSums + 2 * kSums;
 };
 struct KqMisc {
-    unsigned long long b_full[2], b_free[2], dx_full[4], dx_free[4], raw_full[3], raw_free[3], a_full[2][2], a_free[2][2], acc_full[2], acc_free[2], hdr_free[2][2];
+    unsigned long long b_full[2], b_free[2], dx_full[4], dx_free[4], raw_full[3], raw_free[3], a_full[2][2][2], a_free[2][2][2], acc_full[2], acc_free[2], hdr_free[2][2];
     uint32_t tmem_base, marked[2], pad;      // marked: whether the matrix's block is summed stage by stage
     float dx[4][kKqN];
     uint32_t hdr[2][2][128];      // Q4_K, Q5_K: half2 (d, dmin) of a row's block
@@ -111,41 +114,29 @@ __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 
 __device__ __forceinline__ void kq_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// D[tmem] (+)= A[tmem] . B[smem], fp16: A's lane = row, a 32-bit column = two consecutive K; K = 16 per instruction.  Eight of them on consecutive
-// 8-column slices of A, against the four 32-byte steps of a 64-wide B tile and of the tile `next` (in descriptor units) behind it.  One election.
-__device__ __forceinline__ void mma_f16_ta8(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint64_t next, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] . B[smem], fp16: A's lane = row, a 32-bit column = two consecutive K; K = 16 per instruction.  Four of them on consecutive
+// 8-column slices of A, against the four 32-byte steps of a 64-wide B tile.  One election.
+__device__ __forceinline__ void mma_f16_ta4(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n"
         ".reg .pred p, q, t;\n"
         ".reg .b32 r, a;\n"
         ".reg .b64 b;\n"
         "elect.sync r|q, 0xffffffff;\n"
-        "setp.ne.b32 p, %5, 0;\n"
+        "setp.ne.b32 p, %4, 0;\n"
         "setp.eq.b32 t, 0, 0;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, p;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
         "add.u32 a, %1, 8;\n"
         "add.u64 b, %2, 2;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
         "add.u32 a, %1, 16;\n"
         "add.u64 b, %2, 4;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
         "add.u32 a, %1, 24;\n"
         "add.u64 b, %2, 6;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
-        "add.u32 a, %1, 32;\n"
-        "add.u64 b, %2, %3;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
-        "add.u32 a, %1, 40;\n"
-        "add.u64 b, b, 2;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
-        "add.u32 a, %1, 48;\n"
-        "add.u64 b, b, 2;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
-        "add.u32 a, %1, 56;\n"
-        "add.u64 b, b, 2;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %4, t;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
         "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(desc_b), "l"(next), "r"(idesc), "r"(accumulate)
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // the elected lane of a converged warp leaves `value` for those who wait for `bar`, and arrives there
@@ -218,8 +209,8 @@ __device__ __forceinline__ KqTile kq_tile(const KqParams& p, int tile) {
         t.sb0 = (int)((long)p.nblk * t.split / p.splits);
         t.nsb = (int)((long)p.nblk * (t.split + 1) / p.splits) - t.sb0;
     }
-    t.e = __shfl_sync(0xffffffffu, t.e, 0); t.row0 = __shfl_sync(0xffffffffu, t.row0, 0); t.p0 = __shfl_sync(0xffffffffu, t.p0, 0); t.n = __shfl_sync(0xffffffffu, t.n, 0);
-    t.sb0 = __shfl_sync(0xffffffffu, t.sb0, 0); t.nsb = __shfl_sync(0xffffffffu, t.nsb, 0);
+    t.e = uniform(t.e); t.row0 = uniform(t.row0); t.p0 = uniform(t.p0); t.n = uniform(t.n);
+    t.sb0 = uniform(t.sb0); t.nsb = uniform(t.nsb);
     return t;
 }
 
@@ -274,7 +265,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
     using C = KqCfg<FMT>;
     constexpr bool Q6 = C::kQ6;
     constexpr int kAccCols = 2 * kKqN, kColA = 2 * kAccCols;      // per matrix: accumulator, minima or the sum of one stage; then the operand stages
-    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // (known to be uniform: see above)
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);      // (known to be uniform: see above)
     if (warp < 16) {
         // ========================================================================== producers
         regs_down<C::kRegsP>();
@@ -287,15 +278,24 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
             const int nsb = kq_tile(p, tile).nsb;
             for (int s = 0; s < nsb; s++, it++) {
                 const uint8_t* src = smem + C::kOffRing + slot * C::kSlot + mat * C::kMat;
-                if (leader) bar_wait(smem_u32(&misc.raw_full[slot]), sphase);
+                bar_wait(smem_u32(&misc.raw_full[slot]), sphase);
 #pragma unroll 1
                 for (int h = half; h < C::kStages; h += 2, uses++) {
-                    if (leader) {
-                        bar_wait(smem_u32(&misc.a_free[mat][half]), (uses & 1) ^ 1);
-                        if (!Q6 && !half) bar_wait(smem_u32(&misc.hdr_free[mat][it & 1]), ((it >> 1) & 1) ^ 1);
-                    }
-                    group_sync(1 + grp);
-                    tc_fence_after();
+                    // either part of an operand stage is free, is filled and goes to the issuer by itself: one is multiplied while the other is filled
+                    auto open = [&](int part) {
+                        if (leader) {
+                            bar_wait(smem_u32(&misc.a_free[mat][half][part]), (uses & 1) ^ 1);
+                            if (!Q6 && !half && part) bar_wait(smem_u32(&misc.hdr_free[mat][it & 1]), ((it >> 1) & 1) ^ 1);
+                        }
+                        group_sync(1 + grp);
+                        tc_fence_after();
+                    };
+                    auto close = [&](int part) {
+                        tmem_wait_st();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) bar_arrive(smem_u32(&misc.a_full[mat][half][part]));
+                    };
                     uint32_t w[8], o[16];
                     if (!Q6) {
                         src += r * C::kRow;
@@ -306,6 +306,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                             const __half2 sl = part ? h2_byte<2>(sc) : h2_byte<0>(sc), sh = part ? h2_byte<3>(sc) : h2_byte<1>(sc);
                             const uint8_t* q = src + C::kRow - 128 + 32 * (2 * h + part);
                             kq_words8(q, q + 16, w);
+                            open(part);
                             if (FMT == KQ_Q4K) {
 #pragma unroll
                                 for (int i = 0; i < 2; i++) {
@@ -321,16 +322,17 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                                     tmem_st16(dst + 32 * part + 16 * i, o);
                                 }
                             }
-                        }
-                        if (!half) {      // this group also hands on (d, dmin) and the minima, each twice, against the sixteen 16-value activation sums
-                            misc.hdr[mat][it & 1][r] = head.x;
-                            uint8_t* m = smem + C::kOffMins + (mat * 2 + (it & 1)) * C::kMins + (r >> 3) * 256 + (r & 7) * 16;      // K-major core matrices of 8 rows x 16 bytes
+                            if (part && !half) {      // this group also hands on (d, dmin) and the minima, each twice, against the sixteen 16-value activation sums
+                                misc.hdr[mat][it & 1][r] = head.x;
+                                uint8_t* m = smem + C::kOffMins + (mat * 2 + (it & 1)) * C::kMins + (r >> 3) * 256 + (r & 7) * 16;      // K-major core matrices of 8 rows x 16 bytes
 #pragma unroll
-                            for (int i = 0; i < 2; i++) {
-                                const uint32_t mn = i ? kq_six<1>(head.z, head.w >> 4) : kq_six<0>(head.z, 0);
-                                *reinterpret_cast<uint4*>(m + i * 128) = make_uint4(as_u32(h2_byte<0>(mn)), as_u32(h2_byte<1>(mn)), as_u32(h2_byte<2>(mn)), as_u32(h2_byte<3>(mn)));
+                                for (int i = 0; i < 2; i++) {
+                                    const uint32_t mn = i ? kq_six<1>(head.z, head.w >> 4) : kq_six<0>(head.z, 0);
+                                    *reinterpret_cast<uint4*>(m + i * 128) = make_uint4(as_u32(h2_byte<0>(mn)), as_u32(h2_byte<1>(mn)), as_u32(h2_byte<2>(mn)), as_u32(h2_byte<3>(mn)));
+                                }
+                                fence_async_smem();
                             }
-                            fence_async_smem();
+                            close(part);
                         }
                     } else {
                         // quarter (hh, pp) of the block: elements 128 hh + 32 pp + l (ql low nibbles, qh bits 2 pp) and + 64 (high nibbles, bits 4 + 2 pp), l < 32;
@@ -341,12 +343,15 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                         const __half2 sl[2] = {h2_byte<0, 128>(pair), h2_byte<1, 128>(pair)}, sh[2] = {h2_byte<2, 128>(pair), h2_byte<3, 128>(pair)};
                         const __half2 quarter = __float2half2_rn(0.25f);
                         kq_words8(src + kq_q6_word<FMT>(r, 2 * h), src + kq_q6_word<FMT>(r, 2 * h + 1), w);
+                        open(0);
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
                             kq_unpack4(w + 4 * i, __hmul2(sl[i], quarter), __hmul2(sh[i], quarter), o);
                             tmem_st16(dst + 16 * i, o);
                         }
                         kq_words8(src + kq_q6_word<FMT>(r, 8 + 2 * hh), src + kq_q6_word<FMT>(r, 9 + 2 * hh), w);
+                        close(0);
+                        open(1);
                         // 4 sc (b - 2) for the two bits b: in the top mantissa bits of 4 they add b, two places lower in 16 too; 4 sc times that, less 24 sc or 72 sc (exact:
                         // 9 * 128 has 11 bits).  Bits 0-1 of the even bytes go up by 6, of the odd ones stay; 2-3: 4 up, 4 down; 4-5: 4 up, 4 down; 6-7 stay, 6 down
 #pragma unroll
@@ -375,11 +380,8 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                             }
                             tmem_st16(dst + 32 + 16 * i, o);
                         }
+                        close(1);
                     }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(smem_u32(&misc.a_full[mat][half]));
                 }
                 if (lane == 0) bar_arrive(smem_u32(&misc.raw_free[slot]));
                 if (++slot == C::kRing) { slot = 0; sphase ^= 1; }
@@ -475,27 +477,29 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                     uint64_t bd = smem_desc(base + b * C::kB, 16, 1024, kLayoutSw128);      // (the address field counts 16 bytes, and nothing carries out of it)
                     const uint64_t md = smem_desc(base + C::kOffMins + (mat * 2 + b) * C::kMins, 128, 256, kLayoutNone), sd = smem_desc(base + C::kOffSums + b * C::kSums, 16, 256, kLayoutSw32);
                     constexpr uint64_t kStep = kKqN * 128 >> 4;      // Q6_K: both terms of a quarter's 64 weights meet one tile of activations
+                    // the two parts of stage h into d, from nothing or from what it holds
+                    auto stage = [&](int h, uint32_t d, bool add) {
+#pragma unroll 1
+                        for (int part = 0; part < 2; part++) {
+                            bar_wait(smem_u32(&misc.a_full[mat][h & 1][part]), uses & 1);
+                            tc_fence_after();
+                            mma_f16_ta4(d, a0 + (h & 1) * 64 + part * 32, bd, idesc, add || part);
+                            if (!Q6 || part) bd += kStep;
+                            mma_commit(smem_u32(&misc.a_free[mat][h & 1][part]));
+                        }
+                        if (h & 1) uses++;
+                    };
                     if (!marked) {
 #pragma unroll 1
                         for (int h = 0; h < C::kStages; h++) {
-                            bar_wait(smem_u32(&misc.a_full[mat][h & 1]), uses & 1);
-                            tc_fence_after();
-                            mma_f16_ta8(acc, a0 + (h & 1) * 64, bd, Q6 ? 0 : kStep, idesc, h);
-                            bd += (Q6 ? 1 : 2) * kStep;
+                            stage(h, acc, h);
                             if (!Q6 && h == 0) mma_f16(acc + kKqN, md, sd, idesc, 0);
-                            mma_commit(smem_u32(&misc.a_free[mat][h & 1]));
-                            if (h & 1) uses++;
                         }
                     } else {      // the first stage's sum in the accumulator, each other one behind it, where the epilogue adds it; the minima's product last
 #pragma unroll 1
                         for (int h = 0; h < C::kStages; h++) {
-                            bar_wait(smem_u32(&misc.a_full[mat][h & 1]), uses & 1);
                             if (h > 1) taken();
-                            tc_fence_after();
-                            mma_f16_ta8(acc + (h ? kKqN : 0), a0 + (h & 1) * 64, bd, Q6 ? 0 : kStep, idesc, 0);
-                            bd += (Q6 ? 1 : 2) * kStep;
-                            mma_commit(smem_u32(&misc.a_free[mat][h & 1]));
-                            if (h & 1) uses++;
+                            stage(h, acc + (h ? kKqN : 0), false);
                             if (h && h < C::kStages - Q6) give();
                         }
                         if (!Q6) {
@@ -640,13 +644,16 @@ __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
     KqMisc& misc = *reinterpret_cast<KqMisc*>(smem + C::kOffMisc);
-    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int tid = threadIdx.x, warp = uniform(tid >> 5);
     const int total = p.n_tiles ? *p.n_tiles * p.tiles_mul : p.total;
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
             bar_init(smem_u32(&misc.b_full[i]), 1); bar_init(smem_u32(&misc.b_free[i]), 2);
             bar_init(smem_u32(&misc.acc_full[i]), MARKS ? 2 : 1); bar_init(smem_u32(&misc.acc_free[i]), 4);
-            for (int j = 0; j < 2; j++) { bar_init(smem_u32(&misc.a_full[i][j]), 4); bar_init(smem_u32(&misc.a_free[i][j]), 1); bar_init(smem_u32(&misc.hdr_free[i][j]), 4); }
+            for (int j = 0; j < 2; j++) {
+                for (int k = 0; k < 2; k++) { bar_init(smem_u32(&misc.a_full[i][j][k]), 4); bar_init(smem_u32(&misc.a_free[i][j][k]), 1); }
+                bar_init(smem_u32(&misc.hdr_free[i][j]), 4);
+            }
         }
         for (int i = 0; i < 4; i++) { bar_init(smem_u32(&misc.dx_full[i]), 1); bar_init(smem_u32(&misc.dx_free[i]), 8); }
         for (int i = 0; i < C::kRing; i++) { bar_init(smem_u32(&misc.raw_full[i]), 1); bar_init(smem_u32(&misc.raw_free[i]), 16); }
@@ -656,7 +663,7 @@ __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, misc.tmem_base, 0);
+    const uint32_t tmem = uniform(misc.tmem_base);
 
     kq_roles<FMT, MARKS>(maps, p, smem, misc, base, tmem, total);
     tc_fence_before();

@@ -10,6 +10,10 @@
 namespace ktb {
 namespace umma {
 
+// a value that is the same in all lanes of a converged warp, known as such to the compiler: what follows from it stays in uniform registers, where the operands of TMA and
+// tcgen05 instructions have to be anyway, and branches on it need no reconvergence
+template <typename T>
+__device__ __forceinline__ T uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // ---------------------------------------------------------------------------------------------- mbarrier
