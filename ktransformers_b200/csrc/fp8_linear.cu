@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constan
     uint8_t* smem = smem_raw + (base - raw);
     Fp8Misc& misc = *reinterpret_cast<Fp8Misc*>(smem + kFOffMisc);
     float* a_s = reinterpret_cast<float*>(smem + kFOffS);   // [kFT][kb_per_split]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);
     const int row0 = blockIdx.x * 128;
     const int kb0 = blockIdx.y * p.kb_per_split, nk = min(p.kb_per_split, p.nkb - kb0);
     if (tid == 0) {
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = misc.tmem_base;
+    const uint32_t tmem = uniform(misc.tmem_base);
     griddep_launch_dependents();   // a PDL-launched successor may set up and prefetch its own weights while this grid streams
 
     if (warp == 0) {
@@ -246,6 +246,9 @@ __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constan
 //     lanes are tokens, so the token scale is a register and acc += dot * (a_s * b_s) is ONE fma per value and 128 of K.
 //     Two TMEM buffers of BN columns: the MMAs of one K block run while the block before it is promoted.
 // BN: 256 leaves the tensor pipe shared-memory headroom (96 of 128 B per cycle); 128 and 64 keep the chip full when there are few tiles.
+// The roles are known to be uniform (umma.cuh): 351 -> 333 us for 2000 tokens, 7168 -> 18432 (the kernel above, one token 16384 -> 7168: 34.1 -> 32.7); a wave brings
+// 48 KB per 128 x 256 x 128 products through L2, 11 TB/s in all, which is near what L2 gives.  Longer loads from tensor memory with double buffers, two
+// products per instruction and more registers for them made it 340-460 us.
 // Tiles run token tile fastest inside groups of kFGroupM, so that the CTAs of a wave share the weight rows and the tokens through L2.
 constexpr int kFGemmThreads = 320, kFGroupM = 16, kFGemmRing = 192 * 1024, kFGemmTokens = 4096;
 struct Fp8GemmMisc {
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     Fp8GemmMisc& misc = *reinterpret_cast<Fp8GemmMisc*>(smem_raw + (base - raw) + kFGemmRing);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);
     if (tid == 0) {
         for (int s = 0; s < kStages; s++) { bar_init(smem_u32(&misc.full[s]), 1); bar_init(smem_u32(&misc.free[s]), 1); }
         for (int b = 0; b < 2; b++) { bar_init(smem_u32(&misc.d_full[b]), 1); bar_init(smem_u32(&misc.d_free[b]), 8); }
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = misc.tmem_base;
+    const uint32_t tmem = uniform(misc.tmem_base);
     const int tiles = p.mt * p.nt;
     auto place = [&](int tile, int& m0, int& n0) {      // groups of kFGroupM token tiles; inside a group the token tile is fastest
         const int per = kFGroupM * p.nt, g = tile / per, r = tile - g * per, gm = min(kFGroupM, p.mt - g * kFGroupM);

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
     uint8_t* smem = tc_smem + (base - raw);
     const uint32_t kbase = base + 2 * kTcTile, vbase = base + 4 * kTcTile;
     TcMisc& misc = *reinterpret_cast<TcMisc*>(smem + 6 * kTcTile);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);
     const int RH = a.RH, TOKS = 128 / RH, R = a.H / a.G, hblocks = R / RH;
     if (tid == 0) {      // which sequence portion and which of its tokens this CTA covers; the last tiles, which see most keys, come first
         int b = gridDim.y - 1 - blockIdx.y, found = -1, off = 0, len = 0;
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = misc.tmem_base;
+    const uint32_t tmem = uniform(misc.tmem_base);
     const int tok0 = misc.info[1], ntok = misc.info[2];
     const int g = blockIdx.x / hblocks, h0 = g * R + (blockIdx.x % hblocks) * RH;
     const int pos0 = a.pos[tok0], max_pos = pos0 + ntok - 1, lo = first_visible(pos0, a.window, a.chunk);
