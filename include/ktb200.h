@@ -168,6 +168,8 @@ int ktb200_mlp_forward(ktb200_mlp* mlp, int qlen, const void* input_dev, void* o
 int ktb200_moe_forward_shared(ktb200_moe* moe, ktb200_mlp* shared, int qlen, int k, const int64_t* expert_ids_dev,
                               const float* weights_dev, const void* input_dev, void* output_dev,
                               const int* bsz_tensor_dev, void* stream);
+/* 1 when these two calls run a batch of qlen tokens as per-expert tensor-core GEMMs (and `shared` as a call of its own), 0 when through the row kernels */
+int ktb200_moe_takes_gemms(const ktb200_moe* moe, const ktb200_mlp* shared, int qlen, int k);
 
 /* ------------------------------------------------------------------------------------------
  * Activation quantisation exposed for parity tests: from_float(x, Q8_K | Q8_0)

@@ -1,5 +1,7 @@
 // Routed experts, dense linear and gated MLP on the streaming integer GEMV kernels (gemv.cuh).
 // C-ABI entry points declared in include/ktb200.h.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -576,12 +578,29 @@ bool grouped_ok(const ktb200_moe* m, int k);
 int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, const float* weights, const void* input, void* output, const int* bsz, cudaStream_t s);
 }
 }
-// qlen from which the per-expert tensor-core GEMMs (grouped.cu) replace the per-pair GEMV kernels: the reference makes the
-// same split between MOE::forward_one and MOE::forward_many (moe.cpp:367-377, threshold group_min_len)
-static int grouped_min_qlen() {
-    static const int v = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : 48; }();
-    return v;
+// Whether a batch runs as per-expert tensor-core GEMMs (grouped.cu), which read an expert's weights once per 64 of its tokens, or through the row kernels, once per
+// (token, expert) pair: the reference makes the same split between MOE::forward_one and MOE::forward_many (moe.cpp:367-377, threshold group_min_len).
+// KTB200_GROUPED_MIN fixes the line; else up to 8 tokens the row kernels, from 48 the GEMMs, and between them what is expected to take less time.  Measured (us):
+//   row kernels  20 + pairs (and a shared expert's rows with them) x (0.83 ns a row of gate and up, of Q6_K 1.4, + 1.1 ns for four rows of down)
+//   GEMMs        85 (ten launches: 55 on the device and some more host work; a shared expert, a GEMM each of its own, 30 more) + 1.15 x the rounds of tiles x
+//                their blocks x 1,900 cycles (Q5_K 2,200, Q6_K 3,570) for the experts that the batch is expected to hit
+//   256 experts of 2048 x 7168, 8 chosen: 12 tokens 534 against 640, 16: 700 against 764, 24: 1041 against 1023, 40: 1722 against 1313;  64 of 1536 x 2048, 6 chosen: 9 tokens
+//   196 against 130, 40: 779 against 164;  16 of 512 x 1024, 8 chosen: 9 tokens 75 against 56, 40: 282 against 56;  the first with a shared expert, 24 tokens: 1207 against 818
+static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k) {
+    if (!grouped_ok(m, k)) return false;
+    static const int fixed = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : -1; }();
+    if (fixed >= 0) return fixed > 0 && T >= fixed;
+    if (T <= 8 || T >= 48) return T > 8;
+    if (sh && sh->group_max_len < T) return false;      // (the shared expert would be a call of its own; with the row kernels it rides along)
+    const ktb200_moe_config& c = m->cfg;
+    const KqFmt gu = kq_fmt(pick_fmt(c.gate_type, m->gu_soa)), down = kq_fmt(pick_fmt(c.down_type, m->down_layout));
+    const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), hit = k < E ? E * (1.0 - pow(1.0 - k / E, T)) : E;
+    const double rows = 20.0 + T * (std::min<double>(k, E) + (sh ? 1 : 0)) * (2e-3 * I * (kq_is_q6(gu) ? 1.4 : 0.83) + 1.1e-3 * H / 4);
+    auto cycles = [](KqFmt f) { return kq_is_q6(f) ? 3570.0 : f == KQ_Q5K ? 2200.0 : 1900.0; };
+    const double blocks = ceil(hit * I / 128 / sms) * (H / QK_K) * cycles(gu) + ceil(hit * H / kKqRows / sms) * (I / QK_K) * cycles(down);
+    return (sh ? 115.0 : 85.0) + 1.15 * blocks / 1850.0 < 0.95 * rows;
 }
+int ktb200_moe_takes_gemms(const ktb200_moe* m, const ktb200_mlp* shared, int qlen, int k) { return m && m->loaded && qlen > 0 && k > 0 && moe_as_gemms(m, shared, qlen, k); }
 
 static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, const float* weights, const void* input,
                             void* output, const int* bsz, cudaStream_t s, cudaEvent_t mid, const ktb200_mlp* sh = nullptr,
@@ -595,7 +614,7 @@ static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
     if (!ids || !weights || !input || !output) { set_error("forward: null pointer"); return KTB200_EINVAL; }
     DeviceGuard g(m->device);
 
-    if (!mid && !shared_out && grouped_min_qlen() > 0 && qlen >= grouped_min_qlen() && grouped_ok(m, k)) {
+    if (!mid && !shared_out && moe_as_gemms(m, sh, qlen, k)) {
         int rc = moe_forward_grouped(m, qlen, k, ids, weights, input, output, bsz, s);
         if (rc || !sh) return rc;
         return ktb200_mlp_forward(const_cast<ktb200_mlp*>(sh), qlen, input, output, 1, bsz, (void*)s);

@@ -25,6 +25,7 @@ from torch import nn
 from .. import native
 from ..util.custom_gguf import GGML_NAMES, TORCH_TO_GGML_HIDDEN, B200_WEIGHT_TYPES
 from ..util.utils import InferenceState
+from ..models.modeling_deepseek_v3 import DeepseekV3MLP
 from .base_operator import BaseInjectedModule
 
 
@@ -315,7 +316,7 @@ class KTransformersExperts(BaseInjectedModule, KExpertsBase):
 class KTransformersExpertsV2(KTransformersExperts):
     """experts.py:1273-1350: the balance-serve variant whose forward carries `bsz_tensor` (device-side live batch size) and a
     CUDA-graph slot.  With `prefill_op: None` the generate experts serve both phases (one GPU-resident KExpertsB200: per-pair
-    GEMV kernels for decode batches, the grouped tensor-core path from KTB200_GROUPED_MIN tokens up)."""
+    GEMV kernels for small decode batches, the grouped tensor-core path for larger ones and prompts)."""
 
     def forward(self, input_tensor, expert_ids, weights, bsz_tensor=None, cuda_graph_idx=0):
         if self.mode == InferenceState.GENERATE or (self.mode == InferenceState.PREFILL and self.prefill_experts is None):
@@ -340,9 +341,35 @@ class _KDeepseekMoEMixin:
     KExpertsB200 take ONE call, `ktb200_moe_block_forward`: router, routed experts and shared expert in a single
     persistent launch, bit-identical to the three-step path below (include/ktb200.h).  The shared expert for that call
     is a `ktb200_mlp` handle built once from the raw GGUF tensors `<key>.shared_experts.{gate,up,down}_proj.weight`.
+    Larger decode batches whose experts run as tensor-core GEMMs (`ktb200_moe_takes_gemms`) take the same call, which is then a dozen
+    launches of the library instead of the modules' (24 tokens, 256 experts: the modules' host work alone is 200 us), as long as calling the
+    modules would do nothing else: shared projections on raw blocks, no hooks.
     """
 
     BLOCK_MAX_TOKENS = 8
+    BATCH_MAX_TOKENS = 47
+
+    def _one_call(self, n_tok, gen):
+        """whether `n_tok` tokens may go through ktb200_moe_block_forward"""
+        if getattr(gen, "ep_size", 1) != 1:
+            return False
+        if n_tok <= self.BLOCK_MAX_TOKENS:
+            return True
+        if not (self.BLOCK_MAX_TOKENS and n_tok <= min(self.BATCH_MAX_TOKENS, getattr(gen, "max_tokens", 0)) and getattr(gen, "handle", None) is not None):
+            return False
+        mods = [getattr(self, "gate", None), getattr(self, "experts", None)]
+        if self.config.n_shared_experts is not None:
+            from .linear import KLinearB200
+            shared = getattr(self, "shared_experts", None)
+            linears = [getattr(shared, n, None) for n in ("gate_proj", "up_proj", "down_proj")]
+            if type(shared) is not DeepseekV3MLP or not all(isinstance(getattr(p, "generate_linear", None), KLinearB200) and p.mode == InferenceState.GENERATE for p in linears):
+                return False
+            mods += [shared] + linears
+        glob = torch.nn.modules.module
+        if glob._global_forward_hooks or glob._global_forward_pre_hooks or any(m is None or m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in mods):
+            return False
+        top = getattr(getattr(mods[0], "orig_module", None), "top_k", 0)
+        return bool(native.lib().ktb200_moe_takes_gemms(gen.handle, getattr(self, "_ktb_mlp", None), n_tok, top))
 
     def load(self):
         """children first (base_operator.py:45-48), then the shared expert's handle for the single-launch path: handles
@@ -394,7 +421,7 @@ class _KDeepseekMoEMixin:
         inter = self.config.moe_intermediate_size * self.config.n_shared_experts
         h = C.c_void_p()
         native.check(native.lib().ktb200_mlp_create(self.config.hidden_size, inter, raw[0].data_ptr(), raw[1].data_ptr(), raw[2].data_ptr(),
-                                                    types[0], types[1], types[2], gen.hidden_type, self.BLOCK_MAX_TOKENS, gen.dev_index, C.byref(h)))
+                                                    types[0], types[1], types[2], gen.hidden_type, self.BATCH_MAX_TOKENS, gen.dev_index, C.byref(h)))
         native.check(native.lib().ktb200_mlp_load_weights(h, _stream(dev)))
         self._ktb_mlp, self._ktb_mlp_raw = h, raw
         return h
@@ -419,7 +446,7 @@ class _KDeepseekMoEMixin:
                                                                       y.data_ptr(), idx.data_ptr(), wt.data_ptr(), 7, _stream(x.device)))
                 self.last_topk = (idx, wt)
                 return y.view(*orig_shape)
-        if n_tok <= self.BLOCK_MAX_TOKENS and getattr(gen0, "ep_size", 1) == 1:
+        if self._one_call(n_tok, gen0):
             hs = self._block_handles(hidden_states)
             if hs is not None:
                 cfg, moe, mlp = hs
@@ -504,7 +531,7 @@ class KDeepseekV3MoEV2(_KDeepseekMoEMixin, BaseInjectedModule, _V3):
         identity, orig_shape = hidden_states, hidden_states.shape
         n_tok = hidden_states.numel() // orig_shape[-1]
         gen = getattr(getattr(self, "experts", None), "generate_experts", None)
-        if n_tok <= self.BLOCK_MAX_TOKENS and getattr(gen, "ep_size", 1) == 1:
+        if self._one_call(n_tok, gen):
             hs = self._block_handles(hidden_states)
             if hs is not None:
                 cfg, moe, mlp = hs

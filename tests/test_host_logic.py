@@ -417,3 +417,47 @@ def test_prompt_attention_looks_up_only_pages_with_visible_keys(tmp_path):
                     assert k % 64 == 0 and k + 63 >= lo and k <= hi, (lo, hi, k0, i, k)
                     if any(lo <= x <= hi for x in range(k0 + 64 * i, k0 + 64 * i + 64)):
                         assert k == k0 + 64 * i
+
+
+def test_moe_batches_that_may_go_in_one_call(monkeypatch):
+    """KDeepseekV3MoE: up to 8 tokens always (one rank); up to 47 only where the library would run GEMMs and calling the modules would do nothing else."""
+    from types import SimpleNamespace
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3MLP
+    from ktransformers_b200.operators import experts
+    from ktransformers_b200.operators.linear import KLinearB200
+    from ktransformers_b200.util.utils import InferenceState
+
+    asked = []
+    monkeypatch.setattr(native, "lib", lambda: SimpleNamespace(ktb200_moe_takes_gemms=lambda m, s, n, k: asked.append((n, k)) or int(n >= 12)))
+
+    class Block(experts._KDeepseekMoEMixin, torch.nn.Module):
+        pass
+
+    class Projection(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.generate_linear, self.mode = KLinearB200.__new__(KLinearB200), InferenceState.GENERATE
+
+    def block():
+        b = Block()
+        b.config = SimpleNamespace(n_shared_experts=1, hidden_size=8, intermediate_size=8)
+        b.gate, b.experts, b.shared_experts = torch.nn.Identity(), torch.nn.Identity(), DeepseekV3MLP(b.config)
+        b.gate.orig_module = SimpleNamespace(top_k=4)
+        for n in ("gate_proj", "up_proj", "down_proj"):
+            setattr(b.shared_experts, n, Projection())
+        return b
+
+    gen = lambda ep=1, most=1024: SimpleNamespace(ep_size=ep, max_tokens=most, handle=1)
+    b = block()
+    assert [b._one_call(n, gen()) for n in (1, 8, 9, 12, 47, 48)] == [True, True, False, True, True, False] and asked == [(9, 4), (12, 4), (47, 4)]
+    assert not b._one_call(1, gen(ep=2)) and not b._one_call(12, gen(most=10))
+    b.BLOCK_MAX_TOKENS = 0
+    assert not b._one_call(1, gen()) and not b._one_call(12, gen())
+    for change in (lambda b: b.gate.register_forward_hook(print), lambda b: b.shared_experts.register_forward_pre_hook(print), lambda b: b.shared_experts.up_proj.register_forward_hook(print),
+                   lambda b: setattr(b.shared_experts.up_proj, "mode", InferenceState.PREFILL), lambda b: setattr(b.shared_experts.down_proj, "generate_linear", None),
+                   lambda b: setattr(b, "shared_experts", torch.nn.Identity()), lambda b: setattr(b.experts, "forward", print)):
+        b = block()
+        change(b)
+        assert b._one_call(8, gen()) and not b._one_call(12, gen())

@@ -301,3 +301,48 @@ def test_k_quant_long_rows_in_fp32(type, K, R, T):
     off, off_rows = ((v.double() - want).norm().item() for v in (call(x), torch.cat([call(x[t:t + 8].contiguous()) for t in range(0, T, 8)])))
     assert off <= 1.05 * off_rows, (off, off_rows)
     lib.ktb200_linear_destroy(h)
+
+
+# decode batches between the row kernels' 8 tokens and the prompt sizes: what the rule sends to the GEMMs agrees with the row kernels (8 tokens at a time); a shared expert
+# whose handle takes fewer tokens keeps the batch with the row kernels, where it rides along
+@pytest.mark.parametrize("T", [9, 24, 47])
+def test_decode_batches_as_gemms(T):
+    import gpu_util as G
+    E, k, H, I = 32, 6, 2048, 1536
+    gate, up, down = synth_blocks(Q4_K, E * I * H, "cuda", 1), synth_blocks(Q4_K, E * I * H, "cuda", 2), synth_blocks(Q6_K, E * H * I, "cuda", 3)
+    shared = [synth_blocks(t, I * H, "cuda", 4 + i) for i, t in enumerate((Q4_K, Q4_K, Q6_K))]
+    m = G.Moe(E, k, H, I, gate, up, down, Q4_K, Q4_K, Q6_K, BF16, max_tokens=64)
+    lib, handles = native.lib(), []
+    for most in (64, 8):
+        h, keep = C.c_void_p(), [t.clone() for t in shared]
+        native.check(lib.ktb200_mlp_create(H, I, *[t.data_ptr() for t in keep], Q4_K, Q4_K, Q6_K, BF16, most, 0, C.byref(h)))
+        native.check(lib.ktb200_mlp_load_weights(h, _stream()))
+        handles.append((h, keep))
+    (big, _), (small, _) = handles
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = (torch.randn((T, H), generator=g, device="cuda") / 10).bfloat16()
+    w = torch.rand((T, k), generator=g, device="cuda")
+    ids = torch.rand((T, E), generator=g, device="cuda").argsort(-1)[:, :k].contiguous()
+    assert [lib.ktb200_moe_takes_gemms(m.h, None, t, k) for t in (1, 8, T, 48)] == [0, 0, 1, 1]
+    assert lib.ktb200_moe_takes_gemms(m.h, big, T, k) == 1 and lib.ktb200_moe_takes_gemms(m.h, small, T, k) == 0
+
+    def call(sh, n0, n1, y, bsz=None):
+        native.check(lib.ktb200_moe_forward_shared(m.h, sh, n1 - n0, k, ids[n0:n1].data_ptr(), w[n0:n1].data_ptr(), x[n0:n1].data_ptr(), y[n0:n1].data_ptr(),
+                                                   bsz.data_ptr() if bsz is not None else None, _stream()))
+
+    for sh in (None, big, small):
+        y, few = (torch.zeros((T, H), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        n0 = native.launch_count()
+        call(sh, 0, T, y)
+        assert (native.launch_count() - n0 >= 10) == (sh is not small)
+        for t in range(0, T, 8):
+            call(sh, t, min(t + 8, T), few)
+        # the same sums in another order: to the last bf16 place (two with a shared term), and an activation at the edge of two int8 steps moves a row by 1e-3
+        size = few.double().abs().max()
+        assert ((y.double() - few.double()).abs() <= 2.0 ** (-6 if sh else -7) * few.double().abs() + 2e-3 * size).all()
+        held = torch.full_like(y, 7.0)
+        call(sh, 0, T, held, torch.tensor([T - 2], dtype=torch.int32, device="cuda"))
+        assert torch.equal(held[:T - 2], y[:T - 2]) and (held[T - 2:] == 7.0).all()
+    for h, _ in handles:
+        lib.ktb200_mlp_destroy(h)
+    m.close()
