@@ -32,6 +32,8 @@ constexpr int kBulkMaxWarpsDown = 16;    // down kernel: 128 registers per threa
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// (before its shared memory becomes something else)
+__device__ __forceinline__ void mbar_inval(uint32_t bar) { asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
@@ -116,7 +118,7 @@ __device__ __forceinline__ float q4k_block_dot(const uint8_t* wb, const uint8_t*
 // streaming across tokens instead of draining it once per token — and all the chunk's activation rows are staged as
 // Q8_K side by side (`act_tok` bytes each).
 template <bool PAIR, int SLOTS>
-__global__ void __launch_bounds__(kBulkMaxWarps * 32, 1) rows_bulk_q4k_kernel(const RowsParams p, int act_tok, int tc) {
+__device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, int tc) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ int s_np;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -146,16 +148,23 @@ __global__ void __launch_bounds__(kBulkMaxWarps * 32, 1) rows_bulk_q4k_kernel(co
   for (int t0 = 0; t0 < Teff; t0 += tc) {
     const int nt = min(tc, Teff - t0);
     __syncthreads();   // previous chunk: everyone is done with the staging and the pair list (and the barriers are initialised)
-    if (threadIdx.x == 0) {
+    if (warp == 0) {      // the list in (token, slot) order, 32 candidates at a time
         int np = 0;
-        for (int tl = 0; tl < nt; tl++) {
-            for (int s = 0; s < p.slots; s++) {
-                const long e = p.ids ? (long)p.ids[(long)(t0 + tl) * p.slots + s] - p.id_offset : 0;
-                if (e >= 0 && e < p.n_experts) pairs[np++] = (tl << 8) | s;
+        for (int i0 = 0; i0 < nt * nslots; i0 += 32) {
+            const int i = i0 + lane, tl = i / nslots, s = i - tl * nslots;
+            bool own = false;
+            if (i < nt * nslots) {
+                if (s == p.slots) own = p.shared_token < 0 || p.shared_token == t0 + tl;
+                else {
+                    const long e = p.ids ? (long)p.ids[(long)(t0 + tl) * p.slots + s] - p.id_offset : 0;
+                    own = e >= 0 && e < p.n_experts;
+                }
             }
-            if (p.x0 && (p.shared_token < 0 || p.shared_token == t0 + tl)) pairs[np++] = (tl << 8) | p.slots;
+            const unsigned all = __ballot_sync(0xffffffffu, own);
+            if (own) pairs[np + __popc(all & ((1u << lane) - 1))] = (tl << 8) | s;
+            np += __popc(all);
         }
-        s_np = np;
+        if (lane == 0) s_np = np;
     }
     __syncthreads();
     const int total = s_np * p.rows;
@@ -254,7 +263,14 @@ __global__ void __launch_bounds__(kBulkMaxWarps * 32, 1) rows_bulk_q4k_kernel(co
         while (crr >= p.rows) { crr -= p.rows; cpi++; }
     }
   }  // token chunks
+    __syncthreads();      // (no chunk at all: every barrier is initialised)
+    if (lane == 0) {
+#pragma unroll
+        for (int s = 0; s < SLOTS; s++) mbar_inval(bar_u32 + 8 * s);
+    }
 }
+template <bool PAIR, int SLOTS>
+__global__ void __launch_bounds__(kBulkMaxWarps * 32, 1) rows_bulk_q4k_kernel(const RowsParams p, int act_tok, int tc) { rows_bulk_q4k<PAIR, SLOTS>(p, act_tok, tc); }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Item formats of the down-projection kernel.  An item is 4 consecutive rows x nb super-blocks, f = rw*nb + blk.
@@ -332,7 +348,7 @@ struct BulkQ6K4T {   // chunk-major 4-row tiles (see the header comment)
 // activation rows are staged as Q8_K side by side.
 constexpr int kBulkMaxChunkTokens = 16;
 template <class Fmt, int SLOTS>
-__global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(const ReduceParams p, int nrows_max, int pcap) {
+__device__ __forceinline__ void reduce_bulk(const ReduceParams& p, int nrows_max, int pcap) {
     constexpr int RW = 4;
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ int s_np, s_nt;
@@ -371,27 +387,35 @@ __global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(
 
   for (int t0 = 0; t0 < Teff;) {
     __syncthreads();
-    if (threadIdx.x == 0) {   // greedy chunk: tokens t0.. while their owned pairs fit
+    if (warp == 0) {   // greedy chunk: tokens t0.. while their owned pairs fit; a token's slots side by side in the lanes, the next token's ids already on their way
         int np = 0, nt = 0;
+        auto owned = [&](int t, int j) {
+            if (t >= Teff || j >= ns) return false;
+            if (j == k) return p.shared_token < 0 || p.shared_token == t;
+            const long e = p.ids ? (long)p.ids[(long)t * k + j] - p.id_offset : 0;
+            return e >= 0 && e < p.n_experts;
+        };
+        bool ahead = owned(t0, lane);
         while (t0 + nt < Teff && nt < kBulkMaxChunkTokens) {
-            const bool sh_here = p.xw && (p.shared_token < 0 || p.shared_token == t0 + nt);
-            int cnt = sh_here ? 1 : 0;
-            for (int j = 0; j < k; j++) {
-                const long e = p.ids ? (long)p.ids[(long)(t0 + nt) * k + j] - p.id_offset : 0;
-                cnt += (e >= 0 && e < p.n_experts) ? 1 : 0;
-            }
+            const bool first = ahead;
+            ahead = owned(t0 + nt + 1, lane);
+            int cnt = 0;
+            for (int j0 = 0; j0 < ns; j0 += 32) cnt += __popc(__ballot_sync(0xffffffffu, j0 ? owned(t0 + nt, j0 + lane) : first));
             if (nt > 0 && np + cnt > pcap) break;
-            s_first[nt] = np;
-            for (int j = 0; j < k; j++) {
-                const long e = p.ids ? (long)p.ids[(long)(t0 + nt) * k + j] - p.id_offset : 0;
-                if (e >= 0 && e < p.n_experts) pairs[np++] = (nt << 8) | j;
+            if (lane == 0) s_first[nt] = np;
+            for (int j0 = 0; j0 < ns; j0 += 32) {
+                const bool own = j0 ? owned(t0 + nt, j0 + lane) : first;
+                const unsigned all = __ballot_sync(0xffffffffu, own);
+                if (own) pairs[np + __popc(all & ((1u << lane) - 1))] = (nt << 8) | (j0 + lane);
+                np += __popc(all);
             }
-            if (sh_here) pairs[np++] = (nt << 8) | k;
             nt++;
         }
-        s_first[nt] = np;
-        s_np = np;
-        s_nt = nt;
+        if (lane == 0) {
+            s_first[nt] = np;
+            s_np = np;
+            s_nt = nt;
+        }
     }
     __syncthreads();
     const int np = s_np, nt = s_nt;
@@ -491,5 +515,16 @@ __global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(
     t0 += nt;
   }  // token chunks
 }
+template <class Fmt, int SLOTS>
+__global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(const ReduceParams p, int nrows_max, int pcap) { reduce_bulk<Fmt, SLOTS>(p, nrows_max, pcap); }
+
+// both row phases of T tokens in one launch (moe_block.cu), planned in moe.cu
+struct MoeRowsPlan {
+    static constexpr int kWarps = 16, kSlotsUp = 3, kSlotsDown = 2;      // 512 threads: 128 registers
+    RowsParams rows;
+    ReduceParams down;
+    int warps, grid, act_tok, tc, nrows_max, pcap;
+    size_t smem;
+};
 
 }  // namespace ktb

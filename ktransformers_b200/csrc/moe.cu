@@ -209,27 +209,34 @@ static int launch_rows_pipe(const RowsParams& p, int T, int device, cudaStream_t
     return KTB200_OK;
 }
 
-// Q4_K rows through the bulk-copy ring (rows_bulk_q4k_kernel).  Returns 1 when the shape does not suit it.
-template <bool PAIR>
-static int launch_rows_bulk_q4k(const RowsParams& p, int T, int device, cudaStream_t stream) {
-    if (!cfg_bulk()) return 1;
-    const int nblk = p.ncols / QK_K;
-    const int row_bytes = nblk * SZ_Q4_K;
-    if (nblk < 16) return 1;                             // needs >= 16 blocks per row to keep most lanes busy
-    const int nslots = p.slots + (p.x0 ? 1 : 0);
-    const long total = (long)nslots * p.rows;
-    if (total >= (1L << 26) || nslots > 200) return 1;
-    const int act_tok = (nblk * kActBlkStride + nblk * 16 + nblk * 4 + 15) & ~15;
-    const int S = cfg_bulk_slots_up();
+// Shared-memory plan of rows_bulk_q4k<., S> for T tokens of `nslots` sets of rows each: returns the warp count (0 = does not fit)
+static int rows_bulk_plan(int ncols, int nslots, int T, int S, int max_warps, int* act_tok_out, int* tc_out, size_t* smem_out) {
+    const int nblk = ncols / QK_K, row_bytes = nblk * SZ_Q4_K, act_tok = (nblk * kActBlkStride + nblk * 16 + nblk * 4 + 15) & ~15;
+    if (nblk < 16) return 0;                             // needs >= 16 blocks per row to keep most lanes busy
     // tokens per chunk: as many (<= 8) as fit next to 12 rings; then as many warps as fit
     int tc = T < 8 ? T : 8;
     while (tc > 1 && (size_t)tc * (act_tok + nslots * 4) + 64 + (size_t)12 * S * (row_bytes + 8) > kSmemCap) tc--;
     const size_t head = (((size_t)tc * act_tok + (size_t)tc * nslots * 4 + 15) & ~(size_t)15);
-    if (head + 64 >= kSmemCap) return 1;
+    if (head + 64 >= kSmemCap) return 0;
     int W = (int)((kSmemCap - head - 16) / ((size_t)S * (row_bytes + 8)));
-    if (W > cfg_bulk_warps()) W = cfg_bulk_warps();
-    if (W < 4) return 1;
-    const size_t smem = head + (((size_t)W * S * 8 + 15) & ~(size_t)15) + (size_t)W * S * row_bytes;
+    if (W > max_warps) W = max_warps;
+    if (W < 4) return 0;
+    *act_tok_out = act_tok; *tc_out = tc;
+    *smem_out = head + (((size_t)W * S * 8 + 15) & ~(size_t)15) + (size_t)W * S * row_bytes;
+    return W;
+}
+// Q4_K rows through the bulk-copy ring (rows_bulk_q4k_kernel).  Returns 1 when the shape does not suit it.
+template <bool PAIR>
+static int launch_rows_bulk_q4k(const RowsParams& p, int T, int device, cudaStream_t stream) {
+    if (!cfg_bulk()) return 1;
+    const int nslots = p.slots + (p.x0 ? 1 : 0);
+    const long total = (long)nslots * p.rows;
+    if (total >= (1L << 26) || nslots > 200) return 1;
+    const int S = cfg_bulk_slots_up();
+    int act_tok = 0, tc = 0;
+    size_t smem = 0;
+    const int W = rows_bulk_plan(p.ncols, nslots, T, S, cfg_bulk_warps(), &act_tok, &tc, &smem);
+    if (!W) return 1;
     int gx = num_sms(device);            // one CTA per SM walks all T tokens
     if (gx > total) gx = (int)total;
     if (gx < 1) gx = 1;
@@ -393,21 +400,22 @@ static int reduce_bulk_plan(int rows, int ncols, int pcap, int S, int device, in
     return W;
 }
 
+// pair capacity of a token chunk: one token's worth at least; up to 2 tokens' worth (<= 18) when several tokens share the launch and >= 10 warps still fit
+template <class Fmt>
+static int reduce_bulk_pairs(int rows, int ncols, int ns, int T, int S, int device) {
+    if (T <= 1) return ns;
+    int want = 2 * ns < 18 ? 2 * ns : (ns > 18 ? ns : 18);
+    if ((long)T * ns < want) want = T * ns;
+    while (want > ns && reduce_bulk_plan<Fmt>(rows, ncols, want, S, device, nullptr, nullptr, nullptr) < 10) want--;
+    return want;
+}
 // Down projection through the bulk-copy ring.  Returns 1 when the shape does not suit it.
 template <class Fmt>
 static int launch_reduce_bulk(const ReduceParams& p, int T, int device, cudaStream_t stream) {
     if (!cfg_bulk()) return 1;
     const int ns = p.slots + (p.xw ? 1 : 0);
     const int S = cfg_bulk_slots_down();
-    // pair capacity of a token chunk: one token's worth at least; up to 2 tokens' worth (<= 18) when several tokens
-    // share the launch and >= 10 warps still fit
-    int pcap = ns;
-    if (T > 1) {
-        int want = 2 * ns < 18 ? 2 * ns : (ns > 18 ? ns : 18);
-        if ((long)T * ns < want) want = T * ns;
-        while (want > ns && reduce_bulk_plan<Fmt>(p.rows, p.ncols, want, S, device, nullptr, nullptr, nullptr) < 10) want--;
-        pcap = want;
-    }
+    const int pcap = reduce_bulk_pairs<Fmt>(p.rows, p.ncols, ns, T, S, device);
     int gx = 0, nrows_max = 0;
     size_t smem = 0;
     const int W = reduce_bulk_plan<Fmt>(p.rows, p.ncols, pcap, S, device, &gx, &nrows_max, &smem);
@@ -602,6 +610,20 @@ static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k
 }
 int ktb200_moe_takes_gemms(const ktb200_moe* m, const ktb200_mlp* shared, int qlen, int k) { return m && m->loaded && qlen > 0 && k > 0 && moe_as_gemms(m, shared, qlen, k); }
 
+// what the row kernels of a layer's routed experts read
+static void row_params(const ktb200_moe* m, int k, const int64_t* ids, const float* weights, const void* input, void* output, const int* bsz, RowsParams& rp, ReduceParams& dp) {
+    const ktb200_moe_config& c = m->cfg;
+    rp.shared_token = -1;
+    rp.w0 = c.gate_proj; rp.w1 = c.up_proj; rp.type0 = c.gate_type; rp.type1 = c.up_type;
+    rp.n_experts = c.expert_num; rp.rows = c.intermediate_size; rp.ncols = c.hidden_size; rp.slots = k;
+    rp.ids = ids; rp.id_offset = c.expert_id_offset; rp.x = input; rp.hidden_type = c.hidden_type;
+    rp.use_silu = c.use_silu; rp.out_f32 = m->inter; rp.out_hidden = nullptr; rp.bias = nullptr; rp.bsz = bsz;
+    dp.shared_token = -1;
+    dp.w = c.down_proj; dp.type = c.down_type; dp.n_experts = c.expert_num; dp.rows = c.hidden_size;
+    dp.ncols = c.intermediate_size; dp.slots = k; dp.ids = ids; dp.id_offset = c.expert_id_offset;
+    dp.weights = weights; dp.a = m->inter; dp.out = output; dp.hidden_type = c.hidden_type; dp.accumulate = 0; dp.bsz = bsz;
+}
+
 static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, const float* weights, const void* input,
                             void* output, const int* bsz, cudaStream_t s, cudaEvent_t mid, const ktb200_mlp* sh = nullptr,
                             int shared_token = -1, void* shared_out = nullptr) {
@@ -622,11 +644,8 @@ static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
     FmtId fg = pick_fmt(c.gate_type, m->gu_soa), fu = pick_fmt(c.up_type, m->gu_soa);
     if (fg != fu) fg = fu = FMT_GENK;  // mixed gate/up types: the generic path reads the type per matrix
     RowsParams rp{};
-    rp.shared_token = -1;
-    rp.w0 = c.gate_proj; rp.w1 = c.up_proj; rp.type0 = c.gate_type; rp.type1 = c.up_type;
-    rp.n_experts = c.expert_num; rp.rows = c.intermediate_size; rp.ncols = c.hidden_size; rp.slots = k;
-    rp.ids = ids; rp.id_offset = c.expert_id_offset; rp.x = input; rp.hidden_type = c.hidden_type;
-    rp.use_silu = c.use_silu; rp.out_f32 = m->inter; rp.out_hidden = nullptr; rp.bias = nullptr; rp.bsz = bsz;
+    ReduceParams dp{};
+    row_params(m, k, ids, weights, input, output, bsz, rp, dp);
     const FmtId fd = pick_fmt(c.down_type, m->down_layout);
     // the shared expert rides in the same two launches as slot k when its tensors have the routed experts'
     // shapes and layouts (DeepSeek-V3: n_shared_experts = 1, same quant types); otherwise it runs separately
@@ -638,18 +657,40 @@ static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
     int rc = launch_rows<true>(fg, rp, qlen, m->device, s);
     if (rc) return rc;
     if (mid) KTB_CUDA_CHECK(cudaEventRecord(mid, s));
-
-    ReduceParams dp{};
-    dp.shared_token = -1;
-    dp.w = c.down_proj; dp.type = c.down_type; dp.n_experts = c.expert_num; dp.rows = c.hidden_size;
-    dp.ncols = c.intermediate_size; dp.slots = k; dp.ids = ids; dp.id_offset = c.expert_id_offset;
-    dp.weights = weights; dp.a = m->inter; dp.out = output; dp.hidden_type = c.hidden_type; dp.accumulate = 0; dp.bsz = bsz;
     if (fuse) { dp.xw = sh->down; dp.shared_token = shared_token; dp.xw_out = shared_out; dp.xw_out_type = sh->hidden_type; }
     rc = launch_reduce(fd, dp, qlen, m->device, s);
     if (rc || !sh || fuse) return rc;
     return ktb200_mlp_forward(const_cast<ktb200_mlp*>(sh), qlen, input, output, 1, bsz, (void*)s);
 }
 
+extern "C++" {
+namespace ktb {
+template <class Fmt>
+static int rows_plan_down(const ReduceParams& p, int T, int device, MoeRowsPlan* o, size_t* smem) {
+    const int ns = p.slots + (p.xw ? 1 : 0);
+    o->pcap = reduce_bulk_pairs<Fmt>(p.rows, p.ncols, ns, T, MoeRowsPlan::kSlotsDown, device);
+    return reduce_bulk_plan<Fmt>(p.rows, p.ncols, o->pcap, MoeRowsPlan::kSlotsDown, device, &o->grid, &o->nrows_max, smem);
+}
+// The row kernels' parameters and one shared-memory plan for both, with a common number of CTAs and warps, for T tokens in one launch (moe_block.cu); false: they do not suit
+bool moe_rows_plan(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, const int64_t* ids, const float* weights, const void* input, void* output, const int* bsz, MoeRowsPlan* o) {
+    const ktb200_moe_config& c = m->cfg;
+    o->rows = RowsParams{}; o->down = ReduceParams{};
+    row_params(m, k, ids, weights, input, output, bsz, o->rows, o->down);
+    o->rows.ntokens = o->down.ntokens = T;
+    if (sh) { o->rows.x0 = sh->gate; o->rows.x1 = sh->up; o->down.xw = sh->down; }
+    const int ns = k + (sh ? 1 : 0);
+    if (!cfg_bulk() || ns > 31 || (long)ns * c.intermediate_size >= (1L << 26) || c.intermediate_size < num_sms(m->device)) return false;
+    size_t up = 0, down = 0;
+    const FmtId fd = pick_fmt(c.down_type, m->down_layout);
+    const int wd = fd == FMT_Q6K4T ? rows_plan_down<BulkQ6K4T>(o->down, T, m->device, o, &down) : fd == FMT_Q4K ? rows_plan_down<BulkQ4K>(o->down, T, m->device, o, &down) : 0;
+    if (wd < 4) return false;
+    o->warps = rows_bulk_plan(c.hidden_size, ns, T, MoeRowsPlan::kSlotsUp, std::min(wd, (int)MoeRowsPlan::kWarps), &o->act_tok, &o->tc, &up);
+    if (o->warps < 4) return false;
+    o->smem = std::max(up, down);      // (planned for at least as many warps)
+    return true;
+}
+}
+}
 int ktb200_moe_forward_shared(ktb200_moe* m, ktb200_mlp* shared, int qlen, int k, const int64_t* ids, const float* weights,
                               const void* input, void* output, const int* bsz, void* stream) {
     if (shared && !shared->loaded) { set_error("shared expert: Not Loaded"); return KTB200_ESTATE; }

@@ -22,6 +22,7 @@
 //
 // Arithmetic, summation orders and rounding are exactly those of the separate kernels (gate.cuh, gemv_bulk.cuh):
 // the fused launch is bit-identical to ktb200_moe_gate_forward + ktb200_moe_forward_shared (tests/test_gpu_parity.py).
+#include <algorithm>
 #include <cstdlib>
 
 #include "gate.cuh"
@@ -29,6 +30,8 @@
 #include "handles.cuh"
 
 namespace ktb {
+
+bool moe_rows_plan(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, const int64_t* ids, const float* weights, const void* input, void* output, const int* bsz, MoeRowsPlan* o);      // moe.cu
 
 constexpr int kBlockWarps = 15;    // 480 threads -> 128 registers; 15 x 13440-byte rings + staging = 227 KB
 constexpr int kBlockWarpsLo = 12;  // 384 threads -> 168 registers (KTB200_BLK_WARPS <= 12)
@@ -539,6 +542,79 @@ __global__ void __launch_bounds__(MAXW * 32, 1) moe_block_kernel(const BlockPara
     }
 }
 
+
+// ===================================================================================================================
+// The block for 2 to 8 tokens: ONE cooperative launch too, but every phase takes all tokens at once.  The kernel above goes through its phases once per token, of which the
+// router, the selection, two barriers and the ends of the streams are 22 us that nothing overlaps (7 tokens: 450 us); here the router's rows are read once for all tokens, a CTA
+// per token selects, and the (token, slot) pairs form one work list for gate and up and one for down, streamed by the row kernels' bodies (gemv_bulk.cuh).  The order of every sum is
+// the separate launches', so the results are their bits.  What bounds it: the bytes of every pair's expert at ~5 TB/s (an expert that two of a few tokens choose is rare).
+// 256 experts of 2048 x 7168, 8 chosen: 2 tokens 134 -> 124 us, 4 260 -> 222, 7 450 -> 377 (the separate launches 374); 64 of 1024 x 4096, 6 chosen: 7 tokens 214 -> 151.
+template <int NT>
+__device__ __forceinline__ void many_router(const GateParams& g, int nt) {      // gate_dot's order of sums (gate.cuh)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5, E = g.E, S = g.S, n4 = g.H / 4;
+    for (int u = blockIdx.x * W + warp; u < E * S; u += gridDim.x * W) {
+        const int s = u / E, e = u - s * E, c0 = (int)((long)n4 * s / S), nc4 = (int)((long)n4 * (s + 1) / S) - c0;
+        const float4* wrow = reinterpret_cast<const float4*>(g.W + (long)e * g.H) + c0;
+        float acc[NT];
+#pragma unroll
+        for (int i = 0; i < NT; i++) acc[i] = 0.f;
+        for (int cb = lane; cb < nc4; cb += 32 * 4) {
+            float4 w[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (cb + 32 * q < nc4) w[q] = __ldg(wrow + cb + 32 * q);
+#pragma unroll
+            for (int i = 0; i < NT; i++)
+                if (i < nt) {
+                    float4 x[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (cb + 32 * q < nc4) x[q] = load_x4(g.x, (long)i * n4 + c0 + cb + 32 * q, g.hidden_type);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (cb + 32 * q < nc4) {
+                            acc[i] = fmaf(w[q].x, x[q].x, acc[i]);
+                            acc[i] = fmaf(w[q].y, x[q].y, acc[i]);
+                            acc[i] = fmaf(w[q].z, x[q].z, acc[i]);
+                            acc[i] = fmaf(w[q].w, x[q].w, acc[i]);
+                        }
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            const float v = warp_sum(acc[i]);
+            if (i < nt && lane == 0) g.partial[((long)i * S + s) * E + e] = v;
+        }
+    }
+}
+template <class DownFmt>
+__global__ void __launch_bounds__(MoeRowsPlan::kWarps * 32, 1) moe_block_many_kernel(const __grid_constant__ GateParams g, unsigned* sync, const __grid_constant__ MoeRowsPlan plan) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    griddep_launch_dependents();
+    griddep_wait();
+    const int T = g.bsz ? min(g.T, *g.bsz) : g.T;
+    unsigned gen = 0;
+    if (T <= 2) many_router<2>(g, T);
+    else if (T <= 4) many_router<4>(g, T);
+    else many_router<kBlockMaxTokens>(g, T);
+    grid_arrive(sync, gen);
+    grid_wait(sync, gen);
+    for (int t = blockIdx.x; t < T; t += gridDim.x)
+        if ((threadIdx.x >> 5) < kGateWarps) gate_select_token<1>(g, t, reinterpret_cast<float*>(smem), g.idx + (long)t * g.top_k, g.w + (long)t * g.top_k, g.logits_out);
+    grid_arrive(sync, gen);
+    grid_wait(sync, gen);
+    rows_bulk_q4k<true, MoeRowsPlan::kSlotsUp>(plan.rows, plan.act_tok, plan.tc);
+    grid_arrive(sync, gen);
+    grid_wait(sync, gen);
+    reduce_bulk<DownFmt, MoeRowsPlan::kSlotsDown>(plan.down, plan.nrows_max, plan.pcap);
+    // leave the barrier words zeroed for the next launch / graph replay: the last CTA to get here resets them
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(sync + 1, 1u) == gridDim.x - 1) {
+        sync[0] = 0;
+        sync[1] = 0;
+        __threadfence();
+    }
+}
 
 // ===================================================================================================================
 // Expert-parallel MoE block: ONE persistent launch per layer and GPU, exchange over NVLink peer memory inside it.
@@ -1062,6 +1138,12 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
     p.g = GateParams{gc->weight, input, gc->hidden_type, gc->n_experts, gc->hidden_size, qlen, S, k, gc->n_group, gc->topk_group,
                      gc->scoring, gc->topk_method, gc->norm_topk_prob, gc->routed_scaling_factor, gc->bias, m->blk_partial, nullptr,
                      idx, w, bsz, nullptr};
+    MoeRowsPlan many;
+    const bool all_at_once = qlen > 1 && moe_rows_plan(m, sh, qlen, k, idx, w, input, output, bsz, &many);
+    if (all_at_once) {
+        G = many.grid; W = many.warps;
+        smem = std::max(many.smem, ((size_t)2 * gc->n_experts + 32 + 4 * kGateWarps) * sizeof(float));
+    }
     p.w_gate = c.gate_proj; p.w_up = c.up_proj; p.w_down = c.down_proj;
     p.s_gate = sh ? sh->gate : nullptr; p.s_up = sh ? sh->up : nullptr; p.s_down = sh ? sh->down : nullptr;
     p.n_local = c.expert_num; p.id_offset = c.expert_id_offset;
@@ -1072,9 +1154,10 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
     static const int prime_d = [] { const char* e = getenv("KTB200_BLK_PRIME_D"); return e ? atoi(e) : 2; }();
     p.prime_u = prime_u; p.prime_d = prime_d;
 
-    void* args[] = {&p};
+    void *one[] = {&p}, *all[] = {&p.g, &p.sync, &many}, **args = all_at_once ? all : one;
     const void* fn;
-    if (W > kBlockWarpsLo) fn = fd == FMT_Q6K4T ? (const void*)moe_block_kernel<BulkQ6K4T, kBlockWarps> : (const void*)moe_block_kernel<BulkQ4K, kBlockWarps>;
+    if (all_at_once) fn = fd == FMT_Q6K4T ? (const void*)moe_block_many_kernel<BulkQ6K4T> : (const void*)moe_block_many_kernel<BulkQ4K>;
+    else if (W > kBlockWarpsLo) fn = fd == FMT_Q6K4T ? (const void*)moe_block_kernel<BulkQ6K4T, kBlockWarps> : (const void*)moe_block_kernel<BulkQ4K, kBlockWarps>;
     else fn = fd == FMT_Q6K4T ? (const void*)moe_block_kernel<BulkQ6K4T, kBlockWarpsLo> : (const void*)moe_block_kernel<BulkQ4K, kBlockWarpsLo>;
     static const int coop = [] { const char* e = getenv("KTB200_BLK_COOP"); return e ? atoi(e) : 1; }();
     static const int pdl = [] { const char* e = getenv("KTB200_BLK_PDL"); return e ? atoi(e) : 1; }();
@@ -1085,9 +1168,9 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
     };
     {   // once per (variant, device): raise the dynamic shared-memory limit and check that the G CTAs CAN be co-resident —
         // the spin grid barriers need all of them on the SMs at the same time (1 CTA / SM at this shared-memory size)
-        static size_t limit[4][64] = {};
-        static int resident[4][64] = {};
-        const int v = (W > kBlockWarpsLo ? 2 : 0) + (fd == FMT_Q6K4T ? 1 : 0);
+        static size_t limit[6][64] = {};
+        static int resident[6][64] = {};
+        const int v = (all_at_once ? 4 : W > kBlockWarpsLo ? 2 : 0) + (fd == FMT_Q6K4T ? 1 : 0);
         if (limit[v][dev & 63] < smem) {
             KTB_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int per_sm = 0;
