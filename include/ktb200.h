@@ -354,6 +354,31 @@ int ktb200_mla_absorb_q(const void* q_dev, long q_head_stride, long q_token_stri
 int ktb200_mla_absorb_o(const void* attn_latent_dev, const void* w_uv_dev, int num_heads, int v_head_dim, int kv_lora_rank, void* out_dev,
                         int n_tokens, void* stream);
 
+/* ------------------------------------------------------------------------------------------
+ * One decode step of a DeepSeek attention layer (bf16, latents of 512 + 64, projections on GGUF blocks), in one call: q_a, norm, q_b (q_rank 0: `q_a` is the whole query
+ * projection), kv_a, ktb200_mla_step_prep, ktb200_mla_absorb_q, ktb200_mla_decode, ktb200_mla_absorb_o, o (archive/ktransformers/operators/attention.py:395-478).  The linears'
+ * hidden type has to be bf16; biases fp32 or NULL; w_uk [heads][nope][512] and w_uv [heads][v][512] bf16; positions as for ktb200_mla_step_prep; page_table
+ * [batch][table_pages], kv_len [batch] (written); workspace as for ktb200_mla_decode; scratch of ktb200_latent_step_bytes, 256-byte aligned, used on `stream` only.
+ * ------------------------------------------------------------------------------------------ */
+typedef struct ktb200_latent_step_params {
+    int batch, heads, nope_dim, v_dim, q_rank, page_size, max_pages, table_pages;
+    float q_eps, kv_eps, sm_scale;
+    ktb200_linear *q_a, *q_b, *kv_a, *o;
+    const float *q_a_bias, *q_b_bias, *kv_a_bias, *o_bias;
+    const void *q_norm, *kv_norm;
+    const float* inv_freq;
+    const long long* positions; long position_stride; const long long* cache_position;
+    void* kv_cache;
+    const void *w_uk, *w_uv;
+    const int* page_table; int* kv_len;
+    void* workspace; size_t workspace_bytes;
+    const void* x; void* out;
+    void* scratch; size_t scratch_bytes;
+} ktb200_latent_step_params;
+size_t ktb200_latent_step_bytes(int batch, int heads, int nope_dim, int v_dim, int q_rank);
+int ktb200_latent_step(const ktb200_latent_step_params* p, void* stream);
+
+
 /* paged latent KV write: StaticCache.update (archive/ktransformers/models/custom_cache.py:147-200)
  * kv_cache[page_idx[t]][page_offset[t]][0:512] = ckv[t], [512:576] = k_pe[t] */
 int ktb200_mla_kv_write(void* kv_cache, int page_size, const void* ckv, const void* k_pe, const int* page_idx,

@@ -45,6 +45,13 @@ class MlaParams(C.Structure):
                 ("lse_out", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("kv_cache_rows", C.c_long)]
 
 
+class LatentStepParams(C.Structure):
+    _fields_ = ([(n, C.c_int) for n in ("batch", "heads", "nope_dim", "v_dim", "q_rank", "page_size", "max_pages", "table_pages")] + [(n, C.c_float) for n in ("q_eps", "kv_eps", "sm_scale")]
+                + [(n, C.c_void_p) for n in ("q_a", "q_b", "kv_a", "o", "q_a_bias", "q_b_bias", "kv_a_bias", "o_bias", "q_norm", "kv_norm", "inv_freq", "positions")]
+                + [("position_stride", C.c_long)] + [(n, C.c_void_p) for n in ("cache_position", "kv_cache", "w_uk", "w_uv", "page_table", "kv_len", "workspace")]
+                + [("workspace_bytes", C.c_size_t)] + [(n, C.c_void_p) for n in ("x", "out", "scratch")] + [("scratch_bytes", C.c_size_t)])
+
+
 _lib = None
 _lock = threading.Lock()
 
@@ -77,6 +84,8 @@ SYMBOLS = {
     "ktb200_mlp_forward": (_I, [_VP, _I, _VP, _VP, _I, _VP, _VP]),
     "ktb200_moe_forward_shared": (_I, [_VP, _VP, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP]),
     "ktb200_moe_takes_gemms": (_I, [_VP, _VP, _I, _I]),
+    "ktb200_latent_step_bytes": (C.c_size_t, [_I, _I, _I, _I, _I]),
+    "ktb200_latent_step": (_I, [C.POINTER(LatentStepParams), _VP]),
     "ktb200_quantize_activations": (_I, [_VP, _I, _L, _L, _I, _VP, _VP]),
     "ktb200_dequantize": (_I, [_VP, _I, _L, _VP, _I, _VP]),
     "ktb200_moe_gate_forward": (_I, [C.POINTER(GateConfig), _I, _VP, _VP, _VP, _VP, _VP, _VP]),

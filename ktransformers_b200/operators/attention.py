@@ -17,6 +17,7 @@ import torch
 from .. import native
 from ..models.custom_cache import StaticCache
 from ..models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3RMSNorm, DeepseekV3RotaryEmbedding, apply_rotary_pos_emb
+from ..util.utils import InferenceState
 from .base_operator import BaseInjectedModule
 from .flashinfer_wrapper import MLAWrapperSingleton
 
@@ -45,22 +46,57 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
             object.__setattr__(self, "out_absorb", kv_b[:, self.qk_nope_head_dim:, :].contiguous())
         return self.q_absorb, self.out_absorb
 
+    def _quick(self):
+        """attribute look-up with the answers of `self.<name>`, without an exception on the way to what the wrapped module holds"""
+        own, cls, orig = vars(self), type(self), self.orig_module
+        return lambda name: own[name] if name in own else getattr(self, name) if hasattr(cls, name) else getattr(orig, name)
+
+    def _own_linears(self, x, bsz):
+        """The projections' KLinearB200 operators (q_a, q_b or None, kv_a, o) where calling the modules on `x` would launch those and do nothing else, else None: no hooks, no
+        forward of their own, bf16 in and out, the sizes that the step expects, plain norm of the query latent."""
+        from .linear import KLinearB200, KTransformersLinear
+        get, bf16_code = self._quick(), native.GGML_BF16
+        rank, heads = get("q_lora_rank"), get("num_heads")
+        q_out = heads * (get("qk_nope_head_dim") + 64)
+        wanted = [(get("q_proj"), x.shape[-1], q_out), None] if rank is None else [(get("q_a_proj"), x.shape[-1], rank), (get("q_b_proj"), rank, q_out)]
+        wanted += [(get("kv_a_proj_with_mqa"), x.shape[-1], 576), (get("o_proj"), heads * get("v_head_dim"), None)]
+        if not x.is_contiguous() or x.shape[1] != 1:
+            return None
+        if rank is not None:
+            norm = get("q_a_layernorm")
+            if not (_is_plain(norm, DeepseekV3RMSNorm) and norm.weight.dtype == torch.bfloat16 and norm.weight.device == x.device and rank % 2 == 0 and 0 < rank <= 8192):
+                return None
+        found = []
+        for item in wanted:
+            lin = None
+            if item is not None:
+                module, n_in, n_out = item
+                if not _is_plain(module, KTransformersLinear) or (module.mode == InferenceState.PREFILL and module.prefill_linear is not None):
+                    return None
+                lin = module.generate_linear
+                if not (type(lin) is KLinearB200 and "forward" not in vars(lin) and lin.handle is not None and lin.hidden_type == bf16_code and lin.dev_index == x.device.index
+                        and lin.in_features == n_in and n_out in (None, lin.out_features)):
+                    return None
+            found.append(lin)
+        return found
+
     def _step(self, hidden_states, position_ids, cache, cache_position):
         """One new token per sequence with everything between the projections in this library's launches (`ktb200_mla_step_prep` is the latent norm,
         both rotations, the cache write and the lengths): bf16, plain norms and rotation, the static cache.  None for any other form, which the
         module-by-module path below takes.  (The reference's decode branch: archive/ktransformers/operators/attention.py:395-478.)"""
-        rot, kv_norm, x = self.rotary_emb, self.kv_a_layernorm, hidden_states
+        get = self._quick()
+        rot, kv_norm, x = get("rotary_emb"), get("kv_a_layernorm"), hidden_states
         bf16 = torch.bfloat16
         if not (x.dtype == bf16 and x.is_cuda and _is_plain(rot, DeepseekV3RotaryEmbedding) and _is_plain(kv_norm, DeepseekV3RMSNorm) and type(cache) is StaticCache
-                and kv_norm.weight.dtype == bf16 and kv_norm.weight.device == x.device and self.kv_lora_rank == 512 and self.qk_rope_head_dim == 64):
+                and kv_norm.weight.dtype == bf16 and kv_norm.weight.device == x.device and get("kv_lora_rank") == 512 and get("qk_rope_head_dim") == 64):
             return None
         for t in (position_ids, cache_position):
             if t is None or t.dtype != torch.int64 or t.device != x.device:
                 return None
-        bsz, heads, nope = x.shape[0], self.num_heads, self.qk_nope_head_dim
+        bsz, heads, nope = x.shape[0], get("num_heads"), get("qk_nope_head_dim")
         if tuple(position_ids.shape) != (bsz, 1) or cache_position.numel() != 1 or cache.max_batch_size < bsz or rot.inv_freq.dtype != torch.float32 or rot.inv_freq.numel() != 32 or nope % 2:
             return None
-        w = self.mla_wrapper
+        w = get("mla_wrapper")
         if w is None:
             w = self.mla_wrapper = MLAWrapperSingleton.get_instance(str(x.device), bsz, cache.max_pages * bsz, use_cuda_graph=True)
         # the prep kernel writes `bsz` lengths as they come: a wrapper made for fewer sequences or pages (the device's wrapper keeps its first caller's
@@ -69,6 +105,32 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         if lens.numel() < bsz or lens.dtype != torch.int32 or lens.device != x.device or not lens.is_contiguous() or w.max_pages < cache.max_pages:
             return None
         lib, stream = native.lib(), torch.cuda.current_stream(x.device).cuda_stream
+        q_absorb, out_absorb = self.get_absorbed()
+        kv = cache.key_cache[get("layer_idx")]
+        if w.need_plan:
+            indptr = torch.arange(0, bsz + 1, dtype=torch.int32, device=x.device) * cache.max_pages
+            w.plan(None, indptr, cache.page_table_list[self.layer_idx].reshape(-1), (position_ids[:, 0] + 1).to(torch.int32), None, heads, 512, 64, cache.page_size, self.softmax_scale, bf16, kv.dtype)
+            w.max_pages_per_seq = cache.max_pages
+        inv_freq = rot.inv_freq.to(x.device)
+        own = self._own_linears(x, bsz)
+        if own is not None and q_absorb.dtype == bf16 == kv.dtype and kv.is_contiguous() and w.num_heads == heads and bsz <= w.max_batch_size:
+            # everything in one call: made one by one from here, the calls' host work bounds the layer
+            q_a, q_b, kv_a, o_lin = own
+            rank, v_dim = get("q_lora_rank") or 0, get("v_head_dim")
+            q_norm = get("q_a_layernorm") if rank else None
+            out = torch.empty((bsz, 1, o_lin.out_features), dtype=bf16, device=x.device)
+            need = lib.ktb200_latent_step_bytes(bsz, heads, nope, v_dim, rank)
+            scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
+            bias = lambda lin: lin.bias.data_ptr() if lin is not None and lin.has_bias else None
+            p = native.LatentStepParams(bsz, heads, nope, v_dim, rank, cache.page_size, cache.max_pages, w.max_pages, float(q_norm.variance_epsilon) if rank else 0.0,
+                                        float(kv_norm.variance_epsilon), w.sm_scale, q_a.handle, q_b.handle if rank else None, kv_a.handle, o_lin.handle, bias(q_a), bias(q_b), bias(kv_a), bias(o_lin),
+                                        q_norm.weight.data_ptr() if rank else None, kv_norm.weight.data_ptr(), inv_freq.data_ptr(), position_ids.data_ptr(), position_ids.stride(0),
+                                        cache_position.data_ptr(), kv.data_ptr(), q_absorb.data_ptr(), out_absorb.data_ptr(), w.page_table.data_ptr(), lens.data_ptr(), w.workspace.data_ptr(),
+                                        w.workspace.numel(), x.data_ptr(), out.data_ptr(), scratch.data_ptr(), need)
+            native.check(lib.ktb200_latent_step(C.byref(p), stream))
+            if not torch.cuda.is_current_stream_capturing():
+                cache.past_tokens[get("layer_idx")] += 1
+            return out
         if self.q_lora_rank is None:
             q = self.q_proj(x)
         else:
@@ -80,15 +142,8 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
                 qn = norm(qa)
             q = self.q_b_proj(qn)
         kva = self.kv_a_proj_with_mqa(x)
-        q_absorb, out_absorb = self.get_absorbed()
         if not (q.dtype == bf16 == kva.dtype == q_absorb.dtype and q.is_contiguous() and kva.is_contiguous()):
             return None
-        inv_freq = rot.inv_freq.to(x.device)
-        kv = cache.key_cache[self.layer_idx]
-        if w.need_plan:
-            indptr = torch.arange(0, bsz + 1, dtype=torch.int32, device=x.device) * cache.max_pages
-            w.plan(None, indptr, cache.page_table_list[self.layer_idx].reshape(-1), (position_ids[:, 0] + 1).to(torch.int32), None, heads, 512, 64, cache.page_size, self.softmax_scale, bf16, kv.dtype)
-            w.max_pages_per_seq = cache.max_pages
         q_pe = torch.empty((bsz, heads, 64), dtype=bf16, device=x.device)
         q_abs = torch.empty((bsz, heads, 512), dtype=bf16, device=x.device)
         native.check(lib.ktb200_mla_step_prep(q.data_ptr(), heads, nope, kva.data_ptr(), kv_norm.weight.data_ptr(), float(kv_norm.variance_epsilon), inv_freq.data_ptr(),

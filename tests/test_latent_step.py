@@ -100,3 +100,57 @@ def test_hooks_of_the_modules_between_the_projections_still_run():
                    cache_position=torch.zeros(1, dtype=torch.int64, device="cuda"))
             handle.remove()
             assert seen == [name], (name, register)
+
+
+@pytest.mark.parametrize("bsz,heads,q_rank,pos", [(1, 128, 256, 70), (3, 16, None, 0), (2, 24, 512, 63)])
+def test_one_call_equals_the_calls_one_by_one(bsz, heads, q_rank, pos):
+    """Projections on GGUF blocks: the step is one host call (`ktb200_latent_step`) unless something wants to see a module's call; the launches, and so all bits, are the same."""
+    from ktransformers_b200 import native
+    from ktransformers_b200.models.custom_cache import StaticCache
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3Config, DeepseekV3RotaryEmbedding
+    from ktransformers_b200.operators.attention import KDeepseekV2Attention
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapper
+    from ktransformers_b200.operators.linear import KTransformersLinear
+    from ktransformers_b200.util.synth import synth_blocks
+
+    torch.manual_seed(pos + heads)
+    hidden = 512
+    cfg = DeepseekV3Config(hidden_size=hidden, num_attention_heads=heads, q_lora_rank=q_rank, num_hidden_layers=1)
+    plain = DeepseekV3Attention(cfg, layer_idx=0).to(device="cuda", dtype=torch.bfloat16)
+    plain.rotary_emb = DeepseekV3RotaryEmbedding(64).to("cuda")
+    names = (["q_proj"] if q_rank is None else ["q_a_proj", "q_b_proj"]) + ["kv_a_proj_with_mqa", "o_proj"]
+    old = torch.get_default_dtype()
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        for i, n in enumerate(names):
+            orig = getattr(plain, n)
+            lin = KTransformersLinear("blk.0." + n, None, cfg, orig, "cuda", "KLinearB200", "cuda", None)
+            lin.load(w=(synth_blocks(12, orig.in_features * orig.out_features, "cuda", i), 12))
+            setattr(plain, n, lin)
+        op = KDeepseekV2Attention("blk.0.self_attn", None, cfg, plain, "cuda", "cuda")
+    finally:
+        torch.set_default_dtype(old)
+    x = torch.randn(bsz, 1, hidden, device="cuda").to(torch.bfloat16)
+    past = torch.randn(bsz, max(pos, 1), 576, device="cuda").to(torch.bfloat16)
+    where = torch.full((bsz, 1), pos, dtype=torch.int64, device="cuda")
+    got = []
+    for watched in (None, "kv_a_proj_with_mqa", "o_proj"):
+        cache = StaticCache(cfg, max_batch_size=bsz, max_cache_len=pos + 2, device="cuda")
+        rows = cache.key_cache[0].view(bsz, -1, 576)
+        if pos:
+            rows[:, :pos].copy_(past)
+        op.mla_wrapper = MLAWrapper(bsz, cache.max_pages * bsz)
+        seen = []
+        hook = getattr(plain, watched).register_forward_hook(lambda *a: seen.append(1)) if watched else None
+        assert (op._own_linears(x, bsz) is None) == bool(watched)
+        n0 = native.launch_count()
+        with torch.no_grad():
+            y, _, _ = op(x, position_ids=where, past_key_value=cache, cache_position=torch.tensor([pos], device="cuda"))
+        got.append((native.launch_count() - n0, y.clone(), rows[:, :pos + 1].clone(), op.mla_wrapper.kv_len_arr_buf[:bsz].clone(), cache.get_seq_length(0)))
+        if hook:
+            hook.remove()
+            assert seen == [1]
+    for other in got[1:]:
+        assert got[0][0] == other[0] and got[0][4] == other[4] == 1
+        assert all(torch.equal(a, b) for a, b in zip(got[0][1:4], other[1:4]))
+    assert got[0][1].isfinite().all() and got[0][1].abs().max() > 0
