@@ -7,7 +7,7 @@
 //
 //   * every ring slot is filled by ONE `cp.async.bulk.shared.global` issued by one lane and tracked by an
 //     mbarrier (expect_tx / complete_tx): no per-lane copy instructions, no LSU time for the copy;
-//   * slots are one weight row (Q4_K gate/up: nblk x 144 B) or one 4-row item (down) and a warp keeps SLOTS-1
+//   * slots are one output's weight rows (Q4_K gate and up: 2 nblk x 144 B) or one 4-row item (down) and a warp keeps SLOTS-1
 //     of them in flight while it computes on one: smaller slots -> up to 18 warps per SM (was 12);
 //   * unit -> (slot, row) bookkeeping is incremental (one division per token instead of one per unit);
 //   * Q6_K down tensors are re-tiled once at load time into 4-row "chunk-major" items (`repack_q6k4t`, moe.cu):
@@ -24,7 +24,7 @@
 namespace ktb {
 
 constexpr int kActBlkStride = QK_K + 16;   // int8 activation blocks padded to 272 B: 8 lanes x LDS.128 hit 32 distinct banks
-constexpr int kBulkMaxWarps = 18;        // gate/up kernel (<= 96 registers per thread)
+constexpr int kBulkMaxWarps = 16;        // gate/up kernel: 128 registers per thread
 constexpr int kBulkMaxWarpsDown = 16;    // down kernel: 128 registers per thread, and shared memory caps it at 15 anyway
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -70,48 +70,68 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
 // One Q4_K super-block (144 B at `wb`, shared memory, 16-byte aligned) against one padded int8 activation block.
 // bsv = the block's eight 32-value activation sums (int16), dxb = the activation block scale.
 // `act4(i)` returns the i-th 16-byte word of the block's 256 int8 activations (from shared memory or from registers).
-template <class ActFn>
-__device__ __forceinline__ float q4k_block_dot_t(const uint8_t* wb, ActFn&& act4, const uint4 bsv, const float dxb) {
-    const uint4 hdr = *reinterpret_cast<const uint4*>(wb);
-    const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&hdr.x));
-    const uint32_t scl = hdr.y & 0x3f3f3f3fu;                                          // scales 0..3
-    const uint32_t mnl = hdr.z & 0x3f3f3f3fu;                                          // mins   0..3
-    const uint32_t sch = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);         // scales 4..7
-    const uint32_t mnh = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);  // mins   4..7
-    int isum = 0;
+// N rows (`step` bytes apart) at once: a word of activations is loaded once for all of them, and their chains of sums run beside each other.
+template <int N, class ActFn>
+__device__ __forceinline__ void q4k_block_dots(const uint8_t* wb, long step, ActFn&& act4, const uint4 bsv, const float dxb, float (&out)[N]) {
+    uint4 hdr[N];
+    int isum[N];
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+        hdr[n] = *reinterpret_cast<const uint4*>(wb + n * step);
+        isum[n] = 0;
+    }
+    // scales (top: minima) of sub-blocks 0-3 and 4-7 as bytes
+    auto low = [](uint32_t w) { return w & 0x3f3f3f3fu; };
+    auto high = [](uint32_t w, uint32_t top) { return (top & 0x0f0f0f0fu) | ((w >> 2) & 0x30303030u); };
 #pragma unroll
     for (int g = 0; g < 4; g++) {
         const uint4 a0 = act4(4 * g), a1 = act4(4 * g + 1), a2 = act4(4 * g + 2), a3 = act4(4 * g + 3);
-        const uint4 q0 = *reinterpret_cast<const uint4*>(wb + 16 + 32 * g);
-        const uint4 q1 = *reinterpret_cast<const uint4*>(wb + 32 + 32 * g);
-        int slo = 0, shi = 0, slo2 = 0, shi2 = 0;
-        slo = dp4a_s8s8(q0.x & 0x0f0f0f0fu, a0.x, slo); slo2 = dp4a_s8s8(q0.y & 0x0f0f0f0fu, a0.y, slo2);
-        slo = dp4a_s8s8(q0.z & 0x0f0f0f0fu, a0.z, slo); slo2 = dp4a_s8s8(q0.w & 0x0f0f0f0fu, a0.w, slo2);
-        slo = dp4a_s8s8(q1.x & 0x0f0f0f0fu, a1.x, slo); slo2 = dp4a_s8s8(q1.y & 0x0f0f0f0fu, a1.y, slo2);
-        slo = dp4a_s8s8(q1.z & 0x0f0f0f0fu, a1.z, slo); slo2 = dp4a_s8s8(q1.w & 0x0f0f0f0fu, a1.w, slo2);
-        // high nibbles stay in place (x16): the sums are exact multiples of 16
-        shi = dp4a_u8s8(q0.x & 0xf0f0f0f0u, a2.x, shi); shi2 = dp4a_u8s8(q0.y & 0xf0f0f0f0u, a2.y, shi2);
-        shi = dp4a_u8s8(q0.z & 0xf0f0f0f0u, a2.z, shi); shi2 = dp4a_u8s8(q0.w & 0xf0f0f0f0u, a2.w, shi2);
-        shi = dp4a_u8s8(q1.x & 0xf0f0f0f0u, a3.x, shi); shi2 = dp4a_u8s8(q1.y & 0xf0f0f0f0u, a3.y, shi2);
-        shi = dp4a_u8s8(q1.z & 0xf0f0f0f0u, a3.z, shi); shi2 = dp4a_u8s8(q1.w & 0xf0f0f0f0u, a3.w, shi2);
-        const uint32_t scw = (g < 2) ? scl : sch;
-        const int sc0 = (int)((scw >> (16 * (g & 1))) & 0xff), sc1 = (int)((scw >> (16 * (g & 1) + 8)) & 0xff);
-        isum += sc0 * (slo + slo2) + sc1 * ((shi + shi2) >> 4);
+#pragma unroll
+        for (int n = 0; n < N; n++) {
+            const uint4 q0 = *reinterpret_cast<const uint4*>(wb + n * step + 16 + 32 * g);
+            const uint4 q1 = *reinterpret_cast<const uint4*>(wb + n * step + 32 + 32 * g);
+            int slo = 0, shi = 0, slo2 = 0, shi2 = 0;
+            slo = dp4a_s8s8(q0.x & 0x0f0f0f0fu, a0.x, slo); slo2 = dp4a_s8s8(q0.y & 0x0f0f0f0fu, a0.y, slo2);
+            slo = dp4a_s8s8(q0.z & 0x0f0f0f0fu, a0.z, slo); slo2 = dp4a_s8s8(q0.w & 0x0f0f0f0fu, a0.w, slo2);
+            slo = dp4a_s8s8(q1.x & 0x0f0f0f0fu, a1.x, slo); slo2 = dp4a_s8s8(q1.y & 0x0f0f0f0fu, a1.y, slo2);
+            slo = dp4a_s8s8(q1.z & 0x0f0f0f0fu, a1.z, slo); slo2 = dp4a_s8s8(q1.w & 0x0f0f0f0fu, a1.w, slo2);
+            // high nibbles stay in place (x16): the sums are exact multiples of 16
+            shi = dp4a_u8s8(q0.x & 0xf0f0f0f0u, a2.x, shi); shi2 = dp4a_u8s8(q0.y & 0xf0f0f0f0u, a2.y, shi2);
+            shi = dp4a_u8s8(q0.z & 0xf0f0f0f0u, a2.z, shi); shi2 = dp4a_u8s8(q0.w & 0xf0f0f0f0u, a2.w, shi2);
+            shi = dp4a_u8s8(q1.x & 0xf0f0f0f0u, a3.x, shi); shi2 = dp4a_u8s8(q1.y & 0xf0f0f0f0u, a3.y, shi2);
+            shi = dp4a_u8s8(q1.z & 0xf0f0f0f0u, a3.z, shi); shi2 = dp4a_u8s8(q1.w & 0xf0f0f0f0u, a3.w, shi2);
+            const uint32_t scw = g < 2 ? low(hdr[n].y) : high(hdr[n].y, hdr[n].w);
+            const int sc0 = (int)((scw >> (16 * (g & 1))) & 0xff), sc1 = (int)((scw >> (16 * (g & 1) + 8)) & 0xff);
+            isum[n] += sc0 * (slo + slo2) + sc1 * ((shi + shi2) >> 4);
+        }
     }
-    int msum = __dp2a_lo((int)bsv.x, (int)mnl, 0);
-    msum = __dp2a_hi((int)bsv.y, (int)mnl, msum);
-    msum = __dp2a_lo((int)bsv.z, (int)mnh, msum);
-    msum = __dp2a_hi((int)bsv.w, (int)mnh, msum);
-    return (dm.x * dxb) * (float)isum - (dm.y * dxb) * (float)msum;
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+        const uint32_t mnl = low(hdr[n].z), mnh = high(hdr[n].z, hdr[n].w >> 4);
+        int msum = __dp2a_lo((int)bsv.x, (int)mnl, 0);
+        msum = __dp2a_hi((int)bsv.y, (int)mnl, msum);
+        msum = __dp2a_lo((int)bsv.z, (int)mnh, msum);
+        msum = __dp2a_hi((int)bsv.w, (int)mnh, msum);
+        const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&hdr[n].x));
+        out[n] = (dm.x * dxb) * (float)isum[n] - (dm.y * dxb) * (float)msum;
+    }
+}
+template <class ActFn>
+__device__ __forceinline__ float q4k_block_dot_t(const uint8_t* wb, ActFn&& act4, const uint4 bsv, const float dxb) {
+    float out[1];
+    q4k_block_dots<1>(wb, 0, act4, bsv, dxb, out);
+    return out[0];
 }
 __device__ __forceinline__ float q4k_block_dot(const uint8_t* wb, const uint8_t* aq, const uint4 bsv, const float dxb) {
     return q4k_block_dot_t(wb, [&](int i) { return *reinterpret_cast<const uint4*>(aq + 16 * i); }, bsv, dxb);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Gate/up (PAIR) or dense (PAIR = false) rows of Q4_K tensors.  Per warp: a private ring of SLOTS row slots; the
-// warp's stream of sub-units is g(u0), u(u0), g(u0+W), u(u0+W), ... (PAIR) and at any time SLOTS-1 rows are in
-// flight behind the one being consumed.
+// Gate/up (PAIR) or dense (PAIR = false) rows of Q4_K tensors.  Per warp: a private ring of SLOTS slots of one unit each — a row, or (PAIR) the gate and the up row of one
+// output, whose dots share their activation loads — and at any time SLOTS-1 units are in flight behind the one being consumed.
+// A dozen warps an SM wait for their own loads and sums more than for a unit of the SM (43 % of the issue slots and of the shared-memory wavefronts in use): two rows at a time are
+// two chains beside each other and a third fewer loads.  MoE block of 7 tokens 377 -> 362 us (256 experts of 2048 x 7168, 8 chosen), 151 -> 137 (64 of 1024 x 4096, 6); routed
+// experts of 9 tokens, 160 of 1536 x 5120, 6 chosen, 202 -> 183.
 //
 // Tokens are processed in chunks of `tc` (launcher: as many as fit next to >= 12 rings).  Within a chunk ALL
 // (token, slot) pairs this launch owns form ONE work list — expert-parallel shards and decode batches keep the ring
@@ -134,7 +154,8 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     const size_t off = ((size_t)tc * act_tok + (size_t)tc * nslots * 4 + 15) & ~(size_t)15;
     const int bar_bytes = (W * SLOTS * 8 + 15) & ~15;
     const uint32_t bar_u32 = (uint32_t)__cvta_generic_to_shared(smem + off) + warp * SLOTS * 8;
-    uint8_t* ring = smem + off + bar_bytes + (size_t)warp * SLOTS * row_bytes;
+    const int unit_bytes = NM * row_bytes;
+    uint8_t* ring = smem + off + bar_bytes + (size_t)warp * SLOTS * unit_bytes;
     const uint32_t ring_u32 = (uint32_t)__cvta_generic_to_shared(ring);
     if (lane == 0) {
 #pragma unroll
@@ -171,33 +192,28 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     const int u0 = (int)((long)total * blockIdx.x / gridDim.x), u1 = (int)((long)total * (blockIdx.x + 1) / gridDim.x);
     int nu = u1 - u0 - warp;
     nu = nu > 0 ? (nu + W - 1) / W : 0;                     // units of this warp: u0 + warp + i*W
-    const int nsub = nu * NM;
-    // issue cursor: (pair index, row) of the next unit to request, and how many rows were requested
-    int ipi = 0, irr = 0, isub = 0;
+    // issue cursor: (pair index, row) of the next unit to request, and how many were requested
+    int ipi = 0, irr = 0, issued = 0;
     if (nu > 0) { ipi = (u0 + warp) / p.rows; irr = (u0 + warp) - ipi * p.rows; }
     int cpi = ipi, crr = irr;                               // consume cursor
 
     auto issue_one = [&]() {
-        if (isub < nsub) {
+        if (issued < nu) {
             if (lane == 0) {
                 const int pr = pairs[ipi], s = pr & 0xff, tl = pr >> 8;
-                const bool second = PAIR && (isub & 1);
-                const uint8_t* src;
-                if (s == p.slots) {
-                    src = reinterpret_cast<const uint8_t*>(second ? p.x1 : p.x0) + (long)irr * row_bytes;
-                } else {
-                    const long e = p.ids ? (long)p.ids[(long)(t0 + tl) * p.slots + s] - p.id_offset : 0;
-                    src = reinterpret_cast<const uint8_t*>(second ? p.w1 : p.w0) + (e * p.rows + irr) * row_bytes;
-                }
                 const uint32_t bar = bar_u32 + 8 * slot_i;
-                mbar_expect_tx(bar, (uint32_t)row_bytes);
-                bulk_g2s(ring_u32 + slot_i * row_bytes, src, (uint32_t)row_bytes, bar);
+                mbar_expect_tx(bar, (uint32_t)unit_bytes);
+                const bool extra = s == p.slots;
+                const long e = extra || !p.ids ? 0 : (long)p.ids[(long)(t0 + tl) * p.slots + s] - p.id_offset;
+#pragma unroll
+                for (int m = 0; m < NM; m++) {
+                    const void* w = extra ? (m ? p.x1 : p.x0) : (m ? p.w1 : p.w0);
+                    bulk_g2s(ring_u32 + slot_i * unit_bytes + m * row_bytes, reinterpret_cast<const uint8_t*>(w) + (e * p.rows + irr) * row_bytes, (uint32_t)row_bytes, bar);
+                }
             }
-            isub++;
-            if (!PAIR || !(isub & 1)) {
-                irr += W;
-                while (irr >= p.rows) { irr -= p.rows; ipi++; }
-            }
+            issued++;
+            irr += W;
+            while (irr >= p.rows) { irr -= p.rows; ipi++; }
             slot_i = (slot_i + 1 == SLOTS) ? 0 : slot_i + 1;
         }
     };
@@ -225,24 +241,28 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     }
     __syncthreads();
 
-    float acc_first = 0.f;
-    for (int n = 0; n < nsub; n++) {
+    for (int n = 0; n < nu; n++) {
         mbar_wait(bar_u32 + 8 * slot_u, (phase >> slot_u) & 1u);
         phase ^= 1u << slot_u;
-        const uint8_t* row0 = ring + slot_u * row_bytes;
+        const uint8_t* row0 = ring + slot_u * unit_bytes;
         const int pr = pairs[cpi];
         const uint8_t* at = smem + (size_t)(pr >> 8) * act_tok;
         const int16_t* bs32 = reinterpret_cast<const int16_t*>(at + (size_t)nblk * kActBlkStride);
         const float* dx = reinterpret_cast<const float*>(at + (size_t)nblk * (kActBlkStride + 16));
-        float acc = 0.f;
-        for (int blk = lane; blk < nblk; blk += 32)
-            acc += q4k_block_dot(row0 + blk * SZ_Q4_K, at + (size_t)blk * kActBlkStride,
-                                 *reinterpret_cast<const uint4*>(bs32 + blk * 8), dx[blk]);
+        float acc[NM];
+#pragma unroll
+        for (int m = 0; m < NM; m++) acc[m] = 0.f;
+        for (int blk = lane; blk < nblk; blk += 32) {
+            const uint8_t* aq = at + (size_t)blk * kActBlkStride;
+            float d[NM];
+            q4k_block_dots<NM>(row0 + blk * SZ_Q4_K, row_bytes, [&](int i) { return *reinterpret_cast<const uint4*>(aq + 16 * i); }, *reinterpret_cast<const uint4*>(bs32 + blk * 8), dx[blk], d);
+#pragma unroll
+            for (int m = 0; m < NM; m++) acc[m] += d[m];
+        }
         __syncwarp();                       // every lane is done reading the slot: hand it back to the copy engine
         slot_u = (slot_u + 1 == SLOTS) ? 0 : slot_u + 1;
         issue_one();
-        if (PAIR && !(n & 1)) { acc_first = acc; continue; }
-        float g = PAIR ? acc_first : acc, uu = acc;
+        float g = acc[0], uu = acc[NM - 1];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             g += __shfl_xor_sync(0xffffffffu, g, o);
@@ -520,7 +540,7 @@ __global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(
 
 // both row phases of T tokens in one launch (moe_block.cu), planned in moe.cu
 struct MoeRowsPlan {
-    static constexpr int kWarps = 16, kSlotsUp = 3, kSlotsDown = 2;      // 512 threads: 128 registers
+    static constexpr int kWarps = 16, kSlotsUp = 2, kSlotsDown = 2;      // 512 threads: 128 registers
     RowsParams rows;
     ReduceParams down;
     int warps, grid, act_tok, tc, nrows_max, pcap;

@@ -144,7 +144,7 @@ static int cfg_pipe() { static int v = env_int("KTB200_PIPE", 2); return v; }   
 static int cfg_nb() { static int v = env_int("KTB200_NB", 2); return v == 4 ? 4 : 2; }
 // bulk-copy generation (gemv_bulk.cuh): KTB200_BULK=0 disables it, *_SLOTS_* = ring depth, KTB200_BULK_WARPS caps the CTA
 static int cfg_bulk() { static int v = env_int("KTB200_BULK", 1); return v; }
-static int cfg_bulk_slots_up() { static int v = env_int("KTB200_BULK_SLOTS_UP", 3); return v == 2 ? 2 : (v == 4 ? 4 : 3); }
+static int cfg_bulk_slots_up() { static int v = env_int("KTB200_BULK_SLOTS_UP", 2); return v == 3 ? 3 : 2; }
 static int cfg_bulk_slots_down() { static int v = env_int("KTB200_BULK_SLOTS_DOWN", 2); return v == 3 ? 3 : 2; }
 static int cfg_bulk_warps() { static int v = env_int("KTB200_BULK_WARPS", kBulkMaxWarps); return v < 1 ? 1 : (v > kBulkMaxWarps ? kBulkMaxWarps : v); }
 constexpr size_t kSmemCap = 232448 - 512;   // 227 KB opt-in limit minus the kernels' static shared variables
@@ -209,13 +209,13 @@ static int launch_rows_pipe(const RowsParams& p, int T, int device, cudaStream_t
     return KTB200_OK;
 }
 
-// Shared-memory plan of rows_bulk_q4k<., S> for T tokens of `nslots` sets of rows each: returns the warp count (0 = does not fit)
-static int rows_bulk_plan(int ncols, int nslots, int T, int S, int max_warps, int* act_tok_out, int* tc_out, size_t* smem_out) {
-    const int nblk = ncols / QK_K, row_bytes = nblk * SZ_Q4_K, act_tok = (nblk * kActBlkStride + nblk * 16 + nblk * 4 + 15) & ~15;
+// Shared-memory plan of rows_bulk_q4k<., S> for T tokens of `nslots` sets of rows each, `nm` rows a unit: returns the warp count (0 = does not fit)
+static int rows_bulk_plan(int ncols, int nm, int nslots, int T, int S, int max_warps, int* act_tok_out, int* tc_out, size_t* smem_out) {
+    const int nblk = ncols / QK_K, row_bytes = nm * nblk * SZ_Q4_K, act_tok = (nblk * kActBlkStride + nblk * 16 + nblk * 4 + 15) & ~15;
     if (nblk < 16) return 0;                             // needs >= 16 blocks per row to keep most lanes busy
-    // tokens per chunk: as many (<= 8) as fit next to 12 rings; then as many warps as fit
+    // tokens per chunk: as many (<= 8) as fit next to 12 rings (of two rows a unit: 8); then as many warps as fit
     int tc = T < 8 ? T : 8;
-    while (tc > 1 && (size_t)tc * (act_tok + nslots * 4) + 64 + (size_t)12 * S * (row_bytes + 8) > kSmemCap) tc--;
+    while (tc > 1 && (size_t)tc * (act_tok + nslots * 4) + 64 + (size_t)(nm == 2 ? 8 : 12) * S * (row_bytes + 8) > kSmemCap) tc--;
     const size_t head = (((size_t)tc * act_tok + (size_t)tc * nslots * 4 + 15) & ~(size_t)15);
     if (head + 64 >= kSmemCap) return 0;
     int W = (int)((kSmemCap - head - 16) / ((size_t)S * (row_bytes + 8)));
@@ -232,10 +232,10 @@ static int launch_rows_bulk_q4k(const RowsParams& p, int T, int device, cudaStre
     const int nslots = p.slots + (p.x0 ? 1 : 0);
     const long total = (long)nslots * p.rows;
     if (total >= (1L << 26) || nslots > 200) return 1;
-    const int S = cfg_bulk_slots_up();
+    const int S = PAIR ? cfg_bulk_slots_up() : 3;
     int act_tok = 0, tc = 0;
     size_t smem = 0;
-    const int W = rows_bulk_plan(p.ncols, nslots, T, S, cfg_bulk_warps(), &act_tok, &tc, &smem);
+    const int W = rows_bulk_plan(p.ncols, PAIR ? 2 : 1, nslots, T, S, cfg_bulk_warps(), &act_tok, &tc, &smem);
     if (!W) return 1;
     int gx = num_sms(device);            // one CTA per SM walks all T tokens
     if (gx > total) gx = (int)total;
@@ -245,7 +245,7 @@ static int launch_rows_bulk_q4k(const RowsParams& p, int T, int device, cudaStre
         KTB_CUDA_CHECK(cudaFuncSetAttribute(rows_bulk_q4k_kernel<PAIR, SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
         rows_bulk_q4k_kernel<PAIR, SL><<<gx, W * 32, smem, stream>>>(p, act_tok, tc);                                  \
     } while (0)
-    if (S == 2) KTB_BULK_ROWS(2); else if (S == 4) KTB_BULK_ROWS(4); else KTB_BULK_ROWS(3);
+    if (S == 2) KTB_BULK_ROWS(2); else KTB_BULK_ROWS(3);
 #undef KTB_BULK_ROWS
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
@@ -684,7 +684,7 @@ bool moe_rows_plan(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, cons
     const FmtId fd = pick_fmt(c.down_type, m->down_layout);
     const int wd = fd == FMT_Q6K4T ? rows_plan_down<BulkQ6K4T>(o->down, T, m->device, o, &down) : fd == FMT_Q4K ? rows_plan_down<BulkQ4K>(o->down, T, m->device, o, &down) : 0;
     if (wd < 4) return false;
-    o->warps = rows_bulk_plan(c.hidden_size, ns, T, MoeRowsPlan::kSlotsUp, std::min(wd, (int)MoeRowsPlan::kWarps), &o->act_tok, &o->tc, &up);
+    o->warps = rows_bulk_plan(c.hidden_size, 2, ns, T, MoeRowsPlan::kSlotsUp, std::min(wd, (int)MoeRowsPlan::kWarps), &o->act_tok, &o->tc, &up);
     if (o->warps < 4) return false;
     o->smem = std::max(up, down);      // (planned for at least as many warps)
     return true;

@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) moe_block_kernel(const BlockPara
 // router, the selection, two barriers and the ends of the streams are 22 us that nothing overlaps (7 tokens: 450 us); here the router's rows are read once for all tokens, a CTA
 // per token selects, and the (token, slot) pairs form one work list for gate and up and one for down, streamed by the row kernels' bodies (gemv_bulk.cuh).  The order of every sum is
 // the separate launches', so the results are their bits.  What bounds it: the bytes of every pair's expert at ~5 TB/s (an expert that two of a few tokens choose is rare).
-// 256 experts of 2048 x 7168, 8 chosen: 2 tokens 134 -> 124 us, 4 260 -> 222, 7 450 -> 377 (the separate launches 374); 64 of 1024 x 4096, 6 chosen: 7 tokens 214 -> 151.
+// 256 experts of 2048 x 7168, 8 chosen: 2 tokens 134 -> 121 us, 4 260 -> 208, 7 450 -> 362; 64 of 1024 x 4096, 6 chosen: 7 tokens 214 -> 137.
 template <int NT>
 __device__ __forceinline__ void many_router(const GateParams& g, int nt) {      // gate_dot's order of sums (gate.cuh)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5, E = g.E, S = g.S, n4 = g.H / 4;
