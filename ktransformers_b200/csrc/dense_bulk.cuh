@@ -14,6 +14,11 @@ namespace ktb {
 
 constexpr int kDenseMaxTokens = 8;
 constexpr int kDenseWarps = 16;
+// Two CTAs an SM where eight warps or more fit into half of its shared memory (a row or two of activations).  The streams of two neighbouring launches then overlap: a
+// launch's weights are requested while the one before it ends, and with two CTAs of one launch on an SM one quantises or ends while the other streams.  A launch of few units
+// keeps one CTA an SM.  In a graph of such launches: 16384 -> 7168 19.4 -> 18.2 us, 7168 -> 18432 22.2 -> 17.8, 1536 -> 24576 7.8 -> 6.4, 4096 -> 4096 5.75 -> 4.9;
+// 7168 -> 1536 4.95 -> 4.6 with one CTA an SM (5.1 with two), 512 -> 16000 3.3 -> 3.0 (3.4).  Three slots a warp (fewer warps) 10-30 % slower.
+constexpr int kDenseWarpsTwo = 12, kDenseSmemTwo = 114000;
 
 struct DenseParams {
     const uint8_t* w;      // [rows][nblk] Q4_K blocks
@@ -26,8 +31,8 @@ struct DenseParams {
     int act_tok;           // bytes of one staged activation row
 };
 
-template <int SLOTS>
-__global__ void __launch_bounds__(kDenseWarps * 32, 1) dense_q4k_kernel(const DenseParams p) {
+template <int SLOTS, int WARPS, int CTAS>
+__global__ void __launch_bounds__(WARPS * 32, CTAS) dense_q4k_kernel(const DenseParams p) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
     griddep_launch_dependents();

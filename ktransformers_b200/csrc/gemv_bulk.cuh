@@ -8,7 +8,7 @@
 //   * every ring slot is filled by ONE `cp.async.bulk.shared.global` issued by one lane and tracked by an
 //     mbarrier (expect_tx / complete_tx): no per-lane copy instructions, no LSU time for the copy;
 //   * slots are one output's weight rows (Q4_K gate and up: 2 nblk x 144 B) or one 4-row item (down) and a warp keeps SLOTS-1
-//     of them in flight while it computes on one: smaller slots -> up to 18 warps per SM (was 12);
+//     of them in flight while it computes on one: no copy holds a lane;
 //   * unit -> (slot, row) bookkeeping is incremental (one division per token instead of one per unit);
 //   * Q6_K down tensors are re-tiled once at load time into 4-row "chunk-major" items (`repack_q6k4t`, moe.cu):
 //       item = rows 4q..4q+3 of one expert, f = rw*nb + blk (nrb = 4*nb (row, block) pairs)

@@ -263,25 +263,21 @@ static int launch_dense_q4k(const RowsParams& p, int T, int device, cudaStream_t
     else if (nblk <= 32) { d.R = 1; d.G = 1; d.segb = nblk; }
     else { d.R = 1; d.G = (nblk + 31) / 32; if (nblk % d.G) return 1; d.segb = nblk / d.G; }
     d.act_tok = (nblk * kActBlkStride + nblk * 16 + nblk * 4 + 15) & ~15;
-    constexpr int SL = 4;
-    const size_t head = (((size_t)T * d.act_tok + 15) & ~(size_t)15);
-    const size_t seg = (size_t)d.segb * SZ_Q4_K;
-    if (head + 64 >= kSmemCap) return 1;
-    int W = (int)((kSmemCap - head - 16) / (SL * (seg + 8)));
-    if (W > kDenseWarps) W = kDenseWarps;
-    if (W < 4) return 1;
-    const size_t smem = head + (((size_t)W * SL * 8 + 15) & ~(size_t)15) + (size_t)W * SL * seg;
-    const int nunits = (p.rows + d.R - 1) / d.R;
-    int gx = num_sms(device);
-    if (gx > nunits) gx = nunits;
-    static size_t limit[64] = {};
-    if (limit[device & 63] < smem) {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(dense_q4k_kernel<SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        limit[device & 63] = smem;
-    }
-    KTB_CUDA_CHECK(launch_pdl(dense_q4k_kernel<SL>, dim3(gx), dim3(W * 32), smem, stream, d));
-    count_launch();
-    return KTB200_OK;
+    const size_t head = (((size_t)T * d.act_tok + 15) & ~(size_t)15), seg = (size_t)d.segb * SZ_Q4_K;
+    const int nunits = (p.rows + d.R - 1) / d.R, sms = num_sms(device);
+    // CTAs of as many warps (`least` or more) as fit with SL slots each into `cap` bytes
+    auto go = [&](auto fn, int SL, int max_warps, int least, size_t cap, int ctas) -> int {
+        if (head + 64 >= cap) return 1;
+        const int W = std::min<int>(max_warps, (int)((cap - head - 16) / (SL * (seg + 8))));
+        if (W < least) return 1;
+        const size_t smem = head + (((size_t)W * SL * 8 + 15) & ~(size_t)15) + (size_t)W * SL * seg;
+        KTB_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(launch_pdl(fn, dim3(std::min(ctas, nunits)), dim3(W * 32), smem, stream, d));
+        count_launch();
+        return KTB200_OK;
+    };
+    const int rc = go(dense_q4k_kernel<2, kDenseWarpsTwo, 2>, 2, kDenseWarpsTwo, 8, kDenseSmemTwo, nunits > kDenseWarpsTwo * sms ? 2 * sms : sms);
+    return rc != 1 ? rc : go(dense_q4k_kernel<4, kDenseWarps, 1>, 4, kDenseWarps, 4, kSmemCap, sms);
 }
 
 template <bool PAIR>
