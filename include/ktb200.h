@@ -356,8 +356,8 @@ int ktb200_mla_absorb_o(const void* attn_latent_dev, const void* w_uv_dev, int n
 
 /* ------------------------------------------------------------------------------------------
  * One decode step of a DeepSeek attention layer (bf16, latents of 512 + 64, projections on GGUF blocks), in one call: q_a, norm, q_b (q_rank 0: `q_a` is the whole query
- * projection), kv_a, ktb200_mla_step_prep, ktb200_mla_absorb_q, ktb200_mla_decode, ktb200_mla_absorb_o, o (archive/ktransformers/operators/attention.py:395-478).  The linears'
- * hidden type has to be bf16; biases fp32 or NULL; w_uk [heads][nope][512] and w_uv [heads][v][512] bf16; positions as for ktb200_mla_step_prep; page_table
+ * projection), kv_a, ktb200_mla_step_prep, ktb200_mla_absorb_q, ktb200_mla_decode, ktb200_mla_absorb_o, o (archive/ktransformers/operators/attention.py:395-478).  The linears have to be of the
+ * sizes that the step's imply, in bf16 and on one device (KTB200_EINVAL before any launch otherwise); biases fp32 or NULL; w_uk [heads][nope][512] and w_uv [heads][v][512] bf16; positions as for ktb200_mla_step_prep; page_table
  * [batch][table_pages], kv_len [batch] (written); workspace as for ktb200_mla_decode; scratch of ktb200_latent_step_bytes, 256-byte aligned, used on `stream` only.
  * ------------------------------------------------------------------------------------------ */
 typedef struct ktb200_latent_step_params {

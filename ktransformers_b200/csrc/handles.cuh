@@ -19,6 +19,12 @@ static inline FmtId pick_fmt(int type, int layout) {
 }  // namespace ktb
 
 // ------------------------------------------------------------------------------------------
+struct ktb200_linear {
+    int in_size, out_size, proj_type, hidden_type, group_max_len, device;
+    const void* proj;
+    bool loaded, soa;
+};
+
 struct ktb200_mlp {
     int H, I, gate_type, up_type, down_type, hidden_type, group_max_len, device;
     const void *gate, *up, *down;

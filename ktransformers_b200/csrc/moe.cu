@@ -771,12 +771,6 @@ int ktb200_moe_forward_host(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
 }
 
 // ------------------------------------------------------------------------------------------ linear
-struct ktb200_linear {
-    int in_size, out_size, proj_type, hidden_type, group_max_len, device;
-    const void* proj;
-    bool loaded, soa;
-};
-
 // Whether a linear of T rows runs as a tensor-core GEMM (kq_gemm.cu).  The row kernels keep up to 8 rows of activations on the SM and read the weights once for
 // them; beyond, once more for every row.  The GEMM's two or three launches take 19-25 us however small the matrix is, and small ones are done by then: the row kernels
 // take about 8 us and, per row, R (500 + 0.35 K) 1e-6 us (512 -> 512: 14 us at 16 rows, 18 at 32, 30 at 64 against 21-25), of Q6_K 1.7 times that;

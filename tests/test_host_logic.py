@@ -67,6 +67,54 @@ def test_error_codes_map_to_reference_exceptions():
         native.check(lib.ktb200_dequantize(1, 12, 100, 1, 0, None))                    # n not a multiple of the block
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="handles on addresses that no GPU may read")
+def test_latent_step_refuses_linears_that_do_not_fit_its_scratch():
+    """Every linear writes rows of its own size and type into scratch that is laid out for the step's: what does not match is refused before any launch."""
+    import ctypes as C
+
+    from ktransformers_b200 import native
+    lib, Q4_K, BF16, F32 = native.lib(), 12, native.GGML_BF16, native.GGML_F32
+    hidden, heads, nope, v, rank = 1024, 16, 128, 128, 512
+
+    def linear(n_in, n_out, hid=BF16, device=0, load=True):
+        h = C.c_void_p()
+        native.check(lib.ktb200_linear_create(n_in, n_out, 4096, Q4_K, hid, 8, device, C.byref(h)))
+        if load:
+            native.check(lib.ktb200_linear_load_weights(h, None))
+        return h
+
+    def step(q_rank=rank, scratch=1 << 20, less=0, **other):
+        lin = dict(q_a=(hidden, q_rank or heads * (nope + 64)), q_b=(rank, heads * (nope + 64)), kv_a=(hidden, 576), o=(heads * v, hidden))
+        lin = {n: linear(*other[n][0], **other[n][1]) if n in other else linear(*a) for n, a in lin.items()}
+        p = native.LatentStepParams(batch=2, heads=heads, nope_dim=nope, v_dim=v, q_rank=q_rank, page_size=64, max_pages=4, table_pages=4, x=4096, out=4096, q_norm=4096, scratch=scratch,
+                                    scratch_bytes=lib.ktb200_latent_step_bytes(2, heads, nope, v, q_rank) - less, **lin)
+        n0 = native.launch_count()
+        rc = lib.ktb200_latent_step(C.byref(p), None)
+        assert native.launch_count() == n0
+        for h in lin.values():
+            lib.ktb200_linear_destroy(h)
+        return rc
+
+    ok = {n: a for n, a in (("q_a", (hidden, rank)), ("q_b", (rank, heads * 192)), ("kv_a", (hidden, 576)), ("o", (heads * v, hidden)))}
+    for name, (n_in, n_out) in ok.items():
+        with pytest.raises(ValueError, match="latent_step: "):
+            native.check(step(**{name: ((n_in + 256, n_out), {})}))
+        if name != "o":      # (its rows leave to the caller's buffer, of whatever width)
+            with pytest.raises(ValueError, match="latent_step: " + name):
+                native.check(step(**{name: ((n_in, n_out + 64), {})}))
+        with pytest.raises(ValueError, match="latent_step: " + name):
+            native.check(step(**{name: ((n_in, n_out), dict(hid=F32))}))
+        with pytest.raises(ValueError, match="latent_step: "):
+            native.check(step(**{name: ((n_in, n_out), dict(device=1))}))
+        with pytest.raises(native.KTB200Error, match="Not Loaded"):
+            native.check(step(**{name: ((n_in, n_out), dict(load=False))}))
+    with pytest.raises(ValueError, match="latent_step: q_a"):
+        native.check(step(q_rank=0, q_a=((hidden, rank), {})))
+    for bad in (dict(scratch=(1 << 20) + 16), dict(less=1)):
+        with pytest.raises(ValueError, match="latent_step: bad shape"):
+            native.check(step(**bad))
+
+
 # ------------------------------------------------------------------------------------------ GGUF + injection
 E, H, I, K = 4, 256, 256, 2
 
