@@ -41,6 +41,9 @@ void count_launch(int n = 1);
     } while (0)
 
 int num_sms(int device);
+// Raises `kernel`'s limit of dynamic shared memory on the current device to `bytes` and never lowers it (runtime.cu): the limit belongs to the kernel, and threads launch the
+// same one with different sizes
+cudaError_t raise_smem_limit(const void* kernel, size_t bytes);
 // stream-ordered scratch from a bounded pool (runtime.cu); ScratchBlock gives it back behind the work already queued on the stream
 cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out);
 void scratch_prepare(int device);      // when a handle is created: its calls may then be captured from the first on

@@ -130,7 +130,7 @@ extern "C" int ktb200_moe_gate_forward(const ktb200_gate_config* c, int qlen, co
     size_t smem = (size_t)nt * nc4_max * 16;
     const size_t smem_sel = ((size_t)2 * c->n_experts + 32 + 4 * kGateWarps) * sizeof(float);
     if (smem_sel > smem) smem = smem_sel;
-    if (smem > 48 * 1024) KTB_CUDA_CHECK(cudaFuncSetAttribute(gate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) KTB_CUDA_CHECK(raise_smem_limit((const void*)gate_kernel, smem));
     gate_kernel<<<dim3(row_ctas, S), kGateThreads, smem, s>>>(p);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;

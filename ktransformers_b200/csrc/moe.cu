@@ -60,7 +60,7 @@ static int repack_q6k(void* w, long rows_total, int ncols, int device, cudaStrea
         set_error("Q6_K repack: row too long (%d cols)", ncols);
         return KTB200_EINVAL;
     }
-    KTB_CUDA_CHECK(cudaFuncSetAttribute(repack_q6k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KTB_CUDA_CHECK(raise_smem_limit((const void*)repack_q6k_kernel, smem));
     long grid = n_groups < (long)num_sms(device) * 8 ? n_groups : (long)num_sms(device) * 8;
     if (grid < 1) grid = 1;
     repack_q6k_kernel<<<(unsigned)grid, 256, smem, stream>>>(reinterpret_cast<uint8_t*>(w), n_groups, nb);
@@ -115,7 +115,7 @@ static int repack_q6k4t(void* w, long rows_total, int ncols, int device, cudaStr
         set_error("Q6_K tile repack: unsupported shape (%ld rows x %d cols)", rows_total, ncols);
         return KTB200_EINVAL;
     }
-    KTB_CUDA_CHECK(cudaFuncSetAttribute(repack_q6k4t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KTB_CUDA_CHECK(raise_smem_limit((const void*)repack_q6k4t_kernel, smem));
     long grid = n_items < (long)num_sms(device) * 8 ? n_items : (long)num_sms(device) * 8;
     if (grid < 1) grid = 1;
     repack_q6k4t_kernel<<<(unsigned)grid, 256, smem, stream>>>(reinterpret_cast<uint8_t*>(w), n_items, nb);
@@ -128,7 +128,7 @@ static int repack_q6k4t(void* w, long rows_total, int ncols, int device, cudaStr
 template <typename K>
 static int set_smem_attr(K kernel, size_t smem) {
     if (smem > 48 * 1024) {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)kernel, smem));
     }
     return KTB200_OK;
 }
@@ -199,10 +199,10 @@ static int launch_rows_pipe(const RowsParams& p, int T, int device, cudaStream_t
     if (gx < 1) gx = 1;
     dim3 grid(gx, T);
     if (warps == 12) {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(rows_pipe_kernel<Fmt, PAIR, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)rows_pipe_kernel<Fmt, PAIR, 12>, smem));
         rows_pipe_kernel<Fmt, PAIR, 12><<<grid, 12 * 32, smem, stream>>>(p, act, slot);
     } else {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(rows_pipe_kernel<Fmt, PAIR, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)rows_pipe_kernel<Fmt, PAIR, 8>, smem));
         rows_pipe_kernel<Fmt, PAIR, 8><<<grid, 8 * 32, smem, stream>>>(p, act, slot);
     }
     KTB_LAUNCH_CHECK();
@@ -242,7 +242,7 @@ static int launch_rows_bulk_q4k(const RowsParams& p, int T, int device, cudaStre
     if (gx < 1) gx = 1;
 #define KTB_BULK_ROWS(SL)                                                                                              \
     do {                                                                                                               \
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(rows_bulk_q4k_kernel<PAIR, SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)rows_bulk_q4k_kernel<PAIR, SL>, smem)); \
         rows_bulk_q4k_kernel<PAIR, SL><<<gx, W * 32, smem, stream>>>(p, act_tok, tc);                                  \
     } while (0)
     if (S == 2) KTB_BULK_ROWS(2); else KTB_BULK_ROWS(3);
@@ -271,7 +271,7 @@ static int launch_dense_q4k(const RowsParams& p, int T, int device, cudaStream_t
         const int W = std::min<int>(max_warps, (int)((cap - head - 16) / (SL * (seg + 8))));
         if (W < least) return 1;
         const size_t smem = head + (((size_t)W * SL * 8 + 15) & ~(size_t)15) + (size_t)W * SL * seg;
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)fn, smem));
         KTB_CUDA_CHECK(launch_pdl(fn, dim3(std::min(ctas, nunits)), dim3(W * 32), smem, stream, d));
         count_launch();
         return KTB200_OK;
@@ -357,11 +357,11 @@ static int launch_reduce_pipe_q6k8(const ReduceParams& p, int T, int device, cud
     dim3 grid(gx, T);
     if (want_slots != 2 && base + (size_t)24 * slot <= 220 * 1024) {
         const size_t smem = base + (size_t)24 * slot;
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(reduce_pipe_q6k8_kernel<24, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)reduce_pipe_q6k8_kernel<24, 1>, smem));
         reduce_pipe_q6k8_kernel<24, 1><<<grid, 24 * 32, smem, stream>>>(p, slot);
     } else if (base + (size_t)12 * 2 * slot <= 220 * 1024) {
         const size_t smem = base + (size_t)12 * 2 * slot;
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(reduce_pipe_q6k8_kernel<12, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)reduce_pipe_q6k8_kernel<12, 2>, smem));
         reduce_pipe_q6k8_kernel<12, 2><<<grid, 12 * 32, smem, stream>>>(p, slot);
     } else {
         return 1;
@@ -417,10 +417,10 @@ static int launch_reduce_bulk(const ReduceParams& p, int T, int device, cudaStre
     const int W = reduce_bulk_plan<Fmt>(p.rows, p.ncols, pcap, S, device, &gx, &nrows_max, &smem);
     if (!W) return 1;
     if (S == 3) {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(reduce_bulk_kernel<Fmt, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)reduce_bulk_kernel<Fmt, 3>, smem));
         reduce_bulk_kernel<Fmt, 3><<<gx, W * 32, smem, stream>>>(p, nrows_max, pcap);
     } else {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(reduce_bulk_kernel<Fmt, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)reduce_bulk_kernel<Fmt, 2>, smem));
         reduce_bulk_kernel<Fmt, 2><<<gx, W * 32, smem, stream>>>(p, nrows_max, pcap);
     }
     KTB_LAUNCH_CHECK();

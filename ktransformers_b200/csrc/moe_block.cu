@@ -1171,8 +1171,8 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
         static size_t limit[6][64] = {};
         static int resident[6][64] = {};
         const int v = (all_at_once ? 4 : W > kBlockWarpsLo ? 2 : 0) + (fd == FMT_Q6K4T ? 1 : 0);
+        KTB_CUDA_CHECK(raise_smem_limit(fn, smem));
         if (limit[v][dev & 63] < smem) {
-            KTB_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int per_sm = 0;
             KTB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, W * 32, smem));
             resident[v][dev & 63] = per_sm * num_sms(dev);
@@ -1291,8 +1291,8 @@ extern "C" int ktb200_moe_ep_block_forward(const ktb200_gate_config* gc, ktb200_
         static size_t limit[2][64] = {};
         static int resident[2][64] = {};
         const int v = fd == FMT_Q6K4T ? 1 : 0;
+        KTB_CUDA_CHECK(raise_smem_limit(fn, smem));
         if (limit[v][dev & 63] < smem) {
-            KTB_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int per_sm = 0;
             KTB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, W * 32, smem));
             resident[v][dev & 63] = per_sm * num_sms(dev);

@@ -3,7 +3,9 @@
 #include <cstdarg>
 #include <cstdio>
 #include <atomic>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "gemv_bulk.cuh"
 
@@ -34,6 +36,20 @@ int num_sms(int device) {
         cached[device] = n;
     }
     return cached[device];
+}
+
+cudaError_t raise_smem_limit(const void* kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> limits;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& limit = limits[{kernel, device}];
+    if (limit >= bytes) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) limit = bytes;
+    return e;
 }
 
 // Scratch of one call, taken and given back in stream order from a pool of this library's own (one per device): safe for any number of

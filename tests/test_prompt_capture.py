@@ -113,5 +113,51 @@ def test_two_threads_on_two_streams():
     assert not failed, failed
 
 
+# decode sizes: one kernel with two sizes of shared memory, a thread each.  Linears of one row (two CTAs an SM) and of six (one), MLPs through both row kernels
+@pytest.mark.parametrize("kind,rows,sizes", [("linear", 1, [(16384, 512), (1024, 512)]), ("linear", 6, [(14336, 512), (2048, 512)]), ("mlp", 1, [(16384, 512), (4096, 256)]), ("mlp", 4, [(8192, 2048), (4096, 512)])])
+def test_two_threads_with_one_kernel_at_two_sizes(kind, rows, sizes):
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, jobs, failed = native.lib(), [], []
+    for K, R in sizes:
+        h = C.c_void_p()
+        keep = [synth_blocks(t, R * K, "cuda", 1 + i) for i, t in enumerate((Q4_K, Q4_K, Q6_K))]
+        if kind == "linear":
+            native.check(lib.ktb200_linear_create(K, R, keep[0].data_ptr(), Q4_K, BF16, rows, 0, C.byref(h)))
+            native.check(lib.ktb200_linear_load_weights(h, torch.cuda.current_stream().cuda_stream))
+        else:
+            native.check(lib.ktb200_mlp_create(K, R, *[t.data_ptr() for t in keep], Q4_K, Q4_K, Q6_K, BF16, rows, 0, C.byref(h)))
+            native.check(lib.ktb200_mlp_load_weights(h, torch.cuda.current_stream().cuda_stream))
+        x = _inputs(torch.empty((rows, K), dtype=torch.bfloat16, device="cuda"), K)
+        y, want = (torch.zeros((rows, R if kind == "linear" else K), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+
+        def call(y, stream, h=h, x=x):
+            if kind == "linear":
+                return lib.ktb200_linear_forward(h, rows, x.data_ptr(), y.data_ptr(), None, None, stream)
+            return lib.ktb200_mlp_forward(h, rows, x.data_ptr(), y.data_ptr(), 0, None, stream)
+
+        native.check(call(want, torch.cuda.current_stream().cuda_stream))
+        jobs.append((call, y, want, keep))
+    torch.cuda.synchronize()
+
+    def work(call, y, want, keep):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                stream = torch.cuda.current_stream().cuda_stream
+                for i in range(3000):
+                    native.check(call(y, stream))
+                if not torch.equal(y, want):
+                    failed.append("other bits")
+        except Exception as e:
+            failed.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+
+
 if __name__ == "__main__":
     _captured_first(sys.argv[1])
