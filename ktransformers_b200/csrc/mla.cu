@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         if (lane == 0) {
             for (int j = kStages; j < n; j++) {
                 const int s = j % kStages;
-                bar_wait_polling(smem_u32(&misc.k_empty[s]), ((j / kStages) & 1) ^ 1);
+                bar_wait(smem_u32(&misc.k_empty[s]), ((j / kStages) & 1) ^ 1);
                 const int t_base = (tile0 + j) * kLT;
                 const int page = p.page_table[prow + (t_base / p.page_size) % p.max_pages];
                 const int row = page * p.page_size + t_base % p.page_size;
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             constexpr uint32_t idesc_pv = instr_desc(1, 1, 1, 1, 0, 128, kHG);    // A MN-major (V^T from the [token][latent] tile), 128 x 64
             auto issue_qk = [&](int j) {
                 const int s = j % kStages, buf = j & 1;
-                bar_wait_polling(smem_u32(&misc.s_empty[buf]), ((j >> 1) & 1) ^ 1);
-                bar_wait_polling(smem_u32(&misc.k_full[s]), (j / kStages) & 1);
+                bar_wait(smem_u32(&misc.s_empty[buf]), ((j >> 1) & 1) ^ 1);
+                bar_wait(smem_u32(&misc.k_full[s]), (j / kStages) & 1);
                 tc_fence_after();
                 const uint32_t kb = base + s * kStageBytes, qb = base + kOffQ;
 #pragma unroll
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             issue_qk(0);
             for (int j = 0; j < n; j++) {
                 if (j + 1 < n) issue_qk(j + 1);
-                bar_wait_polling(smem_u32(&misc.p_full), j & 1);
+                bar_wait(smem_u32(&misc.p_full), j & 1);
                 tc_fence_after();
                 const int s = j % kStages;
                 const uint32_t kb = base + s * kStageBytes, pb = base + kOffP + (j & 1) * kPStride;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         float m_ref = -INFINITY, m_run = -INFINITY, l = 0.f;   // l: this lane's half of the row sum
         for (int j = 0; j < n; j++) {
             const int buf = j & 1;
-            bar_wait_polling(smem_u32(&misc.s_full[buf]), (j >> 1) & 1);
+            bar_wait(smem_u32(&misc.s_full[buf]), (j >> 1) & 1);
             tc_fence_after();
             if (p.debug && st == 0 && split == 0 && hg == 0 && b == 0 && j < 60) reinterpret_cast<unsigned long long*>(p.debug + 2048)[64 + j] = gtime();
             uint32_t sv[32];
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             const bool any = misc.need[buf][0] | misc.need[buf][1] | misc.need[buf][2] | misc.need[buf][3];
             if (any) {
                 // O^T must be quiescent: the previous PV has to be complete (it also frees the other P buffer)
-                bar_wait_polling(smem_u32(&misc.p_free[(j - 1) & 1]), ((j - 1) >> 1) & 1);
+                bar_wait(smem_u32(&misc.p_free[(j - 1) & 1]), ((j - 1) >> 1) & 1);
                 tc_fence_after();
                 const float a = need ? ex2(m_ref - m_run) : 1.f;
                 if (!upper) misc.alpha[head] = a;
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
                 asm volatile("bar.sync 1, 128;" ::: "memory");   // alpha[] / need[] may be rewritten only after everyone used them
             }
             // this tile's P buffer was last read by PV(j - 2)
-            if (j >= 2) bar_wait_polling(smem_u32(&misc.p_free[buf]), ((j >> 1) & 1) ^ 1);
+            if (j >= 2) bar_wait(smem_u32(&misc.p_free[buf]), ((j >> 1) & 1) ^ 1);
             {
                 float ps = 0.f;
                 uint32_t pk[8], pl[8];
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         // ---- epilogue: O^T / l -> fp32 partial output, base-2 LSE ---------------------------------------------------
         l += __shfl_xor_sync(0xffffffffu, l, 16);
         if (!upper) { misc.l[head] = l; misc.m[head] = m_ref; }
-        bar_wait_polling(smem_u32(&misc.p_free[(n - 1) & 1]), ((n - 1) >> 1) & 1);   // the last PV (and with it every earlier one) is complete
+        bar_wait(smem_u32(&misc.p_free[(n - 1) & 1]), ((n - 1) >> 1) & 1);   // the last PV (and with it every earlier one) is complete
         tc_fence_after();
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (p.debug && st == 0 && split == 0 && hg == 0 && b == 0) {

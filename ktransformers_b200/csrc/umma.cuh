@@ -50,26 +50,6 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
     atomicAdd(&g_bar_wait_gave_up, 1u);
     return false;
 }
-// The same without suspending the thread between polls (test_wait), for a chain of hand-overs with issue slots to spare: a suspended thread wakes late (latent decode
-// attention, 128 k keys: 91 us with bar_wait, 86 with this, 122 with a longer suspension).
-constexpr uint32_t kBarPollLimit = 1u << 27;
-__device__ __forceinline__ bool bar_wait_polling(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kBarPollLimit; it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    atomicAdd(&g_bar_wait_gave_up, 1u);
-    return false;
-}
 // generic-proxy writes to shared memory (st.shared) -> visible to the async proxy (TMA, tcgen05.mma operand reads)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
