@@ -19,7 +19,7 @@ from ..models.custom_cache import StaticCache
 from ..models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3RMSNorm, DeepseekV3RotaryEmbedding, apply_rotary_pos_emb
 from ..util.utils import InferenceState
 from .base_operator import BaseInjectedModule
-from .flashinfer_wrapper import MLAWrapperSingleton
+from .flashinfer_wrapper import MLAWrapper, MLAWrapperSingleton
 
 
 def _is_plain(module, cls) -> bool:
@@ -113,8 +113,10 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
             w.max_pages_per_seq = cache.max_pages
         inv_freq = rot.inv_freq.to(x.device)
         own = self._own_linears(x, bsz)
-        if own is not None and q_absorb.dtype == bf16 == kv.dtype and kv.is_contiguous() and w.num_heads == heads and bsz <= w.max_batch_size:
-            # everything in one call: made one by one from here, the calls' host work bounds the layer
+        if (own is not None and q_absorb.dtype == bf16 == kv.dtype and kv.is_contiguous() and w.num_heads == heads and bsz <= w.max_batch_size
+                and type(w) is MLAWrapper and "run" not in vars(w) and w.page_size == cache.page_size):
+            # everything in one call, the wrapper's `run` included (a `run` of its caller's and a plan in other pages than the cache's keep the calls below): made one by one from
+            # here, the calls' host work bounds the layer
             q_a, q_b, kv_a, o_lin = own
             rank, v_dim = get("q_lora_rank") or 0, get("v_head_dim")
             q_norm = get("q_a_layernorm") if rank else None

@@ -154,3 +154,73 @@ def test_one_call_equals_the_calls_one_by_one(bsz, heads, q_rank, pos):
         assert got[0][0] == other[0] and got[0][4] == other[4] == 1
         assert all(torch.equal(a, b) for a, b in zip(got[0][1:4], other[1:4]))
     assert got[0][1].isfinite().all() and got[0][1].abs().max() > 0
+
+
+def _layer(bsz, heads, q_rank, pos):
+    """(operator on GGUF projections, input, positions, cache(): a new cache with `pos` tokens of a fixed past)"""
+    from ktransformers_b200.models.custom_cache import StaticCache
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3Attention, DeepseekV3Config, DeepseekV3RotaryEmbedding
+    from ktransformers_b200.operators.attention import KDeepseekV2Attention
+    from ktransformers_b200.operators.linear import KTransformersLinear
+    from ktransformers_b200.util.synth import synth_blocks
+
+    torch.manual_seed(pos + heads)
+    cfg = DeepseekV3Config(hidden_size=512, num_attention_heads=heads, q_lora_rank=q_rank, num_hidden_layers=1)
+    plain = DeepseekV3Attention(cfg, layer_idx=0).to(device="cuda", dtype=torch.bfloat16)
+    plain.rotary_emb = DeepseekV3RotaryEmbedding(64).to("cuda")
+    old = torch.get_default_dtype()
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        for i, n in enumerate((["q_proj"] if q_rank is None else ["q_a_proj", "q_b_proj"]) + ["kv_a_proj_with_mqa", "o_proj"]):
+            orig = getattr(plain, n)
+            lin = KTransformersLinear("blk.0." + n, None, cfg, orig, "cuda", "KLinearB200", "cuda", None)
+            lin.load(w=(synth_blocks(12, orig.in_features * orig.out_features, "cuda", i), 12))
+            setattr(plain, n, lin)
+        op = KDeepseekV2Attention("blk.0.self_attn", None, cfg, plain, "cuda", "cuda")
+    finally:
+        torch.set_default_dtype(old)
+    x = torch.randn(bsz, 1, 512, device="cuda").to(torch.bfloat16)
+    past = torch.randn(bsz, max(pos, 1), 576, device="cuda").to(torch.bfloat16)
+
+    def cache():
+        c = StaticCache(cfg, max_batch_size=bsz, max_cache_len=pos + 2, device="cuda")
+        if pos:
+            c.key_cache[0].view(bsz, -1, 576)[:, :pos].copy_(past)
+        return c
+
+    return op, x, torch.full((bsz, 1), pos, dtype=torch.int64, device="cuda"), cache
+
+
+@pytest.mark.parametrize("bsz,heads,q_rank,pos", [(1, 128, 256, 70), (2, 16, None, 200)])
+def test_wrappers_of_the_callers_own_keep_their_run(bsz, heads, q_rank, pos):
+    """A wrapper class or an instance with another `run` is called, and one planned in pages of 32 tokens over the cache's rows reads its table in those: the bits of the one call."""
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapper
+
+    op, x, where, new_cache = _layer(bsz, heads, q_rank, pos)
+    seen, got = [], []
+
+    class Counting(MLAWrapper):
+        def run(self, *args, **kwargs):
+            seen.append("class")
+            return super().run(*args, **kwargs)
+
+    def replaced(cache):
+        w = MLAWrapper(bsz, cache.max_pages * bsz)
+        w.run = lambda *a, **k: (seen.append("instance"), MLAWrapper.run(w, *a, **k))[1]
+        return w
+
+    def other_pages(cache):
+        n = cache.max_pages * cache.page_size // 32
+        w = MLAWrapper(bsz, n * bsz)
+        w.plan(None, torch.arange(bsz + 1, dtype=torch.int32, device="cuda") * n, torch.arange(n * bsz, dtype=torch.int32, device="cuda"), where[:, 0].int() + 1, None, heads, 512, 64, 32,
+               op.softmax_scale, torch.bfloat16, torch.bfloat16)
+        return w
+
+    for make in (lambda cache: MLAWrapper(bsz, cache.max_pages * bsz), lambda cache: Counting(bsz, cache.max_pages * bsz), replaced, other_pages):
+        cache = new_cache()
+        assert cache.page_size == 64
+        op.mla_wrapper = make(cache)
+        with torch.no_grad():
+            got.append(op(x, position_ids=where, past_key_value=cache, cache_position=where[0])[0])
+    assert seen == ["class", "instance"]
+    assert got[0].abs().max() > 0 and all(torch.equal(got[0], g) for g in got[1:])
