@@ -107,14 +107,17 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         lib, stream = native.lib(), torch.cuda.current_stream(x.device).cuda_stream
         q_absorb, out_absorb = self.get_absorbed()
         kv = cache.key_cache[get("layer_idx")]
-        if w.need_plan:
-            indptr = torch.arange(0, bsz + 1, dtype=torch.int32, device=x.device) * cache.max_pages
-            w.plan(None, indptr, cache.page_table_list[self.layer_idx].reshape(-1), (position_ids[:, 0] + 1).to(torch.int32), None, heads, 512, 64, cache.page_size, self.softmax_scale, bf16, kv.dtype)
-            w.max_pages_per_seq = cache.max_pages
+
+        def planned():      # only for a step that takes a path of this function: a plan that it leaves behind is one that the path below neither makes nor checks
+            if w.need_plan:
+                indptr = torch.arange(0, bsz + 1, dtype=torch.int32, device=x.device) * cache.max_pages
+                w.plan(None, indptr, cache.page_table_list[self.layer_idx].reshape(-1), (position_ids[:, 0] + 1).to(torch.int32), None, heads, 512, 64, cache.page_size, self.softmax_scale, bf16, kv.dtype)
+                w.max_pages_per_seq = cache.max_pages
+            return w
+
         inv_freq = rot.inv_freq.to(x.device)
-        own = self._own_linears(x, bsz)
-        if (own is not None and q_absorb.dtype == bf16 == kv.dtype and kv.is_contiguous() and w.num_heads == heads and bsz <= w.max_batch_size
-                and type(w) is MLAWrapper and "run" not in vars(w) and w.page_size == cache.page_size):
+        own = self._own_linears(x, bsz) if q_absorb.dtype == bf16 == kv.dtype and kv.is_contiguous() else None
+        if own is not None and planned().num_heads == heads and bsz <= w.max_batch_size and type(w) is MLAWrapper and "run" not in vars(w) and w.page_size == cache.page_size:
             # everything in one call, the wrapper's `run` included (a `run` of its caller's and a plan in other pages than the cache's keep the calls below): made one by one from
             # here, the calls' host work bounds the layer
             q_a, q_b, kv_a, o_lin = own
@@ -146,6 +149,7 @@ class KDeepseekV2Attention(BaseInjectedModule, DeepseekV3Attention):
         kva = self.kv_a_proj_with_mqa(x)
         if not (q.dtype == bf16 == kva.dtype == q_absorb.dtype and q.is_contiguous() and kva.is_contiguous()):
             return None
+        planned()
         q_pe = torch.empty((bsz, heads, 64), dtype=bf16, device=x.device)
         q_abs = torch.empty((bsz, heads, 512), dtype=bf16, device=x.device)
         native.check(lib.ktb200_mla_step_prep(q.data_ptr(), heads, nope, kva.data_ptr(), kv_norm.weight.data_ptr(), float(kv_norm.variance_epsilon), inv_freq.data_ptr(),

@@ -224,3 +224,19 @@ def test_wrappers_of_the_callers_own_keep_their_run(bsz, heads, q_rank, pos):
             got.append(op(x, position_ids=where, past_key_value=cache, cache_position=where[0])[0])
     assert seen == ["class", "instance"]
     assert got[0].abs().max() > 0 and all(torch.equal(got[0], g) for g in got[1:])
+
+
+def test_a_step_of_another_type_leaves_no_plan_behind():
+    """bf16 hidden states whose queries come out as fp16 are refused where the wrapper is planned ("bf16 only"): not run on a plan that the step made before it knew."""
+    from ktransformers_b200.operators.flashinfer_wrapper import MLAWrapper
+
+    op, x, where, new_cache = _layer(1, 16, None, 3)
+    plain = op.orig_module
+    lin = plain.q_proj
+    plain.q_proj = type("Half", (torch.nn.Module,), dict(forward=lambda self, x: lin(x).half()))()
+    plain.kv_b_proj.half()
+    cache = new_cache()
+    w = op.mla_wrapper = MLAWrapper(1, cache.max_pages)
+    with torch.no_grad(), pytest.raises(AssertionError, match="bf16 only"):
+        op(x, position_ids=where, past_key_value=cache, cache_position=where[0])
+    assert w.need_plan
