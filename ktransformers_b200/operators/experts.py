@@ -371,6 +371,22 @@ class _KDeepseekMoEMixin:
         top = getattr(getattr(mods[0], "orig_module", None), "top_k", 0)
         return bool(native.lib().ktb200_moe_takes_gemms(gen.handle, getattr(self, "_ktb_mlp", None), n_tok, top))
 
+    def _own_classes(self):
+        """whether the modules are this library's classes themselves, with no method of a subclass or an instance that the one call would pass by"""
+        from .gate import KMoEGateB200
+        from .linear import KLinearB200, KTransformersLinear
+        if type(self).moe_kexperts is not _KDeepseekMoEMixin.moe_kexperts or "moe_kexperts" in vars(self):
+            return False
+        gen = self.experts.generate_experts
+        if not (type(self.gate) is KMoEGateB200 and type(self.experts) in (KTransformersExperts, KTransformersExpertsV2) and type(gen) is KExpertsB200 and not {"forward", "_launch"} & vars(gen).keys()):
+            return False
+        if self.config.n_shared_experts is None:
+            return True
+        shared = self.shared_experts
+        linears = [shared.gate_proj, shared.up_proj, shared.down_proj]
+        return (type(shared) is DeepseekV3MLP and shared.act_fn is torch.nn.functional.silu and all(type(p) is KTransformersLinear and type(p.generate_linear) is KLinearB200
+                                                                                                    and "forward" not in vars(p.generate_linear) for p in linears))
+
     def load(self):
         """children first (base_operator.py:45-48), then the shared expert's handle for the single-launch path: handles
         are created here, never inside forward (which may be running under CUDA-graph capture)."""
@@ -387,6 +403,8 @@ class _KDeepseekMoEMixin:
         if gen.ep_size > 1 and getattr(self, "ep_exchange", None) is None:
             return None
         if getattr(self.experts, "mode", None) != InferenceState.GENERATE or getattr(gate, "_w", None) is None:
+            return None
+        if x.numel() > _KDeepseekMoEMixin.BLOCK_MAX_TOKENS * x.shape[-1] and not self._own_classes():
             return None
         m = gate.orig_module
         from .gate import _SCORING, _TOPK

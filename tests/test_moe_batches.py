@@ -1,0 +1,140 @@
+"""KDeepseekV3MoE on batches of 9 to 47 tokens: one call of the library where that runs GEMMs and where calling the modules would do nothing else."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+Q4_K, Q6_K = 12, 14
+
+
+class _Weights:
+    """a weight loader over tensors that are there already"""
+
+    def __init__(self, raw, plain):
+        self.raw, self.plain, self.tensor_device_map = raw, plain, {}
+
+    def has_tensor(self, name):
+        return name in self.raw or name in self.plain
+
+    def get_mmap_tensor(self, name):
+        return self.raw[name][0] if "_exps" in name else self.raw[name][0].cpu().numpy()
+
+    def get_ggml_type(self, name):
+        return self.raw[name][1]
+
+    def load_gguf_tensor(self, name, device="cuda", target_dtype=None):
+        return self.plain[name].to(device=device, dtype=target_dtype or self.plain[name].dtype)
+
+
+def _block(E, k, H, I, serve=False, dtype=torch.bfloat16):
+    from ktransformers_b200.models.modeling_deepseek_v3 import DeepseekV3Config, DeepseekV3MoE
+    from ktransformers_b200.operators.experts import KDeepseekV3MoE, KDeepseekV3MoEV2, KTransformersExperts, KTransformersExpertsV2
+    from ktransformers_b200.operators.gate import KMoEGateB200
+    from ktransformers_b200.operators.linear import KTransformersLinear
+    from ktransformers_b200.util.synth import synth_blocks
+    cfg = DeepseekV3Config(hidden_size=H, moe_intermediate_size=I, n_routed_experts=E, n_shared_experts=1, num_experts_per_tok=k, n_group=1, topk_group=1)
+    key, types, g = "blk.3", {"gate": Q4_K, "up": Q4_K, "down": Q6_K}, torch.Generator(device="cuda").manual_seed(3)
+    raw = {f"{key}.ffn_{n}_exps.weight": (synth_blocks(t, E * H * I, "cuda", 1 + t + len(n)), t) for n, t in types.items()}
+    raw.update({f"{key}.shared_experts.{n}_proj.weight": (synth_blocks(t, H * I, "cuda", 51 + t + len(n)), t) for n, t in types.items()})
+    weights = _Weights(raw, {key + ".gate.weight": torch.randn((E, H), generator=g, device="cuda") * H ** -0.5,
+                             key + ".gate.e_score_correction_bias": torch.rand(E, generator=g, device="cuda") * 0.4 - 0.2})
+    old = torch.get_default_dtype()
+    torch.set_default_dtype(dtype)
+    try:
+        with torch.device("meta"):
+            plain = DeepseekV3MoE(cfg)
+        moe = (KDeepseekV3MoEV2 if serve else KDeepseekV3MoE)(key, weights, cfg, plain, "cuda", "cuda")
+        plain.gate = KMoEGateB200(key + ".gate", weights, cfg, plain.gate, "cuda", "cuda")
+        plain.experts = (KTransformersExpertsV2 if serve else KTransformersExperts)(key, weights, cfg, plain.experts, prefill_device="cuda", prefill_op=None, generate_device="cuda",
+                                                                                   generate_op="KExpertsB200", out_device="cuda")
+        for n in types:
+            name = n + "_proj"
+            setattr(plain.shared_experts, name, KTransformersLinear(f"{key}.shared_experts.{name}", weights, cfg, getattr(plain.shared_experts, name), "cuda", "KLinearB200", "cuda", None))
+        plain.gate.load()
+        plain.experts.load(warmup=False)
+        for n in types:
+            getattr(plain.shared_experts, n + "_proj").load()
+        moe._shared_mlp_handle(plain.experts.generate_experts)
+    finally:
+        torch.set_default_dtype(old)
+    return moe
+
+
+def _x(T, H, seed):
+    return (torch.randn((1, T, H), generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") / 10).bfloat16()
+
+
+def _in_one_call(moe, *args):
+    moe.last_topk = None
+    with torch.no_grad():
+        y = moe(*args)
+    return y, moe.last_topk is not None
+
+
+def _by_modules(moe, x):
+    hook = moe.shared_experts.register_forward_hook(lambda *a: None)
+    try:
+        y, one = _in_one_call(moe, x)
+    finally:
+        hook.remove()
+    assert not one
+    return y
+
+
+def _close(a, b):
+    """the shared expert hands bf16 on between its modules and fp32 inside the library; the routed sums are in another order"""
+    return (a.float() - b.float()).abs().max() <= 0.03 * b.float().abs().max()
+
+
+@pytest.mark.parametrize("T", [9, 24, 47])
+def test_one_call_agrees_with_the_modules(T):
+    moe, serve = _block(64, 6, 2048, 1536), _block(64, 6, 2048, 1536, serve=True)
+    x = _x(T, 2048, T)
+    y, one = _in_one_call(moe, x)
+    assert one and _close(y, _by_modules(moe, x))
+    live = T - 2
+    y2, one = _in_one_call(serve, x, torch.tensor([live], dtype=torch.int32, device="cuda"))
+    assert one and _close(y2[:, :live], y[:, :live]) and (y2[:, live:] == 0).all()
+    # captured, its first call of this size included, and replayed on other tokens
+    held, graph = x.clone(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.no_grad(), torch.cuda.graph(graph):
+        out = moe(held)
+    for seed in (1, 2):
+        held.copy_(_x(T, 2048, seed))
+        graph.replay()
+        got = out.clone()
+        want, one = _in_one_call(moe, held)
+        assert one and torch.equal(got, want), seed
+
+
+def test_modules_with_methods_of_their_own_are_called():
+    from ktransformers_b200.operators.experts import KDeepseekV3MoE
+    x, seen = _x(24, 2048, 5), []
+
+    def sub(obj, method="forward"):
+        cls = type(obj)
+
+        def called(self, *args, **kwargs):
+            seen.append(cls.__name__)
+            return getattr(cls, method)(self, *args, **kwargs)
+
+        obj.__class__ = type("Own" + cls.__name__, (cls,), {method: called})
+
+    def on_instance(obj, method):
+        real = getattr(obj, method)
+        setattr(obj, method, lambda *a, **k: (seen.append(method), real(*a, **k))[1])
+
+    moe = _block(64, 6, 2048, 1536)
+    want = _by_modules(moe, x)
+    for change, name in ((lambda m: sub(m.gate), "KMoEGateB200"), (lambda m: sub(m.experts), "KTransformersExperts"), (lambda m: sub(m.experts.generate_experts), "KExpertsB200"),
+                         (lambda m: sub(m.experts.generate_experts, "_launch"), "KExpertsB200"), (lambda m: sub(m.shared_experts.up_proj), "KTransformersLinear"),
+                         (lambda m: sub(m.shared_experts.down_proj.generate_linear), "KLinearB200"), (lambda m: sub(m, "moe_kexperts"), "KDeepseekV3MoE"),
+                         (lambda m: on_instance(m.experts.generate_experts, "_launch"), "_launch"), (lambda m: on_instance(m.shared_experts.gate_proj.generate_linear, "forward"), "forward"),
+                         (lambda m: on_instance(m.shared_experts, "act_fn"), "act_fn")):
+        m = _block(64, 6, 2048, 1536)
+        assert type(m) is KDeepseekV3MoE and _in_one_call(m, x)[1]
+        change(m)
+        del seen[:]
+        y, one = _in_one_call(m, x)
+        assert not one and seen == [name] and torch.equal(y, want), name
