@@ -585,11 +585,14 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
 // Whether a batch runs as per-expert tensor-core GEMMs (grouped.cu), which read an expert's weights once per 64 of its tokens, or through the row kernels, once per
 // (token, expert) pair: the reference makes the same split between MOE::forward_one and MOE::forward_many (moe.cpp:367-377, threshold group_min_len).
 // KTB200_GROUPED_MIN fixes the line; else up to 8 tokens the row kernels, from 48 the GEMMs, and between them what is expected to take less time.  Measured (us):
-//   row kernels  20 + pairs (and a shared expert's rows with them) x (0.83 ns a row of gate and up, of Q6_K 1.4, + 1.1 ns for four rows of down)
-//   GEMMs        85 (ten launches: 55 on the device and some more host work; a shared expert, a GEMM each of its own, 30 more) + 1.15 x the rounds of tiles x
-//                their blocks x 1,900 cycles (Q5_K 2,200, Q6_K 3,570) for the experts that the batch is expected to hit
-//   256 experts of 2048 x 7168, 8 chosen: 12 tokens 534 against 640, 16: 700 against 764, 24: 1041 against 1023, 40: 1722 against 1313;  64 of 1536 x 2048, 6 chosen: 9 tokens
-//   196 against 130, 40: 779 against 164;  16 of 512 x 1024, 8 chosen: 9 tokens 75 against 56, 40: 282 against 56;  the first with a shared expert, 24 tokens: 1207 against 818
+//   row kernels  20 + 2.7 a token + pairs (and a shared expert's rows with them) x 0.175 a MB of an expert (0.5 where gate and up are not Q4_K or their rows are short)
+//   GEMMs        58 (ten launches; a shared expert, a GEMM each of its own, 30 more) + 1.25 x the rounds of tiles x their blocks x 1,900 cycles (Q5_K 2,200, Q6_K 3,570)
+//                for the experts that the batch is expected to hit, were the choices spread evenly.  With a shared expert they are a router's, and those fall on fewer: with
+//                sigmoid scores and corrections of up to 0.2, 24 tokens with 8 of 256 hit 89 and not 137, counted as 0.9
+//   row kernels against GEMMs, even choices: 256 experts of 2048 x 7168, 8 chosen: 16 tokens 682 against 847, 24 1016 against 1100, 32 1378 against 1389, 47 2024 against 1692
+//   (24 behind that router, a shared expert and the router included: 1217 by modules, 866);  160 of 1536 x 5120, 6 chosen: 16 tokens 306 against 335, 32 595 against 533;  16 of
+//   2048 x 4096, 2 chosen: 12 tokens 117 against 124, 16 150 against 126;  32 of 1536 x 2048, 6 chosen: 9 tokens 192 against 109, with a shared expert 209 against 156;  16 of
+//   512 x 1024, 8 chosen: 9 tokens 76 against 57.  Both sides are good to a sixth
 static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k) {
     if (!grouped_ok(m, k)) return false;
     static const int fixed = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : -1; }();
@@ -598,11 +601,13 @@ static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k
     if (sh && sh->group_max_len < T) return false;      // (the shared expert would be a call of its own; with the row kernels it rides along)
     const ktb200_moe_config& c = m->cfg;
     const KqFmt gu = kq_fmt(pick_fmt(c.gate_type, m->gu_soa)), down = kq_fmt(pick_fmt(c.down_type, m->down_layout));
-    const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), hit = k < E ? E * (1.0 - pow(1.0 - k / E, T)) : E;
-    const double rows = 20.0 + T * (std::min<double>(k, E) + (sh ? 1 : 0)) * (2e-3 * I * (kq_is_q6(gu) ? 1.4 : 0.83) + 1.1e-3 * H / 4);
+    const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), own = std::min<double>(k, E);
+    const double mb = 1e-6 * (I * (row_bytes(c.hidden_size, c.gate_type) + row_bytes(c.hidden_size, c.up_type)) + H * row_bytes(c.intermediate_size, c.down_type));
+    const double rows = 20.0 + T * (2.7 + (own + (sh ? 1 : 0)) * mb * (gu == KQ_Q4K && H >= 16 * QK_K ? 0.175 : 0.5));
     auto cycles = [](KqFmt f) { return kq_is_q6(f) ? 3570.0 : f == KQ_Q5K ? 2200.0 : 1900.0; };
+    const double hit = E * (1.0 - pow(1.0 - own / E, T)) * (sh ? 0.9 : 1.0);
     const double blocks = ceil(hit * I / 128 / sms) * (H / QK_K) * cycles(gu) + ceil(hit * H / kKqRows / sms) * (I / QK_K) * cycles(down);
-    return (sh ? 115.0 : 85.0) + 1.15 * blocks / 1850.0 < 0.95 * rows;
+    return (sh ? 88.0 : 58.0) + 1.25 * blocks / 1850.0 < 0.95 * rows;
 }
 int ktb200_moe_takes_gemms(const ktb200_moe* m, const ktb200_mlp* shared, int qlen, int k) { return m && m->loaded && qlen > 0 && k > 0 && moe_as_gemms(m, shared, qlen, k); }
 
