@@ -52,6 +52,7 @@ struct ktb200_moe {
     unsigned blk_flip;
     const void* pf[3];       // ktb200_moe_block_prefetch_hint: ranges the block kernel pulls into L2 during its down phase
     size_t pf_bytes[3];
+    float own;               // choices of a token that fall on this handle's experts (ktb200_moe_expect_choices); 0: not told
 };
 
 struct DeviceGuard {

@@ -517,7 +517,7 @@ int ktb200_moe_create(const ktb200_moe_config* c, int device, ktb200_moe** out) 
     m->gu_soa = false;
     m->down_layout = LAYOUT_RAW;
     m->inter = nullptr; m->ids_d = nullptr; m->w_d = nullptr; m->in_d = nullptr; m->out_d = nullptr;
-    m->blk_partial = nullptr; m->blk_sync = nullptr; m->blk_flip = 0;
+    m->blk_partial = nullptr; m->blk_sync = nullptr; m->blk_flip = 0; m->own = 0.f;
     for (int r = 0; r < 3; r++) { m->pf[r] = nullptr; m->pf_bytes[r] = 0; }
     const size_t slots = (size_t)c->group_max_len * c->routed_expert_num;
     const size_t hid = (size_t)c->group_max_len * c->hidden_size * type_size(c->hidden_type);
@@ -593,6 +593,8 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
 //   (24 behind that router, a shared expert and the router included: 1217 by modules, 866);  160 of 1536 x 5120, 6 chosen: 16 tokens 306 against 335, 32 595 against 533;  16 of
 //   2048 x 4096, 2 chosen: 12 tokens 117 against 124, 16 150 against 126;  32 of 1536 x 2048, 6 chosen: 9 tokens 192 against 109, with a shared expert 209 against 156;  16 of
 //   512 x 1024, 8 chosen: 9 tokens 76 against 57.  Both sides are good to a sixth
+// A handle that has some of a layer's experts pays for the choices that fall on them (32 of the first 256: 9 tokens 87 against 135, 16 139 against 174, 24 200 against 212, 47 383
+// against 256); a share that is not told, of which an offset is the sign, keeps the row kernels.
 static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k) {
     if (!grouped_ok(m, k)) return false;
     static const int fixed = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : -1; }();
@@ -600,14 +602,21 @@ static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k
     if (T <= 8 || T >= 48) return T > 8;
     if (sh && sh->group_max_len < T) return false;      // (the shared expert would be a call of its own; with the row kernels it rides along)
     const ktb200_moe_config& c = m->cfg;
+    if (!m->own && c.expert_id_offset) return false;
     const KqFmt gu = kq_fmt(pick_fmt(c.gate_type, m->gu_soa)), down = kq_fmt(pick_fmt(c.down_type, m->down_layout));
-    const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), own = std::min<double>(k, E);
+    const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), own = std::min<double>(m->own ? m->own : k, E);
     const double mb = 1e-6 * (I * (row_bytes(c.hidden_size, c.gate_type) + row_bytes(c.hidden_size, c.up_type)) + H * row_bytes(c.intermediate_size, c.down_type));
     const double rows = 20.0 + T * (2.7 + (own + (sh ? 1 : 0)) * mb * (gu == KQ_Q4K && H >= 16 * QK_K ? 0.175 : 0.5));
     auto cycles = [](KqFmt f) { return kq_is_q6(f) ? 3570.0 : f == KQ_Q5K ? 2200.0 : 1900.0; };
     const double hit = E * (1.0 - pow(1.0 - own / E, T)) * (sh ? 0.9 : 1.0);
     const double blocks = ceil(hit * I / 128 / sms) * (H / QK_K) * cycles(gu) + ceil(hit * H / kKqRows / sms) * (I / QK_K) * cycles(down);
     return (sh ? 88.0 : 58.0) + 1.25 * blocks / 1850.0 < 0.95 * rows;
+}
+int ktb200_moe_expect_choices(ktb200_moe* m, float per_token) {
+    if (!m) { set_error("null handle"); return KTB200_EINVAL; }
+    if (!(per_token > 0.f)) { set_error("expect_choices: a positive number of choices per token"); return KTB200_EINVAL; }
+    m->own = per_token;
+    return KTB200_OK;
 }
 int ktb200_moe_takes_gemms(const ktb200_moe* m, const ktb200_mlp* shared, int qlen, int k) { return m && m->loaded && qlen > 0 && k > 0 && moe_as_gemms(m, shared, qlen, k); }
 

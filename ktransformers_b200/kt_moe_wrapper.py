@@ -101,6 +101,8 @@ class KTMoEWrapper:
         w = {n: self._permute(raw[n], self.num_experts, p2l) for n in ("gate", "up", "down")}
         w.update(gate_type=types["gate"], up_type=types["up"], down_type=types["down"])
         self.moe.load(w, device=self.device)
+        if 0 < self.num_gpu_experts < self.num_experts:
+            self.moe.expect_choices(self.num_experts_per_tok * (1 - self.num_gpu_experts / self.num_experts))
         dt = {0: torch.float32, 1: torch.float16, 30: torch.bfloat16}[self.moe.hidden_type]
         self._out = torch.zeros((self.moe.max_tokens, self.hidden_size), dtype=dt, device=self.device)
         self._mask_dev = self.gpu_experts_mask.to(self.device) if self.num_gpu_experts else None

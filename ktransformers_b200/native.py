@@ -84,6 +84,7 @@ SYMBOLS = {
     "ktb200_mlp_forward": (_I, [_VP, _I, _VP, _VP, _I, _VP, _VP]),
     "ktb200_moe_forward_shared": (_I, [_VP, _VP, _I, _I, _VP, _VP, _VP, _VP, _VP, _VP]),
     "ktb200_moe_takes_gemms": (_I, [_VP, _VP, _I, _I]),
+    "ktb200_moe_expect_choices": (_I, [_VP, C.c_float]),
     "ktb200_latent_step_bytes": (C.c_size_t, [_I, _I, _I, _I, _I]),
     "ktb200_latent_step": (_I, [C.POINTER(LatentStepParams), _VP]),
     "ktb200_quantize_activations": (_I, [_VP, _I, _L, _L, _I, _VP, _VP]),

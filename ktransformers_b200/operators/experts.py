@@ -139,12 +139,18 @@ class KExpertsB200(KExpertsBase):
         native.check(lib.ktb200_moe_create(C.byref(cfg), self.dev_index, C.byref(h)))
         self.handle = h
         native.check(lib.ktb200_moe_load_weights(self.handle, _stream(dev)))
+        if self.ep_size > 1:
+            self.expect_choices(self.config.num_experts_per_tok / self.ep_size)
         if warmup:
             native.check(lib.ktb200_moe_warm_up(self.handle, _stream(dev)))
         if self.out_device not in KExpertsB200.output_gpu_map:
             KExpertsB200.output_gpu_map[self.out_device] = torch.zeros(
                 (self.max_tokens, self.config.hidden_size), device=self.out_device,
                 dtype={0: torch.float32, 1: torch.float16, 30: torch.bfloat16}[hidden_type])
+
+    def expect_choices(self, per_token: float):
+        """tells the handle how many of a token's choices fall on its experts (default: all), which a batch's kernels are chosen by"""
+        native.check(native.lib().ktb200_moe_expect_choices(self.handle, per_token))
 
     def unload(self):
         if self.handle is not None:

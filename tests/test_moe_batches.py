@@ -138,3 +138,40 @@ def test_modules_with_methods_of_their_own_are_called():
         del seen[:]
         y, one = _in_one_call(m, x)
         assert not one and seen == [name] and torch.equal(y, want), name
+
+
+@pytest.mark.parametrize("rank", [0, 3])
+def test_shards_count_the_pairs_that_they_have(rank):
+    """One of eight shards of 256 experts, 8 chosen: its row kernels pay for one choice a token.  Where its GEMMs are taken, 47 tokens agree with the row kernels, 8 at a time."""
+    import ctypes as C
+    from types import SimpleNamespace
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.operators.experts import KExpertsB200
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, E, k, H, I = native.lib(), 256, 8, 7168, 2048
+    types = {"gate": Q4_K, "up": Q4_K, "down": Q6_K}
+    per = E // 8
+    shard = {n: synth_blocks(t, per * H * I, "cuda", t + len(n)) for n, t in types.items()}
+    op = KExpertsB200("blk.3", None, SimpleNamespace(num_experts_per_tok=k, hidden_size=H, moe_intermediate_size=I), E, device="cuda", expert_parallel_rank=rank, expert_parallel_size=8,
+                      hidden_dtype=torch.bfloat16)
+    op.load(w={**{n: t.repeat(8) for n, t in shard.items()}, **{n + "_type": t for n, t in types.items()}})
+    assert [lib.ktb200_moe_takes_gemms(op.handle, None, T, k) for T in (8, 9, 16, 24, 47, 48)] == [0, 0, 0, 0, 1, 1]
+    native.check(lib.ktb200_moe_expect_choices(op.handle, 8.0))
+    assert lib.ktb200_moe_takes_gemms(op.handle, None, 24, k) == 1
+    op.expect_choices(1.0)
+    with pytest.raises(ValueError):
+        op.expect_choices(0.0)
+    h, cfg = C.c_void_p(), native.MoeConfig(per, k, H, I, 64, 10, 64, 1, *[t.data_ptr() for t in (op.gate, op.up, op.down)], Q4_K, Q4_K, Q4_K, 30, 32 * rank)
+    native.check(lib.ktb200_moe_create(C.byref(cfg), 0, C.byref(h)))      # (Q4_K all: nothing is laid out again)
+    native.check(lib.ktb200_moe_load_weights(h, torch.cuda.current_stream().cuda_stream))
+    assert lib.ktb200_moe_takes_gemms(h, None, 47, k) == (rank == 0)      # not told: a whole layer of 32, or an unknown share of one
+    lib.ktb200_moe_destroy(h)
+    T, g = 47, torch.Generator(device="cuda").manual_seed(rank)
+    x = _x(T, H, 7)[0]
+    ids, w = torch.rand((T, E), generator=g, device="cuda").argsort(-1)[:, :k].contiguous(), torch.rand((T, k), generator=g, device="cuda")
+    n0 = native.launch_count()
+    y = op.forward(x, ids, w)
+    assert native.launch_count() - n0 == 10
+    few = torch.cat([op.forward(x[t:t + 8], ids[t:t + 8], w[t:t + 8]) for t in range(0, T, 8)])
+    assert few.abs().max() > 0 and ((y.double() - few.double()).abs() <= 2.0 ** -7 * few.double().abs() + 2e-3 * few.double().abs().max()).all()
