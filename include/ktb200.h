@@ -168,7 +168,8 @@ int ktb200_mlp_forward(ktb200_mlp* mlp, int qlen, const void* input_dev, void* o
 int ktb200_moe_forward_shared(ktb200_moe* moe, ktb200_mlp* shared, int qlen, int k, const int64_t* expert_ids_dev,
                               const float* weights_dev, const void* input_dev, void* output_dev,
                               const int* bsz_tensor_dev, void* stream);
-/* 1 when these two calls run a batch of qlen tokens as per-expert tensor-core GEMMs (and `shared` as a call of its own), 0 when through the row kernels */
+/* 1 when these two calls run a batch of qlen tokens as per-expert tensor-core GEMMs (and `shared` as a call of its own), 0 when through the row kernels.
+ * (Without a batch size on the device; with one, three quarters of qlen are taken as live, and a few more batches keep the row kernels.) */
 int ktb200_moe_takes_gemms(const ktb200_moe* moe, const ktb200_mlp* shared, int qlen, int k);
 /* How many of a token's choices fall on the handle's experts on average, for that decision: k x expert_num / all experts for an expert-parallel shard.  Not told: all k, or, with
  * an expert_id_offset, unknown, and batches below 48 tokens keep the row kernels.  (A shard that starts at expert 0 looks like a whole layer: tell it.) */

@@ -595,7 +595,9 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
 //   512 x 1024, 8 chosen: 9 tokens 76 against 57.  Both sides are good to a sixth
 // A handle that has some of a layer's experts pays for the choices that fall on them (32 of the first 256: 9 tokens 87 against 135, 16 139 against 174, 24 200 against 212, 47 383
 // against 256); a share that is not told, of which an offset is the sign, keeps the row kernels.
-static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k) {
+// `padded`: the number of live tokens is on the device.  Row kernels pay for those only, GEMMs for their launches in any case; a batch is padded to the next size that a program has
+// a graph of, so three quarters of it are taken as live, the middle between half of it and all.
+static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, bool padded) {
     if (!grouped_ok(m, k)) return false;
     static const int fixed = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : -1; }();
     if (fixed >= 0) return fixed > 0 && T >= fixed;
@@ -606,9 +608,10 @@ static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k
     const KqFmt gu = kq_fmt(pick_fmt(c.gate_type, m->gu_soa)), down = kq_fmt(pick_fmt(c.down_type, m->down_layout));
     const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), own = std::min<double>(m->own ? m->own : k, E);
     const double mb = 1e-6 * (I * (row_bytes(c.hidden_size, c.gate_type) + row_bytes(c.hidden_size, c.up_type)) + H * row_bytes(c.intermediate_size, c.down_type));
-    const double rows = 20.0 + T * (2.7 + (own + (sh ? 1 : 0)) * mb * (gu == KQ_Q4K && H >= 16 * QK_K ? 0.175 : 0.5));
+    const double live = padded ? 0.75 * T : T;
+    const double rows = 20.0 + live * (2.7 + (own + (sh ? 1 : 0)) * mb * (gu == KQ_Q4K && H >= 16 * QK_K ? 0.175 : 0.5));
     auto cycles = [](KqFmt f) { return kq_is_q6(f) ? 3570.0 : f == KQ_Q5K ? 2200.0 : 1900.0; };
-    const double hit = E * (1.0 - pow(1.0 - own / E, T)) * (sh ? 0.9 : 1.0);
+    const double hit = E * (1.0 - pow(1.0 - own / E, live)) * (sh ? 0.9 : 1.0);
     const double blocks = ceil(hit * I / 128 / sms) * (H / QK_K) * cycles(gu) + ceil(hit * H / kKqRows / sms) * (I / QK_K) * cycles(down);
     return (sh ? 88.0 : 58.0) + 1.25 * blocks / 1850.0 < 0.95 * rows;
 }
@@ -618,7 +621,7 @@ int ktb200_moe_expect_choices(ktb200_moe* m, float per_token) {
     m->own = per_token;
     return KTB200_OK;
 }
-int ktb200_moe_takes_gemms(const ktb200_moe* m, const ktb200_mlp* shared, int qlen, int k) { return m && m->loaded && qlen > 0 && k > 0 && moe_as_gemms(m, shared, qlen, k); }
+int ktb200_moe_takes_gemms(const ktb200_moe* m, const ktb200_mlp* shared, int qlen, int k) { return m && m->loaded && qlen > 0 && k > 0 && moe_as_gemms(m, shared, qlen, k, false); }
 
 // what the row kernels of a layer's routed experts read
 static void row_params(const ktb200_moe* m, int k, const int64_t* ids, const float* weights, const void* input, void* output, const int* bsz, RowsParams& rp, ReduceParams& dp) {
@@ -646,7 +649,7 @@ static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
     if (!ids || !weights || !input || !output) { set_error("forward: null pointer"); return KTB200_EINVAL; }
     DeviceGuard g(m->device);
 
-    if (!mid && !shared_out && moe_as_gemms(m, sh, qlen, k)) {
+    if (!mid && !shared_out && moe_as_gemms(m, sh, qlen, k, bsz != nullptr)) {
         int rc = moe_forward_grouped(m, qlen, k, ids, weights, input, output, bsz, s);
         if (rc || !sh) return rc;
         return ktb200_mlp_forward(const_cast<ktb200_mlp*>(sh), qlen, input, output, 1, bsz, (void*)s);

@@ -175,3 +175,30 @@ def test_shards_count_the_pairs_that_they_have(rank):
     assert native.launch_count() - n0 == 10
     few = torch.cat([op.forward(x[t:t + 8], ids[t:t + 8], w[t:t + 8]) for t in range(0, T, 8)])
     assert few.abs().max() > 0 and ((y.double() - few.double()).abs() <= 2.0 ** -7 * few.double().abs() + 2e-3 * few.double().abs().max()).all()
+
+
+def test_padded_batches_count_their_live_tokens():
+    """16 experts of 2048 x 4096, 2 chosen: 16 tokens are GEMMs, and rows where only the device knows how many of the 16 are live; 40 are GEMMs either way."""
+    import ctypes as C
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, E, k, H, I = native.lib(), 16, 2, 4096, 2048
+    w = [synth_blocks(t, E * H * I, "cuda", 1 + i) for i, t in enumerate((Q4_K, Q4_K, Q6_K))]
+    h, stream = C.c_void_p(), torch.cuda.current_stream().cuda_stream
+    native.check(lib.ktb200_moe_create(C.byref(native.MoeConfig(E, k, H, I, 64, 10, 64, 1, *[t.data_ptr() for t in w], Q4_K, Q4_K, Q6_K, 30, 0)), 0, C.byref(h)))
+    native.check(lib.ktb200_moe_load_weights(h, stream))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for T, padded in ((16, 2), (40, 10)):
+        x, ids, wt = _x(T, H, T)[0], torch.rand((T, E), generator=g, device="cuda").argsort(-1)[:, :k].contiguous(), torch.rand((T, k), generator=g, device="cuda")
+        out = []
+        for bsz, launches in ((None, 10), (T // 2 + 1, padded)):
+            y, n0 = torch.full((T, H), 7.0, dtype=torch.bfloat16, device="cuda"), native.launch_count()
+            live = torch.tensor([bsz or T], dtype=torch.int32, device="cuda")
+            native.check(lib.ktb200_moe_forward(h, T, k, ids.data_ptr(), wt.data_ptr(), x.data_ptr(), y.data_ptr(), live.data_ptr() if bsz else None, stream))
+            assert native.launch_count() - n0 == launches, (T, bsz)
+            out.append(y)
+        n = T // 2 + 1
+        a, b = out[0][:n].double(), out[1][:n].double()
+        assert (out[1][n:] == 7.0).all() and ((a - b).abs() <= 2.0 ** -7 * a.abs() + 2e-3 * a.abs().max()).all()
+    lib.ktb200_moe_destroy(h)
