@@ -595,6 +595,7 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
 //   512 x 1024, 8 chosen: 9 tokens 76 against 57.  Both sides are good to a sixth
 // A handle that has some of a layer's experts pays for the choices that fall on them (32 of the first 256: 9 tokens 87 against 135, 16 139 against 174, 24 200 against 212, 47 383
 // against 256); a share that is not told, of which an offset is the sign, keeps the row kernels.
+// fp32 handles keep the row kernels, which add a row's blocks as a tree over the lanes: the GEMMs add them in one chain, 1.4 x as far from 64 bits for rows of 7168.
 // `padded`: the number of live tokens is on the device.  Row kernels pay for those only, GEMMs for their launches in any case; a batch is padded to the next size that a program has
 // a graph of, so three quarters of it are taken as live, the middle between half of it and all.
 static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, bool padded) {
@@ -604,6 +605,7 @@ static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k
     if (T <= 8 || T >= 48) return T > 8;
     if (sh && sh->group_max_len < T) return false;      // (the shared expert would be a call of its own; with the row kernels it rides along)
     const ktb200_moe_config& c = m->cfg;
+    if (c.hidden_type == KTB200_TYPE_F32) return false;
     if (!m->own && c.expert_id_offset) return false;
     const KqFmt gu = kq_fmt(pick_fmt(c.gate_type, m->gu_soa)), down = kq_fmt(pick_fmt(c.down_type, m->down_layout));
     const double E = c.expert_num, H = c.hidden_size, I = c.intermediate_size, sms = num_sms(m->device), own = std::min<double>(m->own ? m->own : k, E);

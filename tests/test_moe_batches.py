@@ -202,3 +202,31 @@ def test_padded_batches_count_their_live_tokens():
         a, b = out[0][:n].double(), out[1][:n].double()
         assert (out[1][n:] == 7.0).all() and ((a - b).abs() <= 2.0 ** -7 * a.abs() + 2e-3 * a.abs().max()).all()
     lib.ktb200_moe_destroy(h)
+
+
+def test_fp32_batches_keep_the_sums_of_the_row_kernels():
+    """fp32 experts of long rows: 24 tokens give the bits of eight at a time, and so their distance from 64 bits (bf16 ones of the same sizes are GEMMs)."""
+    import ctypes as C
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, E, k, H, I, T = native.lib(), 16, 4, 7168, 512, 24
+    stream, g = torch.cuda.current_stream().cuda_stream, torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn((T, H), generator=g, device="cuda") / 200      # (results grow with its square; at 1 / 10 they reach fp16's largest value, 65504)
+    ids, wt = torch.rand((T, E), generator=g, device="cuda").argsort(-1)[:, :k].contiguous(), torch.rand((T, k), generator=g, device="cuda")
+    for hidden, gemms in ((0, 0), (30, 1), (1, 1)):
+        w, h = [synth_blocks(t, E * H * I, "cuda", 1 + i) for i, t in enumerate((Q4_K, Q4_K, Q4_K))], C.c_void_p()
+        native.check(lib.ktb200_moe_create(C.byref(native.MoeConfig(E, k, H, I, 64, 10, 64, 1, *[t.data_ptr() for t in w], Q4_K, Q4_K, Q4_K, hidden, 0)), 0, C.byref(h)))
+        native.check(lib.ktb200_moe_load_weights(h, stream))
+        assert [lib.ktb200_moe_takes_gemms(h, None, n, k) for n in (8, T, 48)] == [0, gemms, 1]
+        xs = x.to({0: torch.float32, 1: torch.float16, 30: torch.bfloat16}[hidden])
+        y, few = torch.empty_like(xs), torch.empty_like(xs)
+        call = lambda out, a, b: native.check(lib.ktb200_moe_forward(h, b - a, k, ids[a:b].data_ptr(), wt[a:b].data_ptr(), xs[a:b].data_ptr(), out[a:b].data_ptr(), None, stream))
+        call(y, 0, T)
+        for t in range(0, T, 8):
+            call(few, t, t + 8)
+        if hidden == 0:
+            assert torch.equal(y, few) and y.abs().max() > 0
+        else:
+            assert ((y.double() - few.double()).abs() <= 2.0 ** -7 * few.double().abs() + 2e-3 * few.double().abs().max()).all()
+        lib.ktb200_moe_destroy(h)
