@@ -47,6 +47,7 @@ cudaError_t raise_smem_limit(const void* kernel, size_t bytes);
 // stream-ordered scratch from a bounded pool (runtime.cu); ScratchBlock gives it back behind the work already queued on the stream
 cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out);
 void scratch_prepare(int device);      // when a handle is created: its calls may then be captured from the first on
+constexpr int kNoScratch = 2;          // inside the library: the pool could not give a product's scratch (the error's text is set, nothing is launched)
 struct ScratchBlock {
     void* ptr = nullptr;
     cudaStream_t stream;
@@ -54,6 +55,11 @@ struct ScratchBlock {
     ScratchBlock(const ScratchBlock&) = delete;
     ScratchBlock& operator=(const ScratchBlock&) = delete;
     cudaError_t take(int device, size_t bytes) { return scratch_alloc(device, bytes, stream, &ptr); }
+    bool taken(int device, size_t bytes) {
+        const cudaError_t e = take(device, bytes);
+        if (e != cudaSuccess) set_error("scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        return e == cudaSuccess;
+    }
     ~ScratchBlock() { if (ptr) cudaFreeAsync(ptr, stream); }
 };
 

@@ -112,7 +112,7 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
     const size_t n_x = up(KqActs::bytes(rows, H)), n_g = up(rows * I * 4), n_d = up(rows * H * 4), n_a = up(KqActs::bytes(rows, I));
     const size_t n_mid = n_x + 2 * n_g > n_d ? n_x + 2 * n_g : n_d;
     ScratchBlock mem(s);
-    KTB_CUDA_CHECK(mem.take(dev, n_ints + n_tab + n_mid + n_a));
+    if (!mem.taken(dev, n_ints + n_tab + n_mid + n_a)) return kNoScratch;
     uint8_t* at = reinterpret_cast<uint8_t*>(mem.ptr);
     int *counts = reinterpret_cast<int*>(at), *offsets = counts + E + 1, *nt_prefix = offsets + E + 1, *cursor = nt_prefix + E + 1, *pos = cursor + E + 1;
     int4 *tinfo_gu = reinterpret_cast<int4*>(at + n_ints), *tinfo_d = tinfo_gu + ub_gu;

@@ -937,7 +937,7 @@ int kq_mlp(const ktb200_mlp* m, const void* x, int T, void* y, int accumulate, c
         auto up = [](size_t b) { return (b + 255) / 256 * 256; };
         const size_t n_x = up(KqActs::bytes(n, H)), n_a = up(KqActs::bytes(n, I)), n_g = up((size_t)su * n * I * 4), n_d = up((size_t)sd * n * H * 4);
         ScratchBlock mem(s);
-        KTB_CUDA_CHECK(mem.take(dev, n_x + n_a + 2 * n_g + n_d));
+        if (!mem.taken(dev, n_x + n_a + 2 * n_g + n_d)) return kNoScratch;
         uint8_t* at = reinterpret_cast<uint8_t*>(mem.ptr);
         const KqActs xa(at, n, H), aa(at + n_x, n, I);
         float *gu[2] = {reinterpret_cast<float*>(at + n_x + n_a), reinterpret_cast<float*>(at + n_x + n_a + n_g)}, *part = reinterpret_cast<float*>(at + n_x + n_a + 2 * n_g);

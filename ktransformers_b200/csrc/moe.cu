@@ -598,11 +598,12 @@ int moe_forward_grouped(ktb200_moe* m, int qlen, int k, const int64_t* ids, cons
 // fp32 handles keep the row kernels, which add a row's blocks as a tree over the lanes: the GEMMs add them in one chain, 1.4 x as far from 64 bits for rows of 7168.
 // `padded`: the number of live tokens is on the device.  Row kernels pay for those only, GEMMs for their launches in any case; a batch is padded to the next size that a program has
 // a graph of, so three quarters of it are taken as live, the middle between half of it and all.
+constexpr int kMoeRowsTokens = 47;
 static bool moe_as_gemms(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, bool padded) {
     if (!grouped_ok(m, k)) return false;
     static const int fixed = [] { const char* e = getenv("KTB200_GROUPED_MIN"); return e ? atoi(e) : -1; }();
     if (fixed >= 0) return fixed > 0 && T >= fixed;
-    if (T <= 8 || T >= 48) return T > 8;
+    if (T <= 8 || T > kMoeRowsTokens) return T > 8;
     if (sh && sh->group_max_len < T) return false;      // (the shared expert would be a call of its own; with the row kernels it rides along)
     const ktb200_moe_config& c = m->cfg;
     if (c.hidden_type == KTB200_TYPE_F32) return false;
@@ -639,6 +640,7 @@ static void row_params(const ktb200_moe* m, int k, const int64_t* ids, const flo
     dp.weights = weights; dp.a = m->inter; dp.out = output; dp.hidden_type = c.hidden_type; dp.accumulate = 0; dp.bsz = bsz;
 }
 
+static int mlp_forward_impl(const ktb200_mlp* m, int qlen, const void* input, void* output, int accumulate, const int* bsz, cudaStream_t s);
 static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, const float* weights, const void* input,
                             void* output, const int* bsz, cudaStream_t s, cudaEvent_t mid, const ktb200_mlp* sh = nullptr,
                             int shared_token = -1, void* shared_out = nullptr) {
@@ -653,8 +655,9 @@ static int moe_forward_impl(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
 
     if (!mid && !shared_out && moe_as_gemms(m, sh, qlen, k, bsz != nullptr)) {
         int rc = moe_forward_grouped(m, qlen, k, ids, weights, input, output, bsz, s);
-        if (rc || !sh) return rc;
-        return ktb200_mlp_forward(const_cast<ktb200_mlp*>(sh), qlen, input, output, 1, bsz, (void*)s);
+        if (rc == KTB200_OK && sh) rc = mlp_forward_impl(sh, qlen, input, output, 1, bsz, s);
+        if (rc != kNoScratch) return rc;
+        if (qlen > kMoeRowsTokens) return KTB200_ECUDA;      // (a batch that the row kernels take too needs no scratch)
     }
     FmtId fg = pick_fmt(c.gate_type, m->gu_soa), fu = pick_fmt(c.up_type, m->gu_soa);
     if (fg != fu) fg = fu = FMT_GENK;  // mixed gate/up types: the generic path reads the type per matrix
@@ -915,12 +918,15 @@ static int mlp_gemm_min(const ktb200_mlp* m) {
 }
 
 int ktb200_mlp_forward(ktb200_mlp* m, int qlen, const void* input, void* output, int accumulate, const int* bsz, void* stream) {
+    const int rc = mlp_forward_impl(m, qlen, input, output, accumulate, bsz, (cudaStream_t)stream);
+    return rc == kNoScratch ? KTB200_ECUDA : rc;
+}
+static int mlp_forward_impl(const ktb200_mlp* m, int qlen, const void* input, void* output, int accumulate, const int* bsz, cudaStream_t s) {
     if (!m) { set_error("null handle"); return KTB200_EINVAL; }
     if (!m->loaded) { set_error("Not Loaded"); return KTB200_ESTATE; }
     if (qlen <= 0) return KTB200_OK;
     if (qlen > m->group_max_len) { set_error("forward: qlen=%d exceeds group_max_len=%d", qlen, m->group_max_len); return KTB200_EINVAL; }
     DeviceGuard g(m->device);
-    cudaStream_t s = (cudaStream_t)stream;
     if (qlen >= mlp_gemm_min(m) && input && output) {
         const int rc = kq_mlp(m, input, qlen, output, accumulate, bsz, s);
         if (rc != 1) return rc;

@@ -230,3 +230,51 @@ def test_fp32_batches_keep_the_sums_of_the_row_kernels():
         else:
             assert ((y.double() - few.double()).abs() <= 2.0 ** -7 * few.double().abs() + 2e-3 * few.double().abs().max()).all()
         lib.ktb200_moe_destroy(h)
+
+
+def _without_memory_for_scratch(with_shared):
+    """512 experts of 256 x 7168: 47 tokens take some 90 MB of scratch, and 40 MB of the device are left."""
+    import ctypes as C
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, E, k, H, I, T = native.lib(), 512, 8, 7168, 256, 47
+    stream, g = torch.cuda.current_stream().cuda_stream, torch.Generator(device="cuda").manual_seed(1)
+    w, s = [synth_blocks(Q4_K, E * H * I, "cuda", 1 + i) for i in range(3)], [synth_blocks(Q4_K, H * I, "cuda", 5 + i) for i in range(3)]
+    h, sh = C.c_void_p(), C.c_void_p()
+    native.check(lib.ktb200_moe_create(C.byref(native.MoeConfig(E, k, H, I, 64, 10, 64, 1, *[t.data_ptr() for t in w], Q4_K, Q4_K, Q4_K, 30, 0)), 0, C.byref(h)))
+    native.check(lib.ktb200_mlp_create(H, I, *[t.data_ptr() for t in s], Q4_K, Q4_K, Q4_K, 30, 64, 0, C.byref(sh)))
+    native.check(lib.ktb200_moe_load_weights(h, stream))
+    native.check(lib.ktb200_mlp_load_weights(sh, stream))
+    x, ids, wt = _x(64, H, 1)[0], torch.rand((64, E), generator=g, device="cuda").argsort(-1)[:, :k].contiguous(), torch.rand((64, k), generator=g, device="cuda")
+    few, y = torch.zeros_like(x), torch.zeros_like(x)
+
+    def call(out, a, b, shared):
+        return lib.ktb200_moe_forward_shared(h, shared, b - a, k, ids[a:b].data_ptr(), wt[a:b].data_ptr(), x[a:b].data_ptr(), out[a:b].data_ptr(), None, stream)
+
+    shared = sh if with_shared else None
+    assert lib.ktb200_moe_takes_gemms(h, shared, T, k) == 1
+    for t in range(0, T, 8):
+        native.check(call(few, t, min(t + 8, T), shared))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    native.check(call(y, 0, T, shared))
+    assert torch.equal(y[:T], few[:T])
+    assert call(y, 0, 64, shared) not in (0, native.EINVAL) and b"scratch" in lib.ktb200_last_error()      # a prompt's size is refused as ever
+    del hog
+
+
+@pytest.mark.parametrize("shared", [0, 1])
+def test_without_memory_for_scratch_the_row_kernels_run(shared):
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), str(shared)], capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=root))
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+if __name__ == "__main__":
+    import sys
+    _without_memory_for_scratch(int(sys.argv[1]))
