@@ -24,7 +24,8 @@
 namespace ktb {
 
 constexpr int kActBlkStride = QK_K + 16;   // int8 activation blocks padded to 272 B: 8 lanes x LDS.128 hit 32 distinct banks
-constexpr int kBulkMaxWarps = 16;        // gate/up kernel: 128 registers per thread
+constexpr int kBulkMaxWarps = 18;        // rows one at a time: <= 96 registers per thread
+constexpr int kBulkMaxWarpsBoth = 16;    // gate and up rows at once: 128 registers per thread
 constexpr int kBulkMaxWarpsDown = 16;    // down kernel: 128 registers per thread, and shared memory caps it at 15 anyway
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -127,17 +128,18 @@ __device__ __forceinline__ float q4k_block_dot(const uint8_t* wb, const uint8_t*
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Gate/up (PAIR) or dense (PAIR = false) rows of Q4_K tensors.  Per warp: a private ring of SLOTS slots of one unit each — a row, or (PAIR) the gate and the up row of one
-// output, whose dots share their activation loads — and at any time SLOTS-1 units are in flight behind the one being consumed.
-// A dozen warps an SM wait for their own loads and sums more than for a unit of the SM (43 % of the issue slots and of the shared-memory wavefronts in use): two rows at a time are
-// two chains beside each other and a third fewer loads.  MoE block of 7 tokens 377 -> 362 us (256 experts of 2048 x 7168, 8 chosen), 151 -> 137 (64 of 1024 x 4096, 6); routed
-// experts of 9 tokens, 160 of 1536 x 5120, 6 chosen, 202 -> 183.
+// Gate/up (PAIR) or dense (PAIR = false) rows of Q4_K tensors.  Per warp: a private ring of SLOTS slots, and at any time SLOTS-1 of them are in flight behind the one being
+// consumed.  A slot holds one row, gate and up rows alternating (PAIR), or (BOTH) the gate and the up row of one output, whose dots share their activation loads.
+// A dozen warps an SM wait for their own loads and sums more than for a unit of the SM (43 % of the issue slots and of the shared-memory wavefronts in use with one row a slot): two
+// rows at a time are two chains beside each other and a third fewer loads.  MoE block of 7 tokens 377 -> 363 us (256 experts of 2048 x 7168, 8 chosen), 151 -> 137 (64 of 1024 x
+// 4096, 6); routed experts of 9 tokens, 160 of 1536 x 5120, 6 chosen, 202 -> 183.  But slots of two rows take the warps' place, and a CTA that has few rows, or fits few warps, is
+// better off with more warps (launch_rows_bulk_q4k, moe.cu).
 //
 // Tokens are processed in chunks of `tc` (launcher: as many as fit next to >= 12 rings).  Within a chunk ALL
 // (token, slot) pairs this launch owns form ONE work list — expert-parallel shards and decode batches keep the ring
 // streaming across tokens instead of draining it once per token — and all the chunk's activation rows are staged as
 // Q8_K side by side (`act_tok` bytes each).
-template <bool PAIR, int SLOTS>
+template <bool PAIR, int SLOTS, bool BOTH>
 __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, int tc) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ int s_np;
@@ -146,7 +148,7 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     if (p.bsz) Teff = min(Teff, *p.bsz);
     const int nblk = p.ncols / QK_K;
     const int row_bytes = nblk * SZ_Q4_K;
-    constexpr int NM = PAIR ? 2 : 1;
+    constexpr int NM = BOTH ? 2 : 1, NS = PAIR && !BOTH ? 2 : 1;      // rows of a slot, slots of a unit
     const int nslots = p.slots + (p.x0 ? 1 : 0);
     const int total_out = nslots * p.rows;
     // [tc activation rows: q8 [nblk][272] | bs32 [nblk][8] int16 | dx [nblk]] [pair list: tc*nslots ints] [mbarriers] [rings]
@@ -154,8 +156,8 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     const size_t off = ((size_t)tc * act_tok + (size_t)tc * nslots * 4 + 15) & ~(size_t)15;
     const int bar_bytes = (W * SLOTS * 8 + 15) & ~15;
     const uint32_t bar_u32 = (uint32_t)__cvta_generic_to_shared(smem + off) + warp * SLOTS * 8;
-    const int unit_bytes = NM * row_bytes;
-    uint8_t* ring = smem + off + bar_bytes + (size_t)warp * SLOTS * unit_bytes;
+    const int slot_bytes = NM * row_bytes;
+    uint8_t* ring = smem + off + bar_bytes + (size_t)warp * SLOTS * slot_bytes;
     const uint32_t ring_u32 = (uint32_t)__cvta_generic_to_shared(ring);
     if (lane == 0) {
 #pragma unroll
@@ -192,28 +194,32 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     const int u0 = (int)((long)total * blockIdx.x / gridDim.x), u1 = (int)((long)total * (blockIdx.x + 1) / gridDim.x);
     int nu = u1 - u0 - warp;
     nu = nu > 0 ? (nu + W - 1) / W : 0;                     // units of this warp: u0 + warp + i*W
-    // issue cursor: (pair index, row) of the next unit to request, and how many were requested
+    const int nsub = nu * NS;
+    // issue cursor: (pair index, row) of the next unit to request, and how many slots were filled
     int ipi = 0, irr = 0, issued = 0;
     if (nu > 0) { ipi = (u0 + warp) / p.rows; irr = (u0 + warp) - ipi * p.rows; }
     int cpi = ipi, crr = irr;                               // consume cursor
 
     auto issue_one = [&]() {
-        if (issued < nu) {
+        if (issued < nsub) {
             if (lane == 0) {
                 const int pr = pairs[ipi], s = pr & 0xff, tl = pr >> 8;
                 const uint32_t bar = bar_u32 + 8 * slot_i;
-                mbar_expect_tx(bar, (uint32_t)unit_bytes);
+                mbar_expect_tx(bar, (uint32_t)slot_bytes);
                 const bool extra = s == p.slots;
                 const long e = extra || !p.ids ? 0 : (long)p.ids[(long)(t0 + tl) * p.slots + s] - p.id_offset;
 #pragma unroll
-                for (int m = 0; m < NM; m++) {
+                for (int i = 0; i < NM; i++) {
+                    const int m = NS == 2 ? issued & 1 : i;
                     const void* w = extra ? (m ? p.x1 : p.x0) : (m ? p.w1 : p.w0);
-                    bulk_g2s(ring_u32 + slot_i * unit_bytes + m * row_bytes, reinterpret_cast<const uint8_t*>(w) + (e * p.rows + irr) * row_bytes, (uint32_t)row_bytes, bar);
+                    bulk_g2s(ring_u32 + slot_i * slot_bytes + i * row_bytes, reinterpret_cast<const uint8_t*>(w) + (e * p.rows + irr) * row_bytes, (uint32_t)row_bytes, bar);
                 }
             }
             issued++;
-            irr += W;
-            while (irr >= p.rows) { irr -= p.rows; ipi++; }
+            if (NS == 1 || !(issued & 1)) {
+                irr += W;
+                while (irr >= p.rows) { irr -= p.rows; ipi++; }
+            }
             slot_i = (slot_i + 1 == SLOTS) ? 0 : slot_i + 1;
         }
     };
@@ -241,10 +247,11 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
     }
     __syncthreads();
 
-    for (int n = 0; n < nu; n++) {
+    float first = 0.f;
+    for (int n = 0; n < nsub; n++) {
         mbar_wait(bar_u32 + 8 * slot_u, (phase >> slot_u) & 1u);
         phase ^= 1u << slot_u;
-        const uint8_t* row0 = ring + slot_u * unit_bytes;
+        const uint8_t* row0 = ring + slot_u * slot_bytes;
         const int pr = pairs[cpi];
         const uint8_t* at = smem + (size_t)(pr >> 8) * act_tok;
         const int16_t* bs32 = reinterpret_cast<const int16_t*>(at + (size_t)nblk * kActBlkStride);
@@ -262,7 +269,8 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
         __syncwarp();                       // every lane is done reading the slot: hand it back to the copy engine
         slot_u = (slot_u + 1 == SLOTS) ? 0 : slot_u + 1;
         issue_one();
-        float g = acc[0], uu = acc[NM - 1];
+        if (NS == 2 && !(n & 1)) { first = acc[0]; continue; }
+        float g = NS == 2 ? first : acc[0], uu = acc[NM - 1];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             g += __shfl_xor_sync(0xffffffffu, g, o);
@@ -289,8 +297,8 @@ __device__ __forceinline__ void rows_bulk_q4k(const RowsParams& p, int act_tok, 
         for (int s = 0; s < SLOTS; s++) mbar_inval(bar_u32 + 8 * s);
     }
 }
-template <bool PAIR, int SLOTS>
-__global__ void __launch_bounds__(kBulkMaxWarps * 32, 1) rows_bulk_q4k_kernel(const RowsParams p, int act_tok, int tc) { rows_bulk_q4k<PAIR, SLOTS>(p, act_tok, tc); }
+template <bool PAIR, int SLOTS, bool BOTH>
+__global__ void __launch_bounds__((BOTH ? kBulkMaxWarpsBoth : kBulkMaxWarps) * 32, 1) rows_bulk_q4k_kernel(const RowsParams p, int act_tok, int tc) { rows_bulk_q4k<PAIR, SLOTS, BOTH>(p, act_tok, tc); }
 
 // ---------------------------------------------------------------------------------------------------------------
 // Item formats of the down-projection kernel.  An item is 4 consecutive rows x nb super-blocks, f = rw*nb + blk.

@@ -209,11 +209,11 @@ static int launch_rows_pipe(const RowsParams& p, int T, int device, cudaStream_t
     return KTB200_OK;
 }
 
-// Shared-memory plan of rows_bulk_q4k<., S> for T tokens of `nslots` sets of rows each, `nm` rows a unit: returns the warp count (0 = does not fit)
+// Shared-memory plan of rows_bulk_q4k with S slots a warp for T tokens of `nslots` sets of rows each, `nm` rows a slot: returns the warp count (0 = does not fit)
 static int rows_bulk_plan(int ncols, int nm, int nslots, int T, int S, int max_warps, int* act_tok_out, int* tc_out, size_t* smem_out) {
     const int nblk = ncols / QK_K, row_bytes = nm * nblk * SZ_Q4_K, act_tok = (nblk * kActBlkStride + nblk * 16 + nblk * 4 + 15) & ~15;
     if (nblk < 16) return 0;                             // needs >= 16 blocks per row to keep most lanes busy
-    // tokens per chunk: as many (<= 8) as fit next to 12 rings (of two rows a unit: 8); then as many warps as fit
+    // tokens per chunk: as many (<= 8) as fit next to 12 rings (of two rows a slot: 8); then as many warps as fit
     int tc = T < 8 ? T : 8;
     while (tc > 1 && (size_t)tc * (act_tok + nslots * 4) + 64 + (size_t)(nm == 2 ? 8 : 12) * S * (row_bytes + 8) > kSmemCap) tc--;
     const size_t head = (((size_t)tc * act_tok + (size_t)tc * nslots * 4 + 15) & ~(size_t)15);
@@ -226,29 +226,31 @@ static int rows_bulk_plan(int ncols, int nm, int nslots, int T, int S, int max_w
     return W;
 }
 // Q4_K rows through the bulk-copy ring (rows_bulk_q4k_kernel).  Returns 1 when the shape does not suit it.
+// Gate and up rows share a slot where enough warps fit with such slots.  All 16 for one token (a warp then takes few rows, and 13 warps of 7168 columns take two rounds of a CTA's
+// 14 outputs where 18 take one: MLP of 7168 x 2048 16.8 us against 16.2, x 18432 69.1 against 67.3, but 4096 x 14336 44 against 47) and for a few tokens' experts, whose rows come
+// from memory and not from L2 (7168 x 2048, 8 of 128, 12 warps: 4 tokens 175 us against 170, 8 349 against 354; 5120 x 1536, 6 of 160, 16 warps: 83 against 94).  Else 7 (5 or 4
+// warps: 16384 x 4096, 8 tokens 265 us against 251, 20480 x 2048 235 against 216; 7: 12288 x 4096 191 against 193, 10: 7168 x 18432 333 against 363).
 template <bool PAIR>
 static int launch_rows_bulk_q4k(const RowsParams& p, int T, int device, cudaStream_t stream) {
     if (!cfg_bulk()) return 1;
     const int nslots = p.slots + (p.x0 ? 1 : 0);
     const long total = (long)nslots * p.rows;
     if (total >= (1L << 26) || nslots > 200) return 1;
-    const int S = PAIR ? cfg_bulk_slots_up() : 3;
     int act_tok = 0, tc = 0;
     size_t smem = 0;
-    const int W = rows_bulk_plan(p.ncols, PAIR ? 2 : 1, nslots, T, S, cfg_bulk_warps(), &act_tok, &tc, &smem);
-    if (!W) return 1;
-    int gx = num_sms(device);            // one CTA per SM walks all T tokens
-    if (gx > total) gx = (int)total;
-    if (gx < 1) gx = 1;
-#define KTB_BULK_ROWS(SL)                                                                                              \
-    do {                                                                                                               \
-        KTB_CUDA_CHECK(raise_smem_limit((const void*)rows_bulk_q4k_kernel<PAIR, SL>, smem)); \
-        rows_bulk_q4k_kernel<PAIR, SL><<<gx, W * 32, smem, stream>>>(p, act_tok, tc);                                  \
-    } while (0)
-    if (S == 2) KTB_BULK_ROWS(2); else KTB_BULK_ROWS(3);
-#undef KTB_BULK_ROWS
-    KTB_LAUNCH_CHECK();
-    return KTB200_OK;
+    const int gx = (int)std::max(1L, std::min<long>(num_sms(device), total));      // one CTA per SM walks all T tokens
+    auto go = [&](auto fn, int W) -> int {
+        KTB_CUDA_CHECK(raise_smem_limit((const void*)fn, smem));
+        fn<<<gx, W * 32, smem, stream>>>(p, act_tok, tc);
+        KTB_LAUNCH_CHECK();
+        return KTB200_OK;
+    };
+    if constexpr (PAIR) {
+        const int S = cfg_bulk_slots_up(), W = rows_bulk_plan(p.ncols, 2, nslots, T, S, std::min(cfg_bulk_warps(), kBulkMaxWarpsBoth), &act_tok, &tc, &smem);
+        if (W >= (T == 1 || (p.ids && T < 8) ? kBulkMaxWarpsBoth : 7)) return S == 2 ? go(rows_bulk_q4k_kernel<true, 2, true>, W) : go(rows_bulk_q4k_kernel<true, 3, true>, W);
+    }
+    const int W = rows_bulk_plan(p.ncols, 1, nslots, T, 3, cfg_bulk_warps(), &act_tok, &tc, &smem);
+    return W ? go(rows_bulk_q4k_kernel<PAIR, 3, false>, W) : 1;
 }
 
 // Dense Q4_K linear on the segment ring (dense_bulk.cuh).  Returns 1 when the shape does not suit it.

@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(MoeRowsPlan::kWarps * 32, 1) moe_block_many_ke
         if ((threadIdx.x >> 5) < kGateWarps) gate_select_token<1>(g, t, reinterpret_cast<float*>(smem), g.idx + (long)t * g.top_k, g.w + (long)t * g.top_k, g.logits_out);
     grid_arrive(sync, gen);
     grid_wait(sync, gen);
-    rows_bulk_q4k<true, MoeRowsPlan::kSlotsUp>(plan.rows, plan.act_tok, plan.tc);
+    rows_bulk_q4k<true, MoeRowsPlan::kSlotsUp, true>(plan.rows, plan.act_tok, plan.tc);
     grid_arrive(sync, gen);
     grid_wait(sync, gen);
     reduce_bulk<DownFmt, MoeRowsPlan::kSlotsDown>(plan.down, plan.nrows_max, plan.pcap);

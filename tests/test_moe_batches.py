@@ -232,6 +232,59 @@ def test_fp32_batches_keep_the_sums_of_the_row_kernels():
         lib.ktb200_moe_destroy(h)
 
 
+# one row a slot and gate and up in one (launch_rows_bulk_q4k, csrc/moe.cu): 7168 columns take the first for one token and the second for eight, 16384 always the first, 4096 the second
+@pytest.mark.parametrize("H,I,experts", [(4096, 512, 0), (7168, 512, 0), (8192, 256, 0), (16384, 256, 0), (7168, 256, 8), (8192, 256, 8), (16384, 256, 8)])
+@pytest.mark.parametrize("hidden", [0, 30])
+def test_rows_in_either_form_of_slots_give_the_same_bits(H, I, experts, hidden):
+    import ctypes as C
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, k, T = native.lib(), 3, 8
+    stream, g, h = torch.cuda.current_stream().cuda_stream, torch.Generator(device="cuda").manual_seed(H), C.c_void_p()
+    w = [synth_blocks(t, max(experts, 1) * H * I, "cuda", 1 + i) for i, t in enumerate((Q4_K, Q4_K, Q6_K))]
+    x = (torch.randn((T, H), generator=g, device="cuda") / 10).to(torch.float32 if hidden == 0 else torch.bfloat16)
+    if experts:
+        ids, wt = torch.rand((T, experts), generator=g, device="cuda").argsort(-1)[:, :k].contiguous(), torch.rand((T, k), generator=g, device="cuda")
+        native.check(lib.ktb200_moe_create(C.byref(native.MoeConfig(experts, k, H, I, 64, 10, T, 1, *[t.data_ptr() for t in w], Q4_K, Q4_K, Q6_K, hidden, 0)), 0, C.byref(h)))
+        native.check(lib.ktb200_moe_load_weights(h, stream))
+        call = lambda y, a, b: native.check(lib.ktb200_moe_forward(h, b - a, k, ids[a:b].data_ptr(), wt[a:b].data_ptr(), x[a:b].data_ptr(), y[a:b].data_ptr(), None, stream))
+    else:
+        native.check(lib.ktb200_mlp_create(H, I, *[t.data_ptr() for t in w], Q4_K, Q4_K, Q6_K, hidden, T, 0, C.byref(h)))
+        native.check(lib.ktb200_mlp_load_weights(h, stream))
+        call = lambda y, a, b: native.check(lib.ktb200_mlp_forward(h, b - a, x[a:b].data_ptr(), y[a:b].data_ptr(), 0, None, stream))
+    got = []
+    for step in (8, 3, 1):
+        y = torch.zeros_like(x)
+        for t in range(0, T, step):
+            call(y, t, min(t + step, T))
+        got.append(y)
+    assert got[0].isfinite().all() and got[0].abs().max() > 0 and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    (lib.ktb200_moe_destroy if experts else lib.ktb200_mlp_destroy)(h)
+
+
+def test_more_slots_than_a_warp_has_lanes():
+    """40 choices a token of which only the last eight have a weight give the bits of those eight alone."""
+    import ctypes as C
+
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    lib, E, H, I, T, stream = native.lib(), 64, 4096, 256, 5, torch.cuda.current_stream().cuda_stream
+    w, g, h = [synth_blocks(Q4_K, E * H * I, "cuda", 1 + i) for i in range(3)], torch.Generator(device="cuda").manual_seed(2), C.c_void_p()
+    native.check(lib.ktb200_moe_create(C.byref(native.MoeConfig(E, 40, H, I, 64, 10, T, 1, *[t.data_ptr() for t in w], Q4_K, Q4_K, Q4_K, 0, 0)), 0, C.byref(h)))
+    native.check(lib.ktb200_moe_load_weights(h, stream))
+    x = torch.randn((T, H), generator=g, device="cuda") / 10
+    ids, wt = torch.rand((T, E), generator=g, device="cuda").argsort(-1)[:, :40].contiguous(), torch.rand((T, 40), generator=g, device="cuda")
+    wt[:, :32] = 0
+    got = []
+    for i, v in ((ids, wt), (ids[:, 32:].contiguous(), wt[:, 32:].contiguous())):
+        y = torch.zeros_like(x)
+        native.check(lib.ktb200_moe_forward(h, T, i.shape[1], i.data_ptr(), v.data_ptr(), x.data_ptr(), y.data_ptr(), None, stream))
+        got.append(y)
+    assert got[0].abs().max() > 0 and torch.equal(*got)
+    lib.ktb200_moe_destroy(h)
+
+
 def _without_memory_for_scratch(with_shared):
     """512 experts of 256 x 7168: 47 tokens take some 90 MB of scratch, and 40 MB of the device are left."""
     import ctypes as C
