@@ -14,11 +14,15 @@ namespace ktb {
 
 constexpr int kDenseMaxTokens = 8;
 constexpr int kDenseWarps = 16;
-// Two CTAs an SM where eight warps or more fit into half of its shared memory (a row or two of activations).  The streams of two neighbouring launches then overlap: a
+// Two CTAs an SM where eight warps or more fit into half of its shared memory (dense_two_ctas).  The streams of two neighbouring launches then overlap: a
 // launch's weights are requested while the one before it ends, and with two CTAs of one launch on an SM one quantises or ends while the other streams.  A launch of few units
-// keeps one CTA an SM.  In a graph of such launches: 16384 -> 7168 19.4 -> 18.2 us, 7168 -> 18432 22.2 -> 17.8, 1536 -> 24576 7.8 -> 6.4, 4096 -> 4096 5.75 -> 4.9;
-// 7168 -> 1536 4.95 -> 4.6 with one CTA an SM (5.1 with two), 512 -> 16000 3.3 -> 3.0 (3.4).  Three slots a warp (fewer warps) 10-30 % slower.
+// keeps one CTA an SM.  In a graph of such launches: 16384 -> 7168 18.6 -> 16.8 us, 7168 -> 18432 22.0 -> 17.5, 1536 -> 24576 8.6 -> 7.4, 4096 -> 4096 6.0 -> 5.1;
+// 7168 -> 1536 5.0 -> 4.8 with one CTA an SM (5.1 with two), 512 -> 16000 3.3 -> 3.0 (3.4).  Three slots a warp (fewer warps) 10-30 % slower.
 constexpr int kDenseWarpsTwo = 12, kDenseSmemTwo = 114000;
+// More rows of activations are quantised twice an SM by fewer warps each, and few units meet fewer warps: for one or two rows the form is always the faster, beyond where there are
+// enough units of short rows or many units.  Four rows 7168 -> 1536 14.7 us (11.8 as one CTA of more slots), six rows 7168 -> 4096 28.8 (26.6), 512 -> 512 6.0 (5.4),
+// three rows 14336 -> 4096 28.2 (27.0); but four rows 7168 -> 18432 45.8 (51.0), eight rows 2048 -> 8192 15.5 (17.8), 1536 -> 24576 26.8 (28.3).
+inline bool dense_two_ctas(int T, int nblk, int nunits, int sms) { return T <= 2 || nunits > 40 * sms || (nunits > kDenseWarpsTwo * sms && T * nblk <= 80); }
 
 struct DenseParams {
     const uint8_t* w;      // [rows][nblk] Q4_K blocks

@@ -278,7 +278,7 @@ static int launch_dense_q4k(const RowsParams& p, int T, int device, cudaStream_t
         count_launch();
         return KTB200_OK;
     };
-    const int rc = go(dense_q4k_kernel<2, kDenseWarpsTwo, 2>, 2, kDenseWarpsTwo, 8, kDenseSmemTwo, nunits > kDenseWarpsTwo * sms ? 2 * sms : sms);
+    const int rc = dense_two_ctas(T, nblk, nunits, sms) ? go(dense_q4k_kernel<2, kDenseWarpsTwo, 2>, 2, kDenseWarpsTwo, 8, kDenseSmemTwo, nunits > kDenseWarpsTwo * sms ? 2 * sms : sms) : 1;
     return rc != 1 ? rc : go(dense_q4k_kernel<4, kDenseWarps, 1>, 4, kDenseWarps, 4, kSmemCap, sms);
 }
 

@@ -852,3 +852,21 @@ def test_moe_block_forward_host_pinned_and_pageable_match_the_device_call():
         native.check(lib.ktb200_moe_block_forward_host(C.byref(gc), m.h, None, qlen, xn.data_ptr(), yn.data_ptr(), None, None, s))
         assert torch.equal(yn.view(torch.int16), y_d.cpu().view(torch.int16))
     m.close()
+
+
+# two CTAs an SM and one (dense_two_ctas, csrc/dense_bulk.cuh): few units, short rows, the line at 80 staged blocks, many units of long rows, rows of two segments, rows that leave no room
+@pytest.mark.parametrize("K,R", [(512, 512), (1536, 24576), (2048, 8192), (4096, 4096), (5120, 5120), (7168, 1536), (7168, 18432), (14336, 4096), (18432, 7168)])
+def test_linear_rows_do_not_depend_on_the_form_of_the_kernel(K, R):
+    lib, h = native.lib(), C.c_void_p()
+    w = synth_blocks(Q4_K, R * K, "cuda", K)
+    native.check(lib.ktb200_linear_create(K, R, w.data_ptr(), Q4_K, BF16, 8, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, G.stream()))
+    x = torch.randn((8, K), generator=torch.Generator(device="cuda").manual_seed(R), device="cuda").bfloat16()
+    got = []
+    for step in (1, 2, 3, 4, 5, 6, 8):
+        y = torch.zeros((8, R), dtype=torch.bfloat16, device="cuda")
+        for t in range(0, 8, step):
+            native.check(lib.ktb200_linear_forward(h, min(step, 8 - t), x[t:].data_ptr(), y[t:].data_ptr(), None, None, G.stream()))
+        got.append(y)
+    assert got[0].abs().max() > 0 and all(torch.equal(got[0], y) for y in got[1:])
+    lib.ktb200_linear_destroy(h)
