@@ -241,8 +241,9 @@ int ktb200_moe_forward_ep(ktb200_moe* moe, ktb200_mlp* shared, int qlen, int k, 
  *     y = self.experts(hidden_states, topk_idx, topk_weight)    (CPU MOE: operators/llamafile/moe.cpp:146-245)
  *     y += self.shared_experts(identity)                        (n_shared_experts is not None)
  * For decode batches (qlen <= 8) of Q4_K gate/up + Q6_K or Q4_K down experts with rows of 4096..8192 columns this is
- * ONE persistent cooperative launch (router GEMV, grid barrier, top-k in every CTA, gate/up, grid barrier, down +
- * combine; weights stream through the copy engine across the barriers); any other configuration runs as
+ * ONE persistent cooperative launch.  One token: router GEMV, grid barrier, top-k in every CTA, gate/up, grid barrier, down +
+ * combine; weights stream through the copy engine across the barriers.  2 to 8 tokens: the same phases for all tokens at once, a CTA per
+ * token selecting between two barriers of its own, each phase's stream starting behind its barrier.  Any other configuration runs as
  * ktb200_moe_gate_forward + ktb200_moe_forward_shared.  Results are bit-identical between the two.
  * idx_dev int64 [qlen][top_k] and w_dev fp32 [qlen][top_k] receive the routing (as from ktb200_moe_gate_forward).
  * `shared` may be NULL.  Capturable as is (its scratch belongs to the moe handle); when it falls back to the separate
@@ -723,7 +724,8 @@ int ktb200_debug_stream_read(const void* src_dev, long bytes, int mode, int unro
 /* mode 2 of the probe above: the bulk-copy ring of the expert kernels without arithmetic (unroll = ring slots,
  * ctas_per_sm = warps per CTA).
  * Phase trace of ktb200_moe_block_forward (profiles/block_trace.py): while trace_dev != NULL, thread 0 of every CTA
- * writes %globaltimer at the phase boundaries into trace_dev[cta][16] (uint64, >= num_SMs * 16 entries). */
+ * writes %globaltimer at the phase boundaries into trace_dev[cta][16] (uint64, >= num_SMs * 16 entries); with 2 to 8 tokens
+ * entries 0, 2-6 and 9 only (the two quantisations and the down tiles end inside their phases there). */
 void ktb200_debug_block_trace(unsigned long long* trace_dev);
 
 #ifdef __cplusplus

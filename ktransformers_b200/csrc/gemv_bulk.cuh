@@ -375,8 +375,9 @@ struct BulkQ6K4T {   // chunk-major 4-row tiles (see the header comment)
 // pairs form ONE work list (expert-parallel shards and decode batches do not drain the ring per token) and all their
 // activation rows are staged as Q8_K side by side.
 constexpr int kBulkMaxChunkTokens = 16;
-template <class Fmt, int SLOTS>
-__device__ __forceinline__ void reduce_bulk(const ReduceParams& p, int nrows_max, int pcap) {
+// `last`: called by one warp once the last chunk's first items are requested
+template <class Fmt, int SLOTS, class Last>
+__device__ __forceinline__ void reduce_bulk(const ReduceParams& p, int nrows_max, int pcap, Last&& last) {
     constexpr int RW = 4;
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ int s_np, s_nt;
@@ -475,6 +476,7 @@ __device__ __forceinline__ void reduce_bulk(const ReduceParams& p, int nrows_max
     };
 #pragma unroll
     for (int s = 0; s < SLOTS; s++) issue_one();
+    if (warp == W - 1 && t0 + nt >= Teff) last();
 
     {   // quantise the pairs' activation rows (fp32 phase-1 output) into the padded layout: block g = (pair, block)
         float cur[8], nxt[8];
@@ -544,7 +546,7 @@ __device__ __forceinline__ void reduce_bulk(const ReduceParams& p, int nrows_max
   }  // token chunks
 }
 template <class Fmt, int SLOTS>
-__global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(const ReduceParams p, int nrows_max, int pcap) { reduce_bulk<Fmt, SLOTS>(p, nrows_max, pcap); }
+__global__ void __launch_bounds__(kBulkMaxWarpsDown * 32, 1) reduce_bulk_kernel(const ReduceParams p, int nrows_max, int pcap) { reduce_bulk<Fmt, SLOTS>(p, nrows_max, pcap, [] {}); }
 
 // both row phases of T tokens in one launch (moe_block.cu), planned in moe.cu
 struct MoeRowsPlan {

@@ -699,7 +699,7 @@ bool moe_rows_plan(const ktb200_moe* m, const ktb200_mlp* sh, int T, int k, cons
     o->rows.ntokens = o->down.ntokens = T;
     if (sh) { o->rows.x0 = sh->gate; o->rows.x1 = sh->up; o->down.xw = sh->down; }
     const int ns = k + (sh ? 1 : 0);
-    if (!cfg_bulk() || ns > 31 || (long)ns * c.intermediate_size >= (1L << 26) || c.intermediate_size < num_sms(m->device)) return false;
+    if (!cfg_bulk() || ns > 31 || (long)ns * c.intermediate_size >= (1L << 26)) return false;
     size_t up = 0, down = 0;
     const FmtId fd = pick_fmt(c.down_type, m->down_layout);
     const int wd = fd == FMT_Q6K4T ? rows_plan_down<BulkQ6K4T>(o->down, T, m->device, o, &down) : fd == FMT_Q4K ? rows_plan_down<BulkQ4K>(o->down, T, m->device, o, &down) : 0;

@@ -37,7 +37,12 @@ constexpr int kBlockWarps = 15;    // 480 threads -> 128 registers; 15 x 13440-b
 constexpr int kBlockWarpsLo = 12;  // 384 threads -> 168 registers (KTB200_BLK_WARPS <= 12)
 constexpr int kBlockMaxTokens = 8;
 
-struct BlockParams {
+struct BlockExtras {
+    unsigned long long* trace;           // debug: [grid][16] globaltimer stamps of the phase boundaries (null: off)
+    const uint8_t* pf[3];                // ranges to pull into L2 while the down phase streams (the NEXT layer's router rows and
+    unsigned pf_bytes[3];                // shared-expert gate/up rows: ktb200_moe_block_prefetch_hint); null: none
+};
+struct BlockParams : BlockExtras {
     GateParams g;                        // router (W, bias, partial scratch, idx / w / logits outputs, x)
     const void *w_gate, *w_up, *w_down;  // routed experts [n_local][...]
     const void *s_gate, *s_up, *s_down;  // shared expert (null: none)
@@ -51,9 +56,6 @@ struct BlockParams {
     int region_a;                        // bytes of the aliased activation staging
     int ring_bytes;                      // per-warp ring
     int prime_u, prime_d;                // rows / tiles every warp requests BEFORE the router's / the second grid barrier
-    unsigned long long* trace;           // debug: [grid][16] globaltimer stamps of the phase boundaries (null: off)
-    const uint8_t* pf[3];                // ranges to pull into L2 while the down phase streams (the NEXT layer's router rows and
-    unsigned pf_bytes[3];                // shared-expert gate/up rows: ktb200_moe_block_prefetch_hint); null: none
 };
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
@@ -84,11 +86,24 @@ __device__ __forceinline__ void grid_wait(unsigned* counter, unsigned gen) {
 // Programmatic dependent launch: the next layer's launch is processed, and its CTAs start on SMs as they free up,
 // while the tail of this one still runs; everything that depends on the previous kernel comes after griddep_wait().
 
-__device__ __forceinline__ void block_stamp(const BlockParams& p, int i) {
+__device__ __forceinline__ void block_stamp(const BlockExtras& p, int i) {
     if (p.trace && threadIdx.x == 0) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         p.trace[blockIdx.x * 16 + i] = t;
+    }
+}
+
+// the next layer's first bytes (ktb200_moe_block_prefetch_hint) -> L2, this CTA's 1/grid slice of each range in
+// 4 KB pieces: no registers or shared memory held, the down stream keeps its ring
+__device__ __forceinline__ void block_prefetch(const BlockExtras& p, int lane) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        if (p.pf[r]) {
+            const unsigned per = ((p.pf_bytes[r] / gridDim.x) + 15u) & ~15u;
+            const unsigned lo = per * blockIdx.x, hi = min(p.pf_bytes[r], lo + per);
+            for (unsigned o = lo + lane * 4096u; o < hi; o += 32u * 4096u) prefetch_l2_bulk(p.pf[r] + o, min(4096u, hi - o) & ~15u);
+        }
     }
 }
 
@@ -482,16 +497,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) moe_block_kernel(const BlockPara
 #pragma unroll
         for (int s = 0; s < SD; s++) issue_d();
         if (t == Teff - 1 && warp == W - 1) {
-            // the next layer's first bytes (ktb200_moe_block_prefetch_hint) -> L2, this CTA's 1/grid slice of each range in
-            // 4 KB pieces: no registers or shared memory held, the down stream keeps its ring
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                if (p.pf[r]) {
-                    const unsigned per = ((p.pf_bytes[r] / gridDim.x) + 15u) & ~15u;
-                    const unsigned lo = per * blockIdx.x, hi = min(p.pf_bytes[r], lo + per);
-                    for (unsigned o = lo + lane * 4096u; o < hi; o += 32u * 4096u) prefetch_l2_bulk(p.pf[r] + o, min(4096u, hi - o) & ~15u);
-                }
-            }
+            block_prefetch(p, lane);
         }
         __syncthreads();
         block_stamp(p, 7);
@@ -588,27 +594,35 @@ __device__ __forceinline__ void many_router(const GateParams& g, int nt) {      
     }
 }
 template <class DownFmt>
-__global__ void __launch_bounds__(MoeRowsPlan::kWarps * 32, 1) moe_block_many_kernel(const __grid_constant__ GateParams g, unsigned* sync, const __grid_constant__ MoeRowsPlan plan) {
+__global__ void __launch_bounds__(MoeRowsPlan::kWarps * 32, 1) moe_block_many_kernel(const __grid_constant__ GateParams g, unsigned* sync, const __grid_constant__ MoeRowsPlan plan,
+                                                                                      const __grid_constant__ BlockExtras extras) {
     extern __shared__ __align__(16) uint8_t smem[];
     griddep_launch_dependents();
     griddep_wait();
+    block_stamp(extras, 0);
     const int T = g.bsz ? min(g.T, *g.bsz) : g.T;
     unsigned gen = 0;
     if (T <= 2) many_router<2>(g, T);
     else if (T <= 4) many_router<4>(g, T);
     else many_router<kBlockMaxTokens>(g, T);
+    block_stamp(extras, 2);
     grid_arrive(sync, gen);
     grid_wait(sync, gen);
+    block_stamp(extras, 3);
     for (int t = blockIdx.x; t < T; t += gridDim.x)
         if ((threadIdx.x >> 5) < kGateWarps) gate_select_token<1>(g, t, reinterpret_cast<float*>(smem), g.idx + (long)t * g.top_k, g.w + (long)t * g.top_k, g.logits_out);
     grid_arrive(sync, gen);
     grid_wait(sync, gen);
+    block_stamp(extras, 4);
     rows_bulk_q4k<true, MoeRowsPlan::kSlotsUp, true>(plan.rows, plan.act_tok, plan.tc);
     grid_arrive(sync, gen);
+    block_stamp(extras, 5);
     grid_wait(sync, gen);
-    reduce_bulk<DownFmt, MoeRowsPlan::kSlotsDown>(plan.down, plan.nrows_max, plan.pcap);
+    block_stamp(extras, 6);
+    reduce_bulk<DownFmt, MoeRowsPlan::kSlotsDown>(plan.down, plan.nrows_max, plan.pcap, [&] { block_prefetch(extras, threadIdx.x & 31); });
     // leave the barrier words zeroed for the next launch / graph replay: the last CTA to get here resets them
     __syncthreads();
+    block_stamp(extras, 9);
     if (threadIdx.x == 0 && atomicAdd(sync + 1, 1u) == gridDim.x - 1) {
         sync[0] = 0;
         sync[1] = 0;
@@ -1154,7 +1168,8 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
     static const int prime_d = [] { const char* e = getenv("KTB200_BLK_PRIME_D"); return e ? atoi(e) : 2; }();
     p.prime_u = prime_u; p.prime_d = prime_d;
 
-    void *one[] = {&p}, *all[] = {&p.g, &p.sync, &many}, **args = all_at_once ? all : one;
+    BlockExtras& extras = p;
+    void *one[] = {&p}, *all[] = {&p.g, &p.sync, &many, &extras}, **args = all_at_once ? all : one;
     const void* fn;
     if (all_at_once) fn = fd == FMT_Q6K4T ? (const void*)moe_block_many_kernel<BulkQ6K4T> : (const void*)moe_block_many_kernel<BulkQ4K>;
     else if (W > kBlockWarpsLo) fn = fd == FMT_Q6K4T ? (const void*)moe_block_kernel<BulkQ6K4T, kBlockWarps> : (const void*)moe_block_kernel<BulkQ4K, kBlockWarps>;

@@ -870,3 +870,36 @@ def test_linear_rows_do_not_depend_on_the_form_of_the_kernel(K, R):
         got.append(y)
     assert got[0].abs().max() > 0 and all(torch.equal(got[0], y) for y in got[1:])
     lib.ktb200_linear_destroy(h)
+
+
+# the block of several tokens (moe_block_many_kernel) under DeepSeek-V2's scoring, in fp16 and fp32, with ranges to prefetch and a trace
+@pytest.mark.parametrize("Eg,k,ng,tg,scoring,method,norm,scale,hid,dt", [(160, 6, 8, 3, 1, 2, 0, 16.0, BF16, Q6_K), (64, 6, 1, 1, 1, 1, 0, 1.0, F16, Q4_K), (48, 4, 4, 2, 0, 0, 1, 2.5, F32, Q6_K)])
+def test_moe_block_of_several_tokens(Eg, k, ng, tg, scoring, method, norm, scale, hid, dt):
+    H, I = 4096, 512
+    m = G.Moe(Eg, k, H, I, _synth(Q4_K, Eg * I * H, 81), _synth(Q4_K, Eg * I * H, 82), _synth(dt, Eg * H * I, 83), Q4_K, Q4_K, dt, hid)
+    mlp = G.Mlp(H, I, _synth(Q4_K, I * H, 84), _synth(Q4_K, I * H, 85), _synth(dt, H * I, 86), Q4_K, Q4_K, dt, hid)
+    rng, lib = np.random.default_rng(Eg), native.lib()
+    W, bias = rng.standard_normal((Eg, H)).astype(np.float32), rng.standard_normal(Eg).astype(np.float32)
+    gate = G.Gate(W, bias, k, ng, tg, scoring, method, norm, scale, hidden_type=hid)
+    ranges = [torch.zeros(n, dtype=torch.uint8, device="cuda") for n in (1 << 20, 4096 * 148 + 48, 16)]
+    trace = torch.zeros((torch.cuda.get_device_properties(0).multi_processor_count, 16), dtype=torch.int64, device="cuda")
+    native.check(lib.ktb200_moe_block_prefetch_hint(m.h, (C.c_void_p * 3)(*[r.data_ptr() for r in ranges]), (C.c_size_t * 3)(*[r.numel() for r in ranges]), 3))
+    for qlen in (2, 4, 7, 8):
+        x = (rng.standard_normal((qlen, H)) / 100).astype(np.float32)
+        xin = {F32: lambda: x, F16: lambda: x.astype(np.float16), BF16: lambda: f32_to_bf16_bits(x)}[hid]()
+        trace.zero_()
+        lib.ktb200_debug_block_trace(trace.data_ptr())
+        try:
+            n0 = native.launch_count()
+            out, idx, w = G.moe_block_forward(gate, m, mlp, xin)
+            assert native.launch_count() - n0 == 1
+        finally:
+            lib.ktb200_debug_block_trace(None)
+        ridx, rw, _ = G.gate_forward(xin, W, bias, k, ng, tg, scoring, method, norm, scale, hidden_type=hid)
+        assert np.array_equal(idx, ridx) and np.array_equal(w, rw)
+        assert np.array_equal(out, G.moe_forward_shared(m, mlp, ridx, rw, xin)), qlen
+        at = trace.cpu()[:, [0, 2, 3, 4, 5, 6, 9]]
+        assert (at > 0).all() and (at[:, 1:] >= at[:, :-1]).all() and not trace[:, [1, 7, 8, 10]].any()
+        assert at[:, 1].max() <= at[:, 2].min() + 2000 and at[:, 4].max() <= at[:, 5].min() + 2000      # nobody passes a barrier before the last arrives (the timer's steps: 1 us)
+    m.close()
+    mlp.close()
