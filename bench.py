@@ -46,7 +46,7 @@ PREFILL_TOKENS = 1024   # the reference's group_max_len (experts.py:209): one ch
 
 def committed_traffic(kernel):
     """dram__bytes_read.sum + dram__bytes_write.sum per launch of `kernel` from the committed ncu summary
-    (profiles/traffic.json, written by profiles/summarize.py from an `ncu --set full` capture); None when absent."""
+    (profiles/traffic.json, from an `ncu --set full` capture); None when absent."""
     try:
         d = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
         return d.get(kernel, {}).get("dram_bytes_per_launch")
@@ -61,7 +61,7 @@ def measured_peak_gbs():
             return float(json.load(open(p))["hbm_gbs"]), "measured (MEASURED_PEAKS.json hbm_gbs)"
         except Exception:
             pass
-    return 6650.0, "fallback (B200_PROFILING.md)"
+    return 6650.0, "fallback (an earlier measurement on such a GPU)"
 
 
 class ClockSampler:

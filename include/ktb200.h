@@ -723,7 +723,7 @@ int ktb200_debug_stream_read(const void* src_dev, long bytes, int mode, int unro
                              void* stream, float* ms_out);
 /* mode 2 of the probe above: the bulk-copy ring of the expert kernels without arithmetic (unroll = ring slots,
  * ctas_per_sm = warps per CTA).
- * Phase trace of ktb200_moe_block_forward (profiles/block_trace.py): while trace_dev != NULL, thread 0 of every CTA
+ * Phase trace of ktb200_moe_block_forward: while trace_dev != NULL, thread 0 of every CTA
  * writes %globaltimer at the phase boundaries into trace_dev[cta][16] (uint64, >= num_SMs * 16 entries); with 2 to 8 tokens
  * entries 0, 2-6 and 9 only (the two quantisations and the down tiles end inside their phases there). */
 void ktb200_debug_block_trace(unsigned long long* trace_dev);

@@ -1,13 +1,13 @@
 // Fourth generation of the expert GEMV kernels: bulk-copy (TMA engine) staging + one lane per super-block.
 //
-// What ncu said about the cp.async generation (profiles/r01c_kernels.md): DRAM at ~50 % of peak, issue slots
+// What ncu said about the cp.async generation: DRAM at ~50 % of peak, issue slots
 // 40-50 % busy with only 12 warps per SM, and of the ~700 warp instructions a warp spent per 8 KB unit almost
 // 230 were the copy itself (16 LDGSTS per lane, each with its own 64-bit address arithmetic) plus index
 // divisions — LSU/MIO time shared with the LDS of the dot product.  Here:
 //
 //   * every ring slot is filled by ONE `cp.async.bulk.shared.global` issued by one lane and tracked by an
 //     mbarrier (expect_tx / complete_tx): no per-lane copy instructions, no LSU time for the copy;
-//   * slots are one output's weight rows (Q4_K gate and up: 2 nblk x 144 B) or one 4-row item (down) and a warp keeps SLOTS-1
+//   * slots are a weight row or one output's two (Q4_K gate and up: 2 nblk x 144 B) or one 4-row item (down) and a warp keeps SLOTS-1
 //     of them in flight while it computes on one: no copy holds a lane;
 //   * unit -> (slot, row) bookkeeping is incremental (one division per token instead of one per unit);
 //   * Q6_K down tensors are re-tiled once at load time into 4-row "chunk-major" items (`repack_q6k4t`, moe.cu):
@@ -131,11 +131,11 @@ __device__ __forceinline__ float q4k_block_dot(const uint8_t* wb, const uint8_t*
 // Gate/up (PAIR) or dense (PAIR = false) rows of Q4_K tensors.  Per warp: a private ring of SLOTS slots, and at any time SLOTS-1 of them are in flight behind the one being
 // consumed.  A slot holds one row, gate and up rows alternating (PAIR), or (BOTH) the gate and the up row of one output, whose dots share their activation loads.
 // A dozen warps an SM wait for their own loads and sums more than for a unit of the SM (43 % of the issue slots and of the shared-memory wavefronts in use with one row a slot): two
-// rows at a time are two chains beside each other and a third fewer loads.  MoE block of 7 tokens 377 -> 363 us (256 experts of 2048 x 7168, 8 chosen), 151 -> 137 (64 of 1024 x
+// rows at a time are two chains beside each other and a third fewer loads.  MoE block of 7 tokens 377 -> 362 us (256 experts of 2048 x 7168, 8 chosen), 151 -> 137 (64 of 1024 x
 // 4096, 6); routed experts of 9 tokens, 160 of 1536 x 5120, 6 chosen, 202 -> 183.  But slots of two rows take the warps' place, and a CTA that has few rows, or fits few warps, is
 // better off with more warps (launch_rows_bulk_q4k, moe.cu).
 //
-// Tokens are processed in chunks of `tc` (launcher: as many as fit next to >= 12 rings).  Within a chunk ALL
+// Tokens are processed in chunks of `tc` (launcher: as many as fit next to 12 rings, 8 of two rows a slot).  Within a chunk ALL
 // (token, slot) pairs this launch owns form ONE work list — expert-parallel shards and decode batches keep the ring
 // streaming across tokens instead of draining it once per token — and all the chunk's activation rows are staged as
 // Q8_K side by side (`act_tok` bytes each).

@@ -32,7 +32,7 @@
 //      cycles for a block of two matrices).  The warp's number and what the tiles say come through a shuffle, so that the compiler knows them to be the same in all
 //      lanes and keeps a role's state, its branches and the MMAs' operands off the vector pipes (the other roles' share of the issue slots is what an issuer or
 //      an epilogue warp waits for: 157 -> 129 us for the linear below, 2,782 -> 2,600 for the experts; 268 -> 69 branch instructions a block).
-//      A block of two matrices takes 3,100 cycles at 64 tokens a tile (3,440 before), 1,890 at 16 (2,480; Q6_K 3,570, 4,120); HBM brings one every 1,550 (Q6_K 2,270).  Of the 3,150 the drain of an accumulator is
+//      A block of two matrices takes 3,100 cycles at 64 tokens a tile (3,440 before), 1,890 at 16 (2,480; Q6_K 3,570, 4,120); HBM brings one every 1,550 (Q6_K 2,270).  Of the 3,100 the drain of an accumulator is
 //      1,500 (producers issue beside it; 660 alone), the eight MMAs of either stage 600, the rest hand-overs.  Draining in two halves of the tokens, so that one is multiplied
 //      while the other is drained, was slower (140 us, 2,770), and so were both matrices' drains in one thread (244) and other orders of the roles (165).
 //      At 16 tokens the schedulers issue three instructions of four possible ones a cycle, nearly all of them the producers'; their share of polls and address arithmetic is small

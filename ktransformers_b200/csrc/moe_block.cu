@@ -5,11 +5,11 @@
 // operators/llamafile/moe.cpp:146-245) and `y += self.shared_experts(identity)`.
 //
 // Why one kernel: a launch that streams ~100-150 MB lasts 25-30 us on a B200 of which ~6 us are fixed cost (launch
-// gap, pipeline ramp, activation prologue, tail) — profiles/probe_bulk.txt: the bare copy ring needs 27.3 us for the
+// gap, pipeline ramp, activation prologue, tail): the bare copy ring needs 27.3 us for the
 // gate/up bytes that take 21 us at the sustained rate.  Three launches per layer pay that three times.  Here the 148
 // CTAs (one per SM, cooperative launch, 12 warps, 168 registers) stay resident for the whole layer and separate the
-// phases with two grid-wide barriers.  What overlaps what was decided with profiles/block_trace.py (%globaltimer at the
-// phase boundaries of every CTA):
+// phases with two grid-wide barriers.  (2 to 8 tokens: moe_block_many_kernel below.)  What overlaps what was decided with ktb200_debug_block_trace
+// (%globaltimer at the phase boundaries of every CTA):
 //   * a barrier is split into arrive / wait; weights that do not depend on the other CTAs are requested in between
 //     (the shared expert's rows behind barrier 1, the first down tiles — they need the expert ids only — behind
 //     barrier 2), never before the arrive: a fence issued with bulk copies in flight waits for them;
@@ -554,7 +554,8 @@ __global__ void __launch_bounds__(MAXW * 32, 1) moe_block_kernel(const BlockPara
 // router, the selection, two barriers and the ends of the streams are 22 us that nothing overlaps (7 tokens: 450 us); here the router's rows are read once for all tokens, a CTA
 // per token selects, and the (token, slot) pairs form one work list for gate and up and one for down, streamed by the row kernels' bodies (gemv_bulk.cuh).  The order of every sum is
 // the separate launches', so the results are their bits.  What bounds it: the bytes of every pair's expert at ~5 TB/s (an expert that two of a few tokens choose is rare).
-// 256 experts of 2048 x 7168, 8 chosen: 2 tokens 134 -> 121 us, 4 260 -> 208, 7 450 -> 362; 64 of 1024 x 4096, 6 chosen: 7 tokens 214 -> 137.
+// 256 experts of 2048 x 7168, 8 chosen: 2 tokens 134 -> 121 us, 4 261 -> 209, 7 450 -> 363 (on two other GPUs of the same kind 372 and 374); 64 of 1024 x 4096, 6 chosen: 7 tokens
+// 214 -> 137.  Its phases start with empty rings: nothing is requested ahead of a barrier, as the kernel above does.
 template <int NT>
 __device__ __forceinline__ void many_router(const GateParams& g, int nt) {      // gate_dot's order of sums (gate.cuh)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5, E = g.E, S = g.S, n4 = g.H / 4;
@@ -1337,7 +1338,7 @@ extern "C" int ktb200_moe_ep_block_forward(const ktb200_gate_config* gc, ktb200_
 
 // Prefetch hint: while this handle's block kernel streams its down projection, pull up to three byte ranges into L2 — the
 // caller passes what the NEXT layer's launch reads first (its router weight, its shared expert's gate / up tensors).
-// Measured at DeepSeek-V3 shapes (profiles/r02_block_experiments.md): no gain while the down stream already saturates HBM
+// Measured at DeepSeek-V3 shapes: no gain while the down stream already saturates HBM
 // (the prefetch competes with it), so bench.py leaves it off; kept for callers whose next layer is not back to back.
 extern "C" int ktb200_moe_block_prefetch_hint(ktb200_moe* m, const void* const* ptrs, const size_t* bytes, int n) {
     if (!m || n < 0 || n > 3 || (n && (!ptrs || !bytes))) { set_error("prefetch_hint: up to 3 ranges"); return KTB200_EINVAL; }
@@ -1377,6 +1378,6 @@ extern "C" int ktb200_moe_block_forward_host(const ktb200_gate_config* gc, ktb20
     return KTB200_OK;
 }
 
-// Diagnostics (profiles/block_trace.py): when set, thread 0 of every CTA of the following ktb200_moe_block_forward
+// Diagnostics: when set, thread 0 of every CTA of the following ktb200_moe_block_forward
 // launches writes %globaltimer at the phase boundaries into trace[cta][16] (device memory, >= 148*16 u64).
 extern "C" void ktb200_debug_block_trace(unsigned long long* trace_dev) { g_btrace = trace_dev; }

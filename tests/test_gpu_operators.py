@@ -68,7 +68,7 @@ def test_injected_v3_moe_decodes_through_one_launch_and_matches_dense(tmp_path):
         assert isinstance(moe.experts.generate_experts, KExpertsB200) and moe.experts.generate_experts.handle is not None
 
         W = {k: torch.from_numpy(np.array(v)).cuda() for k, v in dense.items()}
-        for n_tok in (1, 3, 12, 64):     # block kernel | per-pair kernels | grouped tensor-core path (qlen >= KTB200_GROUPED_MIN)
+        for n_tok in (1, 3, 12, 64):     # block kernel (one token, several) | modules, row kernels at these sizes (ktb200_moe_takes_gemms) | grouped tensor-core path
             x = (torch.randn(1, n_tok, H, device="cuda") / 10).to(torch.bfloat16)
             n0 = native.launch_count()
             y = moe(x)
