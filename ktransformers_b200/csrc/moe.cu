@@ -142,7 +142,7 @@ static int env_int(const char* name, int dflt) {
 static int cfg_minb() { static int v = env_int("KTB200_MINB", 2); return v == 3 ? 3 : 2; }
 static int cfg_pipe() { static int v = env_int("KTB200_PIPE", 2); return v; }   // 0 off, 1 chunk-per-lane, 2 block-per-lane
 static int cfg_nb() { static int v = env_int("KTB200_NB", 2); return v == 4 ? 4 : 2; }
-// bulk-copy generation (gemv_bulk.cuh): KTB200_BULK=0 disables it, *_SLOTS_* = ring depth, KTB200_BULK_WARPS caps the CTA
+// bulk-copy generation (gemv_bulk.cuh): KTB200_BULK=0 disables it, *_SLOTS_* = ring depth, 2 or 3 (UP: where gate and up share a slot), KTB200_BULK_WARPS caps the CTA
 static int cfg_bulk() { static int v = env_int("KTB200_BULK", 1); return v; }
 static int cfg_bulk_slots_up() { static int v = env_int("KTB200_BULK_SLOTS_UP", 2); return v == 3 ? 3 : 2; }
 static int cfg_bulk_slots_down() { static int v = env_int("KTB200_BULK_SLOTS_DOWN", 2); return v == 3 ? 3 : 2; }

@@ -594,36 +594,38 @@ __device__ __forceinline__ void many_router(const GateParams& g, int nt) {      
         }
     }
 }
-template <class DownFmt>
+// EXTRAS: with the ranges to prefetch and the stamps of ktb200_debug_block_trace (in every launch they take 1 to 2 us of 370)
+template <class DownFmt, bool EXTRAS>
 __global__ void __launch_bounds__(MoeRowsPlan::kWarps * 32, 1) moe_block_many_kernel(const __grid_constant__ GateParams g, unsigned* sync, const __grid_constant__ MoeRowsPlan plan,
                                                                                       const __grid_constant__ BlockExtras extras) {
     extern __shared__ __align__(16) uint8_t smem[];
     griddep_launch_dependents();
     griddep_wait();
-    block_stamp(extras, 0);
+    auto stamp = [&](int i) { if (EXTRAS) block_stamp(extras, i); };
+    stamp(0);
     const int T = g.bsz ? min(g.T, *g.bsz) : g.T;
     unsigned gen = 0;
     if (T <= 2) many_router<2>(g, T);
     else if (T <= 4) many_router<4>(g, T);
     else many_router<kBlockMaxTokens>(g, T);
-    block_stamp(extras, 2);
+    stamp(2);
     grid_arrive(sync, gen);
     grid_wait(sync, gen);
-    block_stamp(extras, 3);
+    stamp(3);
     for (int t = blockIdx.x; t < T; t += gridDim.x)
         if ((threadIdx.x >> 5) < kGateWarps) gate_select_token<1>(g, t, reinterpret_cast<float*>(smem), g.idx + (long)t * g.top_k, g.w + (long)t * g.top_k, g.logits_out);
     grid_arrive(sync, gen);
     grid_wait(sync, gen);
-    block_stamp(extras, 4);
+    stamp(4);
     rows_bulk_q4k<true, MoeRowsPlan::kSlotsUp, true>(plan.rows, plan.act_tok, plan.tc);
     grid_arrive(sync, gen);
-    block_stamp(extras, 5);
+    stamp(5);
     grid_wait(sync, gen);
-    block_stamp(extras, 6);
-    reduce_bulk<DownFmt, MoeRowsPlan::kSlotsDown>(plan.down, plan.nrows_max, plan.pcap, [&] { block_prefetch(extras, threadIdx.x & 31); });
+    stamp(6);
+    reduce_bulk<DownFmt, MoeRowsPlan::kSlotsDown>(plan.down, plan.nrows_max, plan.pcap, [&] { if (EXTRAS) block_prefetch(extras, threadIdx.x & 31); });
     // leave the barrier words zeroed for the next launch / graph replay: the last CTA to get here resets them
     __syncthreads();
-    block_stamp(extras, 9);
+    stamp(9);
     if (threadIdx.x == 0 && atomicAdd(sync + 1, 1u) == gridDim.x - 1) {
         sync[0] = 0;
         sync[1] = 0;
@@ -1172,7 +1174,8 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
     BlockExtras& extras = p;
     void *one[] = {&p}, *all[] = {&p.g, &p.sync, &many, &extras}, **args = all_at_once ? all : one;
     const void* fn;
-    if (all_at_once) fn = fd == FMT_Q6K4T ? (const void*)moe_block_many_kernel<BulkQ6K4T> : (const void*)moe_block_many_kernel<BulkQ4K>;
+    if (all_at_once && (p.trace || p.pf[0] || p.pf[1] || p.pf[2])) fn = fd == FMT_Q6K4T ? (const void*)moe_block_many_kernel<BulkQ6K4T, true> : (const void*)moe_block_many_kernel<BulkQ4K, true>;
+    else if (all_at_once) fn = fd == FMT_Q6K4T ? (const void*)moe_block_many_kernel<BulkQ6K4T, false> : (const void*)moe_block_many_kernel<BulkQ4K, false>;
     else if (W > kBlockWarpsLo) fn = fd == FMT_Q6K4T ? (const void*)moe_block_kernel<BulkQ6K4T, kBlockWarps> : (const void*)moe_block_kernel<BulkQ4K, kBlockWarps>;
     else fn = fd == FMT_Q6K4T ? (const void*)moe_block_kernel<BulkQ6K4T, kBlockWarpsLo> : (const void*)moe_block_kernel<BulkQ4K, kBlockWarpsLo>;
     static const int coop = [] { const char* e = getenv("KTB200_BLK_COOP"); return e ? atoi(e) : 1; }();

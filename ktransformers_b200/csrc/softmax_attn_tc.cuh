@@ -12,9 +12,9 @@
 //                  more than 2^8 (P <= 256 in between, where bf16 and fp32 are as exact as below 1)
 // TMEM: [S0 | O0 | S1 | O1], 128 columns each.  Shared memory: Q 64 KB, K and V 2 x 32 KB each.
 // Bounds: 16 products of 64 cycles per (row tile, key tile) beside 128 exponentials per thread at 4 per cycle and scheduler (1024 cycles for two
-// tiles on one scheduler): 2,050 cycles of tensor pipe for two tiles, 95-105 us for 2048 tokens behind 2048, 64 heads over 8.  It takes 264: a row's maximum, exponentials,
-// conversions and stores run one after the other in its thread, the tile's next product waits for all of them, and there is one score buffer a tile (tensor pipe 45 %
-// active, issue slots 34 %).
+// tiles on one scheduler): 2,050 cycles of tensor pipe for two tiles, 95-105 us for 2048 tokens behind 2048, 64 heads over 8.  It takes 250: a row's maximum, exponentials,
+// conversions and stores run one after the other in its thread, the tile's next product waits for all of them, and there is one score buffer a tile (tensor pipe 48 %
+// active, issue slots 35 %).
 #pragma once
 #include <cuda.h>
 

@@ -87,7 +87,9 @@ def _close(a, b):
 
 
 @pytest.mark.parametrize("T", [9, 24, 47])
-def test_one_call_agrees_with_the_modules(T):
+def test_one_call_agrees_with_the_modules(T, monkeypatch):
+    from ktransformers_b200.operators.experts import KExpertsB200
+    monkeypatch.setattr(KExpertsB200, "output_gpu_map", {})      # (captured calls write to the device's buffer, which has the width of the first experts that were loaded)
     moe, serve = _block(64, 6, 2048, 1536), _block(64, 6, 2048, 1536, serve=True)
     x = _x(T, 2048, T)
     y, one = _in_one_call(moe, x)
