@@ -27,7 +27,8 @@
 // CTA: 28 warps in 7 groups of 4.  Groups 0-3 producers: (matrix 0, first operand stage), (matrix 1, first), (0, second), (1, second), a warp = 32 rows, a stage in
 //      two parts of 32 columns that are filled, multiplied and given back by themselves (whole stages: 129 us for the linear below, 2,640 for the experts):
 //      raw blocks from a TMA ring -> registers -> TMEM; warp 16 TMA of activations, 17 / 18 MMA issuers of matrix 0 / 1, 19 TMA of weights;
-//      groups 5 / 6 epilogue of matrix 0 / 1.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
+//      groups 5 / 6 epilogue of matrix 0 / 1.  With many tokens (kTwoSets) an epilogue of two groups a matrix, half of the tokens each, beside two groups of producers: an
+//      accumulator's drain is one thread's chain of loads and sums, and with 64 tokens the next product waits for it.  One warp of a group polls a barrier and the others wait in a hardware barrier behind it: polling
 //      warps took a third of the issue slots, and the four roles' code is kept in rolled loops: unrolled it overran the instruction cache (10,000
 //      cycles for a block of two matrices).  The warp's number and what the tiles say come through a shuffle, so that the compiler knows them to be the same in all
 //      lanes and keeps a role's state, its branches and the MMAs' operands off the vector pipes (the other roles' share of the issue slots is what an issuer or
@@ -37,7 +38,9 @@
 //      while the other is drained, was slower (140 us, 2,770), and so were both matrices' drains in one thread (244) and other orders of the roles (165).
 //      At 16 tokens the schedulers issue three instructions of four possible ones a cycle, nearly all of them the producers'; their share of polls and address arithmetic is small
 //      (every producer warp polling for itself, barrier addresses in registers: within 1 %).
-//      Measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 2,910 -> 2,540 us (the operator's call); Q4_K linear 777 x 1536 -> 24576 180 -> 126 us (466 TFLOP/s).
+//      Measured, DeepSeek-V3 sizes: routed experts of 1024 tokens 2,910 -> 2,540 us (the operator's call); Q4_K linear 777 x 1536 -> 24576 180 -> 126 us, with two epilogue groups a matrix 112 (520 TFLOP/s).
+//      Tried beside it: nibbles as e4m3 operands against two e4m3 digits of the activations, exact too and 3 instructions for 8 weights, but eight sums a block to be scaled instead of
+//      one (207 us, experts 3,530); 8 epilogue threads' worth of registers so that all columns are loaded before they are scaled (125, 2,660); the headers in warps of their own (123, 2,630).
 // TMEM: [accumulator | minima] x 2 matrices, then 64-column operand stages, 2 per matrix.
 #include <algorithm>
 #include <atomic>
@@ -59,9 +62,6 @@ struct KqCfg {
     static constexpr int kRow = FMT == KQ_Q4K ? 144 : FMT == KQ_Q5K ? 176 : 208;      // bytes of a row's block in a ring slot (Q6_K: without d)
     static constexpr int kStages = kQ6 ? 4 : 2;                                       // operand stages per block
     static constexpr float kScale = FMT == KQ_Q4K ? 1.f : FMT == KQ_Q5K ? 2.f : 4.f;  // what the fp16 integers were divided by
-    // registers: producers, issuers, epilogue.  They draw on the launch's 7 x 72 per warp group
-    static constexpr int kRegsP = 48, kRegsI = 72, kRegsE = 120;
-    static_assert(4 * kRegsP + kRegsI + 2 * kRegsE == 7 * 72, "register split");
     // shared memory
     static constexpr int kRing = 3, kMat = 128 * kRow, kSlot = 2 * kMat;
     static constexpr int kB = kKqN * 512, kOffRing = 2 * kB, kOffMins = kOffRing + kRing * kSlot, kMins = kQ6 ? 0 : 128 * 32;        // minima: [matrix][2]
@@ -74,6 +74,15 @@ struct KqMisc {
     uint32_t hdr[2][2][128];      // Q4_K, Q5_K: half2 (d, dmin) of a row's block
 };
 constexpr int kKqThreads = 896;
+// How the 28 warps are dealt: SETS epilogue groups of four warps a matrix, each with its part of the tile's tokens, and 4 / SETS groups of producers
+template <int SETS>
+struct KqSplit {
+    static constexpr int kProd = 16 / SETS, kEpi = kProd + 4;                 // first warps of the issuers and copies (four), and of the epilogue
+    static constexpr int kHalves = 2 / SETS, kCols = kKqN / SETS;             // groups that share a matrix's operand stages; tokens of an epilogue thread at most
+    // registers: producers, issuers, epilogue.  They draw on the launch's 7 x 72 per warp group
+    static constexpr int kRegsP = SETS == 1 ? 48 : 56, kRegsI = SETS == 1 ? 72 : 40, kRegsE = SETS == 1 ? 120 : 88;
+    static_assert(4 / SETS * kRegsP + kRegsI + 2 * SETS * kRegsE == 7 * 72, "register split");
+};
 template <int FMT>
 constexpr int kq_smem() { return KqCfg<FMT>::kOffMisc + (int)sizeof(KqMisc) + 1024; }
 static_assert(kq_smem<KQ_Q4K>() <= 232448 && kq_smem<KQ_Q5K>() <= 232448 && kq_smem<KQ_Q6K_T4>() <= 232448, "shared memory budget");
@@ -260,32 +269,37 @@ __device__ __forceinline__ int kq_q6_word(int r, int c) {
 }
 struct KqMaps { CUtensorMap q, sums, w[2][3]; };      // activations, their sums; weights of matrix 0 / 1 (Q6_K in 8-row groups: ql, qh, scales)
 
-template <int FMT, bool MARKS>
+template <int FMT, bool MARKS, int SETS>
 __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, uint8_t* smem, KqMisc& misc, uint32_t base, uint32_t tmem, int total) {
     using C = KqCfg<FMT>;
+    using S = KqSplit<SETS>;
     constexpr bool Q6 = C::kQ6;
     constexpr int kAccCols = 2 * kKqN, kColA = 2 * kAccCols;      // per matrix: accumulator, minima or the sum of one stage; then the operand stages
     const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);      // (known to be uniform: see above)
-    if (warp < 16) {
+    if (warp < S::kProd) {
         // ========================================================================== producers
-        regs_down<C::kRegsP>();
-        const int mat = (warp >> 2) & 1, half = warp >> 3, r = tid & 127, grp = warp >> 2;      // row of the tile's matrix = TMEM lane; operand stages half, half + 2
+        regs_down<S::kRegsP>();
+        const int mat = (warp >> 2) & 1, half = warp >> 3, r = tid & 127, grp = warp >> 2;      // row of the tile's matrix = TMEM lane; operand stages half, half + kHalves, ...
         const bool leader = (warp & 3) == 0;
-        const uint32_t dst = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kColA + (mat * 2 + half) * 64;
+        const uint32_t dst0 = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kColA + mat * 128;
         int slot = 0, sphase = 0;
-        unsigned it = 0, uses = 0;       // blocks, and uses of this group's operand stage, so far
+        unsigned it = 0;       // blocks so far
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
             const int nsb = kq_tile(p, tile).nsb;
             for (int s = 0; s < nsb; s++, it++) {
                 const uint8_t* src = smem + C::kOffRing + slot * C::kSlot + mat * C::kMat;
                 bar_wait(smem_u32(&misc.raw_full[slot]), sphase);
+                const uint8_t* const row = src + r * C::kRow;
 #pragma unroll 1
-                for (int h = half; h < C::kStages; h += 2, uses++) {
+                for (int h = half; h < C::kStages; h += S::kHalves) {
+                    const int buf = h & 1;
+                    const unsigned uses = it * (C::kStages / 2) + (h >> 1);      // of the buffer so far
+                    const uint32_t dst = dst0 + buf * 64;
                     // either part of an operand stage is free, is filled and goes to the issuer by itself: one is multiplied while the other is filled
                     auto open = [&](int part) {
                         if (leader) {
-                            bar_wait(smem_u32(&misc.a_free[mat][half][part]), (uses & 1) ^ 1);
-                            if (!Q6 && !half && part) bar_wait(smem_u32(&misc.hdr_free[mat][it & 1]), ((it >> 1) & 1) ^ 1);
+                            bar_wait(smem_u32(&misc.a_free[mat][buf][part]), (uses & 1) ^ 1);
+                            if (!Q6 && !h && part) bar_wait(smem_u32(&misc.hdr_free[mat][it & 1]), ((it >> 1) & 1) ^ 1);
                         }
                         group_sync(1 + grp);
                         tc_fence_after();
@@ -294,17 +308,16 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                         tmem_wait_st();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) bar_arrive(smem_u32(&misc.a_full[mat][half][part]));
+                        if (lane == 0) bar_arrive(smem_u32(&misc.a_full[mat][buf][part]));
                     };
                     uint32_t w[8], o[16];
                     if (!Q6) {
-                        src += r * C::kRow;
-                        const uint4 head = *reinterpret_cast<const uint4*>(src);
+                        const uint4 head = *reinterpret_cast<const uint4*>(row);
                         const uint32_t sc = h ? kq_six<1>(head.y, head.w) : kq_six<0>(head.y, 0);
 #pragma unroll
                         for (int part = 0; part < 2; part++) {      // chunk c = 2h + part: low nibbles are sub-block 2c, high nibbles sub-block 2c + 1
                             const __half2 sl = part ? h2_byte<2>(sc) : h2_byte<0>(sc), sh = part ? h2_byte<3>(sc) : h2_byte<1>(sc);
-                            const uint8_t* q = src + C::kRow - 128 + 32 * (2 * h + part);
+                            const uint8_t* q = row + C::kRow - 128 + 32 * (2 * h + part);
                             kq_words8(q, q + 16, w);
                             open(part);
                             if (FMT == KQ_Q4K) {
@@ -315,14 +328,14 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                                 }
                             } else {
                                 uint32_t qh[8];
-                                kq_words8(src + 16, src + 32, qh);
+                                kq_words8(row + 16, row + 32, qh);
 #pragma unroll
                                 for (int i = 0; i < 2; i++) {
                                     kq_unpack5(w + 4 * i, qh + 4 * i, 2 * (2 * h + part), sl, sh, o);
                                     tmem_st16(dst + 32 * part + 16 * i, o);
                                 }
                             }
-                            if (part && !half) {      // this group also hands on (d, dmin) and the minima, each twice, against the sixteen 16-value activation sums
+                            if (part && !h) {      // the group of a block's first stage also hands on (d, dmin) and the minima, each twice, against the sixteen 16-value activation sums
                                 misc.hdr[mat][it & 1][r] = head.x;
                                 uint8_t* m = smem + C::kOffMins + (mat * 2 + (it & 1)) * C::kMins + (r >> 3) * 256 + (r & 7) * 16;      // K-major core matrices of 8 rows x 16 bytes
 #pragma unroll
@@ -387,8 +400,9 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                 if (++slot == C::kRing) { slot = 0; sphase ^= 1; }
             }
         }
-    } else if (warp < 20) {
-        if (warp == 16) {
+    } else if (warp < S::kEpi) {
+        if (SETS > 1) regs_down<S::kRegsI>();
+        if (warp == S::kProd) {
             // ====================================================================== activations
             const bool one = lane == 0;
             if (one) tma_prefetch_desc(&maps.q);
@@ -420,7 +434,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                 }
             }
             __syncwarp();
-        } else if (warp == 19) {
+        } else if (warp == S::kProd + 3) {
             // ====================================================================== weights: the blocks of 2 x 128 rows as they lie in memory
             const bool one = lane == 0;
             {
@@ -456,7 +470,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
             __syncwarp();
         } else {
             // ====================================================================== tensor-core issuers (converged warps), one per matrix
-            const int mat = warp - 17;
+            const int mat = warp - S::kProd - 1;
             const uint32_t acc = tmem + mat * kAccCols, a0 = tmem + kColA + mat * 128;
             unsigned it = 0, uses = 0, fills = 0;      // blocks, stages / 2, and accumulators handed to the epilogue so far
             for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
@@ -514,15 +528,16 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
             }
         }
     } else {
-        // ========================================================================== epilogue: a thread owns one weight row and the tile's tokens
-        regs_up<C::kRegsE>();
-        const int mat = (warp - 20) >> 2, sp = warp & 3, r = 32 * sp + lane;
+        // ========================================================================== epilogue: a thread owns one weight row and its group's part of the tile's tokens
+        regs_up<S::kRegsE>();
+        const int grp = (warp - S::kEpi) >> 2, mat = grp & 1, sp = warp & 3, r = 32 * sp + lane;
         const bool leader = sp == 0;
-        const uint32_t tacc = tmem + ((uint32_t)(32 * sp) << 16) + mat * kAccCols;
         unsigned it = 0, fills = 0;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
             const KqTile t = kq_tile(p, tile);
             const int row = t.row0 + (p.pair ? 0 : 128 * mat) + r;
+            const int most = SETS == 1 ? kKqN : t.n > 32 ? 32 : 16, col0 = most * (grp >> 1), cols = min(most, t.n - col0);      // (none where <= 0)
+            const uint32_t tacc = tmem + ((uint32_t)(32 * sp) << 16) + mat * kAccCols + col0;
             // a Q6_K block's d comes straight from memory, a block ahead
             const uint16_t* dsrc = nullptr;
             uint16_t dnext = 0;
@@ -533,9 +548,9 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                                                                          : w + (long)(rc >> 3) * 8 * p.nblk * SZ_Q6_K + 1664L * p.nblk + (rc & 7) * p.nblk * 2) + t.sb0;
                 dnext = __ldg(dsrc);
             }
-            f32x2 acc[kKqN / 2];
+            f32x2 acc[S::kCols / 2];
 #pragma unroll
-            for (int n = 0; n < kKqN / 2; n++) acc[n] = 0;
+            for (int n = 0; n < S::kCols / 2; n++) acc[n] = 0;
             for (int s = 0; s < t.nsb; s++, it++) {
                 const uint16_t dcur = dnext;
                 if (Q6 && s + 1 < t.nsb) dnext = __ldg(dsrc + s + 1);
@@ -543,7 +558,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                 auto sums = [&] {
                     if (leader) bar_wait(smem_u32(&misc.acc_full[mat]), fills & 1);
                     fills++;
-                    group_sync(5 + mat);
+                    group_sync(5 + grp);
                     tc_fence_after();
                 };
                 sums();
@@ -551,7 +566,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
 #pragma unroll 1
                     for (int h = 1;; h++) {
 #pragma unroll 1
-                        for (int c = 0; c < t.n; c += 16) {
+                        for (int c = 0; c < cols; c += 16) {
                             uint32_t v[16], m[16];
                             tmem_ld16(tacc + c, v);
                             tmem_ld16(tacc + kKqN + c, m);
@@ -572,19 +587,21 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                 const __half2 dm = as_h2(Q6 ? (uint32_t)dcur : misc.hdr[mat][it & 1][r]);
                 const float dw = __low2float(dm) * C::kScale, dmin = -__high2float(dm);
                 const f32x2 dw2 = pack2(dw, dw), dmin2 = pack2(dmin, dmin);
-                const ulonglong2* dx = reinterpret_cast<const ulonglong2*>(misc.dx[it & 3]);
+                const ulonglong2* dx = reinterpret_cast<const ulonglong2*>(misc.dx[it & 3] + col0);
+                auto give = [&] {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(smem_u32(&misc.acc_free[mat]));
+                };
+                if (SETS > 1 && cols <= 0) give();
 #pragma unroll
-                for (int c = 0; c < kKqN / 16; c++) {
-                    if (16 * c < t.n) {
+                for (int c = 0; c < S::kCols / 16; c++) {
+                    if (16 * c < cols) {
                         uint32_t v[16], m[16];
                         tmem_ld16(tacc + 16 * c, v);
                         if (!Q6) tmem_ld16(tacc + kKqN + 16 * c, m);
                         tmem_wait_ld();
-                        if (16 * c + 16 >= t.n) {      // the last columns are out: the next block may be multiplied while these are scaled
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) bar_arrive(smem_u32(&misc.acc_free[mat]));
-                        }
+                        if (16 * c + 16 >= cols) give();      // the last columns are out: the next block may be multiplied while these are scaled
 #pragma unroll
                         for (int i = 0; i < 4; i++) {
                             const ulonglong2 x = dx[4 * c + i];
@@ -606,12 +623,12 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
             }
             // eight tokens at a time in a rolled loop, the sums moving down to its registers, and no branch per value: with ggml's rounding in branches a tile's output took
             // 11,000 cycles, half of a tile of 6 blocks; now 5,500
-            int left = t.n;
-            if (p.y && p.bsz) left = min(left, *p.bsz - p.t0 - t.p0);
+            int left = cols;
+            if (p.y && p.bsz) left = min(left, *p.bsz - p.t0 - t.p0 - col0);
             if (row >= p.R) left = 0;
             const float bias = p.y && p.bias && left > 0 ? p.bias[row] : 0.f;
             const int type = p.y ? p.hidden_type : KTB200_TYPE_F32;
-            const long first = ((long)t.split * p.T + t.p0) * p.R;
+            const long first = ((long)t.split * p.T + t.p0 + col0) * p.R;
             uint8_t* const out = reinterpret_cast<uint8_t*>(p.y ? p.y : p.out[mat]) + (type == KTB200_TYPE_F32 ? 4 : 2) * first;
             uint32_t at = (uint32_t)row;
 #pragma unroll 1
@@ -630,15 +647,16 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                 }
                 at += 8u * p.R;
 #pragma unroll
-                for (int n = 0; n + 4 < kKqN / 2; n++) acc[n] = acc[n + 4];
+                for (int n = 0; n + 4 < S::kCols / 2; n++) acc[n] = acc[n + 4];
             }
         }
     }
 }
 
-template <int FMT, bool MARKS>
+template <int FMT, bool MARKS, int SETS>
 __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
     using C = KqCfg<FMT>;
+    using S = KqSplit<SETS>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -649,33 +667,33 @@ __device__ __forceinline__ void kq_body(const KqMaps& maps, const KqParams& p) {
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
             bar_init(smem_u32(&misc.b_full[i]), 1); bar_init(smem_u32(&misc.b_free[i]), 2);
-            bar_init(smem_u32(&misc.acc_full[i]), MARKS ? 2 : 1); bar_init(smem_u32(&misc.acc_free[i]), 4);
+            bar_init(smem_u32(&misc.acc_full[i]), MARKS ? 2 : 1); bar_init(smem_u32(&misc.acc_free[i]), 4 * SETS);
             for (int j = 0; j < 2; j++) {
                 for (int k = 0; k < 2; k++) { bar_init(smem_u32(&misc.a_full[i][j][k]), 4); bar_init(smem_u32(&misc.a_free[i][j][k]), 1); }
-                bar_init(smem_u32(&misc.hdr_free[i][j]), 4);
+                bar_init(smem_u32(&misc.hdr_free[i][j]), 4 * SETS);
             }
         }
-        for (int i = 0; i < 4; i++) { bar_init(smem_u32(&misc.dx_full[i]), 1); bar_init(smem_u32(&misc.dx_free[i]), 8); }
-        for (int i = 0; i < C::kRing; i++) { bar_init(smem_u32(&misc.raw_full[i]), 1); bar_init(smem_u32(&misc.raw_free[i]), 16); }
+        for (int i = 0; i < 4; i++) { bar_init(smem_u32(&misc.dx_full[i]), 1); bar_init(smem_u32(&misc.dx_free[i]), 8 * SETS); }
+        for (int i = 0; i < C::kRing; i++) { bar_init(smem_u32(&misc.raw_full[i]), 1); bar_init(smem_u32(&misc.raw_free[i]), S::kProd); }
         bar_fence_init();
     }
-    if (warp == 17) tmem_alloc(smem_u32(&misc.tmem_base), 512);
+    if (warp == S::kProd + 1) tmem_alloc(smem_u32(&misc.tmem_base), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = uniform(misc.tmem_base);
 
-    kq_roles<FMT, MARKS>(maps, p, smem, misc, base, tmem, total);
+    kq_roles<FMT, MARKS, SETS>(maps, p, smem, misc, base, tmem, total);
     tc_fence_before();
     __syncthreads();
-    if (warp == 17) {
+    if (warp == S::kProd + 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
     }
 }
 
-template <int FMT>
-__device__ __noinline__ void kq_body_marked(const KqMaps& maps, const KqParams& p) { kq_body<FMT, true>(maps, p); }
+template <int FMT, int SETS>
+__device__ __noinline__ void kq_body_marked(const KqMaps& maps, const KqParams& p) { kq_body<FMT, true, SETS>(maps, p); }
 // The form for activations with marked blocks is apart from the other, and the quantiser's word says which one a call needs: in one form the calls without marks took 6-10 %
 // longer (777 x 1536 -> 24576 177 -> 194 us: a block's hand-overs wait for its mark, an MMA whose operand depends on it waits for that to be made uniform).
 //   KQ_BOTH             one launch, the marked form as a function: costs the other one 3-4 % (registers), and nothing where launches bound a call (512 -> 512, 64 rows: 25 us)
@@ -683,15 +701,15 @@ __device__ __noinline__ void kq_body_marked(const KqMaps& maps, const KqParams& 
 //                       routed experts 2920 us against 3013 with KQ_BOTH, 2893 without marks): experts, and from kPairBlocks blocks of a tile per CTA on
 enum KqForms { KQ_PLAIN, KQ_MARKED, KQ_BOTH };
 constexpr int kPairBlocks = 40;
-template <int FMT, KqForms FORMS>
+template <int FMT, KqForms FORMS, int SETS>
 __global__ void __launch_bounds__(kKqThreads, 1) kq_gemm_kernel(const __grid_constant__ KqMaps maps, const __grid_constant__ KqParams p) {
     const bool marks = *p.any == p.id;
     if (FORMS == KQ_BOTH) {
-        if (marks) kq_body_marked<FMT>(maps, p);
-        else kq_body<FMT, false>(maps, p);
+        if (marks) kq_body_marked<FMT, SETS>(maps, p);
+        else kq_body<FMT, false, SETS>(maps, p);
     } else {
         if (FORMS == KQ_PLAIN) griddep_launch_dependents();
-        if (marks == (FORMS == KQ_MARKED)) kq_body<FMT, FORMS == KQ_MARKED>(maps, p);
+        if (marks == (FORMS == KQ_MARKED)) kq_body<FMT, FORMS == KQ_MARKED, SETS>(maps, p);
         if (FORMS == KQ_MARKED) griddep_wait();      // (what follows it in the stream follows both)
     }
 }
@@ -837,22 +855,33 @@ static int kq_map_weights(CUtensorMap* m, KqFmt f, const void* w, long rows, int
     }
     return KTB200_OK;
 }
-template <int FMT>
-static int kq_launch(const KqMaps& maps, const KqParams& p, int grid, cudaStream_t s) {
+template <int FMT, int SETS>
+static int kq_launch_as(const KqMaps& maps, const KqParams& p, int grid, cudaStream_t s) {
     constexpr int smem = kq_smem<FMT>();
     if (!p.tinfo && (long)p.total * ((p.nblk + p.splits - 1) / p.splits) < (long)kPairBlocks * grid) {
-        KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_BOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kq_gemm_kernel<FMT, KQ_BOTH><<<grid, kKqThreads, smem, s>>>(maps, p);
+        KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_BOTH, SETS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kq_gemm_kernel<FMT, KQ_BOTH, SETS><<<grid, kKqThreads, smem, s>>>(maps, p);
         KTB_LAUNCH_CHECK();
         return KTB200_OK;
     }
-    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_MARKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kq_gemm_kernel<FMT, KQ_PLAIN><<<grid, kKqThreads, smem, s>>>(maps, p);
+    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_PLAIN, SETS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KTB_CUDA_CHECK(cudaFuncSetAttribute(kq_gemm_kernel<FMT, KQ_MARKED, SETS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kq_gemm_kernel<FMT, KQ_PLAIN, SETS><<<grid, kKqThreads, smem, s>>>(maps, p);
     KTB_LAUNCH_CHECK();
-    KTB_CUDA_CHECK(launch_pdl(kq_gemm_kernel<FMT, KQ_MARKED>, dim3(grid), dim3(kKqThreads), (size_t)smem, s, maps, p));
+    KTB_CUDA_CHECK(launch_pdl(kq_gemm_kernel<FMT, KQ_MARKED, SETS>, dim3(grid), dim3(kKqThreads), (size_t)smem, s, maps, p));
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
+}
+
+// Two epilogue groups a matrix for a Q4_K matrix against more than 48 tokens: measured against one group (us) 777 x 1536 -> 24576 126 -> 112, 333 of it 65.0 -> 60.9, 2048 -> 8192 64 tokens
+// 27.5 -> 25.4, 333 44.5 -> 42.4, 512 -> 4096 64 tokens 18.4 -> 16.5, and the same time where K splits leave the launch to its copies (7168 -> 2048, 65-333 tokens).  With 12-48
+// tokens 1-10 % slower (half as many producers; 1536 -> 24576, 17 tokens 20.8 -> 23.0), and in Q6_K and Q5_K, whose producers do more, at any number (Q6_K 333 tokens 80.7 -> 93.6)
+constexpr int kTwoSets = 49;
+template <int FMT>
+static int kq_launch(const KqMaps& maps, const KqParams& p, int grid, cudaStream_t s) {
+    if constexpr (FMT == KQ_Q4K)
+        if (!p.tinfo && p.T >= kTwoSets) return kq_launch_as<FMT, 2>(maps, p, grid, s);
+    return kq_launch_as<FMT, 1>(maps, p, grid, s);
 }
 
 int kq_gemm(const KqGemm& g, int device, cudaStream_t s) {
