@@ -16,7 +16,34 @@
 
 namespace ktb {
 
-__global__ void __launch_bounds__(kGateThreads) gate_kernel(const GateParams p) {
+// Bound for batches by chains of loads: CTAs of their own for every tile of 8 tokens (they share the rows through L2), a tile's columns in one round of loads while the rows are on
+// their way to L2, 5 CTAs an SM (96 registers), a token's selection (about 5 us of a CTA) beside the others'.  256 x 7168 (us): 8 tokens 34.0 -> 19.7, 24 tokens 77.6 -> 32.0, 200 tokens
+// 560 -> 160, one token 17.7 -> 17.1, against one CTA per rows and columns that took tile after tile, value by value, and 16 selectors.  Shorter selections (picks as a tree, groups
+// ranked by a warp) changed nothing here and in the fused block.
+constexpr int kGateTiles = 16, kGateSelectors = 64;
+// a tile's columns in fp32: four values a load, eight loads of a thread in flight before the first is looked at
+__device__ __forceinline__ float4 gate_floats(uint4 w, int) { return make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)); }
+__device__ __forceinline__ float4 gate_floats(uint2 w, int hidden_type) {
+    if (hidden_type == KTB200_TYPE_BF16)
+        return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
+    return make_float4(fp16_bits_to_f32((uint16_t)(w.x & 0xffff)), fp16_bits_to_f32((uint16_t)(w.x >> 16)), fp16_bits_to_f32((uint16_t)(w.y & 0xffff)), fp16_bits_to_f32((uint16_t)(w.y >> 16)));
+}
+template <typename V>
+__device__ __forceinline__ void gate_stage(const V* x, int row, int nt, int nc4, int hidden_type, float4* xs) {
+    for (int i0 = threadIdx.x; i0 < nt * nc4; i0 += 8 * kGateThreads) {
+        V v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = min(i0 + u * kGateThreads, nt * nc4 - 1), tt = i / nc4;
+            v[u] = __ldg(x + (long)tt * row + (i - tt * nc4));
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (i0 + u * kGateThreads < nt * nc4) xs[i0 + u * kGateThreads] = gate_floats(v[u], hidden_type);
+    }
+}
+
+__global__ void __launch_bounds__(kGateThreads, 5) gate_kernel(const GateParams p) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     float* xs = reinterpret_cast<float*>(smem_raw);   // [tok tile][slice cols]  (phase 1) / scores+choice (phase 2)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -29,12 +56,21 @@ __global__ void __launch_bounds__(kGateThreads) gate_kernel(const GateParams p) 
     const int e = blockIdx.x * kGateWarps + warp;
     const float4* wrow = reinterpret_cast<const float4*>(p.W + (long)(e < p.E ? e : 0) * p.H) + c0;
 
-    for (int t0 = 0; t0 < Teff; t0 += kGateTokTile) {
+    // the rows are under way to L2 while the tokens are fetched
+    if (e < p.E)
+        for (int c = 8 * lane; c < nc4; c += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(wrow + c));
+    const bool vec = (reinterpret_cast<uintptr_t>(p.x) & (p.hidden_type == KTB200_TYPE_F32 ? 15 : 7)) == 0;
+    for (int t0 = blockIdx.z * kGateTokTile; t0 < Teff; t0 += gridDim.z * kGateTokTile) {
         const int nt = min(kGateTokTile, Teff - t0);
         __syncthreads();
-        for (int tt = 0; tt < nt; tt++)
-            for (int c = threadIdx.x; c < nc4 * 4; c += kGateThreads)
-                xs[tt * nc4 * 4 + c] = load_hidden(p.x, (long)(t0 + tt) * p.H + 4L * c0 + c, p.hidden_type);
+        if (vec) {
+            const long x0 = (long)t0 * p.H + 4L * c0;
+            if (p.hidden_type == KTB200_TYPE_F32) gate_stage(reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.x) + x0), p.H / 4, nt, nc4, p.hidden_type, reinterpret_cast<float4*>(xs));
+            else gate_stage(reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.x) + x0), p.H / 4, nt, nc4, p.hidden_type, reinterpret_cast<float4*>(xs));
+        } else {
+            for (int tt = 0; tt < nt; tt++)
+                for (int c = threadIdx.x; c < nc4 * 4; c += kGateThreads) xs[tt * nc4 * 4 + c] = load_hidden(p.x, (long)(t0 + tt) * p.H + 4L * c0 + c, p.hidden_type);
+        }
         __syncthreads();
         if (e < p.E) {
             switch (nt) {   // compile-time token counts: no predicated-off FMAs for the common bs=1 decode
@@ -48,11 +84,11 @@ __global__ void __launch_bounds__(kGateThreads) gate_kernel(const GateParams p) 
 
     // ---- the last CTAs to finish select: one token each (round-robin), in parallel ----------------------------------
     // ticket[0] counts finished CTAs, ticket[1] finished selectors; both are zero again when the launch ends
-    // (graph-replay safe).  A selector that is not the very last CTA spins until all partial sums are written: the whole
-    // grid is resident (<= 16 small CTAs per SM), so the CTAs it waits for are running.
+    // (graph-replay safe).  A selector that is not the very last CTA spins until all partial sums are written: the
+    // few CTAs that are still at work when a selector spins hold their places, or get those of the CTAs that are done.
     __shared__ int s_sel;
-    const unsigned total = gridDim.x * gridDim.y;
-    const int nsel = min(Teff, (int)min(total, 16u));
+    const unsigned total = gridDim.x * gridDim.y * gridDim.z;
+    const int nsel = min(Teff, (int)min(total, (unsigned)kGateSelectors));
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -131,7 +167,8 @@ extern "C" int ktb200_moe_gate_forward(const ktb200_gate_config* c, int qlen, co
     const size_t smem_sel = ((size_t)2 * c->n_experts + 32 + 4 * kGateWarps) * sizeof(float);
     if (smem_sel > smem) smem = smem_sel;
     if (smem > 48 * 1024) KTB_CUDA_CHECK(raise_smem_limit((const void*)gate_kernel, smem));
-    gate_kernel<<<dim3(row_ctas, S), kGateThreads, smem, s>>>(p);
+    const int tiles = (qlen + kGateTokTile - 1) / kGateTokTile;
+    gate_kernel<<<dim3(row_ctas, S, tiles < kGateTiles ? tiles : kGateTiles), kGateThreads, smem, s>>>(p);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
