@@ -20,6 +20,8 @@
 //
 // Storage type T (bf16 or float) for activations and cache rows; rotation, norms, scores, the cap and the soft-max are fp32
 // (angles fp64).  Cache row of a token: [k G*maps*d | v G*dv]; a sequence's page table row is a ring.
+#include <algorithm>
+
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -192,6 +194,161 @@ __global__ void __launch_bounds__(256) rope_norm_cache_write_kernel(const QkvPre
             const float x = column(i);
             dst[i] = from_f<T>(a.v_unit_rms ? x * inv : x);
             if (CONV && last) cv.store_tail(col0 + i, ch0 + i);
+        }
+    }
+}
+
+// The same without a filter or a value blend, for heads of 32 PER columns (and values as wide): a lane owns PER consecutive columns, its rotated partners (layout of halves) come
+// from another lane, and a warp has the loads of kRowBatch units in flight.  Bound by the bytes of the rows: 2048 tokens of 64 + 8 + 8 heads of 128 (84 MB, 13 us) take
+// 37 us, by their instructions (140 a unit and warp); column by column, a unit at a time, 86.
+constexpr int kRowBatch = 4;
+template <typename T, int PER>
+__device__ __forceinline__ void load_row(const T* p, float (&v)[PER]) {
+    constexpr int kWords = PER * (int)sizeof(T) / 4;
+    uint32_t w[kWords];
+    if constexpr (kWords % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords; i += 4) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + i / 4);
+            w[i] = u.x; w[i + 1] = u.y; w[i + 2] = u.z; w[i + 3] = u.w;
+        }
+    } else if constexpr (kWords == 2) {
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+        w[0] = u.x; w[1] = u.y;
+    } else {
+        w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    }
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        if constexpr (sizeof(T) == 4) v[i] = __uint_as_float(w[i]);
+        else v[i] = __uint_as_float(i & 1 ? w[i / 2] & 0xffff0000u : w[i / 2] << 16);
+    }
+}
+template <typename T, int PER>
+__device__ __forceinline__ void store_row(T* p, const float (&v)[PER]) {
+    constexpr int kWords = PER * (int)sizeof(T) / 4;
+    uint32_t w[kWords];
+#pragma unroll
+    for (int i = 0; i < kWords; i++) {
+        if constexpr (sizeof(T) == 4) w[i] = __float_as_uint(v[i]);
+        else w[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+    }
+    if constexpr (kWords % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < kWords; i += 4) reinterpret_cast<uint4*>(p)[i / 4] = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
+    } else if constexpr (kWords == 2) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+    } else {
+        *reinterpret_cast<uint32_t*>(p) = w[0];
+    }
+}
+template <typename T, int PER, bool HALVES>
+__global__ void __launch_bounds__(256) rope_norm_rows_kernel(const QkvPrep a) {
+    __shared__ float2 turn[16 * PER];      // (cos, sin) of the token's angles
+    __shared__ float red[8], row_inv[2];
+    constexpr int d = 32 * PER;
+    static_assert(kRowBatch == 4, "four sums are reduced together");
+    const long t = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int H = a.Hq, G = a.Gk, qk = H + G, units = qk + a.Gv, u0 = blockIdx.y * a.units_per_cta, u1 = min(units, u0 + a.units_per_cta);
+    const int p = a.pos[t], half = a.rot_dims >> 1;
+    const T* row = (const T*)a.proj + t * a.proj_stride;
+    const long crow = ((long)a.page_table[(long)a.slot[t] * a.max_pages + (p / a.page_size) % a.max_pages] * a.page_size + p % a.page_size) * (long)(G + a.Gv) * d;
+    auto source = [&](int hh) { return row + ((hh < H ? a.q_off : hh < qk ? a.k_off - H * d : a.v_off - qk * d) + hh * d + PER * lane); };
+    float v[kRowBatch][PER];
+#pragma unroll
+    for (int b = 0; b < kRowBatch; b++)
+        if (u0 + warp + nw * b < u1) load_row<T, PER>(source(u0 + warp + nw * b), v[b]);
+    if (u0 < qk) {      // this CTA has query or key heads
+        for (int i = threadIdx.x; i < half; i += blockDim.x) {
+            double sn, cs;
+            sincos((double)p * a.inv_freq[i], &sn, &cs);
+            turn[i] = make_float2((float)cs, (float)sn);
+        }
+        if (a.qk_norm == kQkNormRow) {      // a turn keeps x^2 + y^2 of its pair: the row's mean square is that of the un-turned columns
+            const float sq = block_sum(sum_squares(row + a.q_off, H * d, a.vec_rows), red);
+            const float sk = block_sum(sum_squares(row + a.k_off, G * d, a.vec_rows), red);
+            if (threadIdx.x == 0) {
+                row_inv[0] = 1.0f / sqrtf(sq / (float)(H * d) + a.eps);
+                row_inv[1] = 1.0f / sqrtf(sk / (float)(G * d) + a.eps);
+            }
+        }
+        __syncthreads();
+    }
+    // the lane's turns: of its columns (halves: all of the first or of the second half, since a half is a multiple of PER columns; interleaved: PER / 2 pairs).  A column that
+    // its partner's is taken from has the sine's sign turned; columns that do not turn have cosine 1, sine 0
+    const bool turned = PER * lane < a.rot_dims, second = HALVES && PER * lane >= half;
+    const int partner = HALVES ? (second ? lane - half / PER : lane + half / PER) & 31 : lane;
+    float2 cs[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        cs[i] = turned && u0 < qk ? turn[HALVES ? PER * lane + i - (second ? half : 0) : (PER * lane + i) >> 1] : make_float2(1.f, 0.f);
+        if (!(HALVES ? second : i & 1)) cs[i].y = -cs[i].y;
+    }
+    const bool first_w = a.qk_norm == kQkNormHeadFirst, row_w = a.qk_norm == kQkNormRow, head = a.qk_norm == kQkNormHead || first_w, sums = head || a.v_unit_rms;
+    for (int h0 = u0 + warp; h0 < u1; h0 += nw * kRowBatch) {
+        if (h0 != u0 + warp) {
+#pragma unroll
+            for (int b = 0; b < kRowBatch; b++)
+                if (h0 + nw * b < u1) load_row<T, PER>(source(h0 + nw * b), v[b]);
+        }
+        float s[kRowBatch];
+#pragma unroll
+        for (int b = 0; b < kRowBatch; b++) {
+            const int hh = h0 + nw * b;
+            float (&x)[PER] = v[b];
+            s[b] = 0.f;
+            if (hh < u1) {      // (the same for the warp)
+                if (first_w && hh < qk) {      // (the unit-rms factor is one number per row: it follows the rotation)
+                    float w[PER];
+                    load_row<T, PER>((const T*)(hh < H ? a.q_w : a.k_w) + PER * lane, w);
+#pragma unroll
+                    for (int i = 0; i < PER; i++) { s[b] += x[i] * x[i]; x[i] *= w[i]; }
+                }
+                if (a.rot_dims && hh < qk) {
+                    float o[PER];
+#pragma unroll
+                    for (int i = 0; i < PER; i++) o[i] = HALVES ? __shfl_sync(0xffffffffu, x[i], partner) : x[i ^ 1];
+                    if (turned) {
+#pragma unroll
+                        for (int i = 0; i < PER; i++) x[i] = x[i] * cs[i].x + o[i] * cs[i].y;
+                    }
+                }
+                if (!(first_w && hh < qk)) {
+#pragma unroll
+                    for (int i = 0; i < PER; i++) s[b] += x[i] * x[i];
+                }
+            }
+        }
+        // the four sums at once: eight lanes end with one unit's, and take its root
+        float inv = 1.f;
+        if (sums) {
+            const bool hi = lane & 16, mid = lane & 8;
+            const float a0 = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16), a1 = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
+            float sum = (mid ? a1 : a0) + __shfl_xor_sync(0xffffffffu, mid ? a0 : a1, 8);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            inv = 1.0f / sqrtf(sum / (float)d + a.eps);
+        }
+#pragma unroll
+        for (int b = 0; b < kRowBatch; b++) {
+            const int hh = h0 + nw * b;
+            float (&x)[PER] = v[b];
+            const float mine = __shfl_sync(0xffffffffu, inv, 8 * b);
+            if (hh < u1) {
+                if (hh < qk ? head : a.v_unit_rms) {
+#pragma unroll
+                    for (int i = 0; i < PER; i++) x[i] *= mine;
+                } else if (row_w && hh < qk) {
+                    float w[PER];
+                    load_row<T, PER>((const T*)(hh < H ? a.q_w : a.k_w) + (long)(hh < H ? hh : hh - H) * d + PER * lane, w);
+#pragma unroll
+                    for (int i = 0; i < PER; i++) x[i] = x[i] * row_inv[hh < H ? 0 : 1] * w[i];
+                }
+                T* dst = hh < H ? (T*)a.q_out + (t * H + hh) * d : (T*)a.cache + crow + (long)(hh - H) * d;
+                store_row<T, PER>(dst + PER * lane, x);
+            }
         }
     }
 }
@@ -912,6 +1069,30 @@ extern "C" int ktb200_qkv_prep(const ktb200_qkv_prep_params* c, int n_tokens, in
         });
 #undef PAIR_SIZES
 #undef PAIR_LAUNCH
+        KTB_LAUNCH_CHECK();
+        return KTB200_OK;
+    }
+    // whole rows at once: heads and values of 64, 128 or 256 columns, everything in whole vectors of a lane's columns
+    const int per = c->dim / 32;
+    const size_t lane_bytes = std::min<size_t>(16, per * esz);
+    auto whole = [&](const void* p) { return (reinterpret_cast<uintptr_t>(p) & (lane_bytes - 1)) == 0; };
+    const bool weights = c->qk_norm == kQkNormRow || c->qk_norm == kQkNormHeadFirst;
+    const bool rows = !c->conv_w && !c->v_other && (c->dim == 64 || c->dim == 128 || c->dim == 256) && c->vdim == c->dim && c->rot_dims % (2 * per) == 0 && c->q_off % per == 0 && c->k_off % per == 0 &&
+                      c->v_off % per == 0 && c->proj_stride % per == 0 && whole(c->proj) && whole(c->q_out) && whole(c->cache) && (!weights || (whole(c->q_weight) && whole(c->k_weight)));
+    if (rows) {
+        const dim3 grid(n_tokens, grid_y);
+        const bool halves = c->rot_layout == kRotHalves;
+#define ROWS_LAUNCH(PER)                                                                                                \
+    do {                                                                                                                \
+        if (halves) rope_norm_rows_kernel<T, PER, true><<<grid, 256, 0, (cudaStream_t)stream>>>(a);                     \
+        else rope_norm_rows_kernel<T, PER, false><<<grid, 256, 0, (cudaStream_t)stream>>>(a);                           \
+    } while (0)
+        SEQ_DISPATCH(dtype, {
+            if (per == 2) ROWS_LAUNCH(2);
+            else if (per == 4) ROWS_LAUNCH(4);
+            else ROWS_LAUNCH(8);
+        });
+#undef ROWS_LAUNCH
         KTB_LAUNCH_CHECK();
         return KTB200_OK;
     }

@@ -38,3 +38,30 @@ def test_router_batches(T, E, H, hid, shift):
     assert torch.equal(live[0][:T - 3], got[0][:T - 3]) and (live[0][T - 3:] == -1).all()
     none = call(0, T, torch.zeros(1, dtype=torch.int32, device="cuda"))
     assert (none[0] == -1).all() and torch.equal(call(0, T)[0], got[0])        # (the tickets are back at zero)
+
+
+# heads of 64, 128 and 256 columns in both types and layouts, every norm, part of the columns and none turned, one token and many (blocks of units, and fewer units than
+# a block's warps); the general kernel takes the same rows at an odd offset.  Sums of squares are added in another order: a unit of fp32, which may move a bf16 by one place
+@pytest.mark.parametrize("T,H,G,d,rot,layout,norm,unit_v,dtype", [(1, 64, 8, 128, 64, 1, 1, 0, BF16), (300, 16, 2, 128, 128, 1, 3, 1, BF16), (2100, 4, 4, 64, 32, 0, 1, 0, BF16), (37, 6, 3, 256, 64, 1, 2, 0, BF16),
+                                                                  (5, 40, 8, 128, 0, 0, 1, 1, F32), (65, 8, 2, 64, 64, 0, 3, 0, F32), (700, 3, 1, 256, 256, 1, 0, 0, F32), (16, 8, 8, 128, 32, 0, 2, 1, F32)])
+def test_rotated_rows(T, H, G, d, rot, layout, norm, unit_v, dtype):
+    from ktransformers_b200 import native
+    dt, g, n = TORCH[dtype], torch.Generator(device="cuda").manual_seed(T + H), (H + 2 * G) * d
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    proj, inv_freq = rnd(T, n).to(dt), (10000.0 ** (-torch.arange(max(rot // 2, 1), device="cuda").double() / max(rot // 2, 1)))
+    q_w, k_w = ((rnd(H * d) if norm == 2 else rnd(d)).to(dt), (rnd(G * d) if norm == 2 else rnd(d)).to(dt))
+    page, pages = 64, (T + 63) // 64 + 1
+    pos = torch.arange(T, dtype=torch.int32, device="cuda") + 11
+    slot, table = torch.zeros(T, dtype=torch.int32, device="cuda"), torch.randperm(pages, generator=g, device="cuda").to(torch.int32)
+    lib, out = native.seq_lib(), []
+    for pad in (0, 1):      # a row stride of n + 1 and q one column in: no whole vectors
+        p = torch.zeros((T, n + pad), dtype=dt, device="cuda")
+        p[:, pad:] = proj
+        q, cache = torch.zeros((T, H * d), dtype=dt, device="cuda"), torch.full((pages * page, 2 * G * d), 7.0, dtype=dt, device="cuda")
+        native.check_seq(lib.ktb200_rope_norm_cache_write(p.data_ptr(), n + pad, pad, pad + H * d, pad + (H + G) * d, H, G, d, d, rot, layout, inv_freq.data_ptr(), norm, q_w.data_ptr(), k_w.data_ptr(), unit_v,
+                                                          1e-6, None, 0, None, pos.data_ptr(), slot.data_ptr(), table.data_ptr(), pages, page, cache.data_ptr(), q.data_ptr(), T, dtype, _stream()))
+        out.append((q, cache))
+    for a, b in zip(*out):
+        assert torch.isfinite(a.float()).all() and ((a.double() - b.double()).abs() <= (2.0 ** -7 if dtype == BF16 else 2.0 ** -20) * b.double().abs() + 1e-6).all()
+        assert (a != b).double().mean() < (0.01 if dtype == BF16 else 1.0)
+    assert (out[0][1] == 7.0).all(1).sum() == pages * page - T        # (only the tokens' rows were written)
