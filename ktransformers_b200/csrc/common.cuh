@@ -165,6 +165,21 @@ __device__ __forceinline__ uint16_t f32_to_bf16_ggml(float f) {
     if (!(i & 0x7f800000u)) return (uint16_t)((i & 0x80000000u) >> 16);
     return (uint16_t)((i + (0x7fffu + ((i >> 16) & 1))) >> 16);
 }
+// two values in a 16-bit type; bf16 as ggml rounds it (subnormals to zero; NaN keeps its upper bits), without branches where there is no NaN or infinity
+__device__ __forceinline__ uint32_t pack16(float a, float b, bool bf16) {
+    if (!bf16) {
+        const __half2 h = __floats2half2_rn(a, b);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+    float z, fa, fb;
+    asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(fa) : "f"(a));
+    asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(fb) : "f"(b));
+    z = fmaf(a, 0.f, b * 0.f);
+    if (z != z) return (uint32_t)f32_to_bf16_ggml(a) | (uint32_t)f32_to_bf16_ggml(b) << 16;
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(fb), "f"(fa));
+    return d;
+}
 
 __device__ __forceinline__ float load_hidden(const void* base, long idx, int hidden_type) {
     if (hidden_type == KTB200_TYPE_BF16) {

@@ -240,17 +240,17 @@ __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constan
 
 // Prompt portions (more than kFT tokens): y = xq . W^T as a persistent GEMM.  The pass kernel above streams all of W again for every 16
 // tokens (2000 tokens, 7168 -> 18432: 125 passes, 7.9 ms); here a tile is 128 tokens x BN weight rows, both operands come by TMA in the
-// 128-byte-swizzle layout, and what bounds it is the tensor pipe (K = 128 of a 128 x 256 tile: 512 cycles of MMA) beside the promotion of
-// the partial dot to fp32 after every 128 of K that the two block scales ask for (128 fused multiply-adds per thread and 128 of K).
-//     warp 0 TMA ring (4 to 8 stages, 192 KB), warp 1 issuer, warps 2-9 epilogue: a thread owns one token and half of the tile's columns;
+// 128-byte-swizzle layout.  What bounds it is the shared memory's port: a K block of a 128 x 256 tile brings 48 KB in and the four products read 48 KB, 768 cycles at 128 B
+// a cycle (the products alone: 524; measured 735 a block at the 1.53 GHz that such a load leaves).  A pair of CTAs on one tile would halve the reading of W.
+//     warp 0 TMA ring (4 to 8 stages, 192 KB), warp 1 issuer, warps 4-19 epilogue: a thread owns one token and a quarter of the tile's columns;
 //     lanes are tokens, so the token scale is a register and acc += dot * (a_s * b_s) is ONE fma per value and 128 of K.
 //     Two TMEM buffers of BN columns: the MMAs of one K block run while the block before it is promoted.
-// BN: 256 leaves the tensor pipe shared-memory headroom (96 of 128 B per cycle); 128 and 64 keep the chip full when there are few tiles.
-// The roles are known to be uniform (umma.cuh): 351 -> 333 us for 2000 tokens, 7168 -> 18432 (the kernel above, one token 16384 -> 7168: 34.1 -> 32.7); a wave brings
-// 48 KB per 128 x 256 x 128 products through L2, 11 TB/s in all, which is near what L2 gives.  Longer loads from tensor memory with double buffers, two
-// products per instruction and more registers for them made it 340-460 us.
+// BN: 256 where that gives every SM a tile; 128 and 64 keep the chip full when there are few tiles.
+// 2000 tokens, 7168 -> 18432: 338 -> 317 us by scales that are fetched four blocks ahead (a load takes about 1,000 cycles beside the copies; one block ahead each block waited 400 of
+// them), four epilogue warps a scheduler instead of two (a drain's chain of loads and sums: 720 cycles a block), a tile's output without branches in whole sectors (12,800 -> 4,000
+// cycles) and one election for a block's products and barriers.  The roles are known to be uniform (umma.cuh): 351 -> 333 us (the kernel above, one token 16384 -> 7168: 34.1 -> 32.7).
 // Tiles run token tile fastest inside groups of kFGroupM, so that the CTAs of a wave share the weight rows and the tokens through L2.
-constexpr int kFGemmThreads = 320, kFGroupM = 16, kFGemmRing = 192 * 1024, kFGemmTokens = 4096;
+constexpr int kFGemmThreads = 640, kFGroupM = 16, kFGemmRing = 192 * 1024, kFGemmTokens = 4096;
 struct Fp8GemmMisc {
     unsigned long long full[8], free[8], d_full[2], d_free[2];
     uint32_t tmem_base;
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
     const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);
     if (tid == 0) {
         for (int s = 0; s < kStages; s++) { bar_init(smem_u32(&misc.full[s]), 1); bar_init(smem_u32(&misc.free[s]), 1); }
-        for (int b = 0; b < 2; b++) { bar_init(smem_u32(&misc.d_full[b]), 1); bar_init(smem_u32(&misc.d_free[b]), 8); }
+        for (int b = 0; b < 2; b++) { bar_init(smem_u32(&misc.d_full[b]), 1); bar_init(smem_u32(&misc.d_free[b]), 16); }
         bar_fence_init();
         tma_prefetch_desc(&xmap);
         tma_prefetch_desc(&wmap);
@@ -296,6 +296,11 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
     };
     griddep_wait();      // the quantised tokens and their scales come from the kernel before this one
 
+    // registers: 96 a thread at launch, of which the copies and the issuer need a third (32 + 4 x 112 = 5 x 96)
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        __syncwarp();
+    }
     if (warp == 0) {
         if (lane == 0) {
             int s = 0, ph = 1;
@@ -324,80 +329,98 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
                 bar_wait(smem_u32(&misc.d_free[buf]), ((it >> 1) & 1) ^ 1);
                 tc_fence_after();
                 const uint32_t a = base + s * kStageB, b = a + 128 * 128;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    mma_f8(tmem + buf * BN, smem_desc(a + j * 32, 16, 1024, kLayoutSw128), smem_desc(b + j * 32, 16, 1024, kLayoutSw128), idesc, j != 0);
-                mma_commit(smem_u32(&misc.free[s]));
-                mma_commit(smem_u32(&misc.d_full[buf]));
+                mma_f8_x4(tmem + buf * BN, smem_desc(a, 16, 1024, kLayoutSw128), smem_desc(b, 16, 1024, kLayoutSw128), idesc, 0, smem_u32(&misc.free[s]), smem_u32(&misc.d_full[buf]));
                 if (++s == kStages) { s = 0; ph ^= 1; }
             }
-    } else {
-        constexpr int kHalf = BN / 2;
-        const int sp = warp & 3, ch = (warp - 2) >> 2;
-        const uint32_t tcol = tmem + ((uint32_t)(32 * sp) << 16) + ch * kHalf;
+    } else if (warp >= 4) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        constexpr int kPart = BN / 4, kAhead = 4, kLoad = kPart < 32 ? kPart : 32;
+        const int sp = warp & 3, ch = (warp - 4) >> 2;
+        const uint32_t tcol = tmem + ((uint32_t)(32 * sp) << 16) + ch * kPart;
         const int live = p.bsz ? max(0, min(p.T, *p.bsz - p.t0)) : p.T;
         unsigned it = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             int m0, n0;
             place(tile, m0, n0);
-            const int t = m0 + 32 * sp + lane, nb = n0 + ch * kHalf;
+            const int t = m0 + 32 * sp + lane, nb = n0 + ch * kPart;
             const float* xs = p.xs + t;                                                     // t < tpad
             const float* sinv = p.scale_inv + (long)min(nb / 128, (p.N - 1) / 128) * p.nkb;
-            float acc[kHalf], sum[TWO ? kHalf : 1];
+            float acc[kPart], sum[TWO ? kPart : 1];
 #pragma unroll
-            for (int i = 0; i < kHalf; i++) {
+            for (int i = 0; i < kPart; i++) {
                 acc[i] = 0.f;
                 if (TWO) sum[i] = 0.f;
             }
-            float a_s = __ldg(xs), b_s = __ldg(sinv);
-            for (int kb = 0; kb < p.nkb; kb++, it++) {
-                const int buf = it & 1;
-                const float f = a_s * b_s;
-                if (kb + 1 < p.nkb) { a_s = __ldg(xs + (long)(kb + 1) * p.tpad); b_s = __ldg(sinv + kb + 1); }
-                bar_wait(smem_u32(&misc.d_full[buf]), (it >> 1) & 1);
-                tc_fence_after();
+            // The scales of kAhead blocks are under way: a load takes about 1,000 cycles beside the tiles' copies, and one block ahead each block waited 400 of them
+            float a_s[kAhead], b_s[kAhead];
+            auto scales = [&](int i, int kb) {
+                const int k = min(kb, p.nkb - 1);
+                a_s[i] = __ldg(xs + (long)k * p.tpad);
+                b_s[i] = __ldg(sinv + k);
+            };
 #pragma unroll
-                for (int c = 0; c < kHalf; c += 16) {
-                    uint32_t d[16];
-                    tmem_ld16(tcol + buf * BN + c, d);
-                    tmem_wait_ld();
+            for (int i = 0; i < kAhead; i++) scales(i, i);
+            for (int kb0 = 0; kb0 < p.nkb; kb0 += kAhead)
 #pragma unroll
-                    for (int i = 0; i < 16; i++) acc[c + i] = __fmaf_rn(__uint_as_float(d[i]), f, acc[c + i]);
+                for (int i = 0; i < kAhead; i++) {
+                    const int kb = kb0 + i, buf = it & 1;
+                    if (kb >= p.nkb) break;
+                    const float f = a_s[i] * b_s[i];
+                    scales(i, kb + kAhead);
+                    bar_wait(smem_u32(&misc.d_full[buf]), (it >> 1) & 1);
+                    tc_fence_after();
+#pragma unroll
+                    for (int c = 0; c < kPart; c += kLoad) {
+                        uint32_t d[kLoad];
+                        if constexpr (kLoad == 32) tmem_ld32(tcol + buf * BN + c, d); else tmem_ld16(tcol + buf * BN + c, d);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int u = 0; u < kLoad; u++) acc[c + u] = __fmaf_rn(__uint_as_float(d[u]), f, acc[c + u]);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(smem_u32(&misc.d_free[buf]));
+                    if (TWO && ((kb & 7) == 7 || kb + 1 == p.nkb)) {
+#pragma unroll
+                        for (int u = 0; u < kPart; u++) { sum[u] += acc[u]; acc[u] = 0.f; }
+                    }
+                    it++;
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) bar_arrive(smem_u32(&misc.d_free[buf]));
-                if (TWO && ((kb & 7) == 7 || kb + 1 == p.nkb)) {
-#pragma unroll
-                    for (int i = 0; i < kHalf; i++) { sum[i] += acc[i]; acc[i] = 0.f; }
-                }
-            }
             if (TWO) {
 #pragma unroll
-                for (int i = 0; i < kHalf; i++) acc[i] = sum[i];
+                for (int i = 0; i < kPart; i++) acc[i] = sum[i];
             }
             if (t < live) {
                 const long o = (long)t * p.N + nb;
 #pragma unroll
-                for (int c = 0; c < kHalf; c += 8) {
-                    if (p.vec && nb + c + 8 <= p.N) {
-                        if (p.hidden_type == KTB200_TYPE_F32) {
-                            float4* y = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.y) + o + c);
-                            y[0] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
-                            y[1] = make_float4(acc[c + 4], acc[c + 5], acc[c + 6], acc[c + 7]);
-                        } else {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                const float lo = acc[c + 2 * i], hi = acc[c + 2 * i + 1];
-                                w[i] = p.hidden_type == KTB200_TYPE_BF16 ? (uint32_t)f32_to_bf16_ggml(lo) | ((uint32_t)f32_to_bf16_ggml(hi) << 16)
-                                                                         : (uint32_t)__half_as_ushort(__float2half_rn(lo)) | ((uint32_t)__half_as_ushort(__float2half_rn(hi)) << 16);
+                for (int c = 0; c < kPart; c += 16) {
+                    if (p.vec && nb + c + 16 <= p.N) {
+                        // (a thread's row is its own: whole sectors where the rows allow them)
+                        auto sector = [&](uint8_t* y, const uint32_t (&w)[8]) {
+                            if (p.vec == 2) {
+                                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(y), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+                            } else {
+                                reinterpret_cast<uint4*>(y)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                                reinterpret_cast<uint4*>(y)[1] = make_uint4(w[4], w[5], w[6], w[7]);
                             }
-                            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.y) + o + c) = make_uint4(w[0], w[1], w[2], w[3]);
+                        };
+                        uint32_t w[8];
+                        if (p.hidden_type == KTB200_TYPE_F32) {
+                            uint8_t* y = reinterpret_cast<uint8_t*>(reinterpret_cast<float*>(p.y) + o + c);
+#pragma unroll
+                            for (int q = 0; q < 2; q++) {
+#pragma unroll
+                                for (int i = 0; i < 8; i++) w[i] = __float_as_uint(acc[c + 8 * q + i]);
+                                sector(y + 32 * q, w);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) w[i] = pack16(acc[c + 2 * i], acc[c + 2 * i + 1], p.hidden_type == KTB200_TYPE_BF16);
+                            sector(reinterpret_cast<uint8_t*>(reinterpret_cast<uint16_t*>(p.y) + o + c), w);
                         }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 8; i++)
+                        for (int i = 0; i < 16; i++)
                             if (nb + c + i < p.N) store_hidden(p.y, o + c + i, p.hidden_type, acc[c + i]);
                     }
                 }
@@ -458,7 +481,7 @@ static int fp8_forward_gemm(ktb200_fp8_linear* l, int qlen, const void* x, void*
         p.N = l->N; p.nkb = l->nkb; p.t0 = t0; p.bsz = bsz; p.hidden_type = l->hidden_type; p.scale_inv = l->scale_inv;
         p.mt = (p.T + 127) / 128; p.tpad = p.mt * 128;
         p.y = reinterpret_cast<uint8_t*>(y) + (size_t)t0 * l->N * hb;
-        p.vec = (size_t)l->N * hb % 16 == 0 && (uintptr_t)y % 16 == 0;
+        p.vec = (size_t)l->N * hb % 16 || (uintptr_t)y % 16 ? 0 : (size_t)l->N * hb % 32 || (uintptr_t)y % 32 ? 1 : 2;
         ScratchBlock mem(s);
         const size_t xs_bytes = (size_t)l->nkb * p.tpad * sizeof(float);
         KTB_CUDA_CHECK(mem.take(l->device, (size_t)p.T * l->K + xs_bytes));

@@ -192,19 +192,6 @@ __device__ __forceinline__ uint32_t kq_six(uint32_t w, uint32_t top) {
 }
 __device__ __forceinline__ int byte_of(uint32_t w, int i) { return (int)((w >> (8 * i)) & 0xffu); }
 
-// two values in a 16-bit type; bf16 as ggml rounds it (subnormals to zero; NaN keeps its upper bits), without branches where there is no NaN or infinity
-__device__ __forceinline__ uint32_t kq_pack16(float a, float b, bool bf16) {
-    if (!bf16) return as_u32(__floats2half2_rn(a, b));
-    float z, fa, fb;
-    asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(fa) : "f"(a));
-    asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(fb) : "f"(b));
-    z = fmaf(a, 0.f, b * 0.f);
-    if (z != z) return (uint32_t)f32_to_bf16_ggml(a) | (uint32_t)f32_to_bf16_ggml(b) << 16;
-    uint32_t d;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(fb), "f"(fa));
-    return d;
-}
-
 struct KqTile { int e, row0, p0, n, sb0, nsb, split; };
 __device__ __forceinline__ KqTile kq_tile(const KqParams& p, int tile) {
     KqTile t;
@@ -640,7 +627,7 @@ __device__ __forceinline__ void kq_roles(const KqMaps& maps, const KqParams& p, 
                 } else {
 #pragma unroll
                     for (int i = 0; i < 8; i += 2) {
-                        const uint32_t v = kq_pack16(half_of(acc[i >> 1], 0) + bias, half_of(acc[i >> 1], 1) + bias, type == KTB200_TYPE_BF16);
+                        const uint32_t v = pack16(half_of(acc[i >> 1], 0) + bias, half_of(acc[i >> 1], 1) + bias, type == KTB200_TYPE_BF16);
                         if (i < left) reinterpret_cast<uint16_t*>(out)[at + (uint32_t)(i * p.R)] = (uint16_t)v;
                         if (i + 1 < left) reinterpret_cast<uint16_t*>(out)[at + (uint32_t)((i + 1) * p.R)] = (uint16_t)(v >> 16);
                     }

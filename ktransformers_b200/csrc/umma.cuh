@@ -237,5 +237,39 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
         : "memory");
 }
 
+// Four products on consecutive K-steps, whose operands lie DA and DB units of 16 bytes apart (2: a 128-byte swizzled row's steps of 32 bytes), and the barriers that complete when
+// all products so far have (0: not asked for), in one election
+#define KTB_MMA_SS4(KIND)                                                                             \
+    asm volatile(                                                                                     \
+        "{\n"                                                                                        \
+        ".reg .pred p, q, t, c, e;\n"                                                                \
+        ".reg .b32 r;\n"                                                                             \
+        ".reg .b64 a, b;\n"                                                                          \
+        "elect.sync r|q, 0xffffffff;\n"                                                              \
+        "setp.ne.b32 p, %4, 0;\n"                                                                    \
+        "setp.eq.b32 t, 0, 0;\n"                                                                     \
+        "setp.ne.and.b32 c, %5, 0, q;\n"                                                             \
+        "setp.ne.and.b32 e, %6, 0, q;\n"                                                             \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, p;\n"                          \
+        "add.u64 a, %1, %7;\n"                                                                       \
+        "add.u64 b, %2, %8;\n"                                                                       \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], a, b, %3, t;\n"                            \
+        "add.u64 a, a, %7;\n"                                                                        \
+        "add.u64 b, b, %8;\n"                                                                        \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], a, b, %3, t;\n"                            \
+        "add.u64 a, a, %7;\n"                                                                        \
+        "add.u64 b, b, %8;\n"                                                                        \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], a, b, %3, t;\n"                            \
+        "@c tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n"           \
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n"           \
+        "}\n" ::"r"(tmem_d),                                                                         \
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1), "n"(DA), "n"(DB) \
+        : "memory")
+template <int DA = 2, int DB = 2>
+__device__ __forceinline__ void mma_f8_x4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t bar0 = 0, uint32_t bar1 = 0) { KTB_MMA_SS4("f8f6f4"); }
+template <int DA = 2, int DB = 2>
+__device__ __forceinline__ void mma_f16_x4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t bar0 = 0, uint32_t bar1 = 0) { KTB_MMA_SS4("f16"); }
+#undef KTB_MMA_SS4
+
 }  // namespace umma
 }  // namespace ktb

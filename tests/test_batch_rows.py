@@ -65,3 +65,29 @@ def test_rotated_rows(T, H, G, d, rot, layout, norm, unit_v, dtype):
         assert torch.isfinite(a.float()).all() and ((a.double() - b.double()).abs() <= (2.0 ** -7 if dtype == BF16 else 2.0 ** -20) * b.double().abs() + 1e-6).all()
         assert (a != b).double().mean() < (0.01 if dtype == BF16 else 1.0)
     assert (out[0][1] == 7.0).all(1).sum() == pages * page - T        # (only the tokens' rows were written)
+
+
+# results in whole sectors (rows and address multiples of 32 bytes), in vectors of 16 and value by value: the same values wherever they go; blocks of K that are no multiple of the
+# four whose scales are under way; tiles of 256, 128 and 64 columns, the last one ragged
+@pytest.mark.parametrize("T,K,N,hid", [(130, 128, 4096, BF16), (300, 640, 19000, F16), (257, 1152, 19208, BF16), (129, 384, 2064, F32), (1030, 896, 515, BF16), (64, 2048, 1032, F16)])
+def test_fp8_batches_wherever_results_go(T, K, N, hid):
+    from ktransformers_b200 import native
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w, ws = (torch.randn((N, K), generator=g, device="cuda") * 50).to(torch.float8_e4m3fn), torch.rand(((N + 127) // 128, K // 128), generator=g, device="cuda") / K
+    x, dt = torch.randn((T, K), generator=g, device="cuda").to(TORCH[hid]), TORCH[hid]
+    lib, h = native.lib(), C.c_void_p()
+    native.check(lib.ktb200_fp8_linear_create(K, N, w.data_ptr(), ws.data_ptr(), hid, 0, C.byref(h)))
+    out = []
+    for shift in (0, 16 // x.element_size(), 1):
+        room = torch.full((T * N + 32,), 7.0, dtype=dt, device="cuda")
+        native.check(lib.ktb200_fp8_linear_forward(h, T, x.data_ptr(), room[shift:].data_ptr(), None, _stream()))
+        assert (room[:shift] == 7.0).all() and (room[shift + T * N:] == 7.0).all()
+        out.append(room[shift:shift + T * N].clone())
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+    f = x.float().view(T, -1, 128)
+    s = f.abs().amax(-1, keepdim=True) / 448.0
+    x8 = ((f / s).to(torch.float8_e4m3fn).double() * s.double()).view(T, K)
+    want = x8 @ (w.double() * ws.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)).T
+    off = (out[0].view(T, N).double() - want).norm() / want.norm()
+    assert off < {F32: 1e-5, F16: 1e-3, BF16: 4e-3}[hid], off.item()
+    lib.ktb200_fp8_linear_destroy(h)
