@@ -16,15 +16,18 @@
 // 512 columns are the MN-major A operand [latent x tokens] (the swizzle is a function of the shared-memory address only).
 // The output is accumulated TRANSPOSED — O^T[latent 512][head 64] = 4 blocks of 128 TMEM lanes x 64 columns — because a
 // [head][latent] accumulator for 64 heads would need 512 columns in the M=64 tcgen05 layout (half the lanes idle): the
-// whole tensor memory.  TMEM map (512 columns allocated): [0,256) O^T, [256,384) / [384,512) the two S buffers, each FOUR
-// partial accumulators of 32 columns: a 64 x 32 x 16 MMA is 16 cycles of work behind a pipeline several times as deep, so
-// 36 of them chained through ONE accumulator run at the latency, not the throughput (measured: ~75 cycles each); the 36
-// k-steps are dealt round-robin to four independent accumulators and the softmax warps add the four partial scores.
+// whole tensor memory.  TMEM map (512 columns allocated): [0,256) O^T, [256,288) / [288,320) the two S buffers.  A 64 x N x 16 product takes 34 cycles for every N up to 64, in one
+// accumulator as in four.
+// What bounds it: 36 + 8 products a tile of 32 tokens, 1,620 of the 1,900 cycles that a tile takes.  B = 1, 128 heads, 131,072 keys: 91 -> 75 us by queries that come by TMA while the first
+// tiles do (setup 6.6 -> 2.3 us), scores in one accumulator, one election for four products, and a merge in four parts.  Tiles of 64 tokens (half the cycles for scores) took 79-118 us: two
+// stages of them fill the shared memory, a stage comes back only behind the tile's values, and copies and products then share the shared memory's port (120 of 128 B a cycle).
 //
 // Online softmax with a LAZY reference maximum: p = 2^(x - m_ref), m_ref is only raised (and O^T rescaled in TMEM, all
 // four warps) when some head's running maximum exceeds it by more than 8 — p stays <= 256, exact in bf16/fp32 terms —
 // so the steady-state tile costs no TMEM round trip of the accumulator.  Split-KV partials (fp32 O, base-2 LSE) are
 // merged by mla_merge_kernel.
+#include <algorithm>
+
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -49,11 +52,10 @@ constexpr int kPBytes = kHG * kLT * 2;             // 4,096: [8 head groups][4 t
 constexpr int kOffMiscMax = kMaxStages * kStageBytes + kQBytes + 2 * kPBytes;   // 229,376 (P is double-buffered)
 constexpr int kTmemCols = 512;
 constexpr int kColO = 0, kColS = 256;
-constexpr int kSChains = 4;          // independent partial-score accumulators per S buffer
 constexpr float kRescaleThreshold = 8.f;
 
 struct MlaMisc {
-    unsigned long long k_full[kMaxStages], k_empty[kMaxStages], s_full[2], s_empty[2], p_full, p_free[2];
+    unsigned long long q_full, k_full[kMaxStages], k_empty[kMaxStages], s_full[2], s_empty[2], p_full, p_free[2];
     uint32_t tmem_base;
     int need[2][4];
     float alpha[kHG];     // per head: 2^(m_ref_old - m_ref_new) of the current rescale
@@ -99,7 +101,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // ~16 mantissa bits of p instead of 8 (designs that keep attention weights in 32-bit); the second P buffer pair is paid
 // for with one stage of the KV ring.
 template <bool SPLITP>
-__global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const MlaKParams p) {
+__global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap pe_map, const MlaKParams p) {
     constexpr int kStages = SPLITP ? 3 : 4;
     constexpr int kOffQ = kStages * kStageBytes;
     constexpr int kPStride = SPLITP ? 2 * kPBytes : kPBytes;      // hi | lo
@@ -142,6 +144,8 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
     // ---- one-time setup -----------------------------------------------------------------------------------------
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&kv_map);
+        tma_prefetch_desc(&q_map);
+        bar_init(smem_u32(&misc.q_full), 1);
         for (int s = 0; s < kStages; s++) { bar_init(smem_u32(&misc.k_full[s]), 1); bar_init(smem_u32(&misc.k_empty[s]), 1); }
         for (int s = 0; s < 2; s++) { bar_init(smem_u32(&misc.s_full[s]), 1); bar_init(smem_u32(&misc.s_empty[s]), 4); }
         bar_init(smem_u32(&misc.p_full), 4);
@@ -149,6 +153,11 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         bar_init(smem_u32(&misc.p_free[1]), 1);
         bar_fence_init();
         // the first tiles do not depend on anything set up below: request them now
+        // (Q, 64 heads x 576, into the K-major 128-byte-swizzle layout: a region of 64 rows of 128 B per 64 columns.  Rows beyond the last head are other sequences' or zeros, and
+        // their scores go nowhere)
+        const uint32_t qbar = smem_u32(&misc.q_full);
+        bar_expect_tx(qbar, kQBytes);
+        for (int c = 0; c < kChunks; c++) tma_load_2d(base + kOffQ + c * kQRegion, c < 8 ? &q_map : &pe_map, qbar, c < 8 ? c * 64 : 0, b * p.num_heads + h0);
         for (int j = 0; j < n && j < kStages; j++) {
             const int t_base = (tile0 + j) * kLT;
             const int page = p.page_table[prow + (t_base / p.page_size) % p.max_pages];
@@ -161,34 +170,6 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         }
     }
     if (warp == 1) tmem_alloc(smem_u32(&misc.tmem_base), kTmemCols);
-    // Q (64 heads x 576) -> shared memory in the K-major 128-byte-swizzle layout: chunk region c (64 columns) holds 64
-    // rows of 128 B; the 16-byte piece j of row r sits at piece (j ^ (r & 7)).  Rows beyond num_heads are zero.
-    {
-        constexpr int kPieces = kHG * (kDK / 8), kIter = kPieces / kMlaThreads;   // 4608 = 24 x 192
-        static_assert(kPieces % kMlaThreads == 0, "Q pieces");
-        constexpr int kB = 12;
-        static_assert(kIter % kB == 0, "Q batches");
-#pragma unroll
-        for (int i0 = 0; i0 < kIter; i0 += kB) {
-            uint4 v[kB];
-#pragma unroll
-            for (int u = 0; u < kB; u++) {   // 12 independent 16-byte loads in flight per thread
-                const int i = tid + (i0 + u) * kMlaThreads, r = i / (kDK / 8), j = i - r * (kDK / 8);
-                v[u] = make_uint4(0, 0, 0, 0);
-                if (h0 + r < p.num_heads) {
-                    const long hrow = (long)b * p.num_heads + h0 + r;
-                    v[u] = j < 64 ? __ldg(reinterpret_cast<const uint4*>(p.q_nope + hrow * kDV) + j) : __ldg(reinterpret_cast<const uint4*>(p.q_pe + hrow * 64) + (j - 64));
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kB; u++) {
-                const int i = tid + (i0 + u) * kMlaThreads, r = i / (kDK / 8), j = i - r * (kDK / 8);
-                const int c = j >> 3, jj = j & 7;
-                *reinterpret_cast<uint4*>(smem + kOffQ + c * kQRegion + r * 128 + ((jj ^ (r & 7)) << 4)) = v[u];
-            }
-        }
-    }
-    fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -229,12 +210,10 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
                 const uint32_t kb = base + s * kStageBytes, qb = base + kOffQ;
 #pragma unroll
                 for (int c = 0; c < kChunks; c++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        mma_f16(tmem + kColS + (buf * kSChains + (k & (kSChains - 1))) * kLT, smem_desc(qb + c * kQRegion + k * 32, 16, 1024, kLayoutSw128),
-                                smem_desc(kb + c * kKRegion + k * 32, 16, 1024, kLayoutSw128), idesc_qk, c != 0);
-                mma_commit(smem_u32(&misc.s_full[buf]));
+                    mma_f16_x4(tmem + kColS + buf * kLT, smem_desc(qb + c * kQRegion, 16, 1024, kLayoutSw128), smem_desc(kb + c * kKRegion, 16, 1024, kLayoutSw128), idesc_qk, c != 0,
+                               c == kChunks - 1 ? smem_u32(&misc.s_full[buf]) : 0);
             };
+            bar_wait(smem_u32(&misc.q_full), 0);
             issue_qk(0);
             for (int j = 0; j < n; j++) {
                 if (j + 1 < n) issue_qk(j + 1);
@@ -274,20 +253,8 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             tc_fence_after();
             if (p.debug && st == 0 && split == 0 && hg == 0 && b == 0 && j < 60) reinterpret_cast<unsigned long long*>(p.debug + 2048)[64 + j] = gtime();
             uint32_t sv[32];
-            {   // S = sum of the four partial accumulators
-                uint32_t t1[32], t2[32];
-                const uint32_t sa = tmem + lane_base + kColS + buf * kSChains * kLT;
-                tmem_ld32(sa, sv);
-                tmem_ld32(sa + kLT, t1);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 32; i++) sv[i] = __float_as_uint(__uint_as_float(sv[i]) + __uint_as_float(t1[i]));
-                tmem_ld32(sa + 2 * kLT, t1);
-                tmem_ld32(sa + 3 * kLT, t2);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 32; i++) sv[i] = __float_as_uint(__uint_as_float(sv[i]) + (__uint_as_float(t1[i]) + __uint_as_float(t2[i])));
-            }
+            tmem_ld32(tmem + lane_base + kColS + buf * kLT, sv);
+            tmem_wait_ld();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) bar_arrive(smem_u32(&misc.s_empty[buf]));
@@ -423,26 +390,37 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
 
 // out[b][h][:] = sum_s w_s * o_part[b][s][h][:],  w_s = 2^(lse_s - max) / sum ; lse (natural log) optional
 // sink (optional, [num_heads], natural-log units): one more term exp(sink_h) in the denominator that carries no value
-__global__ void __launch_bounds__(128) mla_merge_kernel(const float* o_part, const float* lse_part, int num_splits, int num_heads,
-                                                        __nv_bfloat16* out, float* lse_out, const float* sink) {
+// A CTA per head and sequence, a thread per four columns and part of the splits (128 threads each, kMergeLoads splits a part and round): bound by rounds of loads, 10 of 8 for 74 splits
+// in one part, two of 10 in four parts.
+constexpr int kMergeLoads = 10, kMergeParts = 4;
+__global__ void __launch_bounds__(128 * kMergeParts) mla_merge_kernel(const float* o_part, const float* lse_part, int num_splits, int num_heads,
+                                                                      __nv_bfloat16* out, float* lse_out, const float* sink) {
     __shared__ float ws[128];
     __shared__ float red[8];
+    __shared__ float4 sums[kMergeParts - 1][128];
     griddep_launch_dependents();
     griddep_wait();
     const int bh = blockIdx.x, b = bh / num_heads, h = bh % num_heads;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x & 127, part = threadIdx.x >> 7, parts = blockDim.x >> 7, lane = tid & 31, warp = tid >> 5;
+    const int c = tid * 4, per = (num_splits + parts - 1) / parts, s0 = part * per, s1 = min(num_splits, s0 + per);
+    const float* src = o_part + ((long)b * num_splits * num_heads + h) * kDV + c;
+    const long sstride = (long)num_heads * kDV;
+    float4 v[kMergeLoads];      // (the first round is under way while the weights are made)
+#pragma unroll
+    for (int u = 0; u < kMergeLoads; u++)
+        if (s0 + u < s1) v[u] = __ldcs(reinterpret_cast<const float4*>(src + (s0 + u) * sstride));
     const float my = tid < num_splits ? lse_part[((long)b * num_splits + tid) * num_heads + h] : -INFINITY;   // num_splits <= 128
     float mx = my;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) red[warp] = mx;
+    if (part == 0 && lane == 0) red[warp] = mx;
     __syncthreads();
     mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
     const float snk = sink ? sink[h] * 1.4426950408889634f : -INFINITY;
     mx = fmaxf(mx, snk);
-    const int c = tid * 4;
     __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(out + ((long)b * num_heads + h) * kDV + c);
     if (mx == -INFINITY) {   // kv_len == 0 (e.g. a padded CUDA-graph batch slot): zeros, lse = -inf
+        if (part) return;
         o2[0] = __floats2bfloat162_rn(0.f, 0.f);
         o2[1] = __floats2bfloat162_rn(0.f, 0.f);
         if (lse_out && tid == 0) lse_out[(long)b * num_heads + h] = -INFINITY;
@@ -450,26 +428,34 @@ __global__ void __launch_bounds__(128) mla_merge_kernel(const float* o_part, con
     }
     const float e = tid < num_splits ? exp2f(my - mx) : 0.f;
     float den = warp_sum(e);
-    if (lane == 0) red[4 + warp] = den;
+    if (part == 0 && lane == 0) red[4 + warp] = den;
     __syncthreads();
     den = (red[4] + red[5]) + (red[6] + red[7]);
     if (sink) den += exp2f(snk - mx);
-    ws[tid] = e / den;
+    if (part == 0) ws[tid] = e / den;
     __syncthreads();
     float4 acc = make_float4(0, 0, 0, 0);
-    const float* src = o_part + ((long)b * num_splits * num_heads + h) * kDV + c;
-    const long sstride = (long)num_heads * kDV;
-    for (int s0 = 0; s0 < num_splits; s0 += 8) {
-        float4 v[8];
+    for (int s = s0; s < s1; s += kMergeLoads) {
+        if (s != s0) {
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (s0 + u < num_splits) v[u] = __ldcs(reinterpret_cast<const float4*>(src + (s0 + u) * sstride));
+            for (int u = 0; u < kMergeLoads; u++)
+                if (s + u < s1) v[u] = __ldcs(reinterpret_cast<const float4*>(src + (s + u) * sstride));
+        }
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (s0 + u < num_splits) {
-                const float w = ws[s0 + u];
+        for (int u = 0; u < kMergeLoads; u++)
+            if (s + u < s1) {
+                const float w = ws[s + u];
                 acc.x += w * v[u].x; acc.y += w * v[u].y; acc.z += w * v[u].z; acc.w += w * v[u].w;
             }
+    }
+    if (parts > 1) {
+        if (part) sums[part - 1][tid] = acc;
+        __syncthreads();
+        if (part) return;
+        for (int q = 0; q + 1 < parts; q++) {
+            const float4 x = sums[q][tid];
+            acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+        }
     }
     o2[0] = __floats2bfloat162_rn(acc.x, acc.y);
     o2[1] = __floats2bfloat162_rn(acc.z, acc.w);
@@ -533,6 +519,16 @@ static int mla_launch(const ktb::MlaKParams& in, const void* kv_cache, long kv_c
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) { set_error("mla_decode: cuTensorMapEncodeTiled failed (%d)", (int)cr); return KTB200_ECUDA; }
 
+    // the queries as [sequence and head][columns], boxes of 64 heads x 64 columns
+    CUtensorMap q_map, pe_map;
+    auto q_tensor = [&](CUtensorMap* m, const void* ptr, int width) {
+        const cuuint64_t dim[2] = {(cuuint64_t)width, (cuuint64_t)batch * in.num_heads}, stride[1] = {(cuuint64_t)width * 2};
+        const cuuint32_t qbox[2] = {64, (cuuint32_t)kHG};
+        return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dim, stride, qbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    const CUresult qr = q_tensor(&q_map, in.q_nope, kDV), pr = qr == CUDA_SUCCESS ? q_tensor(&pe_map, in.q_pe, 64) : qr;
+    if (pr != CUDA_SUCCESS) { set_error("mla_decode: cuTensorMapEncodeTiled failed for the queries (%d)", (int)pr); return KTB200_ECUDA; }
     MlaKParams p = in;
     p.num_splits = splits;
     p.o_part = (float*)workspace;
@@ -545,10 +541,10 @@ static int mla_launch(const ktb::MlaKParams& in, const void* kv_cache, long kv_c
         attr_set[dev & 63] = true;
     }
     const int head_groups = (p.num_heads + kHG - 1) / kHG;
-    if (split_p) KTB_CUDA_CHECK(launch_pdl(mla_decode_tc_kernel<true>, dim3(splits, head_groups, batch), dim3(kMlaThreads), (size_t)kMlaSmem, s, map, p));
-    else KTB_CUDA_CHECK(launch_pdl(mla_decode_tc_kernel<false>, dim3(splits, head_groups, batch), dim3(kMlaThreads), (size_t)kMlaSmem, s, map, p));
+    if (split_p) KTB_CUDA_CHECK(launch_pdl(mla_decode_tc_kernel<true>, dim3(splits, head_groups, batch), dim3(kMlaThreads), (size_t)kMlaSmem, s, map, q_map, pe_map, p));
+    else KTB_CUDA_CHECK(launch_pdl(mla_decode_tc_kernel<false>, dim3(splits, head_groups, batch), dim3(kMlaThreads), (size_t)kMlaSmem, s, map, q_map, pe_map, p));
     count_launch();
-    KTB_CUDA_CHECK(launch_pdl(mla_merge_kernel, dim3(batch * p.num_heads), dim3(128), 0, s, (const float*)p.o_part, (const float*)p.lse_part, splits, p.num_heads,
+    KTB_CUDA_CHECK(launch_pdl(mla_merge_kernel, dim3(batch * p.num_heads), dim3(128 * std::min(kMergeParts, (splits + kMergeLoads - 1) / kMergeLoads)), 0, s, (const float*)p.o_part, (const float*)p.lse_part, splits, p.num_heads,
                               (__nv_bfloat16*)out, lse_out, sink));
     count_launch();
     return KTB200_OK;

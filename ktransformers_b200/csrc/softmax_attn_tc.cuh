@@ -116,10 +116,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
         auto scores = [&](int t, int j) {
             const uint32_t qb = base + t * kTcTile, kb = kbase + (j & 1) * kTcTile;
 #pragma unroll
-            for (int k = 0; k < 8; k++)
-                mma_f16(tmem + t * 256, smem_desc(qb + (k >> 2) * (kTcTile / 2) + (k & 3) * 32, 16, 1024, kLayoutSw128),
-                        smem_desc(kb + (k >> 2) * (kTcTile / 2) + (k & 3) * 32, 16, 1024, kLayoutSw128), idesc_qk, k != 0);
-            mma_commit(smem_u32(&misc.s_full[t]));
+            for (int k = 0; k < 2; k++)
+                mma_f16_x4(tmem + t * 256, smem_desc(qb + k * (kTcTile / 2), 16, 1024, kLayoutSw128), smem_desc(kb + k * (kTcTile / 2), 16, 1024, kLayoutSw128), idesc_qk, k != 0,
+                           k ? smem_u32(&misc.s_full[t]) : 0);
         };
         bar_wait(smem_u32(&misc.q_full), 0);
         bar_wait(smem_u32(&misc.k_full[0]), 0);
