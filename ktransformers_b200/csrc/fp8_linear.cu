@@ -14,6 +14,8 @@
 #include <cuda.h>
 #include <cuda_fp8.h>
 
+#include <algorithm>
+#include <climits>
 #include <new>
 
 #include "common.cuh"
@@ -449,6 +451,7 @@ struct ktb200_fp8_linear {
 };
 
 namespace ktb {
+constexpr int kFp8Round = 8;      // what a CTA of the pass kernel costs beside its blocks, in blocks: set-up, quantisation, the atomics of its sums
 // Whether a batch of more than kFT tokens is still faster in passes of kFT.  The GEMM has no K splits, so a matrix of few rows is one serial chain of
 // K / 128 steps a tile: measured 10 us + 0.48 us a step and round of tiles (7168 -> 576: 35-39 us, 16384 -> 64: 76, 18432 -> 1536: 75); a pass takes 17.5 us
 // + 1 us per 2.9 MB of weights, a last one of a few tokens less (7168 -> 576: 28 us at 17 tokens, 36 at 24, 40 at 32, 58 at 48).
@@ -527,13 +530,16 @@ int ktb200_fp8_linear_create(int in_features, int out_features, const void* weig
     if (!l) return KTB200_ENOMEM;
     l->K = in_features; l->N = out_features; l->hidden_type = hidden_type; l->device = device; l->w = weight_e4m3; l->scale_inv = weight_scale_inv;
     l->nkb = in_features / 128; l->row_tiles = (out_features + 127) / 128;
-    // K splits: at most kFMaxKb blocks of B per CTA, and enough CTAs for two resident waves (2 per SM) when the row tiles are few
-    int ks = (4 * num_sms(device) + l->row_tiles - 1) / l->row_tiles;
-    const int ks_min = (l->nkb + kFMaxKb - 1) / kFMaxKb;
-    if (ks < ks_min) ks = ks_min;
-    if (ks > l->nkb) ks = l->nkb;
-    l->kb_per_split = (l->nkb + ks - 1) / ks;
-    if (l->kb_per_split < 4 && l->nkb >= 4) l->kb_per_split = 4;   // a CTA should at least fill its ring
+    // K splits: at most kFMaxKb blocks of B per CTA, at least as many as fill its ring, and of these the number whose CTAs, two an SM, take least one after the other.  Against as many
+    // splits as give four CTAs an SM (us, one and 16 rows): 1536 -> 24576 16.3 -> 11.2, 37 -> 21 (no splits, no atomics); 7168 -> 4096 13.5 -> 10.4, 29 -> 25; 10240 -> 14000 40.6 -> 36.1,
+    // 70 -> 63; 16384 -> 7168 34.3 -> 33.2, 60 -> 56; 18432 -> 7168 35.0 -> 34.7, 57 -> 60; matrices of few tiles as before
+    const int two = 2 * num_sms(device);
+    l->kb_per_split = std::min(l->nkb, 4);
+    long least = LONG_MAX;
+    for (int kb = std::min(l->nkb, 4); kb <= std::min(l->nkb, kFMaxKb); kb++) {
+        const long cost = (long)((l->row_tiles * ((l->nkb + kb - 1) / kb) + two - 1) / two) * (kb + kFp8Round);
+        if (cost < least) { least = cost; l->kb_per_split = kb; }
+    }
     l->ksplit = (l->nkb + l->kb_per_split - 1) / l->kb_per_split;
     const cuuint64_t gdim[2] = {(cuuint64_t)in_features, (cuuint64_t)out_features};
     const cuuint64_t gstr[1] = {(cuuint64_t)in_features};
