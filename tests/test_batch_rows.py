@@ -91,3 +91,30 @@ def test_fp8_batches_wherever_results_go(T, K, N, hid):
     off = (out[0].view(T, N).double() - want).norm() / want.norm()
     assert off < {F32: 1e-5, F16: 1e-3, BF16: 4e-3}[hid], off.item()
     lib.ktb200_fp8_linear_destroy(h)
+
+
+# linears of two to eight rows on either side of the line between the row kernels and the GEMM: one row at a time gives the same sums in another order (half a place of the result and
+# 4e-6 of the largest), and the launches tell which one ran
+@pytest.mark.parametrize("type,K,R,T,hid,launches", [(12, 16384, 7168, 8, BF16, 1), (14, 7168, 18432, 2, BF16, 3), (14, 7168, 18432, 1, BF16, 1), (14, 7168, 18432, 8, F32, 1), (14, 2048, 2048, 8, BF16, 1),
+                                                     (14, 1536, 24584, 5, F16, 3), (14, 1536, 24577, 5, F16, 1), (13, 512, 40002, 7, BF16, 2), (13, 4096, 8200, 3, BF16, 3), (13, 10240, 16000, 8, F16, 3)])
+def test_few_rows_as_gemms(type, K, R, T, hid, launches):
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    g = torch.Generator(device="cuda").manual_seed(T + R)
+    blocks, x = synth_blocks(type, R * K, "cuda", T), torch.randn((T, K), generator=g, device="cuda").to(TORCH[hid])
+    bias, lib, h = torch.randn(R, generator=g, device="cuda"), native.lib(), C.c_void_p()
+    native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), type, hid, T, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, _stream()))
+    y, one = (torch.full((T, R), 7.0, dtype=TORCH[hid], device="cuda") for _ in range(2))
+    run = lambda x, y, n, bsz=None: native.check(lib.ktb200_linear_forward(h, n, x.data_ptr(), y.data_ptr(), bias.data_ptr(), bsz.data_ptr() if bsz is not None else None, _stream()))
+    n0 = native.launch_count()
+    run(x, y, T)
+    assert native.launch_count() - n0 == launches
+    for t in range(T):
+        run(x[t:], one[t:], 1)
+    a, b = y.double(), one.double()
+    assert ((a - b).abs() <= {BF16: 2.0 ** -7, F16: 2.0 ** -10, F32: 2.0 ** -20}[hid] * b.abs() + 4e-6 * b.abs().max()).all()
+    held = torch.full_like(y, 7.0)
+    run(x, held, T, torch.tensor([T - 1], dtype=torch.int32, device="cuda"))
+    assert torch.equal(held[:T - 1], y[:T - 1]) and (held[T - 1:] == 7.0).all()
+    lib.ktb200_linear_destroy(h)
