@@ -96,7 +96,7 @@ def test_fp8_batches_wherever_results_go(T, K, N, hid):
 # linears of two to eight rows on either side of the line between the row kernels and the GEMM: one row at a time gives the same sums in another order (half a place of the result and
 # 4e-6 of the largest), and the launches tell which one ran
 @pytest.mark.parametrize("type,K,R,T,hid,launches", [(12, 16384, 7168, 8, BF16, 1), (14, 7168, 18432, 2, BF16, 3), (14, 7168, 18432, 1, BF16, 1), (14, 7168, 18432, 8, F32, 1), (14, 2048, 2048, 8, BF16, 1),
-                                                     (14, 1536, 24584, 5, F16, 3), (14, 1536, 24577, 5, F16, 1), (13, 512, 40002, 7, BF16, 2), (13, 4096, 8200, 3, BF16, 3), (13, 10240, 16000, 8, F16, 3)])
+                                                     (14, 1536, 24584, 5, F16, 2), (14, 1536, 24577, 5, F16, 1), (13, 512, 40002, 7, BF16, 2), (13, 4096, 8200, 3, BF16, 3), (13, 10240, 16000, 8, F16, 3)])
 def test_few_rows_as_gemms(type, K, R, T, hid, launches):
     from ktransformers_b200 import native
     from ktransformers_b200.util.synth import synth_blocks
