@@ -1,15 +1,18 @@
 // Un-quantised experts of a prompt portion (KExpertsDense, bf16): the (token, choice) pairs sorted by expert, then per expert
 //     a = act(W_gate x, W_up x)  (or relu(W_up x)^2)        y = W_down a        out[t] = sum_j w_j y_tj
-// as two persistent tcgen05 GEMMs over 128-row tiles of the sorted pairs (the reference loops over experts in torch:
-// archive/ktransformers/operators/experts.py:562-678).  Both products of a gated expert share a tile's accumulator columns [gate 128 | up 128], so the
-// activation is applied to the fp32 sums in the epilogue and the pre-activations never reach memory; y stays fp32 up to the weighted sum.
-// Bounds: each expert's weights once per 128 of its pairs from HBM or L2 (48 KB a stage for 512 cycles of the tensor pipe), so at 100-300 pairs per expert the
-// second row tile's reading from L2 shows.  1000 tokens, 32 experts of 1024 x 2048, 4 choices (403 MB of weights, 62 us at 6.5 TB/s): 253 us as library GEMMs
-// with sorting and elementwise launches between them, 148 us like this (shares: products 48 and 31 %, weighted sum 8, sort 7, gather 5); 128 tokens,
-// 64 experts of 1536 x 4096, 6 choices (2.4 GB): 640 -> 434 us, 5.6 TB/s; 47 tokens, 8 experts of 4096 x 4096: 298 -> 172 us.
-//     kernel: warp 0 TMA (4 stages of 16 + 32 KB, 128-byte swizzle; of the 128 rows only pieces of 32 that the tile has), warp 1 issuer, warps 2-9
-//     epilogue; two accumulators of 256 columns, so that a tile's epilogue runs beside the next tile's products.  The launches are chained (programmatic
-//     dependent launch): each waits for all of its predecessor before it touches the workspace.
+// as two persistent tcgen05 GEMMs over tiles of the sorted pairs (the reference loops over experts in torch:
+// archive/ktransformers/operators/experts.py:562-678).  The weights' rows are the M side of the products and the pairs the N side, so that a tile costs what its
+// pairs need in steps of 16 and an expert's pairs are dealt evenly to its tiles; with the pairs on the M side a tile of 20 took as long as one of 128.  Both products
+// of a gated expert share a tile's accumulators [gate | up], so the activation is applied to the fp32 sums in the epilogue and the pre-activations never reach
+// memory; y stays fp32 up to the weighted sum.
+// Bounds: each expert's weights once per tile of its pairs from HBM or L2, so the second tile's reading shows where experts have more than one.  1000 tokens, 32
+// experts of 1024 x 2048, 4 choices (403 MB of weights, 62 us at 6.5 TB/s): 149 us with the pairs on the M side, 133 like this (products 65 and 34, sort 10, gather 7,
+// weighted sum 10); 1200 tokens 176 -> 139; 2400 tokens, 128 experts of 768 x 2048, 8 choices 512 -> 385; 128 tokens, 64 experts of 1536 x 4096, 6 choices (2.4 GB)
+// 430 -> 420, 5.8 TB/s; 1000 tokens, 8 experts of 512 x 1024 (one round of CTAs, latency) 43 -> 43.  Half tiles of weights (M = 64): 170 us, the pairs are read twice.
+//     kernel: warp 0 TMA (32 KB of weights, 16 KB of pairs and 4 stages, or 32 KB and 3; 128-byte swizzle; of the pairs only pieces of 32 that the tile has), warp 1
+//     issuer, warps 4-19 epilogue (neighbouring threads write neighbouring columns of a result row); two sets of accumulators where a tile has up to 128 pairs, so
+//     that its epilogue runs beside the next one's products.  The launches are chained (programmatic dependent launch): each waits for all of its predecessor before
+//     it touches the workspace.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -19,14 +22,14 @@
 namespace ktb {
 using namespace umma;
 
-constexpr int kEgThreads = 320, kEgStage = 128 * 128 + 256 * 128, kEgStages = 4, kEgMaxExperts = 1024;
+constexpr int kEgThreads = 640, kEgRing = 192 * 1024, kEgMaxExperts = 1024, kEgWide = 256;
 enum EgMode { EG_GATED, EG_RELU2, EG_DOWN };
 struct EgMisc {
-    unsigned long long full[kEgStages], free[kEgStages], d_full[2], d_free[2];
+    unsigned long long full[4], free[4], d_full[2], d_free[2];
     uint32_t tmem_base, pad;
-    int prefix[kEgMaxExperts + 1];      // 128-row tiles before every expert
+    int prefix[kEgMaxExperts + 2];      // pair tiles before every expert; whether a tile has up to kEgWide pairs (else 128)
 };
-constexpr int kEgSmem = kEgStages * kEgStage + (int)sizeof(EgMisc) + 1024;
+constexpr int kEgSmem = kEgRing + (int)sizeof(EgMisc) + 1024;
 static_assert(kEgSmem <= 232448, "shared memory budget");
 
 struct EgParams {
@@ -41,7 +44,7 @@ struct EgParams {
 // pair's row goes among the sorted rows; -1: its id names no expert.  One launch of ~6 us for 4000 pairs instead of three (clear, count, scan) and the
 // gather's atomics; beyond that ~1 us per 1000 pairs, 1-2% of what their products take.
 __global__ void __launch_bounds__(1024) eg_sort_kernel(const int64_t* __restrict__ ids, int n, int E, int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ prefix,
-                                                       int64_t* __restrict__ place) {
+                                                       int64_t* __restrict__ place, int col_tiles, int ctas) {
     __shared__ int cursor[kEgMaxExperts];
     __shared__ int2 part[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -68,7 +71,13 @@ __global__ void __launch_bounds__(1024) eg_sort_kernel(const int64_t* __restrict
         for (int j = 0; j < 4; j++) add(e[j]);
     }
     __syncthreads();
-    const int own = tid < E ? cursor[tid] : 0, tiles = (own + 127) / 128;
+    const int own = tid < E ? cursor[tid] : 0;
+    // Tiles of up to 256 pairs where every expert has one and they save a third of the CTAs' rounds, else of 128.  The weights are read once, but the tile has no second
+    // set of accumulators for the next one, and takes ~1.4 times as long.  128 pairs / 256, us, rounds: 32 experts of 1024 x 2048, 4 choices, 1000 tokens 137 / 133 (3 / 2),
+    // 1200 152 / 139 (4 / 2), 900 123 / 127 (2 / 2); 128 of 768 x 2048, 8 choices, 2400 399 / 385 (11 / 6), 2000 346 / 354 (8 / 6); 8 of 512 x 1024 (one round) 43 / 49.
+    const int one = __syncthreads_count(own > 0), two = __syncthreads_count(own > 128), more = __syncthreads_or(own > kEgWide);
+    const bool wide = two && !more && 2 * (((long)(one + two) * col_tiles + ctas - 1) / ctas) >= 3 * (((long)one * col_tiles + ctas - 1) / ctas);
+    const int tiles = wide ? own > 0 : (own + 127) / 128;
     int2 v = make_int2(own, tiles);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -82,7 +91,7 @@ __global__ void __launch_bounds__(1024) eg_sort_kernel(const int64_t* __restrict
         counts[tid] = own;
         offsets[tid] = cursor[tid] = v.x - own;
         prefix[tid] = v.y - tiles;
-        if (tid == E - 1) prefix[E] = v.y;
+        if (tid == E - 1) { prefix[E] = v.y; prefix[E + 1] = wide; }
     }
     __syncthreads();
     for (long i = tid; i - tid < n; i += 4096) {
@@ -114,11 +123,11 @@ __global__ void __launch_bounds__(kEgThreads, 1) eg_gemm_kernel(const __grid_con
                                                                const EgParams p) {
     extern __shared__ uint8_t eg_smem[];
     const uint32_t raw = smem_u32(eg_smem), base = (raw + 1023u) & ~1023u;
-    EgMisc& misc = *reinterpret_cast<EgMisc*>(eg_smem + (base - raw) + kEgStages * kEgStage);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    EgMisc& misc = *reinterpret_cast<EgMisc*>(eg_smem + (base - raw) + kEgRing);
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);
     if (tid == 0) {
-        for (int s = 0; s < kEgStages; s++) { bar_init(smem_u32(&misc.full[s]), 1); bar_init(smem_u32(&misc.free[s]), 1); }
-        for (int b = 0; b < 2; b++) { bar_init(smem_u32(&misc.d_full[b]), 1); bar_init(smem_u32(&misc.d_free[b]), 8); }
+        for (int s = 0; s < 4; s++) { bar_init(smem_u32(&misc.full[s]), 1); bar_init(smem_u32(&misc.free[s]), 1); }
+        for (int b = 0; b < 2; b++) { bar_init(smem_u32(&misc.d_full[b]), 1); bar_init(smem_u32(&misc.d_free[b]), 16); }
         bar_fence_init();
         tma_prefetch_desc(&amap);
         tma_prefetch_desc(&bmap);
@@ -126,118 +135,101 @@ __global__ void __launch_bounds__(kEgThreads, 1) eg_gemm_kernel(const __grid_con
     }
     griddep_launch_dependents();
     griddep_wait();
-    for (int i = tid; i <= p.E; i += kEgThreads) misc.prefix[i] = p.prefix[i];
+    for (int i = tid; i <= p.E + 1; i += kEgThreads) misc.prefix[i] = p.prefix[i];
     if (warp == 1) tmem_alloc(smem_u32(&misc.tmem_base), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = misc.tmem_base;
-    // Columns of a tile.  Half as many where that fills the last round of CTAs so much better that it pays for reading the rows twice as often (a half tile
-    // takes ~0.6 of a whole one's time: its weights are half, its rows are the same).
-    const int row_tiles = misc.prefix[p.E], whole = MODE == EG_GATED ? 128 : 256;
-    const int rounds_whole = (row_tiles * ((p.cols + whole - 1) / whole) + gridDim.x - 1) / gridDim.x, rounds_half = (row_tiles * ((p.cols + whole / 2 - 1) / (whole / 2)) + gridDim.x - 1) / gridDim.x;
-    const bool half = 3 * rounds_half < 5 * rounds_whole;
-    const int tile_cols = half ? whole / 2 : whole, nt = (p.cols + tile_cols - 1) / tile_cols, total = row_tiles * nt;
-    auto place = [&](int tile, int& e, int& m0, int& n0) {      // expert, then column tile, then row tile fastest: neighbouring CTAs share the weights
+    const uint32_t tmem = uniform(misc.tmem_base);
+    const bool wide = uniform(misc.prefix[p.E + 1]);
+    const int sets = wide ? 1 : 2, stages = wide ? 3 : 4, stage = kEgRing / stages, wofs = wide ? 256 * 128 : 128 * 128;
+    const uint32_t second = wide ? 256 : 128;            // accumulator columns: [first matrix | second], a set of 256 each; a wide tile takes all 512
+    constexpr int kTileCols = MODE == EG_GATED ? 128 : 256;
+    const int nt = (p.cols + kTileCols - 1) / kTileCols, total = misc.prefix[p.E] * nt;
+    struct Tile { int e, at, n, n0; };
+    auto place = [&](int tile) {      // expert, then column tile, then pair tile fastest: neighbouring CTAs share the weights.  An expert's tiles have the same number of pairs
         int lo = 0, hi = p.E;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (misc.prefix[mid] * nt <= tile) lo = mid; else hi = mid;
         }
-        const int local = tile - misc.prefix[lo] * nt, mt = misc.prefix[lo + 1] - misc.prefix[lo];
-        e = lo;
-        m0 = (local % mt) * 128;
-        n0 = (local / mt) * tile_cols;
+        const int local = tile - misc.prefix[lo] * nt, mt = misc.prefix[lo + 1] - misc.prefix[lo], count = p.counts[lo], per = (count + mt - 1) / mt, m0 = (local % mt) * per;
+        return Tile{uniform(lo), uniform(p.offsets[lo] + m0), uniform(min(per, count - m0)), uniform((local / mt) * kTileCols)};
     };
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0, ph = 1;
-            for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-                int e, m0, n0;
-                place(tile, e, m0, n0);
-                const int arow = p.offsets[e] + m0, brow = e * p.rows + n0, pieces = min(4, (p.counts[e] - m0 + 31) / 32);      // (of 32 rows; a row's sums need no other row)
-                for (int k = 0; k < p.nk; k++) {
-                    bar_wait(smem_u32(&misc.free[s]), ph);
-                    const uint32_t bar = smem_u32(&misc.full[s]), dst = base + s * kEgStage;
-                    const uint32_t wdst = dst + 128 * 128;
-                    bar_expect_tx(bar, (half ? 128 : 256) * 128 + pieces * 32 * 128);
-                    for (int i = 0; i < pieces; i++) tma_load_2d(dst + i * 32 * 128, &amap, bar, k * 64, arow + i * 32);
-                    if (MODE == EG_GATED) {
-                        for (int i = 0; i < tile_cols; i += 64) tma_load_2d(wdst + i * 128, &bmap, bar, k * 64, brow + i);
-                        for (int i = 0; i < tile_cols; i += 64) tma_load_2d(wdst + (tile_cols + i) * 128, &umap, bar, k * 64, brow + i);
-                    } else {
-                        for (int i = 0; i < tile_cols; i += 64) tma_load_2d(wdst + i * 128, &bmap, bar, k * 64, brow + i);
-                    }
-                    if (++s == kEgStages) { s = 0; ph ^= 1; }
+        int s = 0, ph = 1;
+        for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+            const Tile t = place(tile);
+            const int brow = t.e * p.rows + t.n0, pieces = (t.n + 31) / 32;      // (of 32 pairs; a pair's sums need no other pair)
+            for (int k = 0; k < p.nk; k++) {
+                bar_wait(smem_u32(&misc.free[s]), ph);
+                if (lane == 0) {
+                    const uint32_t bar = smem_u32(&misc.full[s]), dst = base + s * stage, wdst = dst + wofs;
+                    bar_expect_tx(bar, 256 * 128 + pieces * 32 * 128);
+                    for (int i = 0; i < pieces; i++) tma_load_2d(dst + i * 32 * 128, &amap, bar, k * 64, t.at + i * 32);
+                    for (int i = 0; i < 128; i += 64) tma_load_2d(wdst + i * 128, &bmap, bar, k * 64, brow + i);
+                    for (int i = 0; i < 128; i += 64) tma_load_2d(wdst + (128 + i) * 128, MODE == EG_GATED ? &umap : &bmap, bar, k * 64, (MODE == EG_GATED ? brow : brow + 128) + i);
                 }
+                __syncwarp();
+                if (++s == stages) { s = 0; ph ^= 1; }
             }
         }
-        __syncwarp();
     } else if (warp == 1) {
-        const uint32_t idesc = half ? instr_desc(1, 1, 1, 0, 0, 128, 128) : instr_desc(1, 1, 1, 0, 0, 128, 256);      // f32 += bf16 . bf16, K-major both
         int s = 0, ph = 0;
         unsigned it = 0;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, it++) {
-            const int buf = it & 1;
-            bar_wait(smem_u32(&misc.d_free[buf]), ((it >> 1) & 1) ^ 1);
+            const Tile t = place(tile);
+            const uint32_t idesc = instr_desc(1, 1, 1, 0, 0, 128, (t.n + 15) & ~15);      // f32 += bf16 . bf16, K-major both
+            const int buf = it % sets;
+            const uint32_t d = tmem + buf * 256;
+            bar_wait(smem_u32(&misc.d_free[buf]), ((it / sets) & 1) ^ 1);
             for (int k = 0; k < p.nk; k++) {
                 bar_wait(smem_u32(&misc.full[s]), ph);
                 tc_fence_after();
-                const uint32_t a = base + s * kEgStage, b = a + 128 * 128;
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    mma_f16(tmem + buf * 256, smem_desc(a + j * 32, 16, 1024, kLayoutSw128), smem_desc(b + j * 32, 16, 1024, kLayoutSw128), idesc, (k | j) != 0);
-                mma_commit(smem_u32(&misc.free[s]));
-                if (++s == kEgStages) { s = 0; ph ^= 1; }
+                const uint32_t b = base + s * stage, a = b + wofs;
+                const uint64_t bd = smem_desc(b, 16, 1024, kLayoutSw128);
+                mma_f16_x4(d, smem_desc(a, 16, 1024, kLayoutSw128), bd, idesc, k != 0);
+                mma_f16_x4(d + second, smem_desc(a + 128 * 128, 16, 1024, kLayoutSw128), bd, idesc, k != 0, smem_u32(&misc.free[s]), k + 1 == p.nk ? smem_u32(&misc.d_full[buf]) : 0);
+                if (++s == stages) { s = 0; ph ^= 1; }
             }
-            mma_commit(smem_u32(&misc.d_full[buf]));
         }
-    } else {
-        const int sp = warp & 3, ch = (warp - 2) >> 2, row = 32 * sp + lane;
+    } else if (warp >= 4) {
+        // epilogue: a thread owns a row of either matrix and every fourth run of 16 pairs
+        const int sp = warp & 3, part = (warp - 4) >> 2;
         unsigned it = 0;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, it++) {
-            int e, m0, n0;
-            place(tile, e, m0, n0);
-            const int buf = it & 1, n = p.counts[e] - m0;
-            const long pos = (long)p.offsets[e] + m0 + row;
-            const bool live = row < n;
-            const float sc = p.row_scale && live ? p.row_scale[pos] : 1.f;
+            const Tile t = place(tile);
+            const int buf = it % sets, col = t.n0 + 32 * sp + lane;
             const uint32_t tc = tmem + ((uint32_t)(32 * sp) << 16) + buf * 256;
-            bar_wait(smem_u32(&misc.d_full[buf]), (it >> 1) & 1);
+            bar_wait(smem_u32(&misc.d_full[buf]), (it / sets) & 1);
             tc_fence_after();
 #pragma unroll 1
-            for (int c = ch * (tile_cols / 2); c < (ch + 1) * (tile_cols / 2); c += 16) {
+            for (int c = 16 * part; c < t.n; c += 64) {
                 uint32_t v[16], u[16];
                 tmem_ld16(tc + c, v);
-                if (MODE == EG_GATED) tmem_ld16(tc + tile_cols + c, u);
+                tmem_ld16(tc + second + c, u);
                 tmem_wait_ld();
-                if (live) {
-                    float x[16];
+                const long pos = (long)t.at + c;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const float g = __uint_as_float(v[i]);
-                        if (MODE == EG_GATED) x[i] = gated_act(g * sc, __uint_as_float(u[i]) * sc, p.act, p.limit);
-                        else if (MODE == EG_RELU2) { const float r = fmaxf(g * sc, 0.f); x[i] = r * r; }
-                        else x[i] = g;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; i += 8)
-                        if (n0 + c + i < p.cols) {      // (a multiple of 8)
-                            if (MODE == EG_DOWN) {
-                                float4* o = reinterpret_cast<float4*>((float*)p.out + pos * p.cols + n0 + c + i);
-                                o[0] = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
-                                o[1] = make_float4(x[i + 4], x[i + 5], x[i + 6], x[i + 7]);
-                            } else {
-                                uint32_t w[4];
-#pragma unroll
-                                for (int q = 0; q < 4; q++) {
-                                    const __nv_bfloat162 b = __floats2bfloat162_rn(x[i + 2 * q], x[i + 2 * q + 1]);
-                                    w[q] = *reinterpret_cast<const uint32_t*>(&b);
-                                }
-                                *reinterpret_cast<uint4*>((__nv_bfloat16*)p.out + pos * p.cols + n0 + c + i) = make_uint4(w[0], w[1], w[2], w[3]);
-                            }
+                for (int i = 0; i < 16; i++) {
+                    if (c + i >= t.n) break;
+                    const float a = __uint_as_float(v[i]), b = __uint_as_float(u[i]);
+                    if (MODE == EG_DOWN) {
+                        float* o = (float*)p.out + (pos + i) * p.cols;
+                        if (col < p.cols) o[col] = a;
+                        if (col + 128 < p.cols) o[col + 128] = b;
+                    } else {
+                        const float sc = p.row_scale ? p.row_scale[pos + i] : 1.f;
+                        __nv_bfloat16* o = (__nv_bfloat16*)p.out + (pos + i) * p.cols;
+                        if (MODE == EG_GATED) {
+                            if (col < p.cols) o[col] = __float2bfloat16_rn(gated_act(a * sc, b * sc, p.act, p.limit));
+                        } else {
+                            const float ra = fmaxf(a * sc, 0.f), rb = fmaxf(b * sc, 0.f);
+                            if (col < p.cols) o[col] = __float2bfloat16_rn(ra * ra);
+                            if (col + 128 < p.cols) o[col + 128] = __float2bfloat16_rn(rb * rb);
                         }
+                    }
                 }
             }
             tc_fence_before();
@@ -285,7 +277,7 @@ extern "C" int ktb200_experts_combine(const void* rows, const int64_t* place, co
 
 extern "C" size_t ktb200_experts_prompt_workspace(int n_tokens, int top, int n_experts, int width, int ff) {
     const size_t P = (size_t)n_tokens * top;
-    return up256((3 * (size_t)n_experts + 1) * sizeof(int)) + up256(P * 8) + up256(P * 4) + up256(P * width * 2) + up256(P * ff * 2) + up256(P * width * 4);
+    return up256((3 * (size_t)n_experts + 2) * sizeof(int)) + up256(P * 8) + up256(P * 4) + up256(P * width * 2) + up256(P * ff * 2) + up256(P * width * 4);
 }
 
 extern "C" int ktb200_experts_prompt(const void* x, const int64_t* ids, const float* weights, int weights_on_input, int top, int n_experts, const void* w_gate, const void* w_up,
@@ -301,12 +293,12 @@ extern "C" int ktb200_experts_prompt(const void* x, const int64_t* ids, const fl
     KTB_CUDA_CHECK(cudaGetDevice(&dev));
     uint8_t* at = (uint8_t*)workspace;
     auto take = [&](size_t n) { uint8_t* p = at; at += up256(n); return p; };
-    int* counts = (int*)take((3 * (size_t)n_experts + 1) * sizeof(int));
+    int* counts = (int*)take((3 * (size_t)n_experts + 2) * sizeof(int));
     int *offsets = counts + n_experts, *prefix = offsets + n_experts;
     int64_t* place = (int64_t*)take(P * 8);
     float* scale = (float*)take(P * 4);
     void *xs = take(P * width * 2), *a = take(P * ff * 2), *y = take(P * width * 4);
-    eg_sort_kernel<<<1, 1024, 0, s>>>(ids, (int)P, n_experts, counts, offsets, prefix, place);
+    eg_sort_kernel<<<1, 1024, 0, s>>>(ids, (int)P, n_experts, counts, offsets, prefix, place, (ff + (w_gate ? 127 : 255)) / (w_gate ? 128 : 256), num_sms(dev));
     KTB_LAUNCH_CHECK();
     KTB_CUDA_CHECK(launch_pdl(eg_gather_kernel, dim3((unsigned)P), dim3(128), 0, s, (const uint4*)x, weights, top, width / 8, (const int64_t*)place, weights_on_input ? scale : nullptr,
                               (uint4*)xs));

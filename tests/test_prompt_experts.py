@@ -45,6 +45,13 @@ def test_prompt_experts(T, width, ff, E, top, kind):
         assert ((got - want).abs() <= 2.0 ** -8 * room + 1e-6).all(), ((got - want).abs() / (room + 1e-6)).max().item()
 
 
+# several rounds of CTAs: tiles of up to 256 pairs (one an expert), of up to 128 with an expert's pairs dealt to two, to three, and one tile an expert
+@pytest.mark.parametrize("T", [1300, 1800, 2600, 500])
+@pytest.mark.parametrize("kind", ["silu", "relu2"])
+def test_many_tiles(T, kind):
+    test_prompt_experts(T, 136, 1024, 32, 4, kind)
+
+
 def test_negative_ids_name_no_expert():
     """as those at or beyond the experts: the same bits"""
     from ktransformers_b200.operators.experts import KExpertsDense
