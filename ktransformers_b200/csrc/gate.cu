@@ -12,13 +12,17 @@
 //   phase 2  the LAST CTA to finish (atomic ticket, self-resetting, graph-replay safe) selects, all 128 threads
 //            per token — scoring, bias, group top-2 / max, group top-k, expert top-k by iterative arg-max with
 //            REDUX max/min (ties -> lowest index), gather, normalise, scale.
+#include <algorithm>
+
 #include "gate.cuh"
 
 namespace ktb {
 
 // Bound for batches by chains of loads: CTAs of their own for every tile of 8 tokens (they share the rows through L2), a tile's columns in one round of loads while the rows are on
-// their way to L2, 5 CTAs an SM (96 registers), a token's selection (about 5 us of a CTA) beside the others'.  256 x 7168 (us): 8 tokens 34.0 -> 19.7, 24 tokens 77.6 -> 32.0, 200 tokens
-// 560 -> 160, one token 17.7 -> 17.1, against one CTA per rows and columns that took tile after tile, value by value, and 16 selectors.  Shorter selections (picks as a tree, groups
+// their way to L2, a token's selection (about 5 us of a CTA) beside the others'.  256 x 7168 (us): 8 tokens 34.0 -> 19.7, 24 tokens 77.6 -> 32.0, 200 tokens
+// 560 -> 160, against one CTA per rows and columns that took tile after tile, value by value, and 16 selectors.  5 CTAs an SM (96 registers) where there are
+// more than two an SM and more than two tokens (256 x 7168, 8 tokens 27.4 -> 22.5; 128 x 5120, 12 tokens 20.5 -> 18.4), else all the registers a thread's loads in flight want (128 x
+// 5120, 2 tokens 17.9 -> 14.3, 8 tokens, 256 CTAs, 18.3 -> 16.4; 384 x 7168, one token 22.5 -> 20.9).  Shorter selections (picks as a tree, groups
 // ranked by a warp) changed nothing here and in the fused block.
 constexpr int kGateTiles = 16, kGateSelectors = 64;
 // a tile's columns in fp32: four values a load, eight loads of a thread in flight before the first is looked at
@@ -43,7 +47,8 @@ __device__ __forceinline__ void gate_stage(const V* x, int row, int nt, int nc4,
     }
 }
 
-__global__ void __launch_bounds__(kGateThreads, 5) gate_kernel(const GateParams p) {
+template <int PER_SM>      // CTAs an SM that its registers leave room for (1: as many as the compiler wants)
+__global__ void __launch_bounds__(kGateThreads, PER_SM) gate_kernel(const GateParams p) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     float* xs = reinterpret_cast<float*>(smem_raw);   // [tok tile][slice cols]  (phase 1) / scores+choice (phase 2)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -166,9 +171,10 @@ extern "C" int ktb200_moe_gate_forward(const ktb200_gate_config* c, int qlen, co
     size_t smem = (size_t)nt * nc4_max * 16;
     const size_t smem_sel = ((size_t)2 * c->n_experts + 32 + 4 * kGateWarps) * sizeof(float);
     if (smem_sel > smem) smem = smem_sel;
-    if (smem > 48 * 1024) KTB_CUDA_CHECK(raise_smem_limit((const void*)gate_kernel, smem));
-    const int tiles = (qlen + kGateTokTile - 1) / kGateTokTile;
-    gate_kernel<<<dim3(row_ctas, S, tiles < kGateTiles ? tiles : kGateTiles), kGateThreads, smem, s>>>(p);
+    const int tiles = std::min((qlen + kGateTokTile - 1) / kGateTokTile, kGateTiles);
+    auto kernel = qlen > 2 && row_ctas * S * tiles > 2 * num_sms(dev) ? gate_kernel<5> : gate_kernel<1>;
+    if (smem > 48 * 1024) KTB_CUDA_CHECK(raise_smem_limit((const void*)kernel, smem));
+    kernel<<<dim3(row_ctas, S, tiles), kGateThreads, smem, s>>>(p);
     KTB_LAUNCH_CHECK();
     return KTB200_OK;
 }
