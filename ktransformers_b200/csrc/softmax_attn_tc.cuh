@@ -12,9 +12,9 @@
 //                  more than 2^8 (P <= 256 in between, where bf16 and fp32 are as exact as below 1)
 // TMEM: [S0 | O0 | S1 | O1], 128 columns each.  Shared memory: Q 64 KB, K and V 2 x 32 KB each.
 // Bounds: 16 products of 64 cycles per (row tile, key tile) beside 128 exponentials per thread at 4 per cycle and scheduler (1024 cycles for two
-// tiles on one scheduler): 2,050 cycles of tensor pipe for two tiles, 95-105 us for 2048 tokens behind 2048, 64 heads over 8.  It takes about 200 (250 with the weights of all 128 keys
-// handed over at once): a row's scores arrive, maximum, exponentials and stores run one after the other in its thread, 2,500 of the 3,600 cycles of a round, and only the first 64
-// keys' product runs beside them.  Quarters of 32 keys: 260.  Some of the exponentials as a polynomial on the multiply-add pipes: slower from three of eight on, nothing with one or two.
+// tiles on one scheduler): 2,050 cycles of tensor pipe for two tiles, 95-105 us for 2048 tokens behind 2048, 64 heads over 8.  It takes 250: a row's maximum, exponentials,
+// conversions and stores run one after the other in its thread, the tile's next product waits for all of them, and there is one score buffer a tile (tensor pipe 48 %
+// active, issue slots 35 %).
 #pragma once
 #include <cuda.h>
 
@@ -28,7 +28,7 @@ constexpr int kTcThreads = 384, kTcKeys = 128, kTcTile = 128 * 128 * 2, kTcSmem 
 // shorter portions over more SMs
 constexpr int kTcMinCtas = 32;
 struct TcMisc {
-    unsigned long long q_full, k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], p_full[2][2], o_done[2];
+    unsigned long long q_full, k_full[2], k_free[2], v_full[2], v_free[2], s_full[2], p_full[2], o_done[2];
     uint32_t tmem_base;
     int info[3];
 };
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
         bar_init(smem_u32(&misc.q_full), 1);
         for (int i = 0; i < 2; i++) {
             bar_init(smem_u32(&misc.k_full[i]), 1); bar_init(smem_u32(&misc.k_free[i]), 1); bar_init(smem_u32(&misc.v_full[i]), 1); bar_init(smem_u32(&misc.v_free[i]), 1);
-            bar_init(smem_u32(&misc.s_full[i]), 1); bar_init(smem_u32(&misc.p_full[i][0]), 4); bar_init(smem_u32(&misc.p_full[i][1]), 4); bar_init(smem_u32(&misc.o_done[i]), 1);
+            bar_init(smem_u32(&misc.s_full[i]), 1); bar_init(smem_u32(&misc.p_full[i]), 4); bar_init(smem_u32(&misc.o_done[i]), 1);
         }
         bar_fence_init();
     }
@@ -143,13 +143,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
             if (j + 1 < n) bar_wait(smem_u32(&misc.k_full[st ^ 1]), ((j + 1) >> 1) & 1);
 #pragma unroll 1
             for (int t = 0; t < 2; t++) {
+                bar_wait(smem_u32(&misc.p_full[t]), j & 1);
+                tc_fence_after();
 #pragma unroll
-                for (int half = 0; half < 2; half++) {      // (the weights of 64 keys each: the first are multiplied while the others are made)
-                    bar_wait(smem_u32(&misc.p_full[t][half]), j & 1);
-                    tc_fence_after();
-                    mma_f16_ta_x4<128>(tmem + t * 256 + 128, tmem + t * 256 + 32 * half, smem_desc(vb + half * 8192, kTcTile / 2, 1024, kLayoutSw128), idesc_pv, (j | half) != 0,
-                                       half && t == 1 ? smem_u32(&misc.v_free[st]) : 0);
-                }
+                for (int k = 0; k < 8; k++)
+                    mma_f16_ta(tmem + t * 256 + 128, tmem + t * 256 + 8 * k, smem_desc(vb + k * 2048, kTcTile / 2, 1024, kLayoutSw128), idesc_pv, (j | k) != 0);
+                if (t == 1) mma_commit(smem_u32(&misc.v_free[st]));
                 if (j + 1 < n) {
                     scores(t, j + 1);
                     if (t == 1) mma_commit(smem_u32(&misc.k_free[st ^ 1]));
@@ -247,11 +246,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) softmax_attn_tc_kernel(const __
                     sum[i & 1] = add2(sum[i & 1], pack2(__uint_as_float(pk[i] << 16), __uint_as_float(pk[i] & 0xffff0000u)));
                 }
                 tmem_st32(ts + 32 * q, pk);
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) bar_arrive(smem_u32(&misc.p_full[t][q]));
             }
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive(smem_u32(&misc.p_full[t]));
             float a0, a1, a2, a3;
             unpack2(sum[0], a0, a1);
             unpack2(sum[1], a2, a3);

@@ -211,33 +211,6 @@ __device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uin
         "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// four of them on consecutive 8-column slices of A, the B operands DB units of 16 bytes apart, and a barrier as for mma_f16_x4 below.  One election
-template <int DB>
-__device__ __forceinline__ void mma_f16_ta_x4(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t bar = 0) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q, t, c;\n"
-        ".reg .b32 r, a;\n"
-        ".reg .b64 b;\n"
-        "elect.sync r|q, 0xffffffff;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "setp.eq.b32 t, 0, 0;\n"
-        "setp.ne.and.b32 c, %5, 0, q;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "add.u32 a, %1, 8;\n"
-        "add.u64 b, %2, %6;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
-        "add.u32 a, a, 8;\n"
-        "add.u64 b, b, %6;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
-        "add.u32 a, a, 8;\n"
-        "add.u64 b, b, %6;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n"
-        "@c tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n"
-        "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(bar), "n"(DB)
-        : "memory");
-}
 // e4m3 / e5m2 / 6- and 4-bit float inputs, fp32 accumulate: K = 32 per instruction for the 8-bit types
 __device__ __forceinline__ void mma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
