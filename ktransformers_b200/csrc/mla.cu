@@ -53,6 +53,7 @@ constexpr int kOffMiscMax = kMaxStages * kStageBytes + kQBytes + 2 * kPBytes;   
 constexpr int kTmemCols = 512;
 constexpr int kColO = 0, kColS = 256;
 constexpr float kRescaleThreshold = 8.f;
+constexpr int kMaxSplits = 128;          // of a sequence's keys: the merge has a thread and a weight for each
 
 struct MlaMisc {
     unsigned long long q_full, k_full[kMaxStages], k_empty[kMaxStages], s_full[2], s_empty[2], p_full, p_free[2];
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
 constexpr int kMergeLoads = 10, kMergeParts = 4;
 __global__ void __launch_bounds__(128 * kMergeParts) mla_merge_kernel(const float* o_part, const float* lse_part, int num_splits, int num_heads,
                                                                       __nv_bfloat16* out, float* lse_out, const float* sink) {
-    __shared__ float ws[128];
+    __shared__ float ws[kMaxSplits];
     __shared__ float red[8];
     __shared__ float4 sums[kMergeParts - 1][128];
     griddep_launch_dependents();
@@ -409,7 +410,7 @@ __global__ void __launch_bounds__(128 * kMergeParts) mla_merge_kernel(const floa
 #pragma unroll
     for (int u = 0; u < kMergeLoads; u++)
         if (s0 + u < s1) v[u] = __ldcs(reinterpret_cast<const float4*>(src + (s0 + u) * sstride));
-    const float my = tid < num_splits ? lse_part[((long)b * num_splits + tid) * num_heads + h] : -INFINITY;   // num_splits <= 128
+    const float my = tid < num_splits ? lse_part[((long)b * num_splits + tid) * num_heads + h] : -INFINITY;
     float mx = my;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -476,7 +477,7 @@ static int pick_splits(int batch, int num_heads, int max_kv_tiles, int device) {
     int s = (num_sms(device) + groups - 1) / groups;          // one CTA per SM (227 KB of shared memory each)
     const int cap = (max_kv_tiles + 3) / 4;                   // at least 4 tiles (128 tokens) per split
     if (s > cap) s = cap;
-    if (s > 128) s = 128;
+    if (s > kMaxSplits) s = kMaxSplits;
     if (s < 1) s = 1;
     return s;
 }
@@ -488,7 +489,7 @@ static float* g_mla_debug = nullptr;
 extern "C" {
 
 size_t ktb200_mla_workspace_bytes(int batch, int num_heads, int max_splits) {
-    if (max_splits <= 0) max_splits = 128;
+    if (max_splits <= 0) max_splits = ktb::kMaxSplits;
     return (size_t)batch * max_splits * num_heads * (ktb::kDV + 1) * sizeof(float);
 }
 
@@ -499,8 +500,7 @@ static int mla_launch(const ktb::MlaKParams& in, const void* kv_cache, long kv_c
     int dev = 0;
     KTB_CUDA_CHECK(cudaGetDevice(&dev));
     int splits = num_kv_splits > 0 ? num_kv_splits : pick_splits(batch, in.num_heads, max_tiles, dev);
-    if (splits > max_tiles) splits = max_tiles;
-    if (splits < 1) splits = 1;
+    splits = std::max(1, std::min({splits, max_tiles, kMaxSplits}));
     const size_t need = (size_t)batch * splits * in.num_heads * (kDV + 1) * sizeof(float);
     if (need > workspace_bytes) { set_error("mla_decode: workspace too small (%zu < %zu bytes for %d splits)", workspace_bytes, need, splits); return KTB200_EINVAL; }
     cudaStream_t s = (cudaStream_t)stream;

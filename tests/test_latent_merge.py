@@ -8,9 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 # heads that end inside a box (whose other rows are the next sequence's, here not numbers, or lie beyond the last); splits around the ten that a part of the merge loads at once and its
-# four parts; more splits than tiles; a sequence without keys; a page of 32 and of 64
+# four parts; more splits than tiles, and than the merge takes; a sequence without keys; a page of 32 and of 64
 @pytest.mark.parametrize("heads,splits,page,lens", [(16, 1, 64, [33, 700]), (63, 9, 32, [300, 1, 2000]), (100, 10, 64, [4000, 0, 31]), (128, 11, 64, [1500]), (64, 21, 32, [3000, 900]),
-                                                    (130, 40, 64, [5000, 64]), (16, 74, 64, [9000]), (128, 128, 64, [9000, 4097]), (8, 0, 64, [2500, 65, 640])])
+                                                    (130, 40, 64, [5000, 64]), (16, 74, 64, [9000]), (128, 128, 64, [9000, 4097]), (16, 129, 64, [9000]), (16, 200, 32, [20000, 64, 8191]), (8, 0, 64, [2500, 65, 640])])
 def test_queries_and_splits(heads, splits, page, lens):
     from ktransformers_b200 import native
     B, g = len(lens), torch.Generator(device="cuda").manual_seed(heads + splits)
