@@ -217,7 +217,8 @@ typedef struct ktb200_gate_config {
 } ktb200_gate_config;
 /* idx_dev int64 [qlen][top_k] (order: descending biased score, like torch.topk sorted=True — the
  * reference uses sorted=False whose order is unspecified; tests compare as sets), w_dev fp32.
- * logits_dev optional fp32 [qlen][n_experts] scratch/out (NULL -> internal). */
+ * logits_dev optional fp32 [qlen][n_experts] out.  Scratch (qlen x n_experts x up to 8 fp32 values) is taken from the device's stream-ordered pool for
+ * the duration of the call: calls may overlap on several streams, and a captured one keeps memory of its own. */
 int ktb200_moe_gate_forward(const ktb200_gate_config* cfg, int qlen, const void* x_dev, int64_t* idx_dev,
                             float* w_dev, float* logits_dev, const int* bsz_tensor_dev, void* stream);
 /* The same selection on logits [qlen][n_experts] fp32 that the caller computed (one CTA per token: prompt-sized batches). */
@@ -246,8 +247,7 @@ int ktb200_moe_forward_ep(ktb200_moe* moe, ktb200_mlp* shared, int qlen, int k, 
  * token selecting between two barriers of its own, each phase's stream starting behind its barrier.  Any other configuration runs as
  * ktb200_moe_gate_forward + ktb200_moe_forward_shared.  Results are bit-identical between the two.
  * idx_dev int64 [qlen][top_k] and w_dev fp32 [qlen][top_k] receive the routing (as from ktb200_moe_gate_forward).
- * `shared` may be NULL.  Capturable as is (its scratch belongs to the moe handle); when it falls back to the separate
- * launches, ktb200_moe_gate_forward's first-call allocation rule applies.
+ * `shared` may be NULL.  Capturable as is (its scratch belongs to the moe handle; the separate launches' to the call).
  * ------------------------------------------------------------------------------------------ */
 int ktb200_moe_block_forward(const ktb200_gate_config* gate, ktb200_moe* moe, ktb200_mlp* shared, int qlen,
                              const void* input_dev, void* output_dev, int64_t* idx_dev, float* w_dev,

@@ -20,7 +20,6 @@ struct GateParams {
     int64_t* idx;
     float* w;
     const int* bsz;
-    unsigned* ticket;
 };
 
 // Column splits of the router GEMV: as many (row, split) units as fit ONE wave of the persistent MoE-block kernel

@@ -1154,7 +1154,7 @@ extern "C" int ktb200_moe_block_forward(const ktb200_gate_config* gc, ktb200_moe
     const int S = gate_splits(gc->n_experts, gc->hidden_size, num_sms(dev));
     p.g = GateParams{gc->weight, input, gc->hidden_type, gc->n_experts, gc->hidden_size, qlen, S, k, gc->n_group, gc->topk_group,
                      gc->scoring, gc->topk_method, gc->norm_topk_prob, gc->routed_scaling_factor, gc->bias, m->blk_partial, nullptr,
-                     idx, w, bsz, nullptr};
+                     idx, w, bsz};
     MoeRowsPlan many;
     const bool all_at_once = qlen > 1 && moe_rows_plan(m, sh, qlen, k, idx, w, input, output, bsz, &many);
     if (all_at_once) {
@@ -1289,7 +1289,7 @@ extern "C" int ktb200_moe_ep_block_forward(const ktb200_gate_config* gc, ktb200_
     const int S = gate_splits(gc->n_experts, gc->hidden_size, num_sms(dev));
     p.g = GateParams{gc->weight, x_own, gc->hidden_type, gc->n_experts, gc->hidden_size, 1, S, k, gc->n_group, gc->topk_group,
                      gc->scoring, gc->topk_method, gc->norm_topk_prob, gc->routed_scaling_factor, gc->bias, m->blk_partial, nullptr,
-                     idx, w, nullptr, nullptr};
+                     idx, w, nullptr};
     p.w_gate = c.gate_proj; p.w_up = c.up_proj; p.w_down = c.down_proj;
     p.s_gate = sh ? sh->gate : nullptr; p.s_up = sh ? sh->up : nullptr; p.s_down = sh ? sh->down : nullptr;
     p.n_local = c.expert_num; p.id_offset = c.expert_id_offset;

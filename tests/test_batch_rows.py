@@ -37,7 +37,37 @@ def test_router_batches(T, E, H, hid, shift):
     live = call(0, T, torch.tensor([T - 3], dtype=torch.int32, device="cuda"))
     assert torch.equal(live[0][:T - 3], got[0][:T - 3]) and (live[0][T - 3:] == -1).all()
     none = call(0, T, torch.zeros(1, dtype=torch.int32, device="cuda"))
-    assert (none[0] == -1).all() and torch.equal(call(0, T)[0], got[0])        # (the tickets are back at zero)
+    assert (none[0] == -1).all() and torch.equal(call(0, T)[0], got[0])
+
+
+# a captured call keeps its scratch whatever is called after it, and calls that overlap on two streams share none: the bits of calls one by one
+def test_router_calls_share_nothing():
+    from ktransformers_b200 import native
+    E, H, k, big, lib = 256, 2048, 8, 4096, native.lib()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, W, bias = (torch.randn(s, generator=g, device="cuda") for s in ((big, H), (E, H), (E,)))
+    W *= H ** -0.5
+    cfg = native.GateConfig(E, H, k, 8, 4, 0, 0, 1, 2.5, W.data_ptr(), bias.data_ptr(), F32)
+    outs = lambda n: (torch.full((n, k), -1, dtype=torch.int64, device="cuda"), torch.zeros((n, k), device="cuda"))
+    run = lambda lo, n, o: native.check(lib.ktb200_moe_gate_forward(C.byref(cfg), n, x[lo:].data_ptr(), o[0].data_ptr(), o[1].data_ptr(), None, None, _stream()))
+    few, graph = outs(5), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(7, 5, few)
+    whole = outs(big)
+    run(0, big, whole)
+    graph.replay()
+    for a, b in zip(few, whole):
+        assert torch.equal(a, b[7:12])
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], []
+    torch.cuda.synchronize()
+    for i in range(200):
+        with torch.cuda.stream(streams[i & 1]):
+            got.append((i, outs(24)))
+            run(16 * i, 24, got[-1][1])
+    torch.cuda.synchronize()
+    for i, o in got:
+        for a, b in zip(o, whole):
+            assert torch.equal(a, b[16 * i:16 * i + 24])
 
 
 # heads of 64, 128 and 256 columns in both types and layouts, every norm, part of the columns and none turned, one token and many (blocks of units, and fewer units than
