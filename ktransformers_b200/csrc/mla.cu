@@ -16,11 +16,14 @@
 // 512 columns are the MN-major A operand [latent x tokens] (the swizzle is a function of the shared-memory address only).
 // The output is accumulated TRANSPOSED — O^T[latent 512][head 64] = 4 blocks of 128 TMEM lanes x 64 columns — because a
 // [head][latent] accumulator for 64 heads would need 512 columns in the M=64 tcgen05 layout (half the lanes idle): the
-// whole tensor memory.  TMEM map (512 columns allocated): [0,256) O^T, [256,288) / [288,320) the two S buffers.  A 64 x N x 16 product takes 34 cycles for every N up to 64, in one
-// accumulator as in four.
-// What bounds it: 36 + 8 products a tile of 32 tokens, 1,620 of the 1,900 cycles that a tile takes.  B = 1, 128 heads, 131,072 keys: 91 -> 75 us by queries that come by TMA while the first
-// tiles do (setup 6.6 -> 2.3 us), scores in one accumulator, one election for four products, and a merge in four parts.  Tiles of 64 tokens (half the cycles for scores) took 79-118 us: two
-// stages of them fill the shared memory, a stage comes back only behind the tile's values, and copies and products then share the shared memory's port (120 of 128 B a cycle).
+// whole tensor memory.  TMEM map (512 columns allocated): [0,256) O^T, [256,384) / [384,512) the two S buffers, each FOUR partial accumulators of 32 columns.  The products of
+// one accumulator's 36 steps drop what does not fit at each of them: scores of a 2-norm error of 5.3e-7 (log-sum-exp up to 2.9e-6 off), in four sums of nine steps added up in fp32 1.35e-7
+// (1.6e-6).
+// What bounds it: 36 + 8 products a tile of 32 tokens (a 64 x N x 16 product takes 34 cycles for every N up to 64, in one accumulator as in four).  B = 1, 128 heads, 131,072 keys, calls one
+// behind the other: 91 us with Q through registers and the merge in one part; with Q by TMA while the first tiles come (setup 4.8 -> 2.1 us), one election for four products and a merge in four
+// parts 88; with the four sums read by rows in one load of 16 lanes x 128 columns, instead of 4 loads of 32 lanes of which half hold nothing, 78 (4 loads of 16 x 32: 80; one
+// accumulator: 72).  Tiles of 64 tokens (half the cycles for scores) took 79-118 us: two stages of them fill the shared memory, a stage comes back only behind the tile's values, and copies
+// and products then share the shared memory's port (120 of 128 B a cycle).
 //
 // Online softmax with a LAZY reference maximum: p = 2^(x - m_ref), m_ref is only raised (and O^T rescaled in TMEM, all
 // four warps) when some head's running maximum exceeds it by more than 8 — p stays <= 256, exact in bf16/fp32 terms —
@@ -52,6 +55,8 @@ constexpr int kPBytes = kHG * kLT * 2;             // 4,096: [8 head groups][4 t
 constexpr int kOffMiscMax = kMaxStages * kStageBytes + kQBytes + 2 * kPBytes;   // 229,376 (P is double-buffered)
 constexpr int kTmemCols = 512;
 constexpr int kColO = 0, kColS = 256;
+constexpr int kSChains = 4;          // partial-score accumulators per S buffer (read together, kSChains * kLT columns)
+static_assert(kSChains * kLT == 128, "tmem_ld64_rows");
 constexpr float kRescaleThreshold = 8.f;
 constexpr int kMaxSplits = 128;          // of a sequence's keys: the merge has a thread and a weight for each
 
@@ -211,7 +216,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
                 const uint32_t kb = base + s * kStageBytes, qb = base + kOffQ;
 #pragma unroll
                 for (int c = 0; c < kChunks; c++)
-                    mma_f16_x4(tmem + kColS + buf * kLT, smem_desc(qb + c * kQRegion, 16, 1024, kLayoutSw128), smem_desc(kb + c * kKRegion, 16, 1024, kLayoutSw128), idesc_qk, c != 0,
+                    mma_f16_x4<2, 2, kLT>(tmem + kColS + buf * kSChains * kLT, smem_desc(qb + c * kQRegion, 16, 1024, kLayoutSw128), smem_desc(kb + c * kKRegion, 16, 1024, kLayoutSw128), idesc_qk, c != 0,
                                c == kChunks - 1 ? smem_u32(&misc.s_full[buf]) : 0);
             };
             bar_wait(smem_u32(&misc.q_full), 0);
@@ -240,44 +245,46 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         __syncwarp();
     } else {
         // ================================================================ softmax / rescale / epilogue (4 warps)
-        // S rows of a sub-partition live in its TMEM lanes 0..15 (M = 64 layout): lane l < 16 loads the 32 scores of head
-        // 16 sp + l and hands tokens 16..31 to lane l + 16, so that all 32 lanes work: lane = (head, half of the tile).
+        // S rows of a sub-partition live in its TMEM lanes 0..15 (M = 64 layout).  A thread loads columns 8 i + 2 (lane % 4) + {0, 1} of two of them, heads 16 sp + lane / 4 and 8
+        // more, of every partial accumulator: a row's maximum takes two shuffles, and the probabilities lie where their pairs are stored
         const int sp = warp & 3;                       // TMEM sub-partition of this warp
         const uint32_t lane_base = (uint32_t)(32 * sp) << 16;
-        const int upper = lane >> 4;
-        const int head = 16 * sp + (lane & 15);
+        const int head = 16 * sp + (lane >> 2), pair = 2 * (lane & 3);
         const int st = tid - 64;                       // 0..127 among the softmax threads
-        float m_ref = -INFINITY, m_run = -INFINITY, l = 0.f;   // l: this lane's half of the row sum
+        float m_ref[2] = {-INFINITY, -INFINITY}, m_run[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // l: this thread's quarter of the row sum
         for (int j = 0; j < n; j++) {
             const int buf = j & 1;
             bar_wait(smem_u32(&misc.s_full[buf]), (j >> 1) & 1);
             tc_fence_after();
             if (p.debug && st == 0 && split == 0 && hg == 0 && b == 0 && j < 60) reinterpret_cast<unsigned long long*>(p.debug + 2048)[64 + j] = gtime();
-            uint32_t sv[32];
-            tmem_ld32(tmem + lane_base + kColS + buf * kLT, sv);
+            uint32_t sv[2 * kLT];      // [partial accumulator][16]
+            tmem_ld64_rows(tmem + lane_base + kColS + buf * kSChains * kLT, sv);
             tmem_wait_ld();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) bar_arrive(smem_u32(&misc.s_empty[buf]));
-            if (p.debug && j == 0 && !upper && split == 0 && hg == 0 && b == 0)
-                for (int i = 0; i < 32; i++) p.debug[head * 32 + i] = __uint_as_float(sv[i]);
-            const int t_base = (tile0 + j) * kLT + 16 * upper;
-            float x[16];
-            float mt = -INFINITY;
+            const int t_base = (tile0 + j) * kLT + pair;
+            float x[4][2][2];      // [eight tokens][row][token of the pair]
+            float mt[2] = {-INFINITY, -INFINITY};
 #pragma unroll
             for (int i = 0; i < 16; i++) {
-                const uint32_t hi = __shfl_sync(0xffffffffu, sv[16 + i], lane & 15);
-                const float v = __uint_as_float(upper ? hi : sv[i]);
-                x[i] = (t_base + i < L && t_base + i >= L0) ? v * p.scale_log2 : -INFINITY;
-                mt = fmaxf(mt, x[i]);
+                const int t = t_base + 8 * (i >> 2) + (i & 1), r = (i >> 1) & 1;
+                const float v = (__uint_as_float(sv[i]) + __uint_as_float(sv[16 + i])) + (__uint_as_float(sv[32 + i]) + __uint_as_float(sv[48 + i]));
+                if (p.debug && j == 0 && split == 0 && hg == 0 && b == 0) p.debug[(head + 8 * r) * 32 + t - t_base + pair] = v;
+                x[i >> 2][r][i & 1] = (t < L && t >= L0) ? v * p.scale_log2 : -INFINITY;
+                mt[r] = fmaxf(mt[r], x[i >> 2][r][i & 1]);
             }
-            mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 16));
-            m_run = fmaxf(m_run, mt);
             // does any head need its reference raised?  (never on the first tile: O^T is overwritten by the first PV)
-            bool need = false;
-            if (j == 0) m_ref = m_run;
-            else need = m_run - m_ref > kRescaleThreshold;
-            const unsigned any_w = __ballot_sync(0xffffffffu, need);
+            bool need[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                mt[r] = fmaxf(mt[r], __shfl_xor_sync(0xffffffffu, mt[r], 1));
+                mt[r] = fmaxf(mt[r], __shfl_xor_sync(0xffffffffu, mt[r], 2));
+                m_run[r] = fmaxf(m_run[r], mt[r]);
+                if (j == 0) m_ref[r] = m_run[r];
+                need[r] = j != 0 && m_run[r] - m_ref[r] > kRescaleThreshold;
+            }
+            const unsigned any_w = __ballot_sync(0xffffffffu, need[0] || need[1]);
             if (lane == 0) misc.need[buf][warp - 2] = any_w != 0;
             asm volatile("bar.sync 1, 128;" ::: "memory");
             const bool any = misc.need[buf][0] | misc.need[buf][1] | misc.need[buf][2] | misc.need[buf][3];
@@ -285,9 +292,12 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
                 // O^T must be quiescent: the previous PV has to be complete (it also frees the other P buffer)
                 bar_wait(smem_u32(&misc.p_free[(j - 1) & 1]), ((j - 1) >> 1) & 1);
                 tc_fence_after();
-                const float a = need ? ex2(m_ref - m_run) : 1.f;
-                if (!upper) misc.alpha[head] = a;
-                if (need) { l *= a; m_ref = m_run; }
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const float a = need[r] ? ex2(m_ref[r] - m_run[r]) : 1.f;
+                    if (pair == 0) misc.alpha[head + 8 * r] = a;
+                    if (need[r]) { l[r] *= a; m_ref[r] = m_run[r]; }
+                }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll 1
                 for (int q = 0; q < 8; q++) {   // 4 latent blocks x 2 halves of the 64 head columns
@@ -306,24 +316,21 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             // this tile's P buffer was last read by PV(j - 2)
             if (j >= 2) bar_wait(smem_u32(&misc.p_free[buf]), ((j >> 1) & 1) ^ 1);
             {
-                float ps = 0.f;
-                uint32_t pk[8], pl[8];
-#pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    const float p0 = ex2(x[i] - m_ref), p1 = ex2(x[i + 1] - m_ref);
-                    ps += p0 + p1;
-                    pk[i >> 1] = pack_bf16(p0, p1);
-                    if (SPLITP)   // what bf16 rounding dropped (exact in fp32), as a second bf16 term
-                        pl[i >> 1] = pack_bf16(p0 - __uint_as_float(pk[i >> 1] << 16), p1 - __uint_as_float(pk[i >> 1] & 0xffff0000u));
-                }
-                l += ps;
                 // P[head][token] as the K-major no-swizzle B operand: core matrix (8 heads x 8 tokens) = 128 contiguous bytes
-                uint8_t* pdst = smem + kOffP + buf * kPStride + (head >> 3) * 512 + (head & 7) * 16 + upper * 256;
-                *reinterpret_cast<uint4*>(pdst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *reinterpret_cast<uint4*>(pdst + 128) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                if (SPLITP) {
-                    *reinterpret_cast<uint4*>(pdst + kPBytes) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-                    *reinterpret_cast<uint4*>(pdst + kPBytes + 128) = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+                uint8_t* pdst = smem + kOffP + buf * kPStride + (head >> 3) * 512 + (head & 7) * 16 + 2 * pair;
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    float ps = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float p0 = ex2(x[i][r][0] - m_ref[r]), p1 = ex2(x[i][r][1] - m_ref[r]);
+                        ps += p0 + p1;
+                        const uint32_t pk = pack_bf16(p0, p1);
+                        *reinterpret_cast<uint32_t*>(pdst + r * 512 + i * 128) = pk;
+                        if (SPLITP)   // what bf16 rounding dropped (exact in fp32), as a second bf16 term
+                            *reinterpret_cast<uint32_t*>(pdst + kPBytes + r * 512 + i * 128) = pack_bf16(p0 - __uint_as_float(pk << 16), p1 - __uint_as_float(pk & 0xffff0000u));
+                    }
+                    l[r] += ps;
                 }
             }
             // rows of the tile beyond kv_len hold whatever the page contains: P is 0 there, but 0 * NaN is NaN -> zero the V rows
@@ -345,8 +352,12 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             }
         }
         // ---- epilogue: O^T / l -> fp32 partial output, base-2 LSE ---------------------------------------------------
-        l += __shfl_xor_sync(0xffffffffu, l, 16);
-        if (!upper) { misc.l[head] = l; misc.m[head] = m_ref; }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+            l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+            if (pair == 0) { misc.l[head + 8 * r] = l[r]; misc.m[head + 8 * r] = m_ref[r]; }
+        }
         bar_wait(smem_u32(&misc.p_free[(n - 1) & 1]), ((n - 1) >> 1) & 1);   // the last PV (and with it every earlier one) is complete
         tc_fence_after();
         asm volatile("bar.sync 1, 128;" ::: "memory");

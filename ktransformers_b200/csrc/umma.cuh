@@ -115,6 +115,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
+// 16 lanes x 128 columns (the lanes of an M = 64 accumulator that a warp has): thread t gets rows t / 4 (registers 4 i, 4 i + 1) and t / 4 + 8 (4 i + 2, 4 i + 3), columns
+// 8 i + 2 (t % 4) + {0, 1}
+__device__ __forceinline__ void tmem_ld64_rows(uint32_t taddr, uint32_t (&r)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
+        "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
+        "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
+          "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+          "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
+          "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+          "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]),
@@ -238,36 +257,39 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 }
 
 // Four products on consecutive K-steps, whose operands lie DA and DB units of 16 bytes apart (2: a 128-byte swizzled row's steps of 32 bytes), and the barriers that complete when
-// all products so far have (0: not asked for), in one election
+// all products so far have (0: not asked for), in one election.  DD: TMEM columns from one product's accumulator to the next one's (0: one for all four)
 #define KTB_MMA_SS4(KIND)                                                                             \
     asm volatile(                                                                                     \
         "{\n"                                                                                        \
         ".reg .pred p, q, t, c, e;\n"                                                                \
-        ".reg .b32 r;\n"                                                                             \
+        ".reg .b32 r, d;\n"                                                                          \
         ".reg .b64 a, b;\n"                                                                          \
         "elect.sync r|q, 0xffffffff;\n"                                                              \
         "setp.ne.b32 p, %4, 0;\n"                                                                    \
-        "setp.eq.b32 t, 0, 0;\n"                                                                     \
+        "setp.eq.or.b32 t, %9, 0, p;\n"                                                              \
         "setp.ne.and.b32 c, %5, 0, q;\n"                                                             \
         "setp.ne.and.b32 e, %6, 0, q;\n"                                                             \
         "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, p;\n"                          \
         "add.u64 a, %1, %7;\n"                                                                       \
         "add.u64 b, %2, %8;\n"                                                                       \
-        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], a, b, %3, t;\n"                            \
+        "add.u32 d, %0, %9;\n"                                                                       \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [d], a, b, %3, t;\n"                             \
         "add.u64 a, a, %7;\n"                                                                        \
         "add.u64 b, b, %8;\n"                                                                        \
-        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], a, b, %3, t;\n"                            \
+        "add.u32 d, d, %9;\n"                                                                        \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [d], a, b, %3, t;\n"                             \
         "add.u64 a, a, %7;\n"                                                                        \
         "add.u64 b, b, %8;\n"                                                                        \
-        "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], a, b, %3, t;\n"                            \
+        "add.u32 d, d, %9;\n"                                                                        \
+        "@q tcgen05.mma.cta_group::1.kind::" KIND " [d], a, b, %3, t;\n"                             \
         "@c tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n"           \
         "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n"           \
         "}\n" ::"r"(tmem_d),                                                                         \
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1), "n"(DA), "n"(DB) \
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(bar0), "r"(bar1), "n"(DA), "n"(DB), "n"(DD) \
         : "memory")
-template <int DA = 2, int DB = 2>
+template <int DA = 2, int DB = 2, int DD = 0>
 __device__ __forceinline__ void mma_f8_x4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t bar0 = 0, uint32_t bar1 = 0) { KTB_MMA_SS4("f8f6f4"); }
-template <int DA = 2, int DB = 2>
+template <int DA = 2, int DB = 2, int DD = 0>
 __device__ __forceinline__ void mma_f16_x4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t bar0 = 0, uint32_t bar1 = 0) { KTB_MMA_SS4("f16"); }
 #undef KTB_MMA_SS4
 

@@ -44,3 +44,18 @@ def test_queries_and_splits(heads, splits, page, lens):
         # probabilities reach the product as bf16 (2^-9 of each) and the result is rounded to bf16
         assert ((out[b].double() - want).norm() / want.norm()).item() < 4e-3
         assert (lse[b].double() - torch.logsumexp(s, -1)).abs().max() < 1e-3
+
+
+# Scores are sums of 36 products of 16 columns in the tensor core's accumulators, which drop what does not fit at every step: 1.35e-7 (2-norm) in four sums of nine steps that are
+# added up in fp32, 5.3e-7 in one of 36.  With one key a head the log-sum-exp is the score (times log2 e and back: three more roundings of 2^-25 on average)
+def test_scores_are_four_sums():
+    from ktransformers_b200 import native
+    B, heads, g, lib = 64, 64, torch.Generator(device="cuda").manual_seed(3), native.lib()
+    q, pe, kv = (torch.randn(s, generator=g, device="cuda").bfloat16() for s in ((B, heads, 512), (B, heads, 64), (B, 64, 576)))
+    table, kv_len = torch.arange(B, dtype=torch.int32, device="cuda").view(B, 1), torch.ones(B, dtype=torch.int32, device="cuda")
+    out, lse, need = torch.zeros_like(q), torch.zeros((B, heads), device="cuda"), lib.ktb200_mla_workspace_bytes(B, heads, 0)
+    work = torch.zeros(need // 4, device="cuda")
+    p = native.MlaParams(B, heads, 64, 1, 1, 1.0, q.data_ptr(), pe.data_ptr(), kv.data_ptr(), table.data_ptr(), kv_len.data_ptr(), out.data_ptr(), lse.data_ptr(), work.data_ptr(), need)
+    native.check(lib.ktb200_mla_decode(C.byref(p), torch.cuda.current_stream().cuda_stream))
+    want = (torch.cat([q, pe], -1).double() @ kv[:, 0].double()[:, :, None])[..., 0]
+    assert ((lse.double() - want).norm() / want.norm()).item() < 2.5e-7
