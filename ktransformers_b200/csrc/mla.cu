@@ -61,7 +61,7 @@ constexpr float kRescaleThreshold = 8.f;
 constexpr int kMaxSplits = 128;          // of a sequence's keys: the merge has a thread and a weight for each
 
 struct MlaMisc {
-    unsigned long long q_full, k_full[kMaxStages], k_empty[kMaxStages], s_full[2], s_empty[2], p_full, p_free[2];
+    unsigned long long q_full, k_full[kMaxStages], k_empty[kMaxStages], s_full[2], s_empty[2], p_full[2], p_free[2];
     uint32_t tmem_base;
     int need[2][4];
     float alpha[kHG];     // per head: 2^(m_ref_old - m_ref_new) of the current rescale
@@ -154,9 +154,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
         bar_init(smem_u32(&misc.q_full), 1);
         for (int s = 0; s < kStages; s++) { bar_init(smem_u32(&misc.k_full[s]), 1); bar_init(smem_u32(&misc.k_empty[s]), 1); }
         for (int s = 0; s < 2; s++) { bar_init(smem_u32(&misc.s_full[s]), 1); bar_init(smem_u32(&misc.s_empty[s]), 4); }
-        bar_init(smem_u32(&misc.p_full), 4);
-        bar_init(smem_u32(&misc.p_free[0]), 1);
-        bar_init(smem_u32(&misc.p_free[1]), 1);
+        for (int s = 0; s < 2; s++) { bar_init(smem_u32(&misc.p_full[s]), 4); bar_init(smem_u32(&misc.p_free[s]), 1); }
         bar_fence_init();
         // the first tiles do not depend on anything set up below: request them now
         // (Q, 64 heads x 576, into the K-major 128-byte-swizzle layout: a region of 64 rows of 128 B per 64 columns.  Rows beyond the last head are other sequences' or zeros, and
@@ -223,7 +221,8 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             issue_qk(0);
             for (int j = 0; j < n; j++) {
                 if (j + 1 < n) issue_qk(j + 1);
-                bar_wait(smem_u32(&misc.p_full), j & 1);
+                // (a barrier a buffer: P of the next tile may be ready before this warp looks here, and a wait that finds two phases of one barrier completed sees neither)
+                bar_wait(smem_u32(&misc.p_full[j & 1]), (j >> 1) & 1);
                 tc_fence_after();
                 const int s = j % kStages;
                 const uint32_t kb = base + s * kStageBytes, pb = base + kOffP + (j & 1) * kPStride;
@@ -344,7 +343,7 @@ __global__ void __launch_bounds__(kMlaThreads, 1) mla_decode_tc_kernel(const __g
             }
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) bar_arrive(smem_u32(&misc.p_full));
+            if (lane == 0) bar_arrive(smem_u32(&misc.p_full[buf]));
             if (p.debug && st == 0 && split == 0 && hg == 0 && b == 0 && j < 60) {
                 unsigned long long t;
                 asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
