@@ -46,12 +46,12 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
-// bounded wait for a phase of an mbarrier: gives up after kMbarWaitLimit polls (seconds), counts that in g_mbar_wait_gave_up and
-// returns, so that a copy that never completes ends the kernel (with wrong results) instead of holding the GPU
-constexpr uint32_t kMbarWaitLimit = 1u << 24;
+// bounded wait for a phase of an mbarrier: gives up after kMbarWaitLimit polls (a second), counts that in g_mbar_wait_gave_up and
+// returns, so that a copy that never completes ends the kernel (with wrong results) instead of holding the GPU.  Once one has, the others end after kMbarWaitShort polls (16 ms)
+constexpr uint32_t kMbarWaitLimit = 1u << 21, kMbarWaitShort = 1u << 15;
 static __device__ unsigned int g_mbar_wait_gave_up;
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kMbarWaitLimit; it++) {
+    for (uint32_t it = 1; it <= kMbarWaitLimit; it++) {
         uint32_t done;
         asm volatile(
             "{\n"
@@ -63,6 +63,7 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return;
+        if (it % kMbarWaitShort == 0 && *(volatile unsigned int*)&g_mbar_wait_gave_up) break;
     }
     atomicAdd(&g_mbar_wait_gave_up, 1u);
 }

@@ -28,13 +28,13 @@ __device__ __forceinline__ void bar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // Waits until the phase with the given parity has completed (a fresh barrier passes parity 1 at once).  The wait is bounded:
-// after kBarWaitLimit polls (each poll suspends the thread for a hardware-defined while; seconds in all) it gives up, counts the
+// after kBarWaitLimit polls (half a microsecond each where nothing happens, a second in all) it gives up, counts the
 // event in g_bar_wait_gave_up and returns false, so a kernel whose copy or MMA never arrives still ends (with wrong results)
-// instead of occupying the GPU for good.
-constexpr uint32_t kBarWaitLimit = 1u << 24;
+// instead of occupying the GPU for good.  Once one has, the others end after kBarWaitShort polls (16 ms): a kernel has thousands.
+constexpr uint32_t kBarWaitLimit = 1u << 21, kBarWaitShort = 1u << 15;
 static __device__ unsigned int g_bar_wait_gave_up;
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kBarWaitLimit; it++) {
+    for (uint32_t it = 1; it <= kBarWaitLimit; it++) {
         uint32_t done;
         asm volatile(
             "{\n"
@@ -46,6 +46,7 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
             : "r"(bar), "r"(parity)
             : "memory");
         if (done) return true;
+        if (it % kBarWaitShort == 0 && *(volatile unsigned int*)&g_bar_wait_gave_up) break;
     }
     atomicAdd(&g_bar_wait_gave_up, 1u);
     return false;
