@@ -123,6 +123,24 @@ def test_fp8_batches_wherever_results_go(T, K, N, hid):
     lib.ktb200_fp8_linear_destroy(h)
 
 
+# fp32 results of up to 16 rows: the error against 64 bits is that of sums of four blocks of K (one chain of 12 and 16 blocks: 9.5e-8 to 9.9e-8 and 1.01e-7 to 1.05e-7)
+@pytest.mark.parametrize("K,N,most", [(1536, 24576, 9.25e-8), (2048, 20480, 9.5e-8)])
+@pytest.mark.parametrize("T", [1, 3, 16])
+def test_fp8_rows_in_fp32(T, K, N, most):
+    from ktransformers_b200 import native
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = (torch.randn((N, K), generator=g, device="cuda") * 60).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    ws, x = (torch.rand(((N + 127) // 128, K // 128), generator=g, device="cuda") * 0.6 + 0.7) / 5000, torch.randn((T, K), generator=g, device="cuda")
+    y, lib, h = torch.zeros((T, N), device="cuda"), native.lib(), C.c_void_p()
+    native.check(lib.ktb200_fp8_linear_create(K, N, w.data_ptr(), ws.data_ptr(), F32, 0, C.byref(h)))
+    native.check(lib.ktb200_fp8_linear_forward(h, T, x.data_ptr(), y.data_ptr(), None, _stream()))
+    f = x.view(T, -1, 128)
+    s = f.abs().amax(-1, keepdim=True) / 448.0
+    want = ((f / s).to(torch.float8_e4m3fn).double() * s.double()).view(T, K) @ (w.float().double() * ws.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)).T
+    assert ((y.double() - want).norm() / want.norm()).item() < most
+    lib.ktb200_fp8_linear_destroy(h)
+
+
 # linears of two to eight rows on either side of the line between the row kernels and the GEMM: one row at a time gives the same sums in another order (half a place of the result and
 # 4e-6 of the largest), and the launches tell which one ran
 @pytest.mark.parametrize("type,K,R,T,hid,launches", [(12, 16384, 7168, 8, BF16, 1), (14, 7168, 18432, 2, BF16, 3), (14, 7168, 18432, 1, BF16, 1), (14, 7168, 18432, 8, F32, 1), (14, 2048, 2048, 8, BF16, 1),
