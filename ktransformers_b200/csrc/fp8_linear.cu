@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
 }  // namespace ktb
 
 struct ktb200_fp8_linear {
-    int K, N, hidden_type, device, nkb, row_tiles, ksplit, kb_per_split;
+    int K, N, hidden_type, device, nkb, row_tiles, kb_per_split, kb_many;      // (kb_many: for kFp8Many and more rows)
     const void* w;
     const float* scale_inv;
     CUtensorMap map;
@@ -465,7 +465,42 @@ struct ktb200_fp8_linear {
 };
 
 namespace ktb {
-constexpr int kFp8Round = 8;      // what a CTA of the pass kernel costs beside its blocks, in blocks: set-up, quantisation, the atomics of its sums
+// Blocks of K a CTA of the pass kernel takes: at most kFMaxKb, at least as many as fill its ring, and of these the number whose CTAs, two an SM, take least one after the other; kFp8Round is what
+// a CTA costs beside its blocks, in blocks: set-up, quantisation, the atomics of its sums.  Against as many splits as give four CTAs an SM (us, weights from memory, one and 16 rows):
+// 1536 -> 24576 16.3 -> 10.9, 35 -> 20 (no splits, no atomics); 7168 -> 4096 13.7 -> 10.4, 28 -> 23; 10240 -> 14000 39.5 -> 35.5, 68 -> 60; 16384 -> 7168 33.3 -> 32.0, 56 -> 52; matrices of
+// few tiles as before.
+// From kFp8Many rows on, where the CTAs do not run all at once, a block takes longer (kFp8RoundMany) and the last split's CTAs, which have what is left of K, fill the gaps: the least time of
+// CTAs taken in order by whichever place is free.  16 rows: 18432 -> 7168 54.9 -> 52.6, 4224 -> 12864 37.1 -> 32.4, 5120 -> 19456 51.7 -> 49.1, 9728 -> 11136 50.0 -> 47.7, 7680 -> 19904
+// 66.8 -> 68.4; at 9 rows as often slower as faster.
+constexpr int kFp8Round = 8, kFp8RoundMany = 4, kFp8Many = 12;
+static long fp8_span(int tiles, int nkb, int kb, int places) {
+    const int splits = (nkb + kb - 1) / kb, full = tiles * (splits - 1), whole = full / places, rest = full % places;
+    const long c = kb + kFp8RoundMany, d = nkb - kb * (splits - 1) + kFp8RoundMany;      // a whole CTA, one of the last split
+    long at[2] = {whole * c, (whole + 1) * c}, end = at[rest > 0];
+    const int free[2] = {places - rest, rest};
+    for (int left = tiles; left > 0;) {
+        const int i = free[1] > 0 && at[1] < at[0];
+        at[i] += d;
+        left -= free[i];
+        end = std::max(end, at[i]);
+    }
+    return end;
+}
+static int fp8_blocks(int tiles, int nkb, int places, bool many) {
+    int best = std::min(nkb, 4);
+    long least = LONG_MAX;
+    for (int kb = best; kb <= std::min(nkb, kFMaxKb); kb++) {
+        const long cost = (long)((tiles * ((nkb + kb - 1) / kb) + places - 1) / places) * (kb + kFp8Round);
+        if (cost < least) { least = cost; best = kb; }
+    }
+    if (!many || best == nkb || tiles * ((nkb + best - 1) / best) <= places) return best;      // (one split needs no atomics)
+    least = LONG_MAX;
+    for (int kb = std::min(nkb, 4); kb <= std::min(nkb, kFMaxKb); kb++) {
+        const long cost = fp8_span(tiles, nkb, kb, places);
+        if (cost < least) { least = cost; best = kb; }
+    }
+    return best;
+}
 // Whether a batch of more than kFT tokens is still faster in passes of kFT.  The GEMM has no K splits, so a matrix of few rows is one serial chain of
 // K / 128 steps a tile: measured 10 us + 0.48 us a step and round of tiles (7168 -> 576: 35-39 us, 16384 -> 64: 76, 18432 -> 1536: 75); a pass takes 17.5 us
 // + 1 us per 2.9 MB of weights, a last one of a few tokens less (7168 -> 576: 28 us at 17 tokens, 36 at 24, 40 at 32, 58 at 48).
@@ -544,17 +579,9 @@ int ktb200_fp8_linear_create(int in_features, int out_features, const void* weig
     if (!l) return KTB200_ENOMEM;
     l->K = in_features; l->N = out_features; l->hidden_type = hidden_type; l->device = device; l->w = weight_e4m3; l->scale_inv = weight_scale_inv;
     l->nkb = in_features / 128; l->row_tiles = (out_features + 127) / 128;
-    // K splits: at most kFMaxKb blocks of B per CTA, at least as many as fill its ring, and of these the number whose CTAs, two an SM, take least one after the other.  Against as many
-    // splits as give four CTAs an SM (us, one and 16 rows): 1536 -> 24576 16.3 -> 11.2, 37 -> 21 (no splits, no atomics); 7168 -> 4096 13.5 -> 10.4, 29 -> 25; 10240 -> 14000 40.6 -> 36.1,
-    // 70 -> 63; 16384 -> 7168 34.3 -> 33.2, 60 -> 56; 18432 -> 7168 35.0 -> 34.7, 57 -> 60; matrices of few tiles as before
-    const int two = 2 * num_sms(device);
-    l->kb_per_split = std::min(l->nkb, 4);
-    long least = LONG_MAX;
-    for (int kb = std::min(l->nkb, 4); kb <= std::min(l->nkb, kFMaxKb); kb++) {
-        const long cost = (long)((l->row_tiles * ((l->nkb + kb - 1) / kb) + two - 1) / two) * (kb + kFp8Round);
-        if (cost < least) { least = cost; l->kb_per_split = kb; }
-    }
-    l->ksplit = (l->nkb + l->kb_per_split - 1) / l->kb_per_split;
+    const int places = 2 * num_sms(device);
+    l->kb_per_split = fp8_blocks(l->row_tiles, l->nkb, places, false);
+    l->kb_many = fp8_blocks(l->row_tiles, l->nkb, places, true);
     const cuuint64_t gdim[2] = {(cuuint64_t)in_features, (cuuint64_t)out_features};
     const cuuint64_t gstr[1] = {(cuuint64_t)in_features};
     const cuuint32_t box[2] = {128, 128}, estr[2] = {1, 1};
@@ -597,14 +624,14 @@ int ktb200_fp8_linear_forward(ktb200_fp8_linear* l, int qlen, const void* x, voi
         p.y = reinterpret_cast<uint8_t*>(y) + (size_t)t0 * l->N * hb;
         p.scale_inv = l->scale_inv; p.ws = l->ws; p.tickets = l->tickets; p.bsz = bsz; p.t0 = t0;
         p.hidden_type = l->hidden_type; p.T = qlen - t0 < kFT ? qlen - t0 : kFT; p.K = l->K; p.N = l->N; p.nkb = l->nkb;
-        p.kb_per_split = l->kb_per_split; p.ksplit = l->ksplit;
+        p.kb_per_split = p.T < kFp8Many ? l->kb_per_split : l->kb_many; p.ksplit = (l->nkb + p.kb_per_split - 1) / p.kb_per_split;
         if (p.T > 2) {   // quantise once, then the GEMM as a programmatic dependent launch: its weight boxes stream while the quantiser drains
             p.xq = l->xq; p.xs = l->xs;
             fp8_act_quant_kernel<<<(p.T * l->nkb + 7) / 8, 256, 0, (cudaStream_t)stream>>>(p.x, l->hidden_type, p.T, l->K, l->xq, l->xs, 0);
-            KTB_CUDA_CHECK(launch_pdl(kernel, dim3(l->row_tiles, l->ksplit), dim3(192), (size_t)kFSmem, (cudaStream_t)stream, l->map, p));
+            KTB_CUDA_CHECK(launch_pdl(kernel, dim3(l->row_tiles, p.ksplit), dim3(192), (size_t)kFSmem, (cudaStream_t)stream, l->map, p));
             count_launch(2);
         } else {
-            KTB_CUDA_CHECK(launch_pdl(kernel, dim3(l->row_tiles, l->ksplit), dim3(192), (size_t)kFSmem, (cudaStream_t)stream, l->map, p));
+            KTB_CUDA_CHECK(launch_pdl(kernel, dim3(l->row_tiles, p.ksplit), dim3(192), (size_t)kFSmem, (cudaStream_t)stream, l->map, p));
             count_launch(1);
         }
     }

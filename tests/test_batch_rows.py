@@ -141,6 +141,25 @@ def test_fp8_rows_in_fp32(T, K, N, most):
     lib.ktb200_fp8_linear_destroy(h)
 
 
+# 12 and more rows split K by the time of CTAs taken in order (11 splits with a short last one for 10; 3 for 5; 2 for 3); 11 rows as one.  The sums are the same up to their order
+@pytest.mark.parametrize("K,N", [(18432, 7168), (4224, 12864), (2944, 19904)])
+@pytest.mark.parametrize("T,hid", [(12, BF16), (16, F16), (16, F32)])
+def test_fp8_rows_in_other_splits(T, K, N, hid):
+    from ktransformers_b200 import native
+    g = torch.Generator(device="cuda").manual_seed(T)
+    w = (torch.randn((N, K), generator=g, device="cuda") * 60).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    ws, x = (torch.rand(((N + 127) // 128, K // 128), generator=g, device="cuda") * 0.6 + 0.7) / 5000, torch.randn((T, K), generator=g, device="cuda").to(TORCH[hid])
+    y, few, lib, h = torch.zeros((T, N), dtype=x.dtype, device="cuda"), torch.zeros((T, N), dtype=x.dtype, device="cuda"), native.lib(), C.c_void_p()
+    native.check(lib.ktb200_fp8_linear_create(K, N, w.data_ptr(), ws.data_ptr(), hid, 0, C.byref(h)))
+    for _ in range(2):      # (the workspace is zero again after a call)
+        native.check(lib.ktb200_fp8_linear_forward(h, T, x.data_ptr(), y.data_ptr(), None, _stream()))
+        for t in range(0, T, 11):
+            native.check(lib.ktb200_fp8_linear_forward(h, min(11, T - t), x[t:].data_ptr(), few[t:].data_ptr(), None, _stream()))
+        a, b = y.double(), few.double()
+        assert ((a - b).abs() <= {BF16: 2.0 ** -7, F16: 2.0 ** -10, F32: 2.0 ** -20}[hid] * b.abs() + 4e-6 * b.abs().max()).all()
+    lib.ktb200_fp8_linear_destroy(h)
+
+
 # linears of two to eight rows on either side of the line between the row kernels and the GEMM: one row at a time gives the same sums in another order (half a place of the result and
 # 4e-6 of the largest), and the launches tell which one ran
 @pytest.mark.parametrize("type,K,R,T,hid,launches", [(12, 16384, 7168, 8, BF16, 1), (14, 7168, 18432, 2, BF16, 3), (14, 7168, 18432, 1, BF16, 1), (14, 7168, 18432, 8, F32, 1), (14, 2048, 2048, 8, BF16, 1),
