@@ -145,7 +145,9 @@ int ktb200_linear_create(int in_size, int out_size, const void* proj_dev, int pr
                          int group_max_len, int device, ktb200_linear** out);
 void ktb200_linear_destroy(ktb200_linear* lin);
 int ktb200_linear_load_weights(ktb200_linear* lin, void* stream);
-/* y[qlen][out] = x[qlen][in] * W^T ; bias_dev optional fp32 [out] added before rounding */
+/* y[qlen][out] = x[qlen][in] * W^T ; bias_dev optional fp32 [out] added before rounding.  Rows of Q4_K, and rows with fp32 results, have the same bits in every call of up to 8; 2 to 8
+ * rows of Q6_K and Q5_K with 16-bit results may differ in their last place from the same rows alone, in a captured call, or where no scratch could be had (their sums are added in
+ * another order there), and so may rows of any type in calls of more than 8. */
 int ktb200_linear_forward(ktb200_linear* lin, int qlen, const void* input_dev, void* output_dev,
                           const float* bias_dev, const int* bsz_tensor_dev, void* stream);
 

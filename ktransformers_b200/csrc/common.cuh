@@ -47,6 +47,7 @@ cudaError_t raise_smem_limit(const void* kernel, size_t bytes);
 // stream-ordered scratch from a bounded pool (runtime.cu); ScratchBlock gives it back behind the work already queued on the stream
 cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out);
 void scratch_prepare(int device);      // when a handle is created: its calls may then be captured from the first on
+bool capturing(cudaStream_t stream);   // (or not to be told, as on the default stream beside another stream's capture)
 constexpr int kNoScratch = 2;          // inside the library: the pool could not give a product's scratch (the error's text is set, nothing is launched)
 struct ScratchBlock {
     void* ptr = nullptr;

@@ -802,15 +802,16 @@ int ktb200_moe_forward_host(ktb200_moe* m, int qlen, int k, const int64_t* ids, 
 // Two to eight rows of Q6_K and Q5_K with 16-bit results (fp32 results stay with the row kernels, whose sums are closer to 64 bits; a Q4_K row has the same bits in every call of up to
 // eight): the register-staged row kernels take a row's sums one after the other.  Measured in graphs (us; MB of weights), row kernels: at least 3 + MB times 0.58 (two rows), 1.05 (three,
 // four), 2 (more);  GEMM: Q6_K 11.8 + 0.32 MB, Q5_K 12 + 0.35 MB.  16384 -> 7168, Q6_K: two rows 72 against 41, three 144, 42, six 262, 42; 7168 -> 18432, Q5_K: two rows 55, 40, five
-// 227, 40; 512 -> 16000, Q6_K: three rows 52, 12.  Its two or three launches cost the host 25 us, so what the row kernels do in less stays.
+// 227, 40; 512 -> 16000, Q6_K: three rows 52, 12.  Its two or three launches cost the host 25 us, so what the row kernels do in less stays.  The row kernels take no scratch: they also
+// run where a call is captured, so that the graph of a decode step holds no memory, and where the pool has none.
 static bool few_rows_as_gemm(KqFmt f, int R, int K, int T) {
     const double mb = (double)R * K / QK_K * 1e-6 * (f == KQ_Q5K ? SZ_Q5_K : SZ_Q6_K);
     const double rows = 3.0 + mb * (T == 2 ? 0.58 : T <= 4 ? 1.05 : 2.0), gemm = f == KQ_Q5K ? 12.0 + 0.35 * mb : 11.8 + 0.32 * mb;
     return rows > 1.05 * std::max(gemm, 25.0);
 }
-static bool linear_as_gemm(FmtId f, int R, int K, int T, int hidden_type) {
+static bool linear_as_gemm(FmtId f, int R, int K, int T, int hidden_type, cudaStream_t s) {
     if (kq_fmt(f) == KQ_NONE || T < 2) return false;
-    if (T <= 8) return hidden_type != KTB200_TYPE_F32 && kq_fmt(f) != KQ_Q4K && few_rows_as_gemm(kq_fmt(f), R, K, T);
+    if (T <= 8) return hidden_type != KTB200_TYPE_F32 && kq_fmt(f) != KQ_Q4K && few_rows_as_gemm(kq_fmt(f), R, K, T) && !capturing(s);
     if (f == FMT_Q4K && K >= 16 * QK_K && T > 11) return true;
     const double rows = (double)T * R * (500.0 + 0.35 * K) * (kq_is_q6(kq_fmt(f)) ? 1.7 : 1.0);
     return rows > 12.5e6 + 3e3 * (K < 1024 ? K : 1024);
@@ -853,7 +854,7 @@ int ktb200_linear_forward(ktb200_linear* l, int qlen, const void* input, void* o
     if (!input || !output) { set_error("forward: null pointer"); return KTB200_EINVAL; }
     DeviceGuard g(l->device);
     const FmtId fmt = pick_fmt(l->proj_type, l->soa);
-    if (linear_as_gemm(fmt, l->out_size, l->in_size, qlen, l->hidden_type)) {
+    if (linear_as_gemm(fmt, l->out_size, l->in_size, qlen, l->hidden_type, (cudaStream_t)stream)) {
         const int rc = kq_linear(fmt, l->proj, l->out_size, l->in_size, input, l->hidden_type, qlen, output, bias, bsz, l->device, (cudaStream_t)stream);
         if (rc != 1) return rc;
     }

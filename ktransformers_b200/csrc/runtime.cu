@@ -82,6 +82,12 @@ void scratch_prepare(int device) {
     cudaMemPool_t pool;
     if (scratch_pool(device, &pool) != cudaSuccess) cudaGetLastError();      // (tried again, and reported, by the first call that needs it)
 }
+bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
 cudaError_t scratch_alloc(int device, size_t bytes, cudaStream_t stream, void** out) {
     cudaMemPool_t pool;
     cudaError_t e = scratch_pool(device, &pool);

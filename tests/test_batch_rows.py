@@ -185,3 +185,30 @@ def test_few_rows_as_gemms(type, K, R, T, hid, launches):
     run(x, held, T, torch.tensor([T - 1], dtype=torch.int32, device="cuda"))
     assert torch.equal(held[:T - 1], y[:T - 1]) and (held[T - 1:] == 7.0).all()
     lib.ktb200_linear_destroy(h)
+
+
+# such calls take no scratch where they are captured (the row kernels run: one launch, the bits of the rows one by one), and give the same as ever beside a capture
+@pytest.mark.parametrize("type,K,R,T,hid", [(14, 7168, 18432, 2, BF16), (13, 10240, 7168, 8, F16), (14, 2048, 32000, 6, BF16), (14, 7168, 8192, 8, F32)])
+def test_few_rows_captured(type, K, R, T, hid):
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    g = torch.Generator(device="cuda").manual_seed(T + R)
+    blocks, x = synth_blocks(type, R * K, "cuda", T), torch.randn((T, K), generator=g, device="cuda").to(TORCH[hid])
+    lib, h = native.lib(), C.c_void_p()
+    native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), type, hid, T, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, _stream()))
+    one, eager, held = (torch.zeros((T, R), dtype=x.dtype, device="cuda") for _ in range(3))
+    run = lambda x, y, n: native.check(lib.ktb200_linear_forward(h, n, x.data_ptr(), y.data_ptr(), None, None, _stream()))
+    for t in range(T):
+        run(x[t:], one[t:], 1)
+    n0 = native.launch_count()
+    run(x, eager, T)
+    assert (native.launch_count() - n0 > 1) == (hid != F32)        # (fp32 results keep the row kernels everywhere)
+    graph, n0 = torch.cuda.CUDAGraph(), native.launch_count()
+    with torch.cuda.graph(graph):
+        run(x, held, T)
+    assert native.launch_count() - n0 == 1
+    graph.replay()
+    assert torch.equal(held, one)
+    assert ((eager.double() - one.double()).abs() <= {BF16: 2.0 ** -7, F16: 2.0 ** -10, F32: 0.0}[hid] * one.double().abs() + (hid != F32) * 4e-6 * one.double().abs().max()).all()
+    lib.ktb200_linear_destroy(h)
