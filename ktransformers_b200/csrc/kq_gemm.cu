@@ -941,7 +941,12 @@ int kq_linear(FmtId fmt, const void* w, int R, int K, const void* x, int hidden_
         const int splits = kq_splits_of(tiles, nblk, sms, hidden_type);
         ScratchBlock mem(s);
         const size_t act = (KqActs::bytes(n, K) + 255) / 256 * 256;
-        if (!mem.taken(device, act + (splits > 1 ? (size_t)splits * n * R * 4 : 0))) return T <= 8 ? 1 : KTB200_ECUDA;      // (so few rows need none: the row kernels take them)
+        const size_t scratch = act + (splits > 1 ? (size_t)splits * n * R * 4 : 0);
+        if (T <= 8) {      // (so few rows need none: without it the row kernels take them, and the call has no error to tell of)
+            if (mem.take(device, scratch) != cudaSuccess) return 1;
+        } else if (!mem.taken(device, scratch)) {
+            return KTB200_ECUDA;
+        }
         const KqActs a(mem.ptr, n, K);
         int rc = kq_quant(reinterpret_cast<const uint8_t*>(x) + (size_t)t0 * K * hb, hidden_type, n, K, nullptr, 1, kq_is_q6(f), kq_limit(f), a, s);
         if (rc) return rc;

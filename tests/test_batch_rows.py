@@ -212,3 +212,51 @@ def test_few_rows_captured(type, K, R, T, hid):
     assert torch.equal(held, one)
     assert ((eager.double() - one.double()).abs() <= {BF16: 2.0 ** -7, F16: 2.0 ** -10, F32: 0.0}[hid] * one.double().abs() + (hid != F32) * 4e-6 * one.double().abs().max()).all()
     lib.ktb200_linear_destroy(h)
+
+
+def _without_memory_for_scratch():
+    """Takes what the device has, in pieces down to 1 MB, behind a first call of the row kernels (whose code is loaded then)."""
+    from ktransformers_b200 import native
+    from ktransformers_b200.util.synth import synth_blocks
+    T, K, R, g = 4, 7168, 18432, torch.Generator(device="cuda").manual_seed(2)
+    blocks, x = synth_blocks(14, R * K, "cuda", T), torch.randn((T, K), generator=g, device="cuda").bfloat16()
+    lib, h, stream = native.lib(), C.c_void_p(), _stream()
+    native.check(lib.ktb200_linear_create(K, R, blocks.data_ptr(), 14, BF16, T, 0, C.byref(h)))
+    native.check(lib.ktb200_linear_load_weights(h, stream))
+    few, y = (torch.zeros((T, R), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for t in range(T):
+        native.check(lib.ktb200_linear_forward(h, 1, x[t:].data_ptr(), few[t:].data_ptr(), None, None, stream))
+    many = torch.zeros((16, R), dtype=torch.bfloat16, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):      # (the row kernels for as many rows)
+        native.check(lib.ktb200_linear_forward(h, T, x.data_ptr(), y.data_ptr(), None, None, _stream()))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, few)
+    y.zero_()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    rt, p, held = C.CDLL("libcudart.so.12"), C.c_void_p(), 1 << 36
+    while held >= 1 << 20:
+        if rt.cudaMalloc(C.byref(p), C.c_size_t(held)):
+            held >>= 1
+    rt.cudaGetLastError()
+    before, n0 = lib.ktb200_last_error(), native.launch_count()
+    native.check(lib.ktb200_linear_forward(h, T, x.data_ptr(), y.data_ptr(), None, None, stream))
+    assert native.launch_count() - n0 == 1 and lib.ktb200_last_error() == before == b""
+    assert lib.ktb200_linear_forward(h, 16, many.data_ptr(), many.data_ptr(), None, None, stream) not in (0, native.EINVAL) and b"scratch" in lib.ktb200_last_error()      # a prompt's size is refused as ever
+    torch.cuda.synchronize()
+    assert y.cpu().equal(few.cpu())
+
+
+def test_few_rows_without_memory_for_scratch():
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, os.path.abspath(__file__)], capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=root))
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+if __name__ == "__main__":
+    _without_memory_for_scratch()
