@@ -271,19 +271,25 @@ struct Fp8GemmMisc {
     unsigned long long full[8], free[8], d_full[2], d_free[2];
     uint32_t tmem_base;
 };
-constexpr int kFGemmSmem = kFGemmRing + (int)sizeof(Fp8GemmMisc) + 1024;
+constexpr int kFGemmTurn = 16 * 33;      // floats of an epilogue warp: 16 columns of 32 tokens
+constexpr int kFGemmSmem = kFGemmRing + (int)sizeof(Fp8GemmMisc) + 1024, kFGemmSmemTurn = kFGemmSmem + 16 * kFGemmTurn * 4;
+static_assert(kFGemmSmemTurn <= 232448, "shared memory budget");
 
 struct Fp8GemmParams {
     const float* xs;          // [nkb][tpad] token scales, token fastest
     const float* scale_inv;   // [ceil(N/128)][nkb]
     void* y;                  // [T][N]
     const int* bsz;
-    int hidden_type, T, N, nkb, tpad, mt, nt, t0, vec;
+    int hidden_type, T, N, nkb, tpad, mt, nt, t0, vec;      // vec: result rows begin at whole sectors (2), at 16 bytes (1), anywhere (0)
 };
 
 // TWO: fp32 results, where the order of a long fp32 chain shows (K = 12032: 2.0e-7 off in one chain, 1.2e-7 with K splits): the chain is cut
 // every 8 blocks into a second accumulator.
-template <int BN, bool TWO>
+// TURN: result rows that begin anywhere, and fp32 ones that do not begin at a sector.  A thread's columns of its token would be scattered values; the warp turns 16 columns of its 32 tokens
+// around in shared memory, and 16 threads write 16 columns of one row (a kernel of its own: in one with the other form aligned rows took 7 % longer).  Value by value / like this (us):
+// 1200 tokens, 1536 -> 9001 fp32 91 / 44, fp16 150 / 38; 64 tokens, 4096 -> 4101 bf16 22.2 / 19.7; in vectors of 16 bytes / like this: fp32 1200 tokens 1024 -> 16388 62.1 / 56.7, 500 tokens
+// 4096 -> 4100 31.9 / 30.1, 1200 tokens 7168 -> 3004 60.7 / 62.5; bf16 1200 tokens 2048 -> 8200 40.3 / 56.6.
+template <int BN, bool TWO, bool TURN>
 __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Fp8GemmParams p) {
     constexpr int kStageB = 128 * 128 + BN * 128, kStages = kFGemmRing / kStageB, kCols = 2 * BN;
     static_assert(kStages <= 8, "barriers");
@@ -406,7 +412,21 @@ __global__ void __launch_bounds__(kFGemmThreads, 1) fp8_gemm_kernel(const __grid
 #pragma unroll
                 for (int i = 0; i < kPart; i++) acc[i] = sum[i];
             }
-            if (t < live) {
+            if (TURN) {
+                float* turn = reinterpret_cast<float*>(smem_raw + (base - raw) + kFGemmRing + sizeof(Fp8GemmMisc)) + (warp - 4) * kFGemmTurn;
+                const int t1 = m0 + 32 * sp + (lane >> 4);
+#pragma unroll
+                for (int c = 0; c < kPart; c += 16) {
+                    const int col = nb + c + (lane & 15);
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 16; i++) turn[33 * i + lane] = acc[c + i];
+                    __syncwarp();
+#pragma unroll 4
+                    for (int k = 0; k < 32; k += 2)
+                        if (t1 + k < live && col < p.N) store_hidden(p.y, (long)(t1 + k) * p.N + col, p.hidden_type, turn[33 * (lane & 15) + (lane >> 4) + k]);
+                }
+            } else if (t < live) {
                 const long o = (long)t * p.N + nb;
 #pragma unroll
                 for (int c = 0; c < kPart; c += 16) {
@@ -520,10 +540,15 @@ static int fp8_map(CUtensorMap* map, const void* ptr, int K, int n, int rows) {
     if (cr != CUDA_SUCCESS) { set_error("fp8_linear: cuTensorMapEncodeTiled failed (%d)", (int)cr); return KTB200_ECUDA; }
     return KTB200_OK;
 }
+template <int BN, bool TWO, bool TURN>
+static cudaError_t launch_fp8_gemm_as(const CUtensorMap& xmap, const CUtensorMap& wmap, const Fp8GemmParams& p, int grid, cudaStream_t s) {
+    constexpr int smem = TURN ? kFGemmSmemTurn : kFGemmSmem;
+    const cudaError_t e = cudaFuncSetAttribute(fp8_gemm_kernel<BN, TWO, TURN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e != cudaSuccess ? e : launch_pdl(fp8_gemm_kernel<BN, TWO, TURN>, dim3(grid), dim3(kFGemmThreads), (size_t)smem, s, xmap, wmap, p);
+}
 template <int BN, bool TWO>
 static cudaError_t launch_fp8_gemm(const CUtensorMap& xmap, const CUtensorMap& wmap, const Fp8GemmParams& p, int grid, cudaStream_t s) {
-    const cudaError_t e = cudaFuncSetAttribute(fp8_gemm_kernel<BN, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFGemmSmem);
-    return e != cudaSuccess ? e : launch_pdl(fp8_gemm_kernel<BN, TWO>, dim3(grid), dim3(kFGemmThreads), (size_t)kFGemmSmem, s, xmap, wmap, p);
+    return p.vec > TWO ? launch_fp8_gemm_as<BN, TWO, false>(xmap, wmap, p, grid, s) : launch_fp8_gemm_as<BN, TWO, true>(xmap, wmap, p, grid, s);
 }
 static int fp8_forward_gemm(ktb200_fp8_linear* l, int qlen, const void* x, void* y, const int* bsz, cudaStream_t s) {
     const size_t hb = type_size(l->hidden_type);

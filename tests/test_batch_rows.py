@@ -99,13 +99,14 @@ def test_rotated_rows(T, H, G, d, rot, layout, norm, unit_v, dtype):
 
 # results in whole sectors (rows and address multiples of 32 bytes), in vectors of 16 and value by value: the same values wherever they go; blocks of K that are no multiple of the
 # four whose scales are under way; tiles of 256, 128 and 64 columns, the last one ragged
-@pytest.mark.parametrize("T,K,N,hid", [(130, 128, 4096, BF16), (300, 640, 19000, F16), (257, 1152, 19208, BF16), (129, 384, 2064, F32), (1030, 896, 515, BF16), (64, 2048, 1032, F16)])
+@pytest.mark.parametrize("T,K,N,hid", [(130, 128, 4096, BF16), (300, 640, 19000, F16), (257, 1152, 19208, BF16), (129, 384, 2064, F32), (1030, 896, 515, BF16), (64, 2048, 1032, F16),
+                                         (300, 512, 2068, F32), (200, 256, 19001, F32), (4200, 128, 131, BF16)])
 def test_fp8_batches_wherever_results_go(T, K, N, hid):
     from ktransformers_b200 import native
     g = torch.Generator(device="cuda").manual_seed(N)
     w, ws = (torch.randn((N, K), generator=g, device="cuda") * 50).to(torch.float8_e4m3fn), torch.rand(((N + 127) // 128, K // 128), generator=g, device="cuda") / K
     x, dt = torch.randn((T, K), generator=g, device="cuda").to(TORCH[hid]), TORCH[hid]
-    lib, h = native.lib(), C.c_void_p()
+    lib, h, live = native.lib(), C.c_void_p(), torch.tensor([T - 5], dtype=torch.int32, device="cuda")
     native.check(lib.ktb200_fp8_linear_create(K, N, w.data_ptr(), ws.data_ptr(), hid, 0, C.byref(h)))
     out = []
     for shift in (0, 16 // x.element_size(), 1):
@@ -113,6 +114,8 @@ def test_fp8_batches_wherever_results_go(T, K, N, hid):
         native.check(lib.ktb200_fp8_linear_forward(h, T, x.data_ptr(), room[shift:].data_ptr(), None, _stream()))
         assert (room[:shift] == 7.0).all() and (room[shift + T * N:] == 7.0).all()
         out.append(room[shift:shift + T * N].clone())
+        native.check(lib.ktb200_fp8_linear_forward(h, T, x.data_ptr(), room.fill_(7.0)[shift:].data_ptr(), live.data_ptr(), _stream()))
+        assert torch.equal(room[shift:shift + (T - 5) * N], out[-1][:(T - 5) * N]) and (room[shift + (T - 5) * N:] == 7.0).all()
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
     f = x.float().view(T, -1, 128)
     s = f.abs().amax(-1, keepdim=True) / 448.0
