@@ -522,8 +522,10 @@ static int fp8_blocks(int tiles, int nkb, int places, bool many) {
     return best;
 }
 // Whether a batch of more than kFT tokens is still faster in passes of kFT.  The GEMM has no K splits, so a matrix of few rows is one serial chain of
-// K / 128 steps a tile: measured 10 us + 0.48 us a step and round of tiles (7168 -> 576: 35-39 us, 16384 -> 64: 76, 18432 -> 1536: 75); a pass takes 17.5 us
-// + 1 us per 2.9 MB of weights, a last one of a few tokens less (7168 -> 576: 28 us at 17 tokens, 36 at 24, 40 at 32, 58 at 48).
+// K / 128 steps a tile.  The line was fitted to former kernels, 10 us + 0.48 us a step and round of tiles against 17.5 us + 1 us per 2.9 MB of weights a pass, a last one of a few tokens
+// less.  Measured again (40 matrices, graphs): 4 us + 0.25 us a step, and 12 us + 1 us per 5 MB, a last pass of up to 2 tokens 0.6, of up to 8 tokens 0.85 of one.  Where the matrix is
+// narrow and long both lines agree (20480 -> 256, 24 tokens: passes 27, GEMM 47 us); near the line the GEMM is now the faster one by up to 1.45 (7168 -> 576: 24 tokens 26.6 / 19.6; 5120 -> 1024,
+// 18 tokens 22.6 / 15.3), 2 % on the average of all.  The choice stays where callers and tests have it.
 static bool fp8_passes_win(const ktb200_fp8_linear* l, int T, int sms) {
     if (T > 64) return false;
     const int rest = T % kFT, rounds = ((l->N + 63) / 64 + sms - 1) / sms;      // (few tiles: 64 weight rows each)
