@@ -70,8 +70,27 @@ def test_router_calls_share_nothing():
             assert torch.equal(a, b[16 * i:16 * i + 24])
 
 
+def _turned(x, heads, pos, inv_freq, rot, layout, norm, w, eps=1e-6):
+    """[T][heads * d] in 64 bits: the rows turned and normed, and how large a value's terms are"""
+    T, d = x.shape[0], x.shape[1] // heads
+    x = x.double().view(T, heads, d)
+    whole = (x.square().mean((1, 2), keepdim=True) + eps).rsqrt()
+    inv, w = {0: torch.ones_like(whole), 2: whole}.get(norm, (x.square().mean(2, keepdim=True) + eps).rsqrt()), w.double()
+    if norm == 3:
+        x = x * w
+    first = torch.arange(rot // 2, device=x.device) * (1 if layout else 2)
+    second = first + (rot // 2 if layout else 1)
+    a, b, angle, y, size = x[..., first], x[..., second], pos.double()[:, None, None] * inv_freq, x.clone(), x.abs()
+    if rot:
+        y[..., first], y[..., second] = a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()
+        size[..., first] = size[..., second] = (a.square() + b.square()).sqrt()
+    scale = inv * (w.view(heads, d) if norm == 2 else 1.0)
+    return (y * scale).view(T, -1), (size * scale.abs()).view(T, -1)
+
+
 # heads of 64, 128 and 256 columns in both types and layouts, every norm, part of the columns and none turned, one token and many (blocks of units, and fewer units than
-# a block's warps); the general kernel takes the same rows at an odd offset.  Sums of squares are added in another order: a unit of fp32, which may move a bf16 by one place
+# a block's warps); the general kernel takes the same rows at an odd offset.  Both against 64 bits: some ten roundings of fp32 of a value's terms, and of sums of squares of up to 8192
+# columns in order of lanes, and half a place of bf16; between the two, sums in another order may move a bf16 by one place
 @pytest.mark.parametrize("T,H,G,d,rot,layout,norm,unit_v,dtype", [(1, 64, 8, 128, 64, 1, 1, 0, BF16), (300, 16, 2, 128, 128, 1, 3, 1, BF16), (2100, 4, 4, 64, 32, 0, 1, 0, BF16), (37, 6, 3, 256, 64, 1, 2, 0, BF16),
                                                                   (5, 40, 8, 128, 0, 0, 1, 1, F32), (65, 8, 2, 64, 64, 0, 3, 0, F32), (700, 3, 1, 256, 256, 1, 0, 0, F32), (16, 8, 8, 128, 32, 0, 2, 1, F32)])
 def test_rotated_rows(T, H, G, d, rot, layout, norm, unit_v, dtype):
@@ -91,9 +110,16 @@ def test_rotated_rows(T, H, G, d, rot, layout, norm, unit_v, dtype):
         native.check_seq(lib.ktb200_rope_norm_cache_write(p.data_ptr(), n + pad, pad, pad + H * d, pad + (H + G) * d, H, G, d, d, rot, layout, inv_freq.data_ptr(), norm, q_w.data_ptr(), k_w.data_ptr(), unit_v,
                                                           1e-6, None, 0, None, pos.data_ptr(), slot.data_ptr(), table.data_ptr(), pages, page, cache.data_ptr(), q.data_ptr(), T, dtype, _stream()))
         out.append((q, cache))
+    row = table[(pos.long() // page) % pages].long() * page + pos.long() % page
+    parts = list(proj.split((H * d, G * d, G * d), 1))
+    wq, wk = _turned(parts[0], H, pos, inv_freq, rot, layout, norm, q_w), _turned(parts[1], G, pos, inv_freq, rot, layout, norm, k_w)
+    wv = _turned(parts[2], G, pos, inv_freq, 0, layout, 1 if unit_v else 0, k_w)
+    for q, cache in out:
+        for got, (want, size) in ((q, wq), (cache[row][:, :G * d], wk), (cache[row][:, G * d:], wv)):
+            assert ((got.double() - want).abs() <= (2.0 ** -8 if dtype == BF16 else 0.0) * want.abs() + 2.0 ** -20 * size).all()
     for a, b in zip(*out):
         assert torch.isfinite(a.float()).all() and ((a.double() - b.double()).abs() <= (2.0 ** -7 if dtype == BF16 else 2.0 ** -20) * b.double().abs() + 1e-6).all()
-        assert (a != b).double().mean() < (0.01 if dtype == BF16 else 1.0)
+        assert dtype != BF16 or (a != b).double().mean() < 0.01
     assert (out[0][1] == 7.0).all(1).sum() == pages * page - T        # (only the tokens' rows were written)
 
 
