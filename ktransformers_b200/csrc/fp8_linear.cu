@@ -256,13 +256,15 @@ __global__ void __launch_bounds__(192, 2) fp8_linear_kernel(const __grid_constan
 
 // Prompt portions (more than kFT tokens): y = xq . W^T as a persistent GEMM.  The pass kernel above streams all of W again for every 16
 // tokens (2000 tokens, 7168 -> 18432: 125 passes, 7.9 ms); here a tile is 128 tokens x BN weight rows, both operands come by TMA in the
-// 128-byte-swizzle layout.  What bounds it is the shared memory's port: a K block of a 128 x 256 tile brings 48 KB in and the four products read 48 KB, 768 cycles at 128 B
-// a cycle (the products alone: 524; measured 735 a block at the 1.53 GHz that such a load leaves).  A pair of CTAs on one tile would halve the reading of W.
+// 128-byte-swizzle layout.  A K block of a 128 x 256 tile takes 735 cycles (its products alone 524; they read 48 KB of shared memory while the copies bring 48 KB in).
+// 2000 tokens, 7168 -> 18432: 8 rounds of 56 blocks and 8 outputs of 4,000 cycles are 361 k of the 368 k cycles counted, 214 us at the 1.72 GHz of one launch (tensor pipe 64 % active);
+// the quantisation before it 24 us; a call 245 us by itself, and 277-289 in a long row of them, where the power limit takes the clock to 1.48 GHz.  A pair of CTAs on one tile would halve the
+// reading of W.
 //     warp 0 TMA ring (4 to 8 stages, 192 KB), warp 1 issuer, warps 4-19 epilogue: a thread owns one token and a quarter of the tile's columns;
 //     lanes are tokens, so the token scale is a register and acc += dot * (a_s * b_s) is ONE fma per value and 128 of K.
 //     Two TMEM buffers of BN columns: the MMAs of one K block run while the block before it is promoted.
 // BN: 256 where that gives every SM a tile; 128 and 64 keep the chip full when there are few tiles.
-// 2000 tokens, 7168 -> 18432: 338 -> 317 us by scales that are fetched four blocks ahead (a load takes about 1,000 cycles beside the copies; one block ahead each block waited 400 of
+// The same call 338 -> 317 us by scales that are fetched four blocks ahead (a load takes about 1,000 cycles beside the copies; one block ahead each block waited 400 of
 // them), four epilogue warps a scheduler instead of two (a drain's chain of loads and sums: 720 cycles a block), a tile's output without branches in whole sectors (12,800 -> 4,000
 // cycles) and one election for a block's products and barriers.  The roles are known to be uniform (umma.cuh): 351 -> 333 us (the kernel above, one token 16384 -> 7168: 34.1 -> 32.7).
 // Tiles run token tile fastest inside groups of kFGroupM, so that the CTAs of a wave share the weight rows and the tokens through L2.

@@ -11,10 +11,10 @@
 //                  its S in tensor memory; the reference maximum is raised, and O scaled in tensor memory, only when a row's maximum grows by
 //                  more than 2^8 (P <= 256 in between, where bf16 and fp32 are as exact as below 1)
 // TMEM: [S0 | O0 | S1 | O1], 128 columns each.  Shared memory: Q 64 KB, K and V 2 x 32 KB each.
-// Bounds: 16 products of 64 cycles per (row tile, key tile) beside 128 exponentials per thread at 4 per cycle and scheduler (1024 cycles for two
-// tiles on one scheduler): 2,050 cycles of tensor pipe for two tiles, 95-105 us for 2048 tokens behind 2048, 64 heads over 8.  It takes 250: a row's maximum, exponentials,
-// conversions and stores run one after the other in its thread, the tile's next product waits for all of them, and there is one score buffer a tile (tensor pipe 48 %
-// active, issue slots 35 %).
+// Bounds: 16 products of 64 cycles per (row tile, key tile), 2,050 cycles of tensor pipe for two tiles, 95-105 us for 2048 tokens behind 2048, 64 heads over 8; beside them
+// 128 exponentials per thread at 4 per cycle and scheduler, 1,024 cycles a warp and as much as the products for the two warps that share a scheduler.  It takes 247 us: a row's
+// maximum, exponentials, conversions and stores run one after the other in its thread, the tile's next product waits for all of them, and there is one score buffer a tile (tensor
+// pipe 48 % active, issue slots 35 %).
 #pragma once
 #include <cuda.h>
 
