@@ -20,10 +20,10 @@
 // one accumulator's 36 steps drop what does not fit at each of them: scores of a 2-norm error of 5.3e-7 (log-sum-exp up to 2.9e-6 off), in four sums of nine steps added up in fp32 1.35e-7
 // (1.6e-6).
 // What bounds it: 36 + 8 products a tile of 32 tokens (a 64 x N x 16 product takes 34 cycles for every N up to 64, in one accumulator as in four).  B = 1, 128 heads, 131,072 keys, calls one
-// behind the other: 91 us with Q through registers and the merge in one part; with Q by TMA while the first tiles come (setup 4.8 -> 2.1 us), one election for four products and a merge in four
+// behind the other: 92 us with Q through registers and the merge in one part; with Q by TMA while the first tiles come (setup 4.8 -> 2.1 us), one election for four products and a merge in four
 // parts 88; with the four sums read by rows in one load of 16 lanes x 128 columns, instead of 4 loads of 32 lanes of which half hold nothing, 78 (4 loads of 16 x 32: 80; one
-// accumulator: 72).  Tiles of 64 tokens (half the cycles for scores) took 79-118 us: two stages of them fill the shared memory, a stage comes back only behind the tile's values, and copies
-// and products then share the shared memory's port (120 of 128 B a cycle).
+// accumulator: 72); with the waits as they are now 68 (umma.cuh).  Tiles of 64 tokens (half the cycles for scores) took 79-118 us: two stages of them fill the shared memory, a stage comes back only behind
+// the tile's values, and copies and products then share the shared memory's port (120 of 128 B a cycle).
 //
 // Online softmax with a LAZY reference maximum: p = 2^(x - m_ref), m_ref is only raised (and O^T rescaled in TMEM, all
 // four warps) when some head's running maximum exceeds it by more than 8 — p stays <= 256, exact in bf16/fp32 terms —
