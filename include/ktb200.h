@@ -220,7 +220,8 @@ typedef struct ktb200_gate_config {
 /* idx_dev int64 [qlen][top_k] (order: descending biased score, like torch.topk sorted=True — the
  * reference uses sorted=False whose order is unspecified; tests compare as sets), w_dev fp32.
  * logits_dev optional fp32 [qlen][n_experts] out.  Scratch (qlen x n_experts x up to 8 fp32 values) is taken from the device's stream-ordered pool for
- * the duration of the call: calls may overlap on several streams, and a captured one keeps memory of its own. */
+ * the duration of the call: calls may overlap on several streams, and a captured one keeps memory of its own.  Where the pool has none a slower kernel
+ * without scratch gives the same bits. */
 int ktb200_moe_gate_forward(const ktb200_gate_config* cfg, int qlen, const void* x_dev, int64_t* idx_dev,
                             float* w_dev, float* logits_dev, const int* bsz_tensor_dev, void* stream);
 /* The same selection on logits [qlen][n_experts] fp32 that the caller computed (one CTA per token: prompt-sized batches). */

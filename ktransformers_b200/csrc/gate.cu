@@ -96,6 +96,26 @@ __global__ void __launch_bounds__(kGateThreads) gate_select_kernel(const GatePar
     for (int t = blockIdx.x; t < T; t += gridDim.x)
         gate_select_token<0>(p, t, reinterpret_cast<float*>(smem_raw), p.idx + (long)t * p.top_k, p.w + (long)t * p.top_k, p.logits_out);
 }
+// Both for a token in one CTA, its partial sums (the same, in the same order) in shared memory: where the pool has no memory for them.  Every CTA reads all of W through L2 (256 x 7168, one to 148 tokens: 584 us)
+__global__ void __launch_bounds__(kGateThreads) gate_alone_kernel(const GateParams p) {
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    GateParams own = p;
+    own.partial = reinterpret_cast<float*>(smem_raw);
+    float *sel = own.partial + (size_t)p.S * p.E, *xs = sel + 2 * p.E + 32 + 4 * kGateWarps;
+    xs = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(xs) + 15) & ~(uintptr_t)15);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n4 = p.H / 4, T = p.bsz ? min(p.T, *p.bsz) : p.T;
+    for (int t = blockIdx.x; t < T; t += gridDim.x) {
+        for (int s = 0; s < p.S; s++) {
+            const int c0 = (int)((long)n4 * s / p.S), nc4 = (int)((long)n4 * (s + 1) / p.S) - c0;
+            __syncthreads();
+            for (int c = threadIdx.x; c < nc4 * 4; c += kGateThreads) xs[c] = load_hidden(p.x, (long)t * p.H + 4L * c0 + c, p.hidden_type);
+            __syncthreads();
+            for (int e = warp; e < p.E; e += kGateWarps) gate_dot<1>(own, reinterpret_cast<const float4*>(p.W + (long)e * p.H) + c0, xs, nc4, lane, 0, e, s, p.S);
+        }
+        __syncthreads();
+        gate_select_token<0, true>(own, 0, sel, p.idx + (long)t * p.top_k, p.w + (long)t * p.top_k, p.logits_out ? p.logits_out + (long)t * p.E : nullptr);
+    }
+}
 static size_t gate_select_smem(int E) { return ((size_t)2 * E + 32 + 4 * kGateWarps) * sizeof(float); }
 static int gate_select_ctas(int T) { return std::min(T, 148 * 16); }
 
@@ -123,11 +143,18 @@ extern "C" int ktb200_moe_gate_forward(const ktb200_gate_config* c, int qlen, co
     const int row_ctas = (c->n_experts + kGateWarps - 1) / kGateWarps;
     const int S = gate_splits(c->n_experts, c->hidden_size, num_sms(dev));
     ScratchBlock partial(s);
-    if (!partial.taken(dev, (size_t)qlen * c->n_experts * S * sizeof(float))) return KTB200_ECUDA;
+    const bool alone = partial.take(dev, (size_t)qlen * c->n_experts * S * sizeof(float)) != cudaSuccess;
     GateParams p{c->weight, x, c->hidden_type, c->n_experts, c->hidden_size, qlen, S, c->top_k, c->n_group, c->topk_group,
                  c->scoring, c->topk_method, c->norm_topk_prob, c->routed_scaling_factor, c->bias, (float*)partial.ptr, logits,
                  idx, w, bsz};
     const int nc4_max = c->hidden_size / 4 / S + 1;
+    if (alone) {
+        const size_t smem = (size_t)S * c->n_experts * sizeof(float) + gate_select_smem(c->n_experts) + (size_t)nc4_max * 16 + 16;
+        if (smem > 48 * 1024) KTB_CUDA_CHECK(raise_smem_limit((const void*)gate_alone_kernel, smem));
+        gate_alone_kernel<<<gate_select_ctas(qlen), kGateThreads, smem, s>>>(p);
+        KTB_LAUNCH_CHECK();
+        return KTB200_OK;
+    }
     const int nt = qlen < kGateTokTile ? qlen : kGateTokTile;
     const size_t smem = (size_t)nt * nc4_max * 16;
     const int tiles = std::min((qlen + kGateTokTile - 1) / kGateTokTile, kGateTiles);

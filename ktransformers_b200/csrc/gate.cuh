@@ -63,7 +63,8 @@ struct GateSel {
     const float* bias;
     const float* partial;
 };
-template <int BAR>
+// SHARED: the partial sums lie in shared memory
+template <int BAR, bool SHARED = false>
 __device__ void gate_select_token(const GateParams& pin, int t, float* sm, int64_t* idx_out, float* w_out, float* logits_out) {
     const GateSel p{pin.E, pin.S, pin.top_k, pin.n_group, pin.topk_group, pin.scoring, pin.topk_method, pin.norm_topk_prob,
                     pin.routed_scaling_factor, pin.bias, pin.partial};
@@ -83,7 +84,7 @@ __device__ void gate_select_token(const GateParams& pin, int t, float* sm, int64
 #pragma unroll
         for (int i = 0; i < kGateEPT; i++) {
             const int e = tid + kGateThreads * i;
-            pv[s][i] = (s < p.S && e < E) ? __ldcg(pp + e) : 0.f;   // written by other SMs in this launch: read at L2
+            pv[s][i] = (s < p.S && e < E) ? (SHARED ? pp[e] : __ldcg(pp + e)) : 0.f;   // written by other SMs in this launch: read at L2
         }
     }
     float bv[kGateEPT];   // e_score_correction_bias, requested together with the partial sums

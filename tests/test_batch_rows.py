@@ -244,7 +244,7 @@ def test_few_rows_captured(type, K, R, T, hid):
 
 
 def _without_memory_for_scratch():
-    """Takes what the device has, in pieces down to 1 MB, behind a first call of the row kernels (whose code is loaded then)."""
+    """Takes what the device has, in pieces down to 1 MB.  A linear and the router run all the same, in other kernels, with the bits of rows one by one and of the usual ones."""
     from ktransformers_b200 import native
     from ktransformers_b200.util.synth import synth_blocks
     T, K, R, g = 4, 7168, 18432, torch.Generator(device="cuda").manual_seed(2)
@@ -265,25 +265,41 @@ def _without_memory_for_scratch():
     y.zero_()
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
-    rt, p, held = C.CDLL("libcudart.so.12"), C.c_void_p(), 1 << 36
+    E, k, Tr = 256, 8, 24
+    W, xr = torch.randn((E, K), generator=g, device="cuda") * K ** -0.5, torch.randn((Tr, K), generator=g, device="cuda").bfloat16()
+    cfg = native.GateConfig(E, K, k, 8, 4, 0, 0, 1, 2.5, W.data_ptr(), None, BF16)
+    routed = [(torch.full((Tr, k), -1, dtype=torch.int64, device="cuda"), torch.zeros((Tr, k), device="cuda"), torch.zeros((Tr, E), device="cuda")) for _ in range(2)]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    rt, p, held, taken = C.CDLL("libcudart.so.12"), C.c_void_p(), 1 << 36, []
     while held >= 1 << 20:
         if rt.cudaMalloc(C.byref(p), C.c_size_t(held)):
             held >>= 1
+        else:
+            taken.append(p.value)
     rt.cudaGetLastError()
     before, n0 = lib.ktb200_last_error(), native.launch_count()
     native.check(lib.ktb200_linear_forward(h, T, x.data_ptr(), y.data_ptr(), None, None, stream))
     assert native.launch_count() - n0 == 1 and lib.ktb200_last_error() == before == b""
     assert lib.ktb200_linear_forward(h, 16, many.data_ptr(), many.data_ptr(), None, None, stream) not in (0, native.EINVAL) and b"scratch" in lib.ktb200_last_error()      # a prompt's size is refused as ever
-    torch.cuda.synchronize()
-    assert y.cpu().equal(few.cpu())
+    for o in routed:
+        n0 = native.launch_count()
+        native.check(lib.ktb200_moe_gate_forward(C.byref(cfg), Tr, xr.data_ptr(), *[t.data_ptr() for t in o], None, stream))
+        torch.cuda.synchronize()
+        assert native.launch_count() - n0 == (1 if o is routed[0] else 2)
+        while taken:
+            rt.cudaFree(C.c_void_p(taken.pop()))
+    assert torch.equal(y, few)
+    for a, b in zip(*routed):
+        assert torch.equal(a, b)
 
 
-def test_few_rows_without_memory_for_scratch():
+def test_without_memory_for_scratch():
     import os
     import subprocess
     import sys
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, os.path.abspath(__file__)], capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=root))
+    r = subprocess.run([sys.executable, os.path.abspath(__file__)], capture_output=True, text=True, timeout=300, env=dict(os.environ, PYTHONPATH=root, CUDA_MODULE_LOADING="EAGER"))
     assert r.returncode == 0, r.stdout + r.stderr
 
 
